@@ -421,8 +421,6 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
 #pragma unroll
           for (int ch = 0; ch < ROW_CHUNKS; ++ch) raw[ch] = *reinterpret_cast<const uint4*>(src + ((ch ^ swz) << 4));
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&idx_empty[si]);  // the tile lives in registers now
         // group g owns A slot g: free once the MMAs of this group's previous batch have completed
         if (!mbar_wait_warp(&a_empty[grp], ((lb >> 1) & 1) ^ 1, abort_flag, p.status, ERR_WAIT_EMPTY)) { ok = false; break; }
         tc_fence_after();
@@ -435,6 +433,10 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
             tmem_st_32x32(t_lane + A_COL0 + (grp * KBB + kk) * 32, o);
           }
         }
+        // The tile is released only here: every index byte has been used as a table address by now. An arrival right after
+        // the loads were issued let the next tile's TMA write overtake them once the ring wrapped (wrong sums).
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&idx_empty[si]);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();

@@ -98,6 +98,24 @@ def test_gpu_oil_gemm_matches_dequantised_matmul(fmt, M, N, K):
     assert torch.equal(y, y2) or float((y2.float() - ref).norm() / ref.norm()) < 1e-2
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", ["oil4", "oil8", "spark"])
+@pytest.mark.parametrize("M,N,K", [(1, 32000, 4096), (64, 22016, 4096), (64, 4096, 11008), (100, 6144, 4096), (128, 4096, 4096)])
+def test_gpu_oil_gemm_ring_of_index_tiles_wraps(fmt, M, N, K):
+    """More index tiles per CTA than the ring holds, the weights warm in L2 from the second call on: a tile must not be replaced
+    before it has been used. The operands are exact in bf16 and the sums fp32, so the error is the rounding of the result (2^-9)."""
+    from innova_b200.ops import runtime as rt
+    from innova_b200.ops.oil_linear import quantize_weight, oil_linear
+    g = torch.Generator(device="cuda").manual_seed(8)
+    qw = quantize_weight(torch.randn(N, K, device="cuda", generator=g) * 0.02, fmt)
+    x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    ref = x.float() @ qw.dequantize().float().t()
+    for _ in range(4):
+        y = oil_linear(x, qw).float()
+        assert float((y - ref).norm() / ref.norm()) < 2.0 ** -8
+    rt.check_status()
+
+
 def test_fused_finish_fallbacks_cpu():
     from innova_b200 import ops
     from innova_b200.ops.oil_linear import oil_linear, oil_linear_norm, oil_linear_swiglu, quantize_weight
