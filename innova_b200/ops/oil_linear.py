@@ -68,6 +68,15 @@ class QuantWeight:
 
     def dequantize(self) -> torch.Tensor:
         """[N, K] in the scales' dtype."""
+        cb, entries = self.codebook, 1 << self.bits
+        if (self.idx.is_cuda and self.idx.device.index == torch.cuda.current_device() and self.scales.dtype == torch.bfloat16 and cb.dtype == torch.float32 and cb.numel() == entries and self.K % 32 == 0
+                and self.idx.dtype == torch.uint8 and self.idx.numel() * 8 == self.N * self.K * self.bits and self.idx.data_ptr() % 8 == 0
+                and self.scales.numel() * 32 == self.N * self.K
+                and all(t.device == self.idx.device and t.is_contiguous() and not t.requires_grad for t in (self.idx, self.scales, cb))):
+            out = torch.empty(self.N, self.K, dtype=torch.bfloat16, device=self.idx.device)
+            rt.check(rt.lib().inv_weight_dequant(self.idx.data_ptr(), self.scales.data_ptr(), cb.data_ptr(), self.bits, out.data_ptr(), out.numel(),
+                                                 rt.stream_ptr()), "inv_weight_dequant")
+            return out
         if self.fmt == "oil4":
             codes = torch.stack([self.idx & 15, self.idx >> 4], dim=-1).reshape(self.N, self.K)
         elif self.bits == 2:
@@ -87,6 +96,16 @@ def quantize_weight(w: torch.Tensor, fmt: str = "oil4", codebook: Optional[torch
         cb = torch.tensor(TERNARY_TABLE[fmt], dtype=torch.float32, device=w.device)
     else:
         cb = (codebook if codebook is not None else quant.default_codebook(fmt, w.device)).float().to(w.device)
+    if w.is_cuda:
+        src, bits = w.detach().contiguous(), {"oil4": 4, "oil8": 8}.get(fmt, 2)
+        src = src if src.dtype in (torch.float32, torch.bfloat16) else src.float()
+        if src.data_ptr() % 16 == 0:          # codes packed and scales rounded by the quantising kernel itself
+            cb = cb.contiguous()
+            idx = torch.empty(N, K * bits // 8, dtype=torch.uint8, device=w.device)
+            sc = torch.empty(N, K // 32, dtype=torch.bfloat16, device=w.device)
+            rt.check(rt.lib().inv_quantize_weight(src.data_ptr(), int(src.dtype == torch.bfloat16), idx.data_ptr(), sc.data_ptr(), cb.data_ptr(),
+                                                  cb.numel(), N * K, quant.MODES[fmt], rt.stream_ptr()), "inv_quantize_weight")
+            return QuantWeight(fmt, idx, sc, cb, N, K, None if bias is None else bias.to(torch.bfloat16))
     idx, sc, _ = quant.quantize_blockwise(w.contiguous(), fmt, cb)
     idx = idx.view(N, K)
     if fmt == "oil4":

@@ -20,6 +20,8 @@ _native.register_cuda_sigs({
     "inv_block_quant": [_native.vp, _native.i32, _native.vp, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.i64,
                         _native.i32, _native.vp],
     "inv_block_dequant": [_native.vp, _native.vp, _native.vp, _native.i32, _native.vp, _native.i64, _native.vp],
+    "inv_quantize_weight": [_native.vp, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.i64, _native.i32, _native.vp],
+    "inv_weight_dequant": [_native.vp, _native.vp, _native.vp, _native.i32, _native.vp, _native.i64, _native.vp],
     "inv_pack_nibbles": [_native.vp, _native.vp, _native.i64, _native.vp],
 })
 

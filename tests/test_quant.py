@@ -98,6 +98,53 @@ def test_gpu_oil_gemm_matches_dequantised_matmul(fmt, M, N, K):
     assert torch.equal(y, y2) or float((y2.float() - ref).norm() / ref.norm()) < 1e-2
 
 
+def _codes_and_values(qw):
+    """What dequantize() says with plain PyTorch calls."""
+    shifts = {"oil4": (0, 4), "oil8": (0,)}.get(qw.fmt, (0, 2, 4, 6))
+    mask = {"oil4": 15, "oil8": 255}.get(qw.fmt, 3)
+    codes = torch.stack([(qw.idx >> s) & mask for s in shifts], -1).view(qw.N, qw.K)
+    vals = qw.codebook[codes.long()].bfloat16()
+    return codes, (vals.view(qw.N, -1, 32) * qw.scales.view(qw.N, -1, 1)).view(qw.N, qw.K)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("fmt", ["oil4", "oil8", "spark", "oil1"])
+@pytest.mark.parametrize("n", [32, 7 * 32, 8 * 32, 9 * 32, 300 * 32 + 5, 148 * 8 * 64 * 32 + 64])
+def test_gpu_whole_blocks_and_single_values_quantise_alike(n, fmt, dtype):
+    """The kernel of whole blocks against the one that takes a value per lane (any address), bit for bit: uneven codebooks,
+    blocks of zeros, values that are no numbers or too large, the last block cut short."""
+    g = torch.Generator(device="cuda").manual_seed(n % 1000)
+    w = torch.randn(n, device="cuda", generator=g) * 0.02
+    w[:32] = 0.0
+    if n > 200:
+        w[40], w[70], w[100], w[101] = float("nan"), float("inf"), -1e30, 1e-38
+    w = w.to(dtype)
+    off = torch.empty(n + 1, dtype=dtype, device="cuda")[1:].copy_(w)          # not on a 16-byte boundary
+    K = {"oil4": 16, "oil8": 256}.get(fmt, 16)
+    uneven = torch.linspace(-1, 1, K, device="cuda").pow(3).contiguous()
+    for cb in (None, uneven) if fmt in ("oil4", "oil8") else (None,):
+        a, b = quant.quantize_blockwise(w, fmt, cb, want_dequant=True), quant.quantize_blockwise(off, fmt, cb, want_dequant=True)
+        for x, y in zip(a, b):
+            assert torch.equal(torch.nan_to_num(x.float(), 7.0), torch.nan_to_num(y.float(), 7.0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("fmt", ["oil4", "oil8", "spark", "oil1"])
+@pytest.mark.parametrize("N,K", [(1, 64), (3, 192), (128, 4096), (1001, 320)])
+def test_gpu_quantised_matrix_and_back(N, K, fmt, dtype):
+    from innova_b200.ops.oil_linear import quantize_weight
+    w = (torch.randn(N, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(N)) * 0.02).to(dtype)
+    qw = quantize_weight(w, fmt)
+    idx, sc, _ = quant.quantize_blockwise(w, fmt)
+    codes, values = _codes_and_values(qw)
+    assert torch.equal(codes, idx.view(N, K)) and torch.equal(qw.scales, sc.view(N, -1).bfloat16())
+    assert torch.equal(qw.dequantize(), values)
+    off = torch.empty(N * K + 1, dtype=dtype, device="cuda")[1:].copy_(w.view(-1)).view(N, K)
+    assert torch.equal(quantize_weight(off, fmt).idx, qw.idx)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("fmt", ["oil4", "oil8", "spark"])
 @pytest.mark.parametrize("M,N,K", [(1, 32000, 4096), (64, 22016, 4096), (64, 4096, 11008), (100, 6144, 4096), (128, 4096, 4096)])
