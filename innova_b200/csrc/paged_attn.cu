@@ -14,6 +14,7 @@
 #include "inv_api.h"
 
 #include <cuda_fp16.h>
+#include <type_traits>
 
 namespace inv {
 
@@ -21,24 +22,108 @@ constexpr int PAGE = 16;
 __constant__ float c_kv_levels[16] = {-1.0f, -0.755096f, -0.588527f, -0.455957f, -0.341269f, -0.239458f, -0.146295f, -0.046361f,
                                       0.046361f, 0.146295f, 0.239458f, 0.341269f, 0.455957f, 0.588527f, 0.755096f, 1.0f};
 
+// The nearest level of x in [-1, 1] (halfway: the lower one, by the rounded differences) is the number of thresholds at or below
+// x; what is no number takes level 0. The thresholds are the smallest floats for which "(level[j] - x) < (x - level[j - 1])" holds.
+__device__ constexpr float KV_THRESHOLDS[15] = {-0x1.c14df8p-1f, -0x1.57f7acp-1f, -0x1.0b634cp-1f, -0x1.982e00p-2f, -0x1.29550ap-2f,
+                                                -0x1.8b02d4p-3f, -0x1.8a8f38p-4f, 0x1.000002p-29f,  0x1.8a8f3cp-4f,  0x1.8b02d6p-3f,
+                                                0x1.29550ep-2f,  0x1.982e02p-2f,  0x1.0b6350p-1f,  0x1.57f7b0p-1f,  0x1.c14dfap-1f};
 __device__ __forceinline__ int nearest_level16(float x) {
-  int lo = 0;
+  int n = 0;
 #pragma unroll
-  for (int step = 8; step > 0; step >>= 1)
-    if (c_kv_levels[lo + step] <= x) lo += step;
-  if (lo < 15 && (c_kv_levels[lo + 1] - x) < (x - c_kv_levels[lo])) ++lo;
-  return lo;
+  for (int j = 0; j < 15; ++j) n += x >= KV_THRESHOLDS[j] ? 1 : 0;
+  return n;
+}
+// The same in one table read for code that quantises many values: x falls into one of 256 buckets of [-1, 1], none of which holds
+// two thresholds (they are at least 0.09 apart). The margin of 1e-6 covers the rounding of the bucket's edges.
+struct KvBucket {
+  float thr;
+  int base;
+};
+constexpr int KV_BUCKETS = 256;
+__device__ __forceinline__ void kv_buckets_fill(KvBucket* t) {
+  for (int b = threadIdx.x; b < KV_BUCKETS + 2; b += blockDim.x) {
+    const float low = ((float)b - 0.5f) * (2.f / KV_BUCKETS) - 1.f - 1e-6f;
+    KvBucket e{INFINITY, 0};
+    if (b <= KV_BUCKETS) {
+      e.base = nearest_level16(low);
+#pragma unroll
+      for (int j = 0; j < 15; ++j)
+        if (j == e.base) e.thr = KV_THRESHOLDS[j];
+    }
+    t[b] = e;
+  }
+}
+// Level of w / scale with inv = 1 / scale: the product is within a few units in the last place of the quotient, which is only
+// computed where a threshold is that near.
+__device__ __forceinline__ uint32_t kv_code(const KvBucket* t, float w, float scale, float inv) {
+  float x = w * inv;
+  const KvBucket e = t[min(__float_as_int(fmaf(x, KV_BUCKETS / 2, 8388608.f + KV_BUCKETS / 2)) & (2 * KV_BUCKETS - 1), KV_BUCKETS + 1)];
+  if (fabsf(x - e.thr) < 1e-6f) x = w / scale;
+  return e.base + (x >= e.thr ? 1 : 0);
 }
 
-// One warp per (token, kv head, k-or-v): lane handles D/32 consecutive... each lane owns the elements
-// e = lane + 32*j (one per 32-block j), so a block's abs-max is a warp reduction and nibble pairs are
-// formed with a shuffle.
+// Appends S_new tokens of every sequence to the paged cache. grid = (token groups, 2 * Hkv, B): a CTA takes the keys or the values
+// of one head, D / 8 lanes a token with eight values each (a 16-byte load), so that the 16 slots of a page are written as one run
+// of bytes and four neighbouring lanes own a block of 32. Bound by memory: 64 x 512 tokens, 32 heads of 128 in 103 us,
+// 6.7 TB/s (a warp per token and head with 2-byte loads and a binary search per value: 845 us).
 template <bool OIL4>
 __global__ void __launch_bounds__(256) kv_append_kernel(const __nv_bfloat16* __restrict__ k_new, const __nv_bfloat16* __restrict__ v_new, int ld_k,
                                                         int ld_v, const int* __restrict__ page_table, int max_pages,
-                                                        const int* __restrict__ start_pos, int B, int S_new, int Hkv, int D,
+                                                        const int* __restrict__ start_pos, int S_new, int Hkv, int D,
                                                         uint8_t* __restrict__ k_pool, uint8_t* __restrict__ v_pool, __half* __restrict__ k_scale,
                                                         __half* __restrict__ v_scale) {
+  __shared__ KvBucket table[OIL4 ? KV_BUCKETS + 2 : 1];
+  if (OIL4) {
+    kv_buckets_fill(table);
+    __syncthreads();
+  }
+  const int hk = blockIdx.y >> 1, which = blockIdx.y & 1, b = blockIdx.z;
+  const int lanes = D / 8, per_pass = 256 / lanes;          // lanes of a token, tokens of a pass
+  const int sub = threadIdx.x % lanes, tok = threadIdx.x / lanes;
+  const int start = start_pos[b];
+  const int ld = which ? ld_v : ld_k;
+  const __nv_bfloat16* src = (which ? v_new : k_new) + (long)b * S_new * ld + (long)hk * D + sub * 8;
+  uint8_t* pool = which ? v_pool : k_pool;
+  __half* scales = which ? v_scale : k_scale;
+  for (int s0 = blockIdx.x * per_pass; s0 < S_new; s0 += gridDim.x * per_pass) {
+    const int s = s0 + tok;
+    const bool ok = tok < per_pass && s < S_new;
+    const uint4 raw = ok ? *reinterpret_cast<const uint4*>(src + (long)s * ld) : make_uint4(0, 0, 0, 0);
+    const int pos = start + s;
+    const long row = ok ? ((long)page_table[(long)b * max_pages + pos / PAGE] * Hkv + hk) * PAGE + pos % PAGE : 0;
+    if (!OIL4) {
+      if (ok) *reinterpret_cast<uint4*>(pool + (row * D + sub * 8) * 2) = raw;
+      continue;
+    }
+    const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
+    float w[8], amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      w[2 * i] = __uint_as_float(words[i] << 16);
+      w[2 * i + 1] = __uint_as_float(words[i] & 0xffff0000u);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(w[i]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    const float scale = amax < 1e-10f ? 1.f : amax, inv = 1.f / scale;
+    uint32_t codes = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) codes |= kv_code(table, w[i], scale, inv) << (4 * i);
+    if (ok) {
+      *reinterpret_cast<uint32_t*>(pool + row * (D / 2) + sub * 4) = codes;
+      if ((sub & 3) == 0) scales[row * (D / 32) + (sub >> 2)] = __float2half_rn(scale);
+    }
+  }
+}
+
+// The same for source rows off 16 bytes: one warp per (token, kv head, k-or-v), lane l holds the elements l + 32 j.
+template <bool OIL4>
+__global__ void __launch_bounds__(256) kv_append_rows_kernel(const __nv_bfloat16* __restrict__ k_new, const __nv_bfloat16* __restrict__ v_new, int ld_k,
+                                                             int ld_v, const int* __restrict__ page_table, int max_pages,
+                                                             const int* __restrict__ start_pos, int B, int S_new, int Hkv, int D,
+                                                             uint8_t* __restrict__ k_pool, uint8_t* __restrict__ v_pool,
+                                                             __half* __restrict__ k_scale, __half* __restrict__ v_scale) {
   const int lane = threadIdx.x & 31;
   const long warp_id = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   const long total = (long)B * S_new * Hkv * 2;
@@ -88,24 +173,25 @@ __device__ __forceinline__ bool token_visible(int tok, int len, int tail0, unsig
   return tok < len && (tok < tail0 || ((tail_bits >> ((tok - tail0) & 63)) & 1ull));
 }
 
-// Decode attention: one query token per sequence. grid = (splits, Hkv, B), 128 threads.
-// Writes partial (m, l, o[G][D]) per (b, hk, split) to scratch; attn_combine_kernel finishes.
-template <bool OIL4, int D>
+// Decode attention over a bf16 cache: one query token per sequence. grid = (splits, Hkv, B), 128 threads, a warp per 16-token page.
+// With one split the result goes straight to `out_direct`, else partial (m, l, o[G][D]) per (b, hk, split) go to scratch and
+// attn_combine_kernel finishes. Short contexts are bound by the chain of loads, so a page's keys and values are all requested
+// before the scores are computed (a loop over the tokens with one load each took 17 us at one sequence of 32 to 96 tokens).
+template <int D>
 __global__ void __launch_bounds__(128) paged_decode_kernel(const __nv_bfloat16* __restrict__ q, int ld_q, const int* __restrict__ page_table,
                                                            int max_pages, const int* __restrict__ seq_lens, int H, int Hkv,
-                                                           const uint8_t* __restrict__ k_pool, const uint8_t* __restrict__ v_pool,
-                                                           const __half* __restrict__ k_scale, const __half* __restrict__ v_scale, float scale,
-                                                           float* __restrict__ part, int splits, TreeRows tree) {
+                                                           const uint8_t* __restrict__ k_pool, const uint8_t* __restrict__ v_pool, float scale,
+                                                           float* __restrict__ part, int splits, __nv_bfloat16* __restrict__ out_direct, int ld_o,
+                                                           TreeRows tree) {
   constexpr int MAXG = 8;
   constexpr int EPL = D / 32;  // output elements per lane
   constexpr int HALF = D / 2;  // elements per lane in the QK phase (two lanes per token)
+  using VRaw = typename std::conditional<EPL == 4, uint2, uint32_t>::type;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the output projection may start on its weights
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ float sq[MAXG][D];
   __shared__ float sm_m[4][MAXG], sm_l[4][MAXG];
   __shared__ float sm_o[4][MAXG][D];
-  // the 16 levels, one copy per bank: lane l reads lv[code * 32 + l], so a warp never conflicts
-  // (a table in constant memory would serialise the 32 different indices of a warp)
-  __shared__ float lv[16 * 32];
-  for (int i = threadIdx.x; i < 16 * 32; i += blockDim.x) lv[i] = c_kv_levels[i >> 5];
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int G = H / Hkv;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -134,35 +220,15 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const __nv_bfloat16* 
   for (int pg = p0 + warp; pg < p1; pg += 4) {
     const int page = page_table[(long)seq * max_pages + pg];
     const long row0 = ((long)page * Hkv + hk) * PAGE;
-    // ---- scores: lane = (token t, half hf) ----
-    float kf[HALF];
-    if (OIL4) {
-      const uint8_t* kp = k_pool + (row0 + t) * (D / 2) + hf * (HALF / 2);
-      const __half* ks = k_scale + (row0 + t) * (D / 32) + hf * (HALF / 32);
+    // ---- loads: scores' lane = (token t, half hf); in the values a lane owns elements [lane * EPL, lane * EPL + EPL) ----
+    uint4 kraw[HALF / 8];
+    const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(k_pool) + (row0 + t) * D + hf * HALF;
 #pragma unroll
-      for (int j = 0; j < HALF / 32; ++j) {
-        const float s = __half2float(ks[j]);
-        const uint4 raw = *reinterpret_cast<const uint4*>(kp + j * 16);
-        const uint32_t wds[4] = {raw.x, raw.y, raw.z, raw.w};
+    for (int j = 0; j < HALF / 8; ++j) kraw[j] = *reinterpret_cast<const uint4*>(kp + j * 8);
+    VRaw vraw[PAGE];
+    const __nv_bfloat16* vp = reinterpret_cast<const __nv_bfloat16*>(v_pool) + row0 * D + lane * EPL;
 #pragma unroll
-        for (int w = 0; w < 4; ++w)
-#pragma unroll
-          for (int n = 0; n < 8; ++n) kf[j * 32 + w * 8 + n] = lv[(((wds[w] >> (4 * n)) & 15) << 5) + lane] * s;
-      }
-    } else {
-      const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(k_pool) + (row0 + t) * D + hf * HALF;
-#pragma unroll
-      for (int j = 0; j < HALF / 8; ++j) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(kp + j * 8);
-        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          const float2 f = __bfloat1622float2(h2[n]);
-          kf[j * 8 + 2 * n] = f.x;
-          kf[j * 8 + 2 * n + 1] = f.y;
-        }
-      }
-    }
+    for (int tt = 0; tt < PAGE; ++tt) vraw[tt] = *reinterpret_cast<const VRaw*>(vp + tt * D);
     const bool valid = token_visible(pg * PAGE + t, len, tail0, tail_bits);
     float pr[MAXG], alpha[MAXG];
 #pragma unroll
@@ -171,7 +237,14 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const __nv_bfloat16* 
         float s = 0.f;
         const float* qg = &sq[g][hf * HALF];
 #pragma unroll
-        for (int e = 0; e < HALF; ++e) s += kf[e] * qg[e];
+        for (int j = 0; j < HALF / 8; ++j) {
+          const uint32_t w[4] = {kraw[j].x, kraw[j].y, kraw[j].z, kraw[j].w};
+#pragma unroll
+          for (int n = 0; n < 4; ++n) {
+            s += __uint_as_float(w[n] << 16) * qg[j * 8 + 2 * n];
+            s += __uint_as_float(w[n] & 0xffff0000u) * qg[j * 8 + 2 * n + 1];
+          }
+        }
         s += __shfl_xor_sync(0xffffffffu, s, 16);
         s = valid ? s : -INFINITY;
         float mx = s;
@@ -187,33 +260,30 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const __nv_bfloat16* 
         m[g] = m_new;
       }
     }
-    // ---- values: lane owns output elements [lane*EPL, lane*EPL+EPL) ----
 #pragma unroll
     for (int g = 0; g < MAXG; ++g)
       if (g < G)
 #pragma unroll
         for (int e = 0; e < EPL; ++e) o[g][e] *= alpha[g];
-    const int ntok = min(PAGE, len - pg * PAGE);
-    for (int tt = 0; tt < ntok; ++tt) {
-      float vf[EPL];
-      if (OIL4) {
-        const uint8_t* vp = v_pool + (row0 + tt) * (D / 2) + (lane * EPL) / 2;
-        const float s = __half2float(v_scale[(row0 + tt) * (D / 32) + (lane * EPL) / 32]);
-        uint32_t bits = EPL == 4 ? *reinterpret_cast<const uint16_t*>(vp) : *vp;
+    const int ntok = min(PAGE, len - pg * PAGE);  // slots past the sequence's end hold whatever was there
 #pragma unroll
-        for (int e = 0; e < EPL; ++e) vf[e] = lv[(((bits >> (4 * e)) & 15) << 5) + lane] * s;
-      } else {
-        const __nv_bfloat16* vp = reinterpret_cast<const __nv_bfloat16*>(v_pool) + (row0 + tt) * D + lane * EPL;
+    for (int tt = 0; tt < PAGE; ++tt) {
+      if (tt < ntok) {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(&vraw[tt]);
+        float vf[EPL];
 #pragma unroll
-        for (int e = 0; e < EPL; ++e) vf[e] = __bfloat162float(vp[e]);
-      }
-#pragma unroll
-      for (int g = 0; g < MAXG; ++g)
-        if (g < G) {
-          const float pt = __shfl_sync(0xffffffffu, pr[g], tt);
-#pragma unroll
-          for (int e = 0; e < EPL; ++e) o[g][e] += pt * vf[e];
+        for (int e = 0; e < EPL; e += 2) {
+          vf[e] = __uint_as_float(w[e / 2] << 16);
+          vf[e + 1] = __uint_as_float(w[e / 2] & 0xffff0000u);
         }
+#pragma unroll
+        for (int g = 0; g < MAXG; ++g)
+          if (g < G) {
+            const float pt = __shfl_sync(0xffffffffu, pr[g], tt);
+#pragma unroll
+            for (int e = 0; e < EPL; ++e) o[g][e] += pt * vf[e];
+          }
+      }
     }
   }
   // ---- fold the 4 warps ----
@@ -236,6 +306,10 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const __nv_bfloat16* 
       const float f = sm_m[w][g] == -INFINITY ? 0.f : exp2f(sm_m[w][g] - mm);
       acc += sm_o[w][g][e] * f;
       ll += sm_l[w][g] * f;
+    }
+    if (out_direct != nullptr) {
+      out_direct[(long)b * ld_o + (hk * G + g) * D + e] = __float2bfloat16_rn(ll > 0.f ? acc / ll : 0.f);
+      continue;
     }
     out[g * (D + 2) + 2 + e] = acc;
     if (e == 0) {
@@ -288,6 +362,7 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32)) paged_decode_oil4_mm
     const uint32_t v = h2_as_u32(__floats2half2_rn(c_kv_levels[e & 15], c_kv_levels[e >> 4]));
     *reinterpret_cast<uint4*>(&lut[i4 * 4]) = make_uint4(v, v, v, v);
   }
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the table is built while the queries are still being written
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int G = H / Hkv;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -479,6 +554,8 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32)) paged_decode_oil4_mm
 // out[b, h*D + e] = sum_s o_s * 2^(m_s - m) / sum_s l_s * 2^(m_s - m)
 __global__ void attn_combine_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out, int ld_o, int B, int H, int Hkv, int D,
                                     int splits) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int G = H / Hkv;
   const long total = (long)B * H * D;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
@@ -500,6 +577,22 @@ __global__ void attn_combine_kernel(const float* __restrict__ part, __nv_bfloat1
   }
 }
 
+// The kernels of a decode step are a few microseconds each: every one may be launched while the one before it drains, and waits for
+// it (griddepcontrol.wait) before it reads anything.
+template <typename... Params, typename... Args>
+static void launch_early(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 }  // namespace inv
 
 using namespace inv;
@@ -508,17 +601,25 @@ extern "C" int inv_kv_append(const void* k_new, const void* v_new, int ld_k, int
                              int B, int S_new, int Hkv, int D, void* k_pool, void* v_pool, void* k_scale, void* v_scale, int oil4,
                              void* stream) {
   if (D % 32 || B <= 0 || S_new <= 0) return B <= 0 || S_new <= 0 ? 0 : -ERR_BAD_ARG;
-  const long warps = (long)B * S_new * Hkv * 2;
-  const int grid = (int)((warps + 7) / 8);
   cudaStream_t st = (cudaStream_t)stream;
-  if (oil4)
-    kv_append_kernel<true><<<grid, 256, 0, st>>>((const __nv_bfloat16*)k_new, (const __nv_bfloat16*)v_new, ld_k, ld_v, page_table, max_pages,
-                                                 start_pos, B, S_new, Hkv, D, (uint8_t*)k_pool, (uint8_t*)v_pool, (__half*)k_scale,
-                                                 (__half*)v_scale);
-  else
-    kv_append_kernel<false><<<grid, 256, 0, st>>>((const __nv_bfloat16*)k_new, (const __nv_bfloat16*)v_new, ld_k, ld_v, page_table, max_pages,
-                                                  start_pos, B, S_new, Hkv, D, (uint8_t*)k_pool, (uint8_t*)v_pool, (__half*)k_scale,
-                                                  (__half*)v_scale);
+  const __nv_bfloat16 *k = (const __nv_bfloat16*)k_new, *v = (const __nv_bfloat16*)v_new;
+  uint8_t *kp = (uint8_t*)k_pool, *vp = (uint8_t*)v_pool;
+  __half *ks = (__half*)k_scale, *vs = (__half*)v_scale;
+  const bool aligned = ((uintptr_t)k_new | (uintptr_t)v_new | (uintptr_t)k_pool | (uintptr_t)v_pool) % 16 == 0 && ld_k % 8 == 0 && ld_v % 8 == 0;
+  if (aligned && D <= 2048 && Hkv <= 32767 && B <= 65535) {
+    // four passes a CTA where there are enough of them to fill the GPU, which spreads the cost of the table
+    const int passes = (S_new + 2048 / D - 1) / (2048 / D);
+    const long ctas = (long)passes * 2 * Hkv * B;
+    const dim3 grid(ctas > 148 * 32 ? (passes + 3) / 4 : passes, 2 * Hkv, B);
+    if (oil4) kv_append_kernel<true><<<grid, 256, 0, st>>>(k, v, ld_k, ld_v, page_table, max_pages, start_pos, S_new, Hkv, D, kp, vp, ks, vs);
+    else kv_append_kernel<false><<<grid, 256, 0, st>>>(k, v, ld_k, ld_v, page_table, max_pages, start_pos, S_new, Hkv, D, kp, vp, ks, vs);
+  } else {
+    const int grid = (int)(((long)B * S_new * Hkv * 2 + 7) / 8);
+    if (oil4)
+      kv_append_rows_kernel<true><<<grid, 256, 0, st>>>(k, v, ld_k, ld_v, page_table, max_pages, start_pos, B, S_new, Hkv, D, kp, vp, ks, vs);
+    else
+      kv_append_rows_kernel<false><<<grid, 256, 0, st>>>(k, v, ld_k, ld_v, page_table, max_pages, start_pos, B, S_new, Hkv, D, kp, vp, ks, vs);
+  }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
@@ -538,6 +639,7 @@ __global__ void __launch_bounds__(256) decode_qkv_finish_kernel(float* __restric
                                                                 __half* __restrict__ k_scale, __half* __restrict__ v_scale) {
   constexpr int NJ = D / 32, HALFJ = NJ / 2;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int lane = threadIdx.x & 31;
   const long warp_id = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   const int slots = H + 2 * Hkv;
@@ -607,7 +709,7 @@ extern "C" int inv_decode_qkv_finish(float* acc, int ld_acc, const void* bias, c
   const int grid = (int)((warps + 7) / 8);
   cudaStream_t st = (cudaStream_t)stream;
 #define INV_DQF(O, DD)                                                                                                                      \
-  decode_qkv_finish_kernel<O, DD><<<grid, 256, 0, st>>>(acc, ld_acc, (const __nv_bfloat16*)bias, cos_t, sin_t, pos, page_table, max_pages, B, \
+  launch_early(decode_qkv_finish_kernel<O, DD>, dim3(grid), 256, st, acc, ld_acc, (const __nv_bfloat16*)bias, cos_t, sin_t, pos, page_table, max_pages, B, \
                                                         H, Hkv, (__nv_bfloat16*)q_out, ld_q, (uint8_t*)k_pool, (uint8_t*)v_pool,             \
                                                         (__half*)k_scale, (__half*)v_scale)
   if (oil4) {
@@ -630,32 +732,32 @@ static int paged_decode_impl(const void* q, int ld_q, const int* page_table, int
   if (B <= 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
   dim3 grid(splits, Hkv, B);
-#define INV_PD(O, DD)                                                                                                                      \
-  paged_decode_kernel<O, DD><<<grid, 128, 0, st>>>((const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H, Hkv,                 \
-                                                   (const uint8_t*)k_pool, (const uint8_t*)v_pool, (const __half*)k_scale,                 \
-                                                   (const __half*)v_scale, scale, scratch, splits, tree)
+#define INV_PD(DD)                                                                                                                         \
+  launch_early(paged_decode_kernel<DD>, grid, 128, st, (const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H, Hkv,                    \
+                                                (const uint8_t*)k_pool, (const uint8_t*)v_pool, scale, scratch, splits,                    \
+                                                splits == 1 ? (__nv_bfloat16*)out : nullptr, ld_o, tree)
   if (oil4) {
     // four warps per CTA, four CTAs per SM. Eight warps (NW = 8, two CTAs per SM) halve a CTA's serial chain of pages but
     // double the waves of the grid: 35.7 us either way at batch 64, 8 KV heads, 640 tokens of context
 #define INV_PD4(DD, NW)                                                                                                                    \
-  paged_decode_oil4_mma_kernel<DD, NW><<<grid, NW * 32, 0, st>>>((const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H, Hkv,      \
+  launch_early(paged_decode_oil4_mma_kernel<DD, NW>, grid, NW * 32, st, (const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H, Hkv,      \
                                                              (const uint8_t*)k_pool, (const uint8_t*)v_pool, (const __half*)k_scale,       \
                                                              (const __half*)v_scale, scale, scratch, splits,                                \
                                                              splits == 1 ? (__nv_bfloat16*)out : nullptr, ld_o, tree)
     if (D == 64) INV_PD4(64, 4); else INV_PD4(128, 4);
 #undef INV_PD4
-    if (splits == 1) {  // the kernel wrote the final output
-      cudaError_t e1 = cudaGetLastError();
-      return e1 == cudaSuccess ? 0 : -(int)e1;
-    }
   } else {
-    if (D == 64) INV_PD(false, 64); else INV_PD(false, 128);
+    if (D == 64) INV_PD(64); else INV_PD(128);
   }
 #undef INV_PD
+  if (splits == 1) {  // the kernel wrote the final output
+    cudaError_t e1 = cudaGetLastError();
+    return e1 == cudaSuccess ? 0 : -(int)e1;
+  }
   const long n = (long)B * H * D;
   long g = (n + 255) / 256;
   if (g > 148 * 8) g = 148 * 8;
-  attn_combine_kernel<<<(int)g, 256, 0, st>>>(scratch, (__nv_bfloat16*)out, ld_o, B, H, Hkv, D, splits);
+  launch_early(attn_combine_kernel, dim3((int)g), 256, st, scratch, (__nv_bfloat16*)out, ld_o, B, H, Hkv, D, splits);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }

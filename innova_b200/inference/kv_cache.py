@@ -53,23 +53,59 @@ class PagedRows:
 
     def reserve(self, b: int, new_len: int):
         """Make sure sequence ``b`` owns pages for ``new_len`` tokens."""
+        if self._take_pages(b, new_len):
+            pages = self._host_pages[b]
+            self.page_table[b, : len(pages)] = torch.tensor(pages, dtype=torch.int32, device=self.device)
+
+    def reserve_rows(self, rows, new_len: int):
+        """``reserve`` for several sequences with one copy of the page table."""
+        grown = []
+        try:
+            for b in rows:
+                if self._take_pages(b, new_len):
+                    grown.append(b)
+        finally:
+            if grown:
+                flat = [p for b in grown for p in self._host_pages[b]]
+                counts = [len(self._host_pages[b]) for b in grown]
+                if len(set(counts)) == 1 and grown == list(range(grown[0], grown[0] + len(grown))):
+                    table = torch.tensor(flat, dtype=torch.int32, device=self.device).view(len(grown), counts[0])
+                    self.page_table[grown[0]:grown[-1] + 1, : counts[0]] = table
+                else:
+                    where = torch.tensor([b * self.max_pages + i for b, n in zip(grown, counts) for i in range(n)], device=self.device)
+                    self.page_table.view(-1)[where] = torch.tensor(flat, dtype=torch.int32, device=self.device)
+
+    def _take_pages(self, b: int, new_len: int) -> bool:
         need = (new_len + PAGE - 1) // PAGE
         if need > self.max_pages:
             raise MemoryError(f"sequence of {new_len} tokens is longer than the cache's {self.max_pages * PAGE}")
         pages = self._host_pages[b]
         if need - len(pages) > len(self._free):
             raise MemoryError("paged KV cache is out of pages")
-        if len(pages) < need:
-            while len(pages) < need:
-                pages.append(self._free.pop())
-            self.page_table[b, : len(pages)] = torch.tensor(pages, dtype=torch.int32, device=self.device)
+        grown = len(pages) < need
+        while len(pages) < need:
+            pages.append(self._free.pop())
+        return grown
 
     def free(self, b: int):
+        self._drop_pages(b)
+        self.seq_lens[b] = 0
+
+    def free_rows(self, rows):
+        """``free`` for several sequences with one write of the lengths."""
+        rows = list(rows)
+        for b in rows:
+            self._drop_pages(b)
+        if len(set(rows)) == self.max_batch:
+            self.seq_lens.zero_()
+        elif rows:
+            self.seq_lens[torch.tensor(rows, device=self.device)] = 0
+
+    def _drop_pages(self, b: int):
         self._free.extend(reversed(self._host_pages[b][self._released[b]:]))
         self._host_pages[b] = []
         self._released[b] = 0
         self._host_lens[b] = 0
-        self.seq_lens[b] = 0
 
     def release_before(self, b: int, position: int):
         """Give back the pages of sequence ``b`` that hold only tokens before ``position``."""

@@ -137,3 +137,78 @@ def test_gpu_sampler_and_generation():
     assert agree >= 12  # bf16 ties may flip a late token
     out_q = Generator(model, kv_format="oil4", max_batch=2, max_seq=256).generate_tokens(ids, 8)
     assert len(out_q[0]) == 8
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", ["oil4", "bf16"])
+@pytest.mark.parametrize("B,S,Hkv,D,start", [(1, 1, 1, 32, 0), (3, 37, 2, 64, 5), (2, 131, 4, 128, 16), (2, 50, 3, 96, 30), (64, 70, 8, 128, 0)])
+def test_gpu_kv_append_whole_rows_as_single_values(fmt, B, S, Hkv, D, start):
+    """The append of 16-byte pieces against the one that takes a value per lane (rows off 16 bytes), byte for byte: zero blocks,
+    values on and beside the halfway points, infinities and what is no number among them."""
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device="cuda").manual_seed(B + S)
+    kv = torch.randn(B, S, 2 * Hkv * D, device=dev, generator=g).bfloat16()
+    flat = kv.view(-1)
+    flat[: D // 2] = 0.0
+    grid = torch.linspace(-1.0, 1.0, flat[D:].numel(), device=dev).bfloat16()
+    flat[D:][::3] = grid[::3]
+    if S > 30:
+        kv[0, 3, 1], kv[0, 4, 2], kv[0, 5, 3] = float("inf"), float("nan"), -float("inf")
+        kv[0, 6, 4], kv[0, 7] = 3e38, 1e-39
+    odd = torch.empty(B * S * (2 * Hkv * D + 1) + 1, dtype=torch.bfloat16, device=dev)[1:].view(B, S, 2 * Hkv * D + 1)
+    odd[..., : 2 * Hkv * D] = kv
+    caches = []
+    for src in (kv, odd):
+        c = PagedKVCache(1, Hkv, D, B, S + start + 16, dev, fmt)
+        c.reserve_rows(range(B), S + start)
+        c.append(0, src[..., : Hkv * D], src[..., Hkv * D:2 * Hkv * D], list(range(B)), [start] * B)
+        caches.append(c)
+    for name in ("k_pool", "v_pool") + (("k_scale", "v_scale") if fmt == "oil4" else ()):
+        a, b = (getattr(c, name)[0].view(torch.uint8) for c in caches)
+        assert torch.equal(a, b), name
+
+
+def test_reserve_and_free_rows_as_one_by_one():
+    for rows, lens in (([0, 1, 2], [33, 33]), ([2, 0], [5, 40]), ([1], [17, 64])):
+        one, many = (PagedKVCache(1, 1, 32, 4, 64, "cpu", "bf16", num_pages=10) for _ in range(2))
+        for n in lens:
+            for b in rows:
+                one.reserve(b, n)
+            many.reserve_rows(rows, n)
+        assert torch.equal(one.page_table, many.page_table) and one._free == many._free and one._host_pages == many._host_pages
+        one.seq_lens.fill_(9), many.seq_lens.fill_(9)
+        for b in rows:
+            one.free(b)
+        many.free_rows(rows)
+        assert torch.equal(one.seq_lens, many.seq_lens) and one._free == many._free
+    full = PagedKVCache(1, 1, 32, 4, 64, "cpu", "bf16", num_pages=5)
+    with pytest.raises(MemoryError):
+        full.reserve_rows([0, 1, 2], 40)
+    assert len(full._host_pages[0]) == 3 and full.page_table[0, :3].tolist() == full._host_pages[0]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,H,Hkv,n,splits", [(128, 16, 4, 1, 1), (128, 16, 4, 97, 1), (64, 8, 1, 203, 1), (128, 16, 4, 203, 3), (64, 4, 4, 16, 1)])
+def test_gpu_bf16_decode_attention_direct_and_split(D, H, Hkv, n, splits):
+    """Against fp64 attention; the slots behind the last token hold what is no number and must not count. fp32 inside: what is left is
+    the rounding of the result."""
+    from innova_b200.ops import runtime as rt
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    c = PagedKVCache(1, Hkv, D, 1, 256, dev, "bf16")
+    for pool in (c.k_pool, c.v_pool):
+        pool[0].view(torch.bfloat16).fill_(float("nan"))
+    c.reserve(0, n)
+    k, v = (torch.randn(1, n, Hkv * D, device=dev, generator=g).bfloat16() for _ in range(2))
+    c.append(0, k, v, [0], [0])
+    c.commit([0], [n])
+    q = torch.randn(1, H * D, device=dev, generator=g).bfloat16()
+    out = torch.empty_like(q)
+    scr = torch.empty(H * splits * (D + 2), device=dev)
+    rt.check(rt.lib().inv_paged_decode(q.data_ptr(), q.stride(0), c.page_table.data_ptr(), c.max_pages, c.seq_lens.data_ptr(), 1, H, Hkv, D,
+                                       c.k_pool[0].data_ptr(), c.v_pool[0].data_ptr(), 0, 0, 0, D ** -0.5, out.data_ptr(), out.stride(0),
+                                       scr.data_ptr(), splits, rt.stream_ptr()), "inv_paged_decode")
+    qd, kd, vd = q.double().view(Hkv, H // Hkv, D), k.double().view(n, Hkv, D), v.double().view(n, Hkv, D)
+    p = torch.softmax(torch.einsum("hgd,thd->hgt", qd, kd) * D ** -0.5, -1)
+    ref = torch.einsum("hgt,thd->hgd", p, vd).reshape(1, -1)
+    assert float((out.double() - ref).norm() / ref.norm()) < 2.0 ** -8
