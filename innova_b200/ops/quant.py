@@ -168,6 +168,7 @@ def dequantize_blockwise(idx: torch.Tensor, scales: torch.Tensor, fmt: str = "oi
 class _SteFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, w, fmt, cb, block):
+        ctx.set_materialize_grads(False)     # a gradient that went to ``main_grad`` arrives as None: nothing to fill, widen and add
         if w.is_cuda and block == BLOCK:
             src = w.contiguous()
             out = torch.empty_like(src)

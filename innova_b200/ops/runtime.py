@@ -14,7 +14,7 @@ ERR_NAMES = {
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())   # no Stream object made for every launch
 
 
 def status_tensor(device=None) -> torch.Tensor:

@@ -313,3 +313,25 @@ def test_speculative_tree_decoder_gpu_equals_greedy():
     # bf16 logits of the batched draft rows and of the tree rows may break a near tie differently: the prefix must agree
     agree = next((i for i, (a, b) in enumerate(zip(got, ref)) if a != b), len(ref))
     assert agree >= 12 and dec.stats.target_calls < 24
+
+
+@pytest.mark.gpu
+def test_gpu_quantised_weight_gradient_goes_to_main_grad_alone():
+    """Through the straight-through quantiser the fp32 gradient accumulates in place and autograd has nothing left to hand on; a weight
+    without ``main_grad`` still gets its ``.grad``."""
+    from innova_b200 import ops
+    from innova_b200.ops.quant import ste_fake_quant
+    g = torch.Generator(device="cuda").manual_seed(3)
+    w0 = (torch.randn(192, 128, device="cuda", generator=g) * 0.1).bfloat16()
+    x = torch.randn(64, 128, device="cuda", generator=g).bfloat16()
+    dy = torch.randn(64, 192, device="cuda", generator=g).bfloat16()
+    want = dy.double().t() @ x.double()
+    for fused in (True, False):
+        w = w0.clone().requires_grad_()
+        if fused:
+            w.main_grad = torch.ones(192, 128, device="cuda")
+        ops.linear(x, ste_fake_quant(w, "oil8")).backward(dy)
+        if fused:
+            assert w.grad is None and float((w.main_grad.double() - 1 - want).norm() / want.norm()) < 1e-5
+        else:
+            assert float((w.grad.double() - want).norm() / want.norm()) < 2.0 ** -8
