@@ -466,6 +466,144 @@ __global__ void __launch_bounds__(256, 1) norm_bwd_rows_kernel(const __nv_bfloat
   }
 }
 
+// ----------------------------------------------------------------------------------------------
+// Backward for 1024 < D <= 8192. A CTA owns a row: eight columns per thread and NV such pieces, so that the column sums stay in
+// registers (the general form keeps them in shared memory, an atomic per element and sum: 4096 x 2048 in 63 us). R rows are
+// reduced together over one barrier and the x, dy and dres of the next R are in flight meanwhile, 48 KB per SM, which is what the
+// memory system needs.
+// ----------------------------------------------------------------------------------------------
+template <bool RMS, int NV, bool RES>
+__global__ void __launch_bounds__(256, 1) norm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                                                               const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
+                                                               const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
+                                                               __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int T, int D) {
+  constexpr int R = NV == 1 ? 4 : NV == 2 ? 2 : 1;
+  __shared__ float2 red[2][R][8];  // sums of a group of rows per warp, alternating between groups
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint4 g[NV];
+  float dg[NV][8], db[RMS ? 1 : NV][8];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int c = (k * 256 + tid) * 8;
+    g[k] = c < D ? *reinterpret_cast<const uint4*>(gamma + c) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      dg[k][j] = 0.f;
+      if (!RMS) db[k][j] = 0.f;
+    }
+  }
+  struct Rows {
+    uint4 x[R][NV], d[R][NV], r[RES ? R : 1][RES ? NV : 1];
+    float mean[R], rstd[R];
+  };
+  // rows past T and columns past D count as zeros
+  auto fetch = [&](int row0, Rows& v) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int row = row0 + i;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        const int c = (k * 256 + tid) * 8;
+        const bool in = row < T && c < D;
+        const size_t at = (size_t)row * D + c;
+        v.x[i][k] = in ? *reinterpret_cast<const uint4*>(x + at) : make_uint4(0, 0, 0, 0);
+        v.d[i][k] = in ? *reinterpret_cast<const uint4*>(dy + at) : make_uint4(0, 0, 0, 0);
+        if (RES) v.r[i][k] = in ? *reinterpret_cast<const uint4*>(dres + at) : make_uint4(0, 0, 0, 0);
+      }
+      v.mean[i] = !RMS && row < T ? mean_in[row] : 0.f;
+      v.rstd[i] = row < T ? rstd_in[row] : 0.f;
+    }
+  };
+  int turn = 0;
+  auto process = [&](int row0, const Rows& v) {
+    float2 s[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      s[i] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        if ((k * 256 + tid) * 8 >= D) continue;
+        float xv[8], dv[8], gv[8];
+        unpack8(v.x[i][k], xv);
+        unpack8(v.d[i][k], dv);
+        unpack8(g[k], gv);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float gg = dv[j] * gv[j];
+          s[i].x += gg;
+          s[i].y += gg * ((xv[j] - v.mean[i]) * v.rstd[i]);
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        if (!RMS) s[i].x += __shfl_xor_sync(0xffffffffu, s[i].x, o);
+        s[i].y += __shfl_xor_sync(0xffffffffu, s[i].y, o);
+      }
+      if (lane == 0) red[turn][i][warp] = s[i];
+    }
+    __syncthreads();  // the next group writes the other half, so one barrier a group is enough
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int row = row0 + i;
+      if (row >= T) continue;
+      float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        s1 += red[turn][i][w].x;
+        s2 += red[turn][i][w].y;
+      }
+      s1 = RMS ? 0.f : s1 / D;
+      s2 /= D;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        const int c = (k * 256 + tid) * 8;
+        if (c >= D) continue;
+        float xv[8], dv[8], gv[8], o[8];
+        unpack8(v.x[i][k], xv);
+        unpack8(v.d[i][k], dv);
+        unpack8(g[k], gv);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float xh = (xv[j] - v.mean[i]) * v.rstd[i];
+          o[j] = v.rstd[i] * (dv[j] * gv[j] - s1 - xh * s2);
+          dg[k][j] += dv[j] * xh;
+          if (!RMS) db[k][j] += dv[j];
+        }
+        if (RES) {
+          float r[8];
+          unpack8(v.r[i][k], r);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] += r[j];
+        }
+        store8(dx + (size_t)row * D + c, o);
+      }
+    }
+    turn ^= 1;
+  };
+  const int step = gridDim.x * R;
+  Rows a, b;
+  fetch(blockIdx.x * R, a);
+  for (int row = blockIdx.x * R; row < T; row += 2 * step) {
+    fetch(row + step, b);
+    process(row, a);
+    if (row + step < T) {
+      fetch(row + 2 * step, a);
+      process(row + step, b);
+    }
+  }
+  float* out = partial + (size_t)blockIdx.x * 2 * D;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int c = (k * 256 + tid) * 8;
+    if (c >= D) continue;
+#pragma unroll
+    for (int j = 0; j < 8; j += 4) {
+      *reinterpret_cast<float4*>(out + c + j) = make_float4(dg[k][j], dg[k][j + 1], dg[k][j + 2], dg[k][j + 3]);
+      if (!RMS) *reinterpret_cast<float4*>(out + D + c + j) = make_float4(db[k][j], db[k][j + 1], db[k][j + 2], db[k][j + 3]);
+    }
+  }
+}
+
 // dgamma[D] += sum_b partial[b][0][:], dbeta[D] += sum_b partial[b][1][:], colsum[D] = sum_b partial_cs[b][:].
 // grid (ceil(D / 32), 3): a CTA owns 32 columns of one of the three sums; its 8 warps take the partial rows round robin
 // (coalesced 128-byte reads) and meet in shared memory.
@@ -567,6 +705,19 @@ static int norm_bwd_launch(const void* dy, const void* x, const void* gamma, con
     } else {
       if (nch == 1) INV_NB_ROWS(false, 1); else if (nch == 2) INV_NB_ROWS(false, 2); else if (nch == 3) INV_NB_ROWS(false, 3); else INV_NB_ROWS(false, 4);
     }
+  } else if (D <= 8192 && reinterpret_cast<uintptr_t>(scratch) % 16 == 0) {
+    // the sums of wider rows no longer fit the registers next to two groups of rows
+#define INV_NB_WIDE(R, N)                                                                                                             \
+  do {                                                                                                                                \
+    if (DR) norm_bwd_wide_kernel<R, N, true><<<grid, 256, 0, st>>>(DY, X, G, mean, rstd, DR, DX, scratch, T, D);                      \
+    else norm_bwd_wide_kernel<R, N, false><<<grid, 256, 0, st>>>(DY, X, G, mean, rstd, DR, DX, scratch, T, D);                        \
+  } while (0)
+    if (rms) {
+      if (D <= 2048) INV_NB_WIDE(true, 1); else if (D <= 4096) INV_NB_WIDE(true, 2); else INV_NB_WIDE(true, 4);
+    } else {
+      if (D <= 2048) INV_NB_WIDE(false, 1); else if (D <= 4096) INV_NB_WIDE(false, 2); else INV_NB_WIDE(false, 4);
+    }
+#undef INV_NB_WIDE
   } else if (rms) {
     norm_bwd_kernel<true><<<grid, 256, smem, st>>>(DY, X, G, mean, rstd, DR, DX, scratch, T, D);
   } else {

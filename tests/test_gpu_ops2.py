@@ -335,3 +335,37 @@ def test_gpu_quantised_weight_gradient_goes_to_main_grad_alone():
             assert w.grad is None and float((w.main_grad.double() - 1 - want).norm() / want.norm()) < 1e-5
         else:
             assert float((w.grad.double() - want).norm() / want.norm()) < 2.0 ** -8
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rms", [True, False])
+@pytest.mark.parametrize("T,D", [(1, 1032), (3, 2048), (600, 2048), (37, 2056), (1300, 4096), (9, 5120), (150, 8192), (5, 8200)])
+@pytest.mark.parametrize("on_residual", [True, False])
+def test_gpu_norm_backward_of_wide_rows(T, D, rms, on_residual):
+    """dx, dgamma and dbeta of rows wider than a warp's registers against fp64; dx is rounded to bf16 (2^-9), the sums are fp32."""
+    from innova_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(D + T)
+
+    def rand(*s):
+        return torch.randn(*s, device="cuda", generator=g).bfloat16()
+
+    x, gamma, beta, dy, dres = rand(T, D), rand(D), rand(D), rand(T, D), rand(T, D)
+    params = [t.clone().requires_grad_() for t in ((x, gamma) if rms else (x, gamma, beta))]
+    for p in params[1:]:
+        p.main_grad = torch.zeros(D, device="cuda")
+    if on_residual:
+        y, r = ops.norm_residual(params[0], params[1], None if rms else params[2], 1e-5, rms)
+        torch.autograd.backward([y, r], [dy, dres])
+    else:
+        y = ops.rms_norm(*params, 1e-5) if rms else ops.layer_norm(*params, 1e-5)
+        y.backward(dy)
+    ref = [p.detach().double().requires_grad_() for p in params]
+    if rms:
+        yr = ref[0] * torch.rsqrt(ref[0].square().mean(-1, keepdim=True) + 1e-5) * ref[1]
+    else:
+        yr = torch.nn.functional.layer_norm(ref[0], (D,), ref[1], ref[2], 1e-5)
+    yr.backward(dy.double())
+    want = ref[0].grad + (dres.double() if on_residual else 0)
+    assert float((params[0].grad.double() - want).norm() / want.norm()) < 2.0 ** -8
+    for p, q in zip(params[1:], ref[1:]):
+        assert float((p.main_grad.double() - q.grad).norm() / q.grad.norm()) < 1e-4
