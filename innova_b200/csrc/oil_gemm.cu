@@ -27,6 +27,7 @@
 // streams the same number of index bytes whatever N and K are, and the partial sums of a range are added to the
 // fp32 output with reductions. Every wait is bounded.
 #include "sm100_common.cuh"
+#include "oil_expand.cuh"
 #include "inv_api.h"
 
 #include <mutex>
@@ -100,58 +101,9 @@ static int make_tmap_bytes(CUtensorMap* out, const void* ptr, uint64_t inner, ui
 template <int BITS>
 __device__ __forceinline__ void expand_row(const uint4* raw, __nv_bfloat16 s0, __nv_bfloat16 s1, const uint32_t* lut, const float* cb, int lane,
                                            uint32_t* o) {
-  if (BITS == 2) {
-    // 4-entry codebook (ternary {-1, 0, +1, 0} for SPARK / OIL1 weights, or the OIL2 levels): the four scaled
-    // entries sit in one 64-bit register and every 2-bit code selects 16 bits of it
-    const uint32_t w[4] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w};
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const __nv_bfloat162 sc2 = __halves2bfloat162(h ? s1 : s0, h ? s1 : s0);
-      const __nv_bfloat162 e01 = __hmul2(__floats2bfloat162_rn(cb[0], cb[1]), sc2);
-      const __nv_bfloat162 e23 = __hmul2(__floats2bfloat162_rn(cb[2], cb[3]), sc2);
-      const uint64_t tbl = (uint64_t)(*reinterpret_cast<const uint32_t*>(&e01)) | ((uint64_t)(*reinterpret_cast<const uint32_t*>(&e23)) << 32);
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {  // a 32-bit word = 16 codes = 8 output pairs
-        const uint32_t codes = w[h * 2 + j];
-#pragma unroll
-        for (int b = 0; b < 8; ++b) {
-          const uint32_t lo = (uint32_t)(tbl >> (16 * ((codes >> (4 * b)) & 3))) & 0xffffu;
-          const uint32_t hi = (uint32_t)(tbl >> (16 * ((codes >> (4 * b + 2)) & 3))) << 16;
-          o[h * 16 + j * 8 + b] = lo | hi;
-        }
-      }
-    }
-  } else if (BITS == 4) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const __nv_bfloat162 sc2 = __halves2bfloat162(h ? s1 : s0, h ? s1 : s0);
-      const uint32_t w[4] = {raw[h].x, raw[h].y, raw[h].z, raw[h].w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const uint32_t pair = lut[(((w[j] >> (8 * b)) & 255) << 5) + lane];
-          const __nv_bfloat162 v = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&pair), sc2);
-          o[h * 16 + j * 4 + b] = *reinterpret_cast<const uint32_t*>(&v);
-        }
-    }
-  } else {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const __nv_bfloat162 sc2 = __halves2bfloat162(h ? s1 : s0, h ? s1 : s0);
-      const uint32_t w[8] = {raw[h * 2].x, raw[h * 2].y, raw[h * 2].z, raw[h * 2].w, raw[h * 2 + 1].x, raw[h * 2 + 1].y, raw[h * 2 + 1].z, raw[h * 2 + 1].w};
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const uint32_t two = w[j] >> (16 * b);
-          const uint32_t lo = lut[((two & 255) << 5) + lane] & 0xffffu, hi = lut[(((two >> 8) & 255) << 5) + lane] << 16;
-          const uint32_t pair = lo | hi;
-          const __nv_bfloat162 v = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&pair), sc2);
-          o[h * 16 + j * 2 + b] = *reinterpret_cast<const uint32_t*>(&v);
-        }
-    }
-  }
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(raw);
+  expand_block<BITS>(w, s0, lut, cb, lane, o);
+  expand_block<BITS>(w + BITS, s1, lut, cb, lane, o + 16);
 }
 
 // Walks a CTA's work in order: `dp_rounds` whole tiles (tile = round * grid + cta, every batch of K), then its share of
@@ -227,8 +179,8 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sX = smem;                                  // 2 slots x KBB activation tiles (X_TILE is a multiple of 2 KB)
   uint8_t* sIdx = sX + 2 * KBB * X_TILE;               // IDX_STAGES x IDX_TILE (swizzled by TMA: 1 KB aligned)
-  uint32_t* lut = reinterpret_cast<uint32_t*>(sIdx + IDX_STAGES * IDX_TILE);  // 256 entries x 32 bank copies
-  float* stage = reinterpret_cast<float*>(lut + 256 * 32);  // epilogue staging: per group STG_TOK tokens x STG_PITCH
+  __shared__ __align__(128) uint32_t lut[BITS == 2 ? 32 : 256 * 32];   // 256 entries x 32 bank copies, at a fixed address
+  float* stage = reinterpret_cast<float*>(sIdx + IDX_STAGES * IDX_TILE);  // epilogue staging: per group STG_TOK tokens x STG_PITCH
   uint64_t* bars = reinterpret_cast<uint64_t*>(stage + 2 * STG_TOK * STG_PITCH);
   uint64_t* idx_full = bars;
   uint64_t* idx_empty = idx_full + MAX_IDX_STAGES;
@@ -380,11 +332,7 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
     if (grp == 1 && pc.valid) pc.advance();
     if (pc.valid) fetch_scales(pc.tile, pc.bb);  // in flight while the table is built
     if (BITS != 2) {
-      // eight lanes write the 32 bank copies of one entry as 16-byte stores: a warp covers four entries (512 contiguous bytes)
-      for (int e = (warp - 2) * 4 + (lane >> 3); e < 256; e += 32) {
-        const uint32_t v = (BITS == 4) ? pack_bf16x2(cb[e & 15], cb[e >> 4]) : pack_bf16x2(cb[e], 0.f);
-        *reinterpret_cast<uint4*>(lut + e * 32 + (lane & 7) * 4) = make_uint4(v, v, v, v);
-      }
+      oil_lut_fill<BITS>(lut, cb, threadIdx.x - 64, 256);
       asm volatile("bar.sync 1, 256;" ::: "memory");
     }
     if (threadIdx.x == 64) OG_STAMP(4);
@@ -762,8 +710,9 @@ static int oil_gemm_launch(const void* x, int ldx, const void* idx, const void* 
   if ((rc = make_tmap_bytes(&ti, idx, (uint64_t)row_bytes, (uint64_t)N, rowb, BN))) return rc;
   if ((rc = make_tmap_2d_bf16(&tx, x, (uint64_t)K, (uint64_t)M, (uint64_t)ldx, BK, (uint32_t)p.Mpad))) return rc;
   const int idx_tile = BN * rowb;
-  const int fixed = 1024 + 2 * kbb * p.Mpad * BK * 2 + 256 * 32 * 4 + 2 * STG_TOK * STG_PITCH * 4 + (2 * MAX_IDX_STAGES + 12) * 8 + 16 + 1024 + 64;
-  int stages = (227 * 1024 - fixed) / idx_tile;
+  const int table = bits == 2 ? 128 : 256 * 32 * 4;   // static shared memory
+  const int fixed = 1024 + 2 * kbb * p.Mpad * BK * 2 + 2 * STG_TOK * STG_PITCH * 4 + (2 * MAX_IDX_STAGES + 12) * 8 + 16 + 1024 + 64;
+  int stages = (227 * 1024 - table - fixed) / idx_tile;
   if (stages > MAX_IDX_STAGES) stages = MAX_IDX_STAGES;
   stages &= ~1;  // even: a ring stage is then always read by the same expanding group, which sees every phase of its barrier
   if (stages < 2) return -ERR_BAD_ARG;
@@ -771,9 +720,9 @@ static int oil_gemm_launch(const void* x, int ldx, const void* idx, const void* 
   const int smem = fixed + stages * idx_tile;
   static bool configured = false;
   if (!configured) {
-    cudaFuncSetAttribute(oil_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    cudaFuncSetAttribute(oil_gemm_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    cudaFuncSetAttribute(oil_gemm_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(oil_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 128);
+    cudaFuncSetAttribute(oil_gemm_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (227 - 32) * 1024);
+    cudaFuncSetAttribute(oil_gemm_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (227 - 32) * 1024);
     configured = true;
   }
   // at least two batches per CTA (one per expanding group): shorter ranges cost more in prologue and reductions

@@ -24,6 +24,8 @@ _native.register_cuda_sigs({
                      _native.i32, _native.i32, _native.vp, _native.vp, _native.i32],
     "inv_oil_gemm_finish": [_native.vp, _native.vp, _native.vp, _native.vp, _native.i64, _native.i32, _native.i32, _native.i32, _native.i32,
                             _native.i32, _native.vp],
+    "inv_oil_skinny": [_native.vp, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp, _native.f32, _native.vp, _native.vp,
+                       _native.i32, _native.vp, _native.i32, _native.i32, _native.i32, _native.i32, _native.i32, _native.vp],
     "inv_oil_gemm_peers": [_native.vp, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp, _native.i32, _native.i32, _native.i32,
                            _native.i32, _native.i32, _native.vp, _native.vp],
     "inv_oil_gemm_rs": [_native.vp, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp, _native.i32, _native.i32, _native.i32,
@@ -135,6 +137,30 @@ def _gemm_into_acc(xs: torch.Tensor, qw: QuantWeight, acc: torch.Tensor):
                                    acc.data_ptr(), acc.stride(0), xs.shape[0], qw.N, qw.K, 0, status, rt.stream_ptr(), 0), "inv_oil_gemm")
 
 
+SKINNY_TOKENS = 16        # up to here one launch without tensor memory, accumulator and finish pass is faster
+SKINNY_PLAIN, SKINNY_SWIGLU, SKINNY_SUMS = 0, 1, 2
+
+
+def skinny_smem_fits(M: int, K: int) -> bool:
+    return (K + 255) // 256 * 128 * (4 * M + 1) <= 180 * 1024
+
+
+def skinny_fits(x2: torch.Tensor, qw: QuantWeight) -> bool:
+    """Whether ``_skinny`` takes x2 [M, K]: a few tokens whose rows fit shared memory."""
+    M = x2.shape[0]
+    return (1 <= M <= SKINNY_TOKENS and skinny_smem_fits(M, qw.K) and x2.data_ptr() % 16 == 0 and x2.stride(0) % 8 == 0
+            and x2.stride(1) == 1 and qw.idx.data_ptr() % 32 == 0 and qw.scales.data_ptr() % 4 == 0)
+
+
+def _skinny(x2: torch.Tensor, qw: QuantWeight, out: torch.Tensor, mode: int = SKINNY_PLAIN, residual: Optional[torch.Tensor] = None, norm=None):
+    """One launch for ``out`` [M, N] (or [M, N / 2], or fp32 sums) from x2 [M, K]; ``norm = (weight, eps)``: of rms_norm(x2) * weight."""
+    rt.check(rt.lib().inv_oil_skinny(x2.data_ptr(), x2.stride(0), qw.idx.data_ptr(), qw.scales.data_ptr(), qw.codebook.data_ptr(), qw.bits,
+                                     None if norm is None else norm[0].data_ptr(), 0.0 if norm is None else float(norm[1]), rt.ptr(qw.bias),
+                                     rt.ptr(residual), 0 if residual is None else residual.stride(0), out.data_ptr(), out.stride(0), x2.shape[0],
+                                     qw.N, qw.K, mode, rt.stream_ptr()), "inv_oil_skinny")
+    return out
+
+
 def oil_linear(x: torch.Tensor, qw: QuantWeight, residual: Optional[torch.Tensor] = None, split_k: int = 0) -> torch.Tensor:
     """x [..., K] bf16 -> [..., N] bf16."""
     shp = x.shape
@@ -148,8 +174,10 @@ def oil_linear(x: torch.Tensor, qw: QuantWeight, residual: Optional[torch.Tensor
         x2 = x2.contiguous()
     M = x2.shape[0]
     out = torch.empty((M, qw.N), dtype=torch.bfloat16, device=x.device)
-    acc = _acc_for(x, qw, M)
     res2 = None if residual is None else residual.reshape(-1, qw.N)
+    if skinny_fits(x2, qw):
+        return _skinny(x2, qw, out, residual=res2).view(*shp[:-1], qw.N)
+    acc = _acc_for(x, qw, M)
     for m0 in range(0, M, 256):
         m1 = min(M, m0 + 256)
         _gemm_into_acc(x2[m0:m1], qw, acc)
@@ -172,6 +200,8 @@ def oil_linear_swiglu(x: torch.Tensor, qw: QuantWeight) -> torch.Tensor:
         x2 = x2.contiguous()
     M = x2.shape[0]
     out = torch.empty((M, Fh), dtype=torch.bfloat16, device=x.device)
+    if skinny_fits(x2, qw):
+        return _skinny(x2, qw, out, SKINNY_SWIGLU).view(*shp[:-1], Fh)
     acc = _acc_for(x, qw, M)
     for m0 in range(0, M, 256):
         m1 = min(M, m0 + 256)
@@ -211,6 +241,10 @@ def oil_linear_norm(x: torch.Tensor, qw: QuantWeight, residual: torch.Tensor, no
         return y, rms_norm(y, norm_w, eps)
     if not x2.is_contiguous():
         x2 = x2.contiguous()
+    if skinny_fits(x2, qw):
+        from .functional import rms_norm
+        y = _skinny(x2, qw, torch.empty((M, qw.N), dtype=torch.bfloat16, device=x.device), residual=residual.reshape(M, qw.N))
+        return y, rms_norm(y, norm_w, eps)
     acc = _acc_for(x, qw, M)
     _gemm_into_acc(x2, qw, acc)
     return finish_norm(acc, M, qw.N, qw.bias, residual.reshape(M, qw.N), norm_w, eps)

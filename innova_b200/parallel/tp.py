@@ -26,7 +26,8 @@ from .. import ops
 from ..inference.kv_cache import PagedKVCache, PAGE
 from ..models.config import TransformerConfig
 from ..ops import runtime as rt
-from ..ops.oil_linear import QuantWeight, _acc_for, _gemm_into_acc, finish_norm, oil_linear, oil_linear_norm, oil_linear_swiglu, quantize_weight
+from ..ops.oil_linear import (SKINNY_SUMS, SKINNY_SWIGLU, SKINNY_TOKENS, QuantWeight, _acc_for, _gemm_into_acc, _skinny, finish_norm, oil_linear,
+                              oil_linear_norm, oil_linear_swiglu, quantize_weight, skinny_smem_fits)
 
 
 class TPContext:
@@ -143,6 +144,11 @@ def tp_reduce_linear(x: torch.Tensor, qw: QuantWeight, ctx: Optional[TPContext],
     return out
 
 
+# Prompts of up to this many tokens in all multiply with the packed weights. 22016 x 4096 at 128 tokens: 61 us against 88 us for
+# expanding the matrix and one wide product; at 256 tokens, which read the weights twice, 116 against 103.
+FEW_PROMPT_TOKENS = 128
+
+
 class TPDecoder:
     """Llama-style decoder, OIL4 (or OIL8) weights sharded over the ranks of ``group``, random-init from
     ``seed`` (every rank draws the full matrix on its GPU, keeps its shard, quantises it, drops the rest)."""
@@ -192,7 +198,8 @@ class TPDecoder:
         self.rope = ops.rope_tables(max_seq, D, cfg.rope_theta, self.dev)
         self.cache = PagedKVCache(cfg.num_layers, self.Hkv, D, max_batch, max_seq, self.dev, kv_format)
         self.max_batch, self.max_seq = max_batch, max_seq
-        self._graph = None
+        self._side = self._graph = None          # stream of the captured step; the last capture, which keeps its memory pool alive
+        self._warmed = set()
         torch.cuda.synchronize()
 
     def weight_bytes(self) -> int:
@@ -207,29 +214,45 @@ class TPDecoder:
         cfg, c = self.cfg, self.cache
         B, S = ids.shape
         H, Hkv, D = self.H, self.Hkv, self.D
-        for b in range(c.max_batch):
-            c.free(b)
-        for b in range(B):
-            c.reserve(b, self.max_seq)  # every page a sequence can need, so that the decode graph never allocates
+        c.free_rows(range(c.max_batch))
+        c.reserve_rows(range(B), self.max_seq)  # every page a sequence can need, so that the decode graph never allocates
         x = self.emb[ids]
-        start = [0] * B
+        rows, start = list(range(B)), [0] * B
+        few = self.world == 1 and B * S <= FEW_PROMPT_TOKENS
+        h = ops.rms_norm(x, self.layers[0]["n1"], cfg.norm_eps)
         for li, l in enumerate(self.layers):
-            h = ops.rms_norm(x, l["n1"], cfg.norm_eps)
-            qkv = ops.linear(h, l["qkv"].dequantize())
+            qkv = oil_linear(h, l["qkv"]) if few else ops.linear(h, l["qkv"].dequantize())
             qkv = ops.rope_qk(qkv, self.rope[0], self.rope[1], H, Hkv, D)
-            c.append(li, qkv[..., H * D:(H + Hkv) * D], qkv[..., (H + Hkv) * D:], list(range(B)), start)
+            c.append(li, qkv[..., H * D:(H + Hkv) * D], qkv[..., (H + Hkv) * D:], rows, start)
             a = ops.flash_attention(qkv, H, Hkv, D, causal=True)
-            o = ops.linear(a, l["o"].dequantize())
+            nxt = self.layers[li + 1]["n1"] if li + 1 < len(self.layers) else None   # the last norm is taken of the last tokens only
+            if few:
+                x2, h = oil_linear_norm(a.view(B * S, -1), l["o"], x.view(B * S, -1), l["n2"], cfg.norm_eps)
+                act = oil_linear_swiglu(h, l["gu"])
+                if nxt is not None:
+                    x2, h = oil_linear_norm(act, l["down"], x2, nxt, cfg.norm_eps)
+                    h = h.view(B, S, -1)
+                else:
+                    x2 = oil_linear(act, l["down"], x2)
+                x = x2.view(B, S, -1)
+                continue
             if self.world > 1:
+                o = ops.linear(a, l["o"].dequantize())
                 dist.all_reduce(o)
-            x = x + o
+                x = x + o
+            else:
+                x = ops.linear(a, l["o"].dequantize(), residual=x, mode="add")
             h = ops.rms_norm(x, l["n2"], cfg.norm_eps)
             act = ops.swiglu(ops.linear(h, l["gu"].dequantize()))
-            d = ops.linear(act, l["down"].dequantize())
             if self.world > 1:
+                d = ops.linear(act, l["down"].dequantize())
                 dist.all_reduce(d)
-            x = x + d
-        c.commit(list(range(B)), [S] * B)
+                x = x + d
+            else:
+                x = ops.linear(act, l["down"].dequantize(), residual=x, mode="add")
+            if nxt is not None:
+                h = ops.rms_norm(x, nxt, cfg.norm_eps)
+        c.commit(rows, [S] * B)
         return self._logits(x[:, -1].contiguous())
 
     def _logits(self, last: torch.Tensor, normed: bool = False) -> torch.Tensor:
@@ -243,18 +266,45 @@ class TPDecoder:
         return lg[:, : self.cfg.vocab_size]
 
     # ------------------------------------------------------------------ one decode step (capturable)
+    def _attend(self, li: int, sums: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
+        """Attention of one new token per sequence: fp32 QKV sums [B, (H + 2 Hkv) D] -> [B, H * D]; appends keys and values."""
+        c, B = self.cache, pos.shape[0]
+        H, Hkv, D = self.H, self.Hkv, self.D
+        lib, st = rt.lib(), rt.stream_ptr()
+        q2 = torch.empty(B, H * D, dtype=torch.bfloat16, device=self.dev)
+        rt.check(lib.inv_decode_qkv_finish(sums.data_ptr(), sums.stride(0), rt.ptr(self.layers[li]["qkv"].bias), self.rope[0].data_ptr(),
+                                           self.rope[1].data_ptr(), pos.data_ptr(), c.page_table.data_ptr(), c.max_pages, B, H, Hkv, D, q2.data_ptr(),
+                                           q2.stride(0), c.k_pool[li].data_ptr(), c.v_pool[li].data_ptr(), rt.ptr(c.k_scale[li]),
+                                           rt.ptr(c.v_scale[li]), int(c.fmt == "oil4"), st), "inv_decode_qkv_finish")
+        a = torch.empty(B, H * D, dtype=torch.bfloat16, device=self.dev)
+        rt.check(lib.inv_paged_decode(q2.data_ptr(), q2.stride(0), c.page_table.data_ptr(), c.max_pages, c.seq_lens.data_ptr(), B, H, Hkv, D,
+                                      c.k_pool[li].data_ptr(), c.v_pool[li].data_ptr(), rt.ptr(c.k_scale[li]), rt.ptr(c.v_scale[li]),
+                                      int(c.fmt == "oil4"), float(D ** -0.5), a.data_ptr(), a.stride(0), self._scratch.data_ptr(),
+                                      self._splits, st), "inv_paged_decode")
+        return a
+
     @torch.no_grad()
     def _decode_step(self, tokens: torch.Tensor) -> torch.Tensor:
         """tokens [B] -> logits [B, vocab]. Uses and advances the device-side sequence lengths."""
         cfg, c = self.cfg, self.cache
         B = tokens.shape[0]
-        H, Hkv, D = self.H, self.Hkv, self.D
         lens = c.seq_lens[:B]
         pos = lens.clone()                      # position of the new token
         lens.add_(1)
         x = self.emb[tokens]
-        scale = D ** -0.5
-        lib, st = rt.lib(), rt.stream_ptr()
+        if self.ctx is None and B <= SKINNY_TOKENS and skinny_smem_fits(B, max(qw.K for l in self.layers for qw in (l["qkv"], l["o"], l["down"]))):
+            # A few tokens: every projection is one launch that takes the norm in front of it and the residual or SwiGLU behind it
+            eps = cfg.norm_eps
+
+            def rows(n, dtype=torch.bfloat16):
+                return torch.empty(B, n, dtype=dtype, device=self.dev)
+
+            for li, l in enumerate(self.layers):
+                sums = _skinny(x, l["qkv"], rows(l["qkv"].N, torch.float32), SKINNY_SUMS, norm=(l["n1"], eps))
+                x = _skinny(self._attend(li, sums, pos), l["o"], rows(cfg.hidden_size), residual=x)
+                act = _skinny(x, l["gu"], rows(l["gu"].N // 2), SKINNY_SWIGLU, norm=(l["n2"], eps))
+                x = _skinny(act, l["down"], rows(cfg.hidden_size), residual=x)
+            return _skinny(x, self.head, rows(self.head.N), norm=(self.norm_w, eps)).float()[:, : cfg.vocab_size]
         h = ops.rms_norm(x, self.layers[0]["n1"], cfg.norm_eps)
         for li, l in enumerate(self.layers):
             # QKV projection: the GEMM leaves fp32 sums, one finish kernel adds the bias, applies RoPE, writes the queries
@@ -262,16 +312,7 @@ class TPDecoder:
             qw = l["qkv"]
             acc = _acc_for(h, qw, B)
             _gemm_into_acc(h.reshape(B, -1), qw, acc)
-            q2 = torch.empty(B, H * D, dtype=torch.bfloat16, device=self.dev)
-            rt.check(lib.inv_decode_qkv_finish(acc.data_ptr(), acc.stride(0), rt.ptr(qw.bias), self.rope[0].data_ptr(), self.rope[1].data_ptr(),
-                                               pos.data_ptr(), c.page_table.data_ptr(), c.max_pages, B, H, Hkv, D, q2.data_ptr(), q2.stride(0),
-                                               c.k_pool[li].data_ptr(), c.v_pool[li].data_ptr(), rt.ptr(c.k_scale[li]), rt.ptr(c.v_scale[li]),
-                                               int(c.fmt == "oil4"), st), "inv_decode_qkv_finish")
-            a = torch.empty(B, H * D, dtype=torch.bfloat16, device=self.dev)
-            rt.check(lib.inv_paged_decode(q2.data_ptr(), q2.stride(0), c.page_table.data_ptr(), c.max_pages, c.seq_lens.data_ptr(), B, H, Hkv, D,
-                                          c.k_pool[li].data_ptr(), c.v_pool[li].data_ptr(), rt.ptr(c.k_scale[li]), rt.ptr(c.v_scale[li]),
-                                          int(c.fmt == "oil4"), float(scale), a.data_ptr(), a.stride(0), self._scratch.data_ptr(),
-                                          self._splits, st), "inv_paged_decode")
+            a = self._attend(li, acc, pos)
             # every projection's finish pass carries what follows it: the residual add and the next RMSNorm, or SwiGLU
             x, h = tp_reduce_linear(a, l["o"], self.ctx, residual=x, norm=(l["n2"], cfg.norm_eps))
             act = oil_linear_swiglu(h, l["gu"])
@@ -283,7 +324,9 @@ class TPDecoder:
     def generate(self, ids: torch.Tensor, max_new_tokens: int, use_graph: bool = True):
         """Greedy generation. Returns (tokens [B, max_new_tokens], prefill seconds, decode seconds), device-timed."""
         B, S = ids.shape
-        self._splits = max(1, min(8, (148 * 2) // max(1, B * self.Hkv)))
+        # one CTA of four warps walks up to 12 pages faster than splits and the launch that folds them; beyond, a page per warp
+        pages = -(-min(S + max_new_tokens, self.max_seq) // PAGE)
+        self._splits = 1 if pages <= 12 else max(1, min(8, (148 * 2) // max(1, B * self.Hkv), pages // 4))
         self._scratch = torch.empty(B * self.H * self._splits * (self.D + 2), dtype=torch.float32, device=self.dev)
         e = [torch.cuda.Event(enable_timing=True) for _ in range(3)]
         e[0].record()
@@ -293,21 +336,31 @@ class TPDecoder:
         out = [tok]
         static_tok = tok.clone()
         if use_graph:
-            # warm up on a side stream (allocations, lazy kernel attributes), restore the state, then capture
+            # The first time, a step runs on a side stream (allocations, lazy kernel attributes) and the state is restored. A capture takes
+            # its buffers, one step's worth, from the pool of the one before it, which is never replayed again (torch.cuda.graph
+            # empties the allocator's cache instead: 10 ms and more of a call in allocations).
             saved = self.cache.seq_lens.clone()
-            s = torch.cuda.Stream()
+            if self._side is None:
+                self._side = torch.cuda.Stream()
+            s = self._side
             s.wait_stream(torch.cuda.current_stream())
             with torch.cuda.stream(s):
-                self._decode_step(static_tok)
+                if self.ctx is not None or (B, self._splits) not in self._warmed:
+                    self._decode_step(static_tok)
+                    self.cache.seq_lens.copy_(saved)
+                    self._warmed.add((B, self._splits))
+                if self.ctx is not None:
+                    self.ctx.turn = 0
+                    self.ctx.xturn = 0
+                graph = torch.cuda.CUDAGraph()
+                graph.capture_begin(pool=None if self._graph is None else self._graph.pool())
+                try:
+                    static_logits = self._decode_step(static_tok)
+                    static_next = static_logits.argmax(-1)
+                finally:
+                    graph.capture_end()
+            self._graph = graph
             torch.cuda.current_stream().wait_stream(s)
-            self.cache.seq_lens.copy_(saved)
-            if self.ctx is not None:
-                self.ctx.turn = 0
-                self.ctx.xturn = 0
-            graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph):
-                static_logits = self._decode_step(static_tok)
-                static_next = static_logits.argmax(-1)
             self.cache.seq_lens.copy_(saved)
             e[1].record()
             for _ in range(max_new_tokens - 1):

@@ -228,3 +228,42 @@ def test_ste_quantizer_static_codebook_and_mixed_blocks():
     assert torch.equal(w.grad, torch.ones_like(w))                                          # identity gradient through every format
     assert STEQuantizer(use_ste=False)(w, "oil4") is w
     STEQuantizer.reset_static_codebooks()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", ["oil4", "oil8", "spark", "oil1"])
+@pytest.mark.parametrize("M,N,K", [(1, 16, 64), (1, 3072, 2048), (3, 1000, 192), (8, 24, 5632), (9, 2048, 1344), (16, 11264, 2048), (7, 4096, 11008),
+                                   (13, 40, 128), (16, 5000, 5056)])
+def test_gpu_few_tokens_one_launch(fmt, M, N, K):
+    """The skinny product against fp64 on the same bf16 operands, in its three forms, with the norm in front and without. Its sums are
+    fp32, so what is left is the rounding of the results (2^-9) and, with the norm, of the normed row (another 2^-9)."""
+    from innova_b200.ops.functional import rms_norm
+    from innova_b200.ops.oil_linear import (SKINNY_SUMS, SKINNY_SWIGLU, _skinny, oil_linear, oil_linear_norm, oil_linear_swiglu, quantize_weight)
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + K)
+    bias = torch.randn(N, device="cuda", generator=g).bfloat16()
+    qw = quantize_weight(torch.randn(N, K, device="cuda", generator=g) * 0.05, fmt, bias=bias)
+    x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    res = torch.randn(M, N, device="cuda", generator=g).bfloat16()
+    nw = torch.randn(K, device="cuda", generator=g).bfloat16()
+    w = qw.dequantize().double()
+
+    def off(y, ref):
+        return float((y.double() - ref).norm() / ref.norm())
+
+    def out(n, dtype=torch.bfloat16):
+        return torch.full((M, n), float("nan"), dtype=dtype, device="cuda")
+
+    prod = x.double() @ w.t()
+    plain = prod + bias.double() + res.double()
+    y = _skinny(x, qw, out(N), residual=res)
+    assert off(y, plain) < 2.0 ** -8 and torch.equal(y, _skinny(x, qw, out(N), residual=res))
+    assert off(_skinny(x, qw, out(N, torch.float32), SKINNY_SUMS), prod) < 1e-5
+    gate, up = (prod + bias.double()).bfloat16().double().chunk(2, -1)
+    glu = torch.nn.functional.silu(gate) * up
+    assert off(_skinny(x, qw, out(N // 2), SKINNY_SWIGLU), glu) < 2.0 ** -7
+    normed = rms_norm(x, nw, 1e-5).double() @ w.t()
+    assert off(_skinny(x, qw, out(N, torch.float32), SKINNY_SUMS, norm=(nw, 1e-5)), normed) < 2.0 ** -8
+    nwo = torch.randn(N, device="cuda", generator=g).bfloat16()
+    assert off(oil_linear(x, qw, residual=res), plain) < 2.0 ** -8 and off(oil_linear_swiglu(x, qw), glu) < 2.0 ** -7
+    y, hn = oil_linear_norm(x, qw, res, nwo, 1e-5)
+    assert off(y, plain) < 2.0 ** -8 and off(hn, rms_norm(y, nwo, 1e-5).double()) < 2.0 ** -8
