@@ -284,6 +284,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 
 static EncodeTiledFn get_encode_fn() {
   static EncodeTiledFn fn = nullptr;
+  bind_context();
   static std::once_flag once;
   std::call_once(once, []() {
     void* f = nullptr;

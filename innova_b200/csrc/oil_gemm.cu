@@ -72,6 +72,7 @@ typedef CUresult (*EncodeTiledFnO)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static EncodeTiledFnO og_encode_fn() {
   static EncodeTiledFnO fn = nullptr;
+  bind_context();
   static std::once_flag once;
   std::call_once(once, []() {
     void* f = nullptr;

@@ -577,22 +577,6 @@ __global__ void attn_combine_kernel(const float* __restrict__ part, __nv_bfloat1
   }
 }
 
-// The kernels of a decode step are a few microseconds each: every one may be launched while the one before it drains, and waits for
-// it (griddepcontrol.wait) before it reads anything.
-template <typename... Params, typename... Args>
-static void launch_early(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
-}
-
 }  // namespace inv
 
 using namespace inv;
@@ -709,7 +693,7 @@ extern "C" int inv_decode_qkv_finish(float* acc, int ld_acc, const void* bias, c
   const int grid = (int)((warps + 7) / 8);
   cudaStream_t st = (cudaStream_t)stream;
 #define INV_DQF(O, DD)                                                                                                                      \
-  launch_early(decode_qkv_finish_kernel<O, DD>, dim3(grid), 256, st, acc, ld_acc, (const __nv_bfloat16*)bias, cos_t, sin_t, pos, page_table, max_pages, B, \
+  launch_early(decode_qkv_finish_kernel<O, DD>, dim3(grid), 256, 0, st, acc, ld_acc, (const __nv_bfloat16*)bias, cos_t, sin_t, pos, page_table, max_pages, B, \
                                                         H, Hkv, (__nv_bfloat16*)q_out, ld_q, (uint8_t*)k_pool, (uint8_t*)v_pool,             \
                                                         (__half*)k_scale, (__half*)v_scale)
   if (oil4) {
@@ -733,14 +717,14 @@ static int paged_decode_impl(const void* q, int ld_q, const int* page_table, int
   cudaStream_t st = (cudaStream_t)stream;
   dim3 grid(splits, Hkv, B);
 #define INV_PD(DD)                                                                                                                         \
-  launch_early(paged_decode_kernel<DD>, grid, 128, st, (const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H, Hkv,                    \
+  launch_early(paged_decode_kernel<DD>, grid, 128, 0, st, (const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H, Hkv,                    \
                                                 (const uint8_t*)k_pool, (const uint8_t*)v_pool, scale, scratch, splits,                    \
                                                 splits == 1 ? (__nv_bfloat16*)out : nullptr, ld_o, tree)
   if (oil4) {
     // four warps per CTA, four CTAs per SM. Eight warps (NW = 8, two CTAs per SM) halve a CTA's serial chain of pages but
     // double the waves of the grid: 35.7 us either way at batch 64, 8 KV heads, 640 tokens of context
 #define INV_PD4(DD, NW)                                                                                                                    \
-  launch_early(paged_decode_oil4_mma_kernel<DD, NW>, grid, NW * 32, st, (const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H, Hkv,      \
+  launch_early(paged_decode_oil4_mma_kernel<DD, NW>, grid, NW * 32, 0, st, (const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H, Hkv,      \
                                                              (const uint8_t*)k_pool, (const uint8_t*)v_pool, (const __half*)k_scale,       \
                                                              (const __half*)v_scale, scale, scratch, splits,                                \
                                                              splits == 1 ? (__nv_bfloat16*)out : nullptr, ld_o, tree)
@@ -757,7 +741,7 @@ static int paged_decode_impl(const void* q, int ld_q, const int* page_table, int
   const long n = (long)B * H * D;
   long g = (n + 255) / 256;
   if (g > 148 * 8) g = 148 * 8;
-  launch_early(attn_combine_kernel, dim3((int)g), 256, st, scratch, (__nv_bfloat16*)out, ld_o, B, H, Hkv, D, splits);
+  launch_early(attn_combine_kernel, dim3((int)g), 256, 0, st, scratch, (__nv_bfloat16*)out, ld_o, B, H, Hkv, D, splits);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }

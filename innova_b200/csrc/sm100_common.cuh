@@ -332,4 +332,33 @@ __device__ __forceinline__ float silu_grad_f(float x) {
   return s * (1.0f + x * (1.0f - s));
 }
 
+// The driver's tensor-map encoder wants the device's context current on the calling thread, which the runtime only binds with a
+// thread's first real call: an autograd thread whose first work is a product has made none.
+static inline void bind_context() {
+  static thread_local bool bound = false;
+  int device = 0;
+  if (!bound && cudaGetDevice(&device) == cudaSuccess) bound = cudaSetDevice(device) == cudaSuccess;
+}
+
+// ---------------------------------------------------------------- programmatic dependent launch
+// Kernels of a decode step take a few microseconds each. One launched by launch_early may start while the kernel before it drains;
+// all of its threads pass wait_previous() before they touch anything an earlier kernel reads or writes (what comes before may only
+// read weights). release_next() lets the next kernel do the same.
+__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... Params, typename... Args>
+static inline void launch_early(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 }  // namespace inv

@@ -369,3 +369,45 @@ def test_gpu_norm_backward_of_wide_rows(T, D, rms, on_residual):
     assert float((params[0].grad.double() - want).norm() / want.norm()) < 2.0 ** -8
     for p, q in zip(params[1:], ref[1:]):
         assert float((p.main_grad.double() - q.grad).norm() / q.grad.norm()) < 1e-4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,pad", [(1, 8, 32, 0), (5, 17, 104, 8), (16, 10000, 2048, 0), (17, 2048, 5632, 0), (33, 4608, 264, 8), (64, 9600, 1040, 0),
+                                       (3, 40, 16, 0), (32, 5000, 200, 0)])
+def test_gpu_decode_projection_over_tiles_and_pieces(M, N, K, pad):
+    """Rows of whole 32-byte pieces and others, more tiles than CTAs, K shorter than the ring; plain and gated, against fp64 on the same
+    bf16 operands (fp32 sums)."""
+    from innova_b200.ops import skinny_gemm
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    x = torch.randn(M, K + pad, device="cuda", generator=g).bfloat16()[:, :K]
+    w = (torch.randn(2 * N, K + pad, device="cuda", generator=g) * K ** -0.5).bfloat16()[:, :K]
+    gate, up = (x.double() @ t.double().t() for t in (w[:N], w[N:]))
+    plain = skinny_gemm(x, w, n=N)
+    assert float((plain.double() - gate).norm() / gate.norm()) < 1e-5
+    want = torch.nn.functional.silu(gate) * up
+    got = skinny_gemm(x, w, n=N, silu_half=N)
+    assert float((got.double() - want).norm() / want.norm()) < 1e-5
+
+
+@pytest.mark.gpu
+def test_gpu_first_call_of_a_thread_may_be_a_product():
+    """A thread whose first CUDA work is a tensor-map product (a backward that starts with a weight gradient) has no context bound yet."""
+    import threading
+    from innova_b200 import ops
+    a, b = (torch.randn(192, 128, device="cuda").bfloat16() for _ in range(2))
+    out, errors = torch.empty(192, 192, dtype=torch.bfloat16, device="cuda"), []
+    torch.cuda.synchronize()
+
+    def work():
+        try:
+            ops.gemm(a, b, out=out)
+        except RuntimeError as e:
+            errors.append(e)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    torch.cuda.synchronize()
+    assert not errors
+    ref = a.double() @ b.double().t()
+    assert float((out.double() - ref).norm() / ref.norm()) < 2.0 ** -8
