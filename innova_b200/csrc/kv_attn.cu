@@ -89,6 +89,8 @@ __global__ void __launch_bounds__(512) qkv_prep_kernel(const QkvPrep p) {
   __shared__ float red[2][16];
   __shared__ __align__(16) float2 turn[KV_MAX_PAIRS];
   const int tid = threadIdx.x, nt = blockDim.x;
+  release_next();
+  wait_previous();
   const size_t t = blockIdx.x;
   const TI* row = static_cast<const TI*>(p.in) + t * p.in_ld;
   const int per = p.Dp / 8, nq = p.H * per, n = (p.H + p.G) * per;
@@ -309,6 +311,8 @@ __global__ void __launch_bounds__(NW * 32) kv_attend_mma_kernel(const KvAttend p
   const cg::cluster_group cluster = cg::this_cluster();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
   const int splits = gridDim.x, split = blockIdx.x;
+  release_next();
+  wait_previous();
   const size_t t = blockIdx.z;
   const int group = p.H / p.G, blocks = (group + 7) / 8, g = blockIdx.y / blocks;
   const int h0 = g * group + (blockIdx.y % blocks) * 8, nh = min(8, (g + 1) * group - h0);
@@ -454,11 +458,11 @@ static int launch_prep(const QkvPrep& p, int T, cudaStream_t st) {
   const int rounds = (n + cap - 1) / cap;
   const int threads = ((n + rounds - 1) / rounds + 31) / 32 * 32;
   switch (rounds) {
-    case 1: qkv_prep_kernel<TI, TC, 1><<<T, threads, 0, st>>>(p); break;
-    case 2: qkv_prep_kernel<TI, TC, 2><<<T, threads, 0, st>>>(p); break;
-    case 3: qkv_prep_kernel<TI, TC, 3><<<T, threads, 0, st>>>(p); break;
-    case 4: qkv_prep_kernel<TI, TC, 4><<<T, threads, 0, st>>>(p); break;
-    default: qkv_prep_kernel<TI, TC, 0><<<T, 512, 0, st>>>(p); break;
+    case 1: launch_early(qkv_prep_kernel<TI, TC, 1>, dim3(T), threads, 0, st, p); break;
+    case 2: launch_early(qkv_prep_kernel<TI, TC, 2>, dim3(T), threads, 0, st, p); break;
+    case 3: launch_early(qkv_prep_kernel<TI, TC, 3>, dim3(T), threads, 0, st, p); break;
+    case 4: launch_early(qkv_prep_kernel<TI, TC, 4>, dim3(T), threads, 0, st, p); break;
+    default: launch_early(qkv_prep_kernel<TI, TC, 0>, dim3(T), 512, 0, st, p); break;
   }
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
@@ -493,12 +497,14 @@ static int launch_mma(const KvAttend& p, int splits, int n_tok, cudaStream_t st)
   cfg.blockDim = dim3(NW * 32);
   cfg.dynamicSmemBytes = bytes;
   cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = splits;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = splits;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kv_attend_mma_kernel<D, NW>, p);
   return e == cudaSuccess ? 0 : -(int)e;
 }

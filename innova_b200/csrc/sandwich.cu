@@ -63,6 +63,13 @@ template <typename YT, typename HT, int NV>
 __global__ void __launch_bounds__(512) sandwich_kernel(const SandwichParams p) {
   __shared__ float red[2][16];
   const int tid = threadIdx.x, nt = blockDim.x, E4 = p.E / 4;
+  release_next();
+  float4 wp, wn;               // one piece per thread: the weights are on their way while the sublayer before finishes
+  if (NV == 1 && tid < E4) {
+    if (p.y && p.post_w) wp = reinterpret_cast<const float4*>(p.post_w)[tid];
+    if (p.norm_w) wn = reinterpret_cast<const float4*>(p.norm_w)[tid];
+  }
+  wait_previous();
   const size_t row = p.rows ? (size_t)p.rows[blockIdx.x] : (size_t)blockIdx.x;
   float* x = p.x + row * (size_t)p.E;
   float4 xr[NV], yr[NV];
@@ -92,7 +99,7 @@ __global__ void __launch_bounds__(512) sandwich_kernel(const SandwichParams p) {
 #pragma unroll
       for (int i = 0; i < NV; ++i)
         if (tid + i * nt < E4) {
-          const float4 w = reinterpret_cast<const float4*>(p.post_w)[tid + i * nt];
+          const float4 w = NV == 1 ? wp : reinterpret_cast<const float4*>(p.post_w)[tid + i * nt];
           yr[i].x *= r * (p.offset + w.x); yr[i].y *= r * (p.offset + w.y); yr[i].z *= r * (p.offset + w.z); yr[i].w *= r * (p.offset + w.w);
         }
     }
@@ -114,7 +121,7 @@ __global__ void __launch_bounds__(512) sandwich_kernel(const SandwichParams p) {
 #pragma unroll
   for (int i = 0; i < NV; ++i)
     if (tid + i * nt < E4) {
-      const float4 w = reinterpret_cast<const float4*>(p.norm_w)[tid + i * nt];
+      const float4 w = NV == 1 ? wn : reinterpret_cast<const float4*>(p.norm_w)[tid + i * nt];
       Four<HT>::st(p.h, (size_t)blockIdx.x * p.h_ld + 4 * (tid + i * nt),
                    make_float4(xr[i].x * r * (p.offset + w.x), xr[i].y * r * (p.offset + w.y), xr[i].z * r * (p.offset + w.z), xr[i].w * r * (p.offset + w.w)));
     }
@@ -125,6 +132,8 @@ template <typename YT, typename HT>
 __global__ void __launch_bounds__(512) sandwich_any_kernel(const SandwichParams p) {
   __shared__ float red[2][16];
   const int tid = threadIdx.x, nt = blockDim.x, E = p.E;
+  release_next();
+  wait_previous();
   const size_t row = p.rows ? (size_t)p.rows[blockIdx.x] : (size_t)blockIdx.x;
   float* x = p.x + row * (size_t)E;
   const size_t tok = p.ids ? (size_t)p.ids[row] * p.table_ld : 0, yo = row * (size_t)p.y_ld;
@@ -161,12 +170,12 @@ static int sandwich_launch(const SandwichParams& p, int n, bool vec, cudaStream_
   const int e4 = p.E / 4, few = (e4 + 511) / 512;
   const int want = n <= 148 || e4 < 256 ? 1 : e4 < 512 ? 2 : 4, rounds = few > want ? few : want;
   const int threads = ((e4 + rounds - 1) / rounds + 31) / 32 * 32;
-  if (!vec || rounds > 12) sandwich_any_kernel<YT, HT><<<n, 256, 0, st>>>(p);
-  else if (rounds <= 1) sandwich_kernel<YT, HT, 1><<<n, threads, 0, st>>>(p);
-  else if (rounds <= 2) sandwich_kernel<YT, HT, 2><<<n, threads, 0, st>>>(p);
-  else if (rounds <= 4) sandwich_kernel<YT, HT, 4><<<n, threads, 0, st>>>(p);
-  else if (rounds <= 8) sandwich_kernel<YT, HT, 8><<<n, threads, 0, st>>>(p);
-  else sandwich_kernel<YT, HT, 12><<<n, threads, 0, st>>>(p);
+  if (!vec || rounds > 12) launch_early(sandwich_any_kernel<YT, HT>, dim3(n), 256, 0, st, p);
+  else if (rounds <= 1) launch_early(sandwich_kernel<YT, HT, 1>, dim3(n), threads, 0, st, p);
+  else if (rounds <= 2) launch_early(sandwich_kernel<YT, HT, 2>, dim3(n), threads, 0, st, p);
+  else if (rounds <= 4) launch_early(sandwich_kernel<YT, HT, 4>, dim3(n), threads, 0, st, p);
+  else if (rounds <= 8) launch_early(sandwich_kernel<YT, HT, 8>, dim3(n), threads, 0, st, p);
+  else launch_early(sandwich_kernel<YT, HT, 12>, dim3(n), threads, 0, st, p);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
