@@ -476,7 +476,8 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
 // out_bf16[m, n] = bf16(acc[m, n] + bias[n] (+ residual[m, n])); clears acc for the next use. Four columns per thread.
 __global__ void oil_gemm_finish_kernel(float* __restrict__ acc, const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ residual,
                                        __nv_bfloat16* __restrict__ out, long M, int N, int ld_acc, int ld_out, int ld_res, int clear, int vec) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the next GEMM may start fetching and expanding its weights
+  release_next();  // the next GEMM may start fetching and expanding its weights
+  wait_previous();
   const long m = blockIdx.y;
   if (vec) {
     for (int n = (blockIdx.x * blockDim.x + threadIdx.x) * 4; n < N; n += gridDim.x * blockDim.x * 4) {
@@ -509,7 +510,8 @@ __global__ void oil_gemm_finish_kernel(float* __restrict__ acc, const __nv_bfloa
 // The gate / up projection's finish and the SwiGLU in one pass. F % 4 == 0.
 __global__ void oil_gemm_finish_swiglu_kernel(float* __restrict__ acc, const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out, int F,
                                               int ld_acc, int ld_out) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  release_next();
+  wait_previous();
   const long m = blockIdx.y;
   for (int f = (blockIdx.x * blockDim.x + threadIdx.x) * 4; f < F; f += gridDim.x * blockDim.x * 4) {
     float4 g = *reinterpret_cast<float4*>(acc + m * ld_acc + f);
@@ -600,7 +602,8 @@ __global__ void __launch_bounds__(256) oil_gemm_finish_norm_kernel(float* __rest
                                                                    int N, int ld_acc, int ld_x, int ld_res, int ld_h, int W, int rank,
                                                                    HeadBarrier hb) {
   constexpr int MAXV = 16;  // float4 groups per thread: 256 * 16 * 4 = 16384 columns
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  release_next();
+  wait_previous();
   const long m = blockIdx.x;
   uint32_t epoch = 1;
   if (hb.state != nullptr) {  // tensor parallel: every rank's GEMM has added its partial sums into this rank's accumulator
@@ -924,7 +927,7 @@ extern "C" int inv_oil_gemm_finish(float* acc, const void* bias, const void* res
   int gx = (N + per_block - 1) / per_block;
   if (gx > 32) gx = 32;
   dim3 grid(gx, (unsigned)M);
-  oil_gemm_finish_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(acc, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual,
+  launch_early(oil_gemm_finish_kernel, grid, 256, 0, (cudaStream_t)stream, acc, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual,
                                                                   (__nv_bfloat16*)out, M, N, ld_acc, ld_out, ld_res, clear, vec ? 1 : 0);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
@@ -937,7 +940,7 @@ extern "C" int inv_oil_gemm_finish_swiglu(float* acc, const void* bias, void* ou
   int gx = (F + 1023) / 1024;
   if (gx > 32) gx = 32;
   dim3 grid(gx, (unsigned)M);
-  oil_gemm_finish_swiglu_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(acc, (const __nv_bfloat16*)bias, (__nv_bfloat16*)out, F, ld_acc, ld_out);
+  launch_early(oil_gemm_finish_swiglu_kernel, grid, 256, 0, (cudaStream_t)stream, acc, (const __nv_bfloat16*)bias, (__nv_bfloat16*)out, F, ld_acc, ld_out);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
@@ -949,7 +952,7 @@ extern "C" int inv_oil_gemm_finish_norm(float* acc, const void* bias, const void
   if ((N % 4) || N > 16384 || (ld_acc % 4) || (ld_x % 4) || (ld_res % 4) || (ld_h % 4) || ((uintptr_t)acc % 16) || ((uintptr_t)x_out % 8) ||
       ((uintptr_t)h_out % 8) || ((uintptr_t)bias % 8) || ((uintptr_t)residual % 8) || ((uintptr_t)norm_w % 8))
     return -ERR_BAD_ARG;
-  oil_gemm_finish_norm_kernel<<<(unsigned)M, 256, 0, (cudaStream_t)stream>>>(acc, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual,
+  launch_early(oil_gemm_finish_norm_kernel, dim3((unsigned)M), 256, 0, (cudaStream_t)stream, acc, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual,
                                                                               (__nv_bfloat16*)x_out, (const __nv_bfloat16*)norm_w, eps,
                                                                               (__nv_bfloat16*)h_out, N, ld_acc, ld_x, ld_res, ld_h, 1, 0,
                                                                               make_head_barrier(nullptr, nullptr, nullptr, 1, nullptr));

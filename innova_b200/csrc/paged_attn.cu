@@ -721,14 +721,19 @@ static int paged_decode_impl(const void* q, int ld_q, const int* page_table, int
                                                 (const uint8_t*)k_pool, (const uint8_t*)v_pool, scale, scratch, splits,                    \
                                                 splits == 1 ? (__nv_bfloat16*)out : nullptr, ld_o, tree)
   if (oil4) {
-    // four warps per CTA, four CTAs per SM. Eight warps (NW = 8, two CTAs per SM) halve a CTA's serial chain of pages but
-    // double the waves of the grid: 35.7 us either way at batch 64, 8 KV heads, 640 tokens of context
+    // Four warps per CTA and four CTAs per SM, or, where all CTAs fit at two per SM, eight warps: half the chain of pages (64
+    // sequences, 4 KV heads, 512 to 576 tokens). At batch 64, 8 KV heads, 640 tokens the two are alike, 35.7 us.
+    const bool few = (long)splits * Hkv * B <= 148 * 2;
 #define INV_PD4(DD, NW)                                                                                                                    \
   launch_early(paged_decode_oil4_mma_kernel<DD, NW>, grid, NW * 32, 0, st, (const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H, Hkv,      \
                                                              (const uint8_t*)k_pool, (const uint8_t*)v_pool, (const __half*)k_scale,       \
                                                              (const __half*)v_scale, scale, scratch, splits,                                \
                                                              splits == 1 ? (__nv_bfloat16*)out : nullptr, ld_o, tree)
-    if (D == 64) INV_PD4(64, 4); else INV_PD4(128, 4);
+    if (few) {
+      if (D == 64) INV_PD4(64, 8); else INV_PD4(128, 8);
+    } else {
+      if (D == 64) INV_PD4(64, 4); else INV_PD4(128, 4);
+    }
 #undef INV_PD4
   } else {
     if (D == 64) INV_PD(64); else INV_PD(128);
