@@ -117,10 +117,17 @@ def skinny_gemm(x, w, n=None, silu_half: int = 0, out_dtype=torch.float32, softc
     return out[:, :n]
 
 
-def _accumulate_wgrad(weight, dy2, x2):
-    """weight.main_grad[N,K] += dy2[T,N]^T @ x2[T,K]; returns a grad tensor only when there is no main_grad."""
+def main_grads(*params):
+    """The ``main_grad`` of each parameter, for a forward pass to keep: a saved tensor that comes back through saved-tensor hooks
+    (gradient checkpointing recomputes it) is another object without the attribute."""
+    return tuple(getattr(p, "main_grad", None) for p in params)
+
+
+def _accumulate_wgrad(weight, dy2, x2, kept=None):
+    """weight.main_grad[N,K] += dy2[T,N]^T @ x2[T,K]; returns a grad tensor only when there is no main_grad (nor ``kept``, the one that
+    the forward pass saw)."""
     N, K = weight.shape
-    mg = getattr(weight, "main_grad", None)
+    mg = getattr(weight, "main_grad", kept)
     if mg is not None:
         gemm(dy2, x2, out=mg.view(N, K), a_mn=True, b_mn=True, epilogue=EPI_ATOMIC)
         return None
@@ -129,9 +136,9 @@ def _accumulate_wgrad(weight, dy2, x2):
     return g.to(weight.dtype)
 
 
-def _accumulate_bgrad(bias, dy2, colsum=None):
+def _accumulate_bgrad(bias, dy2, colsum=None, kept=None):
     """``colsum``: fp32 column sums of ``dy2`` when its producer already computed them (``rt.take_colsum``)."""
-    mg = getattr(bias, "main_grad", None)
+    mg = getattr(bias, "main_grad", kept)
     T, N = dy2.shape
     if colsum is not None:
         if mg is not None:
@@ -171,6 +178,7 @@ class _LinearFn(torch.autograd.Function):
             gemm(x2, weight, out=y2, bias=bias)
         ctx.mode = mode
         ctx.has_bias = bias is not None
+        ctx.main_grads = main_grads(weight, bias)
         ctx.save_for_backward(x2, weight, bias, pre)
         ctx.xshape = shp
         return y
@@ -193,8 +201,8 @@ class _LinearFn(torch.autograd.Function):
         dx = None
         if ctx.needs_input_grad[0]:
             dx = gemm(dy2, weight, b_mn=True).view(ctx.xshape)
-        dw = _accumulate_wgrad(weight, dy2, x2) if ctx.needs_input_grad[1] else None
-        db = _accumulate_bgrad(bias, dy2, cs) if (ctx.has_bias and ctx.needs_input_grad[2]) else None
+        dw = _accumulate_wgrad(weight, dy2, x2, ctx.main_grads[0]) if ctx.needs_input_grad[1] else None
+        db = _accumulate_bgrad(bias, dy2, cs, ctx.main_grads[1]) if (ctx.has_bias and ctx.needs_input_grad[2]) else None
         return dx, dw, db, dres, None
 
 
@@ -249,6 +257,7 @@ class _MlpGeluFn(torch.autograd.Function):
             gemm(act, w2, out=y.view(-1, N), epilogue=EPI_ADD, bias=b2, aux_in=residual.reshape(-1, N))
         else:
             gemm(act, w2, out=y.view(-1, N), bias=b2)
+        ctx.main_grads = main_grads(w1, b1, w2, b2)
         ctx.save_for_backward(x2, pre, act, w1, b1, w2, b2)
         ctx.has_res = residual is not None
         ctx.xshape = shp
@@ -263,11 +272,12 @@ class _MlpGeluFn(torch.autograd.Function):
             dy2 = dy2.contiguous()
         cs = rt.take_colsum(dy2)
         dpre = gemm(dy2, w2, b_mn=True, epilogue=EPI_MUL, aux_in=pre)
-        dw2 = _accumulate_wgrad(w2, dy2, act)
-        db2 = _accumulate_bgrad(b2, dy2, cs) if b2 is not None else None
+        kw1, kb1, kw2, kb2 = ctx.main_grads
+        dw2 = _accumulate_wgrad(w2, dy2, act, kw2)
+        db2 = _accumulate_bgrad(b2, dy2, cs, kb2) if b2 is not None else None
         dx = gemm(dpre, w1, b_mn=True).view(ctx.xshape)
-        dw1 = _accumulate_wgrad(w1, dpre, x2)
-        db1 = _accumulate_bgrad(b1, dpre) if b1 is not None else None
+        dw1 = _accumulate_wgrad(w1, dpre, x2, kw1)
+        db1 = _accumulate_bgrad(b1, dpre, kept=kb1) if b1 is not None else None
         return dx, dw1, db1, dw2, db2, (dy if ctx.has_res else None)
 
 
