@@ -34,6 +34,9 @@ _CUDA_SIGS = {
     "inv_rope": [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp],
     "inv_add": [vp, vp, vp, i64, vp],
     "inv_l2_flush": [vp, i64, vp],
+    "inv_ce_count": [vp, i32, f32, vp, vp],
+    "inv_ce_mean": [vp, i32, vp, vp, vp],
+    "inv_scale_bf16": [vp, vp, vp, i64, vp],
     "inv_cross_entropy": [vp, vp, vp, vp, i32, i32, i32, f32, f32, i32, vp],
     "inv_sumsq": [vp, i64, vp, vp],
     "inv_adamw": [vp, vp, vp, vp, vp, i64, vp, vp, i32, vp],

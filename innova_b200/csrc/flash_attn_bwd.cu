@@ -483,34 +483,40 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   }
 }
 
-// delta[b,h,s] = sum_d O[b,s,h,d] * dO[b,s,h,d]. One warp per 32/(D/8) (token, head) pairs.
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta, int B,
-                                  int S, int H, int D, int ld_o, int ld_do) {
+// delta[b,h,s] = sum_d O[b,s,h,d] * dO[b,s,h,d].
+// Vectors of eight values, D / 8 lanes per (token, head). Index type I: 32 bits wherever the count allows (64-bit divisions by H cost
+// more than the loads); four vectors in flight per thread. 65536 x 12 heads of 64: 54 us (one vector per thread, 64-bit: 65.6).
+template <typename I>
+__global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
+                                                         float* __restrict__ delta, I total, int S, int H, int D, int ld_o, int ld_do) {
+  constexpr int U = 4;
   const int lanes_per = D / 8;  // 8 or 16
-  const long gid = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const long pair = gid / lanes_per;
-  const int v = (int)(gid % lanes_per);
-  const long total = (long)B * S * H;
-  float s = 0.f;
-  if (pair < total) {
-    const int h = (int)(pair % H);
-    const long t = pair / H;
-    uint4 a = *reinterpret_cast<const uint4*>(o + t * ld_o + h * D + v * 8);
-    uint4 g = *reinterpret_cast<const uint4*>(d_o + t * ld_do + h * D + v * 8);
-    const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
-    const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&g);
+  const int v = threadIdx.x % lanes_per;
+  const I first = (I)blockIdx.x * (U * 256 / lanes_per) + threadIdx.x / lanes_per;
+  uint4 a[U], g[U];
+  I t[U];
+  int h[U];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(g2[i]);
-      s += x.x * y.x + x.y * y.y;
-    }
+  for (int u = 0; u < U; ++u) {
+    const I pair = first + (I)(u * (256 / lanes_per));
+    const bool in = pair < total;
+    t[u] = in ? pair / (I)H : 0;
+    h[u] = in ? (int)(pair - t[u] * (I)H) : 0;
+    a[u] = in ? *reinterpret_cast<const uint4*>(o + (size_t)t[u] * ld_o + h[u] * D + v * 8) : make_uint4(0, 0, 0, 0);
+    g[u] = in ? *reinterpret_cast<const uint4*>(d_o + (size_t)t[u] * ld_do + h[u] * D + v * 8) : make_uint4(0, 0, 0, 0);
   }
-  for (int off = lanes_per / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (pair < total && v == 0) {
-    const int h = (int)(pair % H);
-    const long t = pair / H;
-    const long bb = t / S, ss = t % S;
-    delta[(bb * H + h) * S + ss] = s;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const uint32_t x[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, y[4] = {g[u].x, g[u].y, g[u].z, g[u].w};
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      s += __uint_as_float(x[i] << 16) * __uint_as_float(y[i] << 16) + __uint_as_float(x[i] & 0xffff0000u) * __uint_as_float(y[i] & 0xffff0000u);
+    for (int off = lanes_per / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (v == 0 && first + (I)(u * (256 / lanes_per)) < total) {
+      const I bb = t[u] / (I)S;
+      delta[((size_t)bb * H + h[u]) * S + (size_t)(t[u] - bb * (I)S)] = s;
+    }
   }
 }
 
@@ -560,9 +566,14 @@ extern "C" int inv_flash_attn_bwd(const void* q, const void* k, const void* v, c
   cudaError_t e = cudaMemsetAsync(dq_acc, 0, (size_t)T * H * head_dim * 4, st);
   if (e != cudaSuccess) return -(int)e;
   {
-    const long threads = T * H * (head_dim / 8);
-    attn_delta_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, B, S, H,
-                                                                        head_dim, ld_o, ld_do);
+    const long total = T * H, per_cta = 4 * 256 / (head_dim / 8);
+    const unsigned ctas = (unsigned)((total + per_cta - 1) / per_cta);
+    if (total < (1l << 31))
+      attn_delta_kernel<uint32_t><<<ctas, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, (uint32_t)total, S, H, head_dim, ld_o,
+                                                        ld_do);
+    else
+      attn_delta_kernel<uint64_t><<<ctas, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, (uint64_t)total, S, H, head_dim, ld_o,
+                                                        ld_do);
   }
   CUtensorMap tq, tk, tv, tdo, tdq;
   int rc;

@@ -11,7 +11,7 @@ import torch
 import torch.nn.functional as F
 
 from . import runtime as rt
-from .gemm import EPI_ATOMIC, gemm
+from .gemm import EPI_ATOMIC, gemm, main_grads
 
 
 def _acc_grad(param, g32):
@@ -40,6 +40,7 @@ class _NormFn(torch.autograd.Function):
         rstd = torch.empty(T, dtype=torch.float32, device=x.device)
         rt.check(rt.lib().inv_norm_fwd(x2.data_ptr(), 0, gamma.data_ptr(), rt.ptr(beta), y.data_ptr(), 0, mean.data_ptr(),
                                        rstd.data_ptr(), T, D, float(eps), int(rms), rt.stream_ptr()), "inv_norm_fwd")
+        ctx.main_grads = main_grads(gamma, beta)
         ctx.save_for_backward(x2, gamma, beta, mean, rstd)
         ctx.rms = rms
         ctx.xshape = shp
@@ -67,8 +68,8 @@ def _norm_backward(ctx, dy, dres):
     dx = torch.empty_like(x2)
     grid = rt.lib().inv_norm_bwd_grid(T)
     scr = rt.scratch("norm_bwd", grid * 3 * D * 4, x2.device)
-    mg_g = getattr(gamma, "main_grad", None)
-    mg_b = getattr(beta, "main_grad", None) if beta is not None else None
+    mg_g = getattr(gamma, "main_grad", ctx.main_grads[0])
+    mg_b = getattr(beta, "main_grad", ctx.main_grads[1]) if beta is not None else None
     dg = mg_g if mg_g is not None else torch.zeros(D, dtype=torch.float32, device=x2.device)
     db = None
     if beta is not None:
@@ -317,6 +318,15 @@ def cross_entropy(logits, labels, vocab=None, smoothing=0.0):
     return _CrossEntropyFn.apply(logits, labels, vocab, smoothing)
 
 
+def _scaled(x, factor):
+    """bf16(x * factor), the fp32 factor on the device; x [T, D] bf16, dense."""
+    if x.data_ptr() % 16:
+        return (x.float() * factor).to(torch.bfloat16)
+    out = torch.empty_like(x)
+    rt.check(rt.lib().inv_scale_bf16(x.data_ptr(), factor.data_ptr(), out.data_ptr(), x.numel(), rt.stream_ptr()), "inv_scale_bf16")
+    return out
+
+
 class _LMHeadCEFn(torch.autograd.Function):
     """loss = mean CE(x W^T, labels), evaluated in chunks of tokens so that no [T, V] tensor exists.
 
@@ -336,18 +346,21 @@ class _LMHeadCEFn(torch.autograd.Function):
         T = x2.shape[0]
         Vp = weight.shape[0]
         lab = labels.reshape(-1).contiguous()
-        n_valid = (lab >= 0).sum().clamp(min=1).float()
+        counts = torch.empty(2, dtype=torch.float32, device=x.device)    # labels that count, grad_scale over them
+        lib, st = rt.lib(), rt.stream_ptr()
+        as_number = not torch.is_tensor(grad_scale)
+        rt.check(lib.inv_ce_count(lab.data_ptr(), T, float(grad_scale) if as_number else 1.0, counts.data_ptr(), st), "inv_ce_count")
+        inv_n = counts[1] if as_number else (grad_scale.to(x.device) / counts[0]).float()
         loss = torch.empty(T, dtype=torch.float32, device=x.device)
         dx = torch.empty_like(x2)
         mg = getattr(weight, "main_grad", None)
         dw = mg.view(Vp, D) if mg is not None else torch.zeros((Vp, D), dtype=torch.float32, device=x.device)
-        inv_n = (grad_scale / n_valid)
         logits = torch.empty((min(chunk, T), Vp), dtype=torch.bfloat16, device=x.device)
         # The kernel takes gscale as a host float; the valid count lives on the device, so the chunk
         # gradient is produced unscaled (bf16 holds softmax - onehot in [-1, 1] well) and 1/n_valid is
         # folded into the two GEMMs that consume it through a rescaled copy of their other operand.
         # Here: dx is scaled afterwards; dw accumulates alpha-scaled by staging x * inv_n.
-        xs = (x2.float() * inv_n).to(torch.bfloat16)
+        xs = _scaled(x2, inv_n)
         for t0 in range(0, T, chunk):
             t1 = min(T, t0 + chunk)
             n = t1 - t0
@@ -361,13 +374,15 @@ class _LMHeadCEFn(torch.autograd.Function):
         ctx.xshape = x.shape
         ctx.ret_dw = None if mg is not None else dw
         ctx.wdtype = weight.dtype
-        return loss.sum() / n_valid
+        mean = torch.empty((), dtype=torch.float32, device=x.device)
+        rt.check(lib.inv_ce_mean(loss.data_ptr(), T, counts.data_ptr(), mean.data_ptr(), st), "inv_ce_mean")
+        return mean
 
     @staticmethod
     def backward(ctx, dloss):
         dx, inv_n = ctx.saved_tensors
         # dloss equals grad_scale by contract, and inv_n already holds grad_scale / n_valid
-        dxo = (dx * inv_n.to(dx.dtype)).view(ctx.xshape)
+        dxo = _scaled(dx, inv_n).view(ctx.xshape)
         dw = None if ctx.ret_dw is None else ctx.ret_dw.to(ctx.wdtype)
         return dxo, dw, None, None, None, None, None
 

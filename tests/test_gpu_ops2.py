@@ -411,3 +411,70 @@ def test_gpu_first_call_of_a_thread_may_be_a_product():
     assert not errors
     ref = a.double() @ b.double().t()
     assert float((out.double() - ref).norm() / ref.norm()) < 2.0 ** -8
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,V,ld", [(3, 7, 8), (5, 4096, 4096), (40, 50257, 50304), (9, 8195, 8256), (2, 12, 64)])
+@pytest.mark.parametrize("smoothing", [0.0, 0.1])
+def test_gpu_cross_entropy_rows(T, V, ld, smoothing):
+    """Losses and gradients against fp64 over widths that end inside a vector, rows far from zero, -inf columns and ignored labels.
+    Losses are fp32 sums of exponentials (about 2^-22 each); the gradient's exponentials and products are bf16 (four roundings of 2^-9)."""
+    from innova_b200.ops import runtime as rt
+    g = torch.Generator(device="cuda").manual_seed(V)
+    lg = (torch.randn(T, ld, device="cuda", generator=g) * 4).bfloat16()
+    lg[0] -= 200
+    lg[:, V:] = float("inf")
+    if smoothing == 0:
+        lg[1, : min(V, 6)] = float("-inf")
+    labels = torch.randint(0, V, (T,), device="cuda", generator=g)
+    labels[1], labels[-1] = V - 1, -100
+    loss = torch.full((T,), float("nan"), device="cuda")
+    x = lg[:, :V].double().requires_grad_()
+    logp = torch.log_softmax(x, -1)
+    ok = labels >= 0
+    nll = -logp.gather(1, labels.clamp(min=0).view(-1, 1)).view(-1)
+    want = torch.where(ok, (1 - smoothing) * nll - (smoothing * logp.mean(-1) if smoothing else 0), torch.zeros_like(nll))
+    grad = (torch.softmax(x, -1) - (1 - smoothing) * torch.nn.functional.one_hot(labels.clamp(min=0), V) - smoothing / V) * ok.view(-1, 1)
+    out = lg.clone()
+    rt.check(rt.lib().inv_cross_entropy(out.data_ptr(), labels.data_ptr(), loss.data_ptr(), 0, T, V, ld, 1.0, smoothing, 1, rt.stream_ptr()),
+             "inv_cross_entropy")
+    assert float((loss.double() - want).abs().max()) < 1e-4
+    assert not out[:, V:].any()
+    assert float((out[:, :V].double() - grad).norm() / grad.norm()) < 4 * 2.0 ** -9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,D", [(1, 8), (1000, 72), (3, 2051)])
+def test_gpu_head_loss_counts_labels_and_scales(T, D):
+    """The counts, the mean and the scaled copies behind the fused head: against the same in plain PyTorch."""
+    from innova_b200.ops import runtime as rt
+    from innova_b200.ops.functional import _scaled
+    g = torch.Generator(device="cuda").manual_seed(T)
+    labels = torch.randint(-1, 3, (T,), device="cuda", generator=g)
+    loss = torch.rand(T, device="cuda", generator=g)
+    counts, mean = torch.empty(2, device="cuda"), torch.empty((), device="cuda")
+    rt.check(rt.lib().inv_ce_count(labels.data_ptr(), T, 3.0, counts.data_ptr(), rt.stream_ptr()), "inv_ce_count")
+    n = (labels >= 0).sum().clamp(min=1).float()
+    assert torch.equal(counts, torch.stack([n, 3.0 / n]))
+    rt.check(rt.lib().inv_ce_mean(loss.data_ptr(), T, counts.data_ptr(), mean.data_ptr(), rt.stream_ptr()), "inv_ce_mean")
+    assert abs(float(mean) - float(loss.double().sum() / n.double())) <= 1e-6 * float(mean)
+    x = torch.randn(T, D, device="cuda", generator=g).bfloat16()
+    assert torch.equal(_scaled(x, counts[1]), (x.float() * counts[1]).bfloat16())
+
+
+@pytest.mark.gpu
+def test_gpu_checkpointed_layers_accumulate_in_place():
+    """Gradients under gradient checkpointing go to main_grad like those without it, and leave no .grad behind."""
+    from innova_b200.models import DenseModel, gpt2_small, tiny_dense
+    ids = torch.randint(0, 200, (2, 64), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    for make, kw in ((tiny_dense, dict(ste_format="oil8")), (gpt2_small, dict(hidden_size=128, num_heads=2, head_dim=64, ffn_hidden_size=256,
+                                                                              vocab_size=256, max_seq_len=64))):
+        grads = []
+        for ckpt in (False, True):
+            m = DenseModel(make(num_layers=2, gradient_checkpointing=ckpt, **kw), dtype=torch.bfloat16, device=torch.device("cuda"), seed=5).train()
+            for p in m.parameters():
+                p.main_grad = torch.zeros(p.shape, dtype=torch.float32, device="cuda")
+            m(ids, ids).backward()
+            assert all(p.grad is None for p in m.parameters())
+            grads.append(torch.cat([p.main_grad.reshape(-1) for p in m.parameters()]).double())
+        assert float((grads[0] - grads[1]).norm() / grads[0].norm()) < 2.0 ** -8    # fp32 sums in another order, a bf16 rounding apart
