@@ -141,15 +141,14 @@ SKINNY_TOKENS = 16        # up to here one launch without tensor memory, accumul
 SKINNY_PLAIN, SKINNY_SWIGLU, SKINNY_SUMS = 0, 1, 2
 
 
-def skinny_smem_fits(M: int, K: int) -> bool:
-    return (K + 255) // 256 * 128 * (4 * M + 1) <= 180 * 1024
+def skinny_takes(qw: QuantWeight, M: int) -> bool:
+    """Whether ``_skinny`` multiplies M rows with this matrix: few of them, within shared memory, and the codes on whole sectors."""
+    return (1 <= M <= SKINNY_TOKENS and (qw.K + 255) // 256 * 128 * (4 * M + 1) <= 180 * 1024 and qw.idx.data_ptr() % 32 == 0
+            and qw.scales.data_ptr() % 4 == 0)
 
 
 def skinny_fits(x2: torch.Tensor, qw: QuantWeight) -> bool:
-    """Whether ``_skinny`` takes x2 [M, K]: a few tokens whose rows fit shared memory."""
-    M = x2.shape[0]
-    return (1 <= M <= SKINNY_TOKENS and skinny_smem_fits(M, qw.K) and x2.data_ptr() % 16 == 0 and x2.stride(0) % 8 == 0
-            and x2.stride(1) == 1 and qw.idx.data_ptr() % 32 == 0 and qw.scales.data_ptr() % 4 == 0)
+    return skinny_takes(qw, x2.shape[0]) and x2.data_ptr() % 16 == 0 and x2.stride(0) % 8 == 0 and x2.stride(1) == 1
 
 
 def _skinny(x2: torch.Tensor, qw: QuantWeight, out: torch.Tensor, mode: int = SKINNY_PLAIN, residual: Optional[torch.Tensor] = None, norm=None):

@@ -26,8 +26,8 @@ from .. import ops
 from ..inference.kv_cache import PagedKVCache, PAGE
 from ..models.config import TransformerConfig
 from ..ops import runtime as rt
-from ..ops.oil_linear import (SKINNY_SUMS, SKINNY_SWIGLU, SKINNY_TOKENS, QuantWeight, _acc_for, _gemm_into_acc, _skinny, finish_norm, oil_linear,
-                              oil_linear_norm, oil_linear_swiglu, quantize_weight, skinny_smem_fits)
+from ..ops.oil_linear import (SKINNY_SUMS, SKINNY_SWIGLU, QuantWeight, _acc_for, _gemm_into_acc, _skinny, finish_norm, oil_linear,
+                              oil_linear_norm, oil_linear_swiglu, quantize_weight, skinny_takes)
 
 
 class TPContext:
@@ -292,7 +292,9 @@ class TPDecoder:
         pos = lens.clone()                      # position of the new token
         lens.add_(1)
         x = self.emb[tokens]
-        if self.ctx is None and B <= SKINNY_TOKENS and skinny_smem_fits(B, max(qw.K for l in self.layers for qw in (l["qkv"], l["o"], l["down"]))):
+        mats = [self.head] + [l[k] for l in self.layers for k in ("qkv", "o", "gu", "down")]
+        norms = [self.norm_w] + [l[k] for l in self.layers for k in ("n1", "n2")]
+        if self.ctx is None and all(skinny_takes(qw, B) for qw in mats) and all(w.data_ptr() % 16 == 0 for w in norms):
             # A few tokens: every projection is one launch that takes the norm in front of it and the residual or SwiGLU behind it
             eps = cfg.norm_eps
 
