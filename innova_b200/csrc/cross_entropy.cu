@@ -11,6 +11,13 @@
 namespace inv {
 
 constexpr int CE_THREADS = 512;
+constexpr float kL2E = 1.4426950408889634f, CE_LARGE = 1e38f;
+
+// What a sum relative to the maximum m becomes relative to the maximum mn >= m.
+__device__ __forceinline__ float ce_ratio(float m, float mn) {
+  if (fmaxf(fabsf(m), fabsf(mn)) >= CE_LARGE) return exp2f((m - mn) * kL2E);
+  return exp2f(__fmul_rn(m, kL2E) - __fmul_rn(mn, kL2E));
+}
 
 // logits: [T, ld] bf16, columns [V, ld) are padding. labels < 0 are ignored.
 // loss[t] = (1-eps)*nll + eps*(lse - mean(x));  if grad != 0: logits <- dloss/dlogits * gscale.
@@ -23,28 +30,32 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   __nv_bfloat16* x = logits + (size_t)row * ld;
   const long label = labels[row];
   const int nvec = ld / 8, whole = V / 8;  // vectors of eight columns, those without padding
-  const float kL2E = 1.4426950408889634f;
-  // m is the maximum and mc = m * log2(e) as rounded: s sums 2^(x log2(e) - mc), and the logarithm below adds the same mc back
+  // m is the maximum and mc = m * log2(e) as rounded: s sums 2^(x log2(e) - mc), and the logarithm below adds the same mc back.
+  // Above CE_LARGE in size (logits masked with their type's lowest value) the product is no longer finite, and s sums
+  // 2^((x - m) log2(e)) instead.
   float m = -INFINITY, mc = 0.f, s = 0.f, sx = 0.f;
+  bool large = false;
   // A thread's vectors are read two at a time. Maximum on packed pairs, one fused multiply-add, one exponential and one addition per
   // value: 16384 x 50257 in 674 us (a test per column and a sum of the logits nobody asked for: 740 us; the rows of the resident
   // CTAs stay in L2 for the second pass, so 500 us is what the bytes take).
+  auto raise = [&](float to) {
+    s = m == -INFINITY ? 0.f : s * ce_ratio(m, to);
+    m = to;
+    mc = __fmul_rn(to, kL2E);
+    large = fabsf(to) >= CE_LARGE;
+  };
   auto add = [&](const uint4& v) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(w);
     const __nv_bfloat162 h2 = __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3]));
     const float lm = fmaxf(__low2float(h2), __high2float(h2));
-    if (lm > m) {
-      const float c = __fmul_rn(lm, kL2E);
-      s = m == -INFINITY ? 0.f : s * exp2f(mc - c);
-      m = lm;
-      mc = c;
-    }
+    if (lm > m) raise(lm);
     float t = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float lo = __uint_as_float(w[j] << 16), hi = __uint_as_float(w[j] & 0xffff0000u);
-      t += exp2f(fmaf(lo, kL2E, -mc)) + exp2f(fmaf(hi, kL2E, -mc));
+      if (large) t += exp2f((lo - m) * kL2E) + exp2f((hi - m) * kL2E);
+      else t += exp2f(fmaf(lo, kL2E, -mc)) + exp2f(fmaf(hi, kL2E, -mc));
       if (smoothing != 0.f) sx += lo + hi;
     }
     s += t;
@@ -58,13 +69,8 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   if (i < whole) add(*reinterpret_cast<const uint4*>(x + i * 8));
   if (threadIdx.x < V - whole * 8) {  // the columns before the padding, one per thread
     const float f = __bfloat162float(x[whole * 8 + threadIdx.x]);
-    if (f > m) {
-      const float c = __fmul_rn(f, kL2E);
-      s = m == -INFINITY ? 0.f : s * exp2f(mc - c);
-      m = f;
-      mc = c;
-    }
-    s += exp2f(fmaf(f, kL2E, -mc));
+    if (f > m) raise(f);
+    s += exp2f(large ? (f - m) * kL2E : fmaf(f, kL2E, -mc));
     if (smoothing != 0.f) sx += f;
   }
   // warp then block reduction of (m, s) pairs
@@ -74,7 +80,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
     float s2 = __shfl_xor_sync(0xffffffffu, s, o);
     sx += __shfl_xor_sync(0xffffffffu, sx, o);
     float mn = fmaxf(m, m2);
-    s = (m == -INFINITY ? 0.f : s * exp2f(__fmul_rn(m, kL2E) - __fmul_rn(mn, kL2E))) + (m2 == -INFINITY ? 0.f : s2 * exp2f(__fmul_rn(m2, kL2E) - __fmul_rn(mn, kL2E)));
+    s = (m == -INFINITY ? 0.f : s * ce_ratio(m, mn)) + (m2 == -INFINITY ? 0.f : s2 * ce_ratio(m2, mn));
     m = mn;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -94,7 +100,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
       float s2 = __shfl_xor_sync(0xffffffffu, s, o);
       sx += __shfl_xor_sync(0xffffffffu, sx, o);
       float mn = fmaxf(m, m2);
-      s = (m == -INFINITY ? 0.f : s * exp2f(__fmul_rn(m, kL2E) - __fmul_rn(mn, kL2E))) + (m2 == -INFINITY ? 0.f : s2 * exp2f(__fmul_rn(m2, kL2E) - __fmul_rn(mn, kL2E)));
+      s = (m == -INFINITY ? 0.f : s * ce_ratio(m, mn)) + (m2 == -INFINITY ? 0.f : s2 * ce_ratio(m2, mn));
       m = mn;
     }
     if (lane == 0) {
@@ -108,7 +114,8 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   s = bc[1];
   sx = bc[2];
   mc = __fmul_rn(m, kL2E);
-  const float lse = (mc + __log2f(s)) * 0.6931471805599453f;
+  large = fabsf(m) >= CE_LARGE;
+  const float lse = large ? m + __logf(s) : (mc + __log2f(s)) * 0.6931471805599453f;
   const bool valid = label >= 0 && label < V;
   if (threadIdx.x == 0) {
     float l = 0.f;
@@ -151,7 +158,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   if (valid) {
     __syncthreads();
     if (threadIdx.x == 0) {
-      const float pl = exp2f(fmaf(xl, kL2E, -mc)) / s;
+      const float pl = exp2f(large ? (xl - m) * kL2E : fmaf(xl, kL2E, -mc)) / s;
       x[label] = __float2bfloat16((pl - smoothing / V - (1.f - smoothing)) * g);
     }
   }

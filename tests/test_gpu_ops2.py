@@ -444,6 +444,31 @@ def test_gpu_cross_entropy_rows(T, V, ld, smoothing):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("V,first", [(4099, 4096), (4096, 2048), (50257, 50000), (9, 8), (5, 4)])
+def test_gpu_cross_entropy_of_logits_masked_with_the_lowest_value(V, first):
+    """Columns at the type's lowest value count as masked, wherever a thread meets them (the product with log2(e) is not finite). The
+    bounds are those of the test above."""
+    from innova_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(V)
+    lg = torch.zeros(3, (V + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)
+    low = torch.finfo(torch.bfloat16).min
+    lg[:, :V] = torch.randn(3, V, device="cuda", generator=g) * 4
+    lg[0, :first] = low
+    lg[1, :V][torch.rand(V, device="cuda", generator=g) < 0.9] = low
+    lg[2, :V] = low
+    lg[:, V - 1] = 1.5
+    labels = torch.full((3,), V - 1, device="cuda")
+    ref = lg[:, :V].double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(ref, labels)
+    want.backward()
+    x = lg.clone().requires_grad_()
+    loss = ops.cross_entropy(x, labels, vocab=V)
+    loss.backward()
+    assert abs(float(loss.detach()) - float(want.detach())) < 1e-4
+    assert float((x.grad[:, :V].double() - ref.grad).norm()) <= 4 * 2.0 ** -9 * float(ref.grad.norm()) + 2.0 ** -20
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("T,D", [(1, 8), (1000, 72), (3, 2051)])
 def test_gpu_head_loss_counts_labels_and_scales(T, D):
     """The counts, the mean and the scaled copies behind the fused head: against the same in plain PyTorch."""
