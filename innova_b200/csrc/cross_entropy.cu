@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   __nv_bfloat16* x = logits + (size_t)row * ld;
   const long label = labels[row];
   const int nvec = ld / 8, whole = V / 8;  // vectors of eight columns, those without padding
-  // m is the maximum and mc = m * log2(e) as rounded: s sums 2^(x log2(e) - mc), and the logarithm below adds the same mc back.
+  // m is the maximum and mc = m * log2(e) as rounded: s sums 2^(x log2(e) - mc), and the logarithm below counts with the same mc.
   // Above CE_LARGE in size (logits masked with their type's lowest value) the product is no longer finite, and s sums
   // 2^((x - m) log2(e)) instead.
   float m = -INFINITY, mc = 0.f, s = 0.f, sx = 0.f;
@@ -115,7 +115,8 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   sx = bc[2];
   mc = __fmul_rn(m, kL2E);
   large = fabsf(m) >= CE_LARGE;
-  const float lse = large ? m + __logf(s) : (mc + __log2f(s)) * 0.6931471805599453f;
+  // the bracket gives back what the rounding of mc took, so that m is rounded once, in the last addition
+  const float lse = m + 0.6931471805599453f * (large ? __log2f(s) : __log2f(s) + fmaf(-m, kL2E, mc));
   const bool valid = label >= 0 && label < V;
   if (threadIdx.x == 0) {
     float l = 0.f;

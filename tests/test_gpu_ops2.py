@@ -469,6 +469,24 @@ def test_gpu_cross_entropy_of_logits_masked_with_the_lowest_value(V, first):
 
 
 @pytest.mark.gpu
+def test_gpu_cross_entropy_rounds_the_log_sum_once():
+    """Rows whose maximum stands alone and far from zero: what is lost is the rounding of the result (2^-24 of it) and the logarithm and
+    exponential of numbers near 1 (2^-21 in all)."""
+    from innova_b200.ops import runtime as rt
+    T, V = 512, 64
+    g = torch.Generator(device="cuda").manual_seed(4)
+    top = ((torch.rand(T, device="cuda", generator=g) - 0.5) * 8000).bfloat16()
+    lg = (top.float().view(T, 1) - 200).bfloat16().repeat(1, V)
+    lg[torch.arange(T), torch.randint(0, V, (T,), device="cuda", generator=g)] = top
+    want = torch.logsumexp(lg.double(), -1)
+    loss, lse = (torch.empty(T, device="cuda") for _ in range(2))
+    labels = torch.zeros(T, dtype=torch.int64, device="cuda")
+    rt.check(rt.lib().inv_cross_entropy(lg.data_ptr(), labels.data_ptr(), loss.data_ptr(), lse.data_ptr(), T, V, V, 1.0, 0.0, 0, rt.stream_ptr()),
+             "inv_cross_entropy")
+    assert bool(((lse.double() - want).abs() <= 2.0 ** -24 * want.abs() + 2.0 ** -21).all())
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("T,D", [(1, 8), (1000, 72), (3, 2051)])
 def test_gpu_head_loss_counts_labels_and_scales(T, D):
     """The counts, the mean and the scaled copies behind the fused head: against the same in plain PyTorch."""
