@@ -192,7 +192,7 @@ def main():
 
         def base():
             i[0] += 1
-            y = oil_linear(act, qws[i[0] % 8]).float()
+            y = oil_linear(act, qws[i[0] % 8], resident=True).float()
             dist.all_reduce(y)
             return (y + res.float()).bfloat16()
 

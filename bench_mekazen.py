@@ -117,7 +117,7 @@ def kernel_section(size="2k"):
     # residual step (two norms and the residual) and, as the like kernel, the RMS norm of the dense decoder
     for T in (8192, 64):
         x, y, w = rand(T, E), rand(T, E).to(bf if T > 64 else torch.float32), rand(E)
-        report("sandwich_step", f"T{T} E{E}", cold(lambda: sandwich_step(x, bf, 1e-5, 1.0, y=y, post_w=w, norm_w=w)), T * E * (8 + y.element_size() + 2) / 1e9)
+        report("sandwich_step", f"T{T} E{E}", cold(lambda: sandwich_step(x, bf, 1e-5, 1.0, y=y, post_w=w, norm_w=w, resident=True)), T * E * (8 + y.element_size() + 2) / 1e9)
         xb, wb = x.to(bf), w.to(bf)
         report("rms_norm", f"T{T} E{E}", cold(lambda: ops.rms_norm(xb, wb, 1e-5)), T * E * 4 / 1e9, like="sandwich_step")
     # norm, rotation and append; like kernels: rotation in place, append to the dense decoder's cache
@@ -161,9 +161,9 @@ def kernel_section(size="2k"):
             report("paged_decode", f"B{B} H{H} G{G} D{D} keys {n}", cold(lambda: kv.decode_attention(0, q, H, 0.09)), gb, fl, like="kv_attend")
         wl, xl = rand(4096, E).to(bf), rand(B, E).to(bf)
         if B <= 32:
-            report("skinny_gemm", f"M{B} N4096 K{E}", cold(lambda: ops.skinny_gemm(xl, wl)), wl.numel() * 2 / 1e9)
+            report("skinny_gemm", f"M{B} N4096 K{E}", cold(lambda: ops.skinny_gemm(xl, wl, resident=True)), wl.numel() * 2 / 1e9)
             wh = rand(V, E).to(bf)
-            report("skinny_gemm softcap", f"M{B} N{V} K{E}", cold(lambda: ops.skinny_gemm(xl, wh, softcap=30.0)), (wh.numel() * 2 + B * V * 4) / 1e9)
+            report("skinny_gemm softcap", f"M{B} N{V} K{E}", cold(lambda: ops.skinny_gemm(xl, wh, softcap=30.0, resident=True)), (wh.numel() * 2 + B * V * 4) / 1e9)
         report("gemm", f"M{B} N4096 K{E}", cold(lambda: ops.gemm(xl, wl)), wl.numel() * 2 / 1e9, like="skinny_gemm")
     # attention, prompts
     for B, S in ((1, 4096), (4, 2048)):

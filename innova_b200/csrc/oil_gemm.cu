@@ -247,8 +247,8 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
         if (++si == IDX_STAGES) { si = 0; ph ^= 1; }
       }
     } else if (lane == 1) {
-      // Programmatic dependent launch: this grid may start while the kernel that produces the activations is still
-      // running. Everything that touches only the (static) weights runs ahead: index tiles are fetched and expanded
+      // Launched early, this grid may start while the kernel that produces the activations is still running.
+      // Everything that touches only the (then resident) weights runs ahead: index tiles are fetched and expanded
       // into tensor memory; the activation loads, and with them the MMAs and the epilogue, wait here for the
       // previous grid to complete.
       asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -679,7 +679,7 @@ static HeadBarrier make_head_barrier(const uint64_t* peer_flags, void* local_fla
 
 
 static int oil_gemm_launch(const void* x, int ldx, const void* idx, const void* scales, const float* codebook, int bits, float* acc, int ldo,
-                           int M, int N, int K, int* status, cudaStream_t st, int multimem, const uint64_t* peers = nullptr, int n_peers = 0,
+                           int M, int N, int K, int* status, cudaStream_t st, bool early, int multimem, const uint64_t* peers = nullptr, int n_peers = 0,
                            size_t peer_off = 0, int owner_cols = 0) {
   using namespace og;
   static int num_sms = 0;
@@ -744,7 +744,7 @@ static int oil_gemm_launch(const void* x, int ldx, const void* idx, const void* 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;
   cudaError_t e;
   if (bits == 2) e = cudaLaunchKernelEx(&cfg, oil_gemm_kernel<2>, ti, tx, p);
   else if (bits == 4) e = cudaLaunchKernelEx(&cfg, oil_gemm_kernel<4>, ti, tx, p);
@@ -752,15 +752,16 @@ static int oil_gemm_launch(const void* x, int ldx, const void* idx, const void* 
   return e == cudaSuccess ? 0 : -(int)e;
 }
 
-// acc (fp32 [M, ldo]) must be zero on entry or hold a partial sum to add to. M <= 256, K % 64 == 0.
+// acc (fp32 [M, ldo]) must be zero on entry or hold a partial sum to add to. M <= 256, K % 64 == 0. early: the weights are resident
+// (launch_step), here and below.
 extern "C" int inv_oil_gemm(const void* x, int ldx, const void* idx, const void* scales, const float* codebook, int bits, float* acc, int ldo,
-                            int M, int N, int K, int split_k, int* status, void* stream, int multimem) {
+                            int M, int N, int K, int split_k, int* status, void* stream, int multimem, int early) {
   (void)split_k;  // the split is stream-K: equal (tile, batch) ranges per CTA
   if ((bits != 2 && bits != 4 && bits != 8) || M < 1 || M > 256 || (K % 64) || (ldx % 8) || N < 1) return -ERR_BAD_ARG;
   for (int m0 = 0; m0 < M; m0 += og::MAXM) {
     const int m = M - m0 < og::MAXM ? M - m0 : og::MAXM;
     const int rc = oil_gemm_launch((const __nv_bfloat16*)x + (size_t)m0 * ldx, ldx, idx, scales, codebook, bits, acc + (size_t)m0 * ldo, ldo, m, N, K,
-                                   status, (cudaStream_t)stream, multimem);
+                                   status, (cudaStream_t)stream, early != 0, multimem);
     if (rc) return rc;
   }
   return 0;
@@ -769,12 +770,12 @@ extern "C" int inv_oil_gemm(const void* x, int ldx, const void* idx, const void*
 // The same GEMM with the partial sums added into n_peers buffers (each rank's copy of a replicated accumulator, given
 // as addresses that already include the column offset): one launch, the weights are read once.
 extern "C" int inv_oil_gemm_peers(const void* x, int ldx, const void* idx, const void* scales, const float* codebook, int bits,
-                                  const uint64_t* peers, int n_peers, int ldo, int M, int N, int K, int* status, void* stream) {
+                                  const uint64_t* peers, int n_peers, int ldo, int M, int N, int K, int* status, int early, void* stream) {
   if ((bits != 2 && bits != 4 && bits != 8) || M < 1 || M > 256 || (K % 64) || (ldx % 8) || N < 1 || n_peers < 1 || n_peers > 8) return -ERR_BAD_ARG;
   for (int m0 = 0; m0 < M; m0 += og::MAXM) {
     const int m = M - m0 < og::MAXM ? M - m0 : og::MAXM;
     const int rc = oil_gemm_launch((const __nv_bfloat16*)x + (size_t)m0 * ldx, ldx, idx, scales, codebook, bits,
-                                   reinterpret_cast<float*>(peers[0]) + (size_t)m0 * ldo, ldo, m, N, K, status, (cudaStream_t)stream, 2, peers, n_peers,
+                                   reinterpret_cast<float*>(peers[0]) + (size_t)m0 * ldo, ldo, m, N, K, status, (cudaStream_t)stream, early != 0, 2, peers, n_peers,
                                    (size_t)m0 * ldo);
     if (rc) return rc;
   }
@@ -785,14 +786,14 @@ extern "C" int inv_oil_gemm_peers(const void* x, int ldx, const void* idx, const
 // entry); column n of every rank's partial product is added into peers[n / owner_cols] only. After a barrier rank r holds
 // the complete sums of columns [r * owner_cols, (r + 1) * owner_cols).
 extern "C" int inv_oil_gemm_rs(const void* x, int ldx, const void* idx, const void* scales, const float* codebook, int bits,
-                               const uint64_t* peers, int W, int owner_cols, int ldo, int M, int N, int K, int* status, void* stream) {
+                               const uint64_t* peers, int W, int owner_cols, int ldo, int M, int N, int K, int* status, int early, void* stream) {
   if ((bits != 2 && bits != 4 && bits != 8) || M < 1 || M > 256 || (K % 64) || (ldx % 8) || N < 1 || W < 1 || W > 8 || owner_cols < 4 ||
       (owner_cols % 4) || owner_cols * W < N)
     return -ERR_BAD_ARG;
   for (int m0 = 0; m0 < M; m0 += og::MAXM) {
     const int m = M - m0 < og::MAXM ? M - m0 : og::MAXM;
     const int rc = oil_gemm_launch((const __nv_bfloat16*)x + (size_t)m0 * ldx, ldx, idx, scales, codebook, bits,
-                                   reinterpret_cast<float*>(peers[0]) + (size_t)m0 * ldo, ldo, m, N, K, status, (cudaStream_t)stream, 3, peers, W,
+                                   reinterpret_cast<float*>(peers[0]) + (size_t)m0 * ldo, ldo, m, N, K, status, (cudaStream_t)stream, early != 0, 3, peers, W,
                                    (size_t)m0 * ldo, owner_cols);
     if (rc) return rc;
   }

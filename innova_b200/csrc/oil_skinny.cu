@@ -7,9 +7,9 @@
 // form) and its eight warps take every eighth 256-wide slice of K straight from memory into registers: a lane loads two blocks of 32
 // codes of a row (one whole 32-byte sector of the 4-bit format) with their scales, expands them through the lookup table and feeds
 // warp-level MMA fragments (weights are the 16-row side, tokens the 8-column side; both read k in the same permuted order, which a
-// dot product does not notice). Sums meet in shared memory, in one fixed order. The weights, which no earlier kernel of a step
-// writes, are requested before the kernel waits for the previous grid. The rows of x stay in shared memory in fragment order; the
-// host entry states the limits.
+// dot product does not notice). Sums meet in shared memory, in one fixed order. Resident weights are requested before the
+// kernel waits for the previous grid; others are multiplied by a plainly launched kernel. The rows of x stay in shared memory in
+// fragment order; the host entry states the limits.
 #include "oil_expand.cuh"
 #include "inv_api.h"
 
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(os::THREADS, 2) oil_skinny_kernel(const OilSki
 }
 
 template <int BITS, int MT>
-static int launch_oil_skinny(const OilSkinnyParams& p, cudaStream_t st) {
+static int launch_oil_skinny(const OilSkinnyParams& p, bool early, cudaStream_t st) {
   using namespace os;
   const int slices = (p.K + SLICE - 1) / SLICE;
   const int smem = slices * 128 * (4 * p.M + 1) + WARPS * ROWS * (MT * 8 + 1) * 4;
@@ -246,17 +246,8 @@ static int launch_oil_skinny(const OilSkinnyParams& p, cudaStream_t st) {
   }
   if (smem > limit) return -ERR_BAD_ARG;
   const int per_sm = 2 * (smem + (BITS == 2 ? 3 : 35) * 1024) <= 226 * 1024 ? 2 : 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.n_tiles < 148 * per_sm ? p.n_tiles : 148 * per_sm);
-  cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, oil_skinny_kernel<BITS, MT>, p);
+  launch_step(early, oil_skinny_kernel<BITS, MT>, dim3(p.n_tiles < 148 * per_sm ? p.n_tiles : 148 * per_sm), THREADS, smem, st, p);
+  const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
 
@@ -267,10 +258,11 @@ using namespace inv;
 // M <= 32 tokens, K % 64 == 0, and x (M * K rounded up to 256, 2 bytes each, and a little) within 180 KB of shared memory. x and norm_w on 16
 // bytes, the codes on 32, the scales on 4, ldx % 8 == 0. mode 0: out bf16 [M, N] = product + bias + residual. mode 1: out bf16
 // [M, N / 2] = silu(gate + bias) * (up + bias), gate rows [0, N / 2), up rows behind them. mode 2: out fp32 [M, N] = product. norm_w
-// (optional): x is rms_norm(x) * norm_w, as its own kernel would round it.
+// (optional): x is rms_norm(x) * norm_w, as its own kernel would round it. early: codes, scales and codebook are
+// resident (launch_step).
 extern "C" int inv_oil_skinny(const void* x, int ldx, const void* idx, const void* scales, const float* codebook, int bits, const void* norm_w,
                               float eps, const void* bias, const void* residual, int ld_res, void* out, int ldo, int M, int N, int K, int mode,
-                              void* stream) {
+                              int early, void* stream) {
   if ((bits != 2 && bits != 4 && bits != 8) || M < 1 || M > 32 || (K % 64) || K < 64 || (ldx % 8) || N < 1 || mode < 0 || mode > 2 ||
       (mode == 1 && (N % 2)) || ((uintptr_t)x | (uintptr_t)norm_w) % 16 || (uintptr_t)idx % 32 || (uintptr_t)scales % 4 ||
       (long)((K + 255) / 256) * 128 * (4 * M + 1) > 180 * 1024)
@@ -279,7 +271,8 @@ extern "C" int inv_oil_skinny(const void* x, int ldx, const void* idx, const voi
                     (const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual, ld_res, out, ldo, M, N, K, mode,
                     mode == 1 ? (N / 2 + 7) / 8 : (N + 15) / 16};
   cudaStream_t st = (cudaStream_t)stream;
-#define INV_OS(B) (M <= 8 ? launch_oil_skinny<B, 1>(p, st) : M <= 16 ? launch_oil_skinny<B, 2>(p, st) : launch_oil_skinny<B, 4>(p, st))
+  const bool pdl = early != 0;
+#define INV_OS(B) (M <= 8 ? launch_oil_skinny<B, 1>(p, pdl, st) : M <= 16 ? launch_oil_skinny<B, 2>(p, pdl, st) : launch_oil_skinny<B, 4>(p, pdl, st))
   return bits == 2 ? INV_OS(2) : bits == 4 ? INV_OS(4) : INV_OS(8);
 #undef INV_OS
 }

@@ -165,17 +165,17 @@ __global__ void __launch_bounds__(512) sandwich_any_kernel(const SandwichParams 
 }
 
 template <typename YT, typename HT>
-static int sandwich_launch(const SandwichParams& p, int n, bool vec, cudaStream_t st) {
+static int sandwich_launch(const SandwichParams& p, int n, bool vec, bool early, cudaStream_t st) {
   // few rows: one short pass over a row, its latency is all there is; many: enough values per thread to pay for the two block sums
   const int e4 = p.E / 4, few = (e4 + 511) / 512;
   const int want = n <= 148 || e4 < 256 ? 1 : e4 < 512 ? 2 : 4, rounds = few > want ? few : want;
   const int threads = ((e4 + rounds - 1) / rounds + 31) / 32 * 32;
-  if (!vec || rounds > 12) launch_early(sandwich_any_kernel<YT, HT>, dim3(n), 256, 0, st, p);
-  else if (rounds <= 1) launch_early(sandwich_kernel<YT, HT, 1>, dim3(n), threads, 0, st, p);
-  else if (rounds <= 2) launch_early(sandwich_kernel<YT, HT, 2>, dim3(n), threads, 0, st, p);
-  else if (rounds <= 4) launch_early(sandwich_kernel<YT, HT, 4>, dim3(n), threads, 0, st, p);
-  else if (rounds <= 8) launch_early(sandwich_kernel<YT, HT, 8>, dim3(n), threads, 0, st, p);
-  else launch_early(sandwich_kernel<YT, HT, 12>, dim3(n), threads, 0, st, p);
+  if (!vec || rounds > 12) launch_step(early, sandwich_any_kernel<YT, HT>, dim3(n), 256, 0, st, p);
+  else if (rounds <= 1) launch_step(early, sandwich_kernel<YT, HT, 1>, dim3(n), threads, 0, st, p);
+  else if (rounds <= 2) launch_step(early, sandwich_kernel<YT, HT, 2>, dim3(n), threads, 0, st, p);
+  else if (rounds <= 4) launch_step(early, sandwich_kernel<YT, HT, 4>, dim3(n), threads, 0, st, p);
+  else if (rounds <= 8) launch_step(early, sandwich_kernel<YT, HT, 8>, dim3(n), threads, 0, st, p);
+  else launch_step(early, sandwich_kernel<YT, HT, 12>, dim3(n), threads, 0, st, p);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
@@ -199,18 +199,18 @@ __global__ void __launch_bounds__(256) softcap_kernel(float* x, int ld, int cols
 
 using namespace inv;
 
-// Types: y_f32 / h_f32 say whether y and h (and the embedding table) are fp32, otherwise bf16 (h fp32 needs y fp32).
+// early: post_w and norm_w are resident (launch_step). Types: y_f32 / h_f32 say whether y and h (and the embedding table) are fp32, otherwise bf16 (h fp32 needs y fp32).
 extern "C" int inv_sandwich_step(float* x, const int* ids, const void* table, int table_ld, float scale, const void* y, int y_ld, int y_f32,
                                  const float* post_w, const float* norm_w, float offset, float eps, void* h, int h_ld, int h_f32, const int* rows, int n,
-                                 int write_x, int E, void* stream) {
+                                 int write_x, int E, int early, void* stream) {
   if (E < 1 || (h_f32 && !y_f32)) return -ERR_BAD_ARG;
   if (n <= 0) return 0;
   const SandwichParams p{x, ids, table, table_ld, scale, y, y_ld, post_w, norm_w, offset, eps, h, h_ld, rows, write_x, E};
   cudaStream_t st = (cudaStream_t)stream;
   const bool vec = E % 4 == 0 && (!y || y_ld % 4 == 0) && (!norm_w || h_ld % 4 == 0) && (!ids || table_ld % 4 == 0);
-  if (h_f32) return sandwich_launch<float, float>(p, n, vec, st);
-  if (y_f32) return sandwich_launch<float, __nv_bfloat16>(p, n, vec, st);
-  return sandwich_launch<__nv_bfloat16, __nv_bfloat16>(p, n, vec, st);
+  if (h_f32) return sandwich_launch<float, float>(p, n, vec, early != 0, st);
+  if (y_f32) return sandwich_launch<float, __nv_bfloat16>(p, n, vec, early != 0, st);
+  return sandwich_launch<__nv_bfloat16, __nv_bfloat16>(p, n, vec, early != 0, st);
 }
 
 extern "C" int inv_softcap(float* x, int ld, int rows, int cols, float cap, void* stream) {

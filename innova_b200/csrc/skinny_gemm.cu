@@ -6,7 +6,8 @@
 // warp-level MMA fragments: a lane loads eight or sixteen consecutive k of a row and both operands read them in the same permuted
 // order, which a dot product does not notice. (A 128-row tcgen05 tile would be mostly padding here, and its tensor-memory set-up
 // and drain cost more than the whole product.) A warp keeps a ring of slices in registers, 64 KB per CTA and two CTAs per SM; the
-// ring is filled before the kernel waits for the previous one and refilled across tiles, so that the weights never stop flowing.
+// ring is filled before the kernel waits for the previous one (resident weights; others are multiplied by a plainly launched kernel) and
+// refilled across tiles, so that the weights never stop flowing.
 //
 // SILU: W holds gate rows [0, N) and up rows [half, half + N); the output is silu(gate) * up.
 // cap > 0 (plain form): the output is cap * tanh(out / cap), the soft limit of logits.
@@ -144,10 +145,10 @@ __global__ void __launch_bounds__(SG_THREADS, 2) skinny_gemm_kernel(const __nv_b
 
 template <int MT, int P, bool SILU>
 static int launch_skinny(const void* x, int ldx, const void* W, int ldw, int M, int N, int K, int half, void* out, int ldo, int out_f32, float cap,
-                         cudaStream_t st) {
+                         bool early, cudaStream_t st) {
   constexpr int bytes = SG_WARPS * MT * 16 * (2 * 8 + 4) * 4;
   const int tiles = SILU ? (N + 7) / 8 : (N + 15) / 16;
-  launch_early(skinny_gemm_kernel<MT, P, SILU>, dim3(tiles < 148 * 2 ? tiles : 148 * 2), SG_THREADS, bytes, st, (const __nv_bfloat16*)x, ldx,
+  launch_step(early, skinny_gemm_kernel<MT, P, SILU>, dim3(tiles < 148 * 2 ? tiles : 148 * 2), SG_THREADS, bytes, st, (const __nv_bfloat16*)x, ldx,
                (const __nv_bfloat16*)W, ldw, M, N, K, half, out, ldo, out_f32, cap, tiles);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
@@ -157,9 +158,10 @@ static int launch_skinny(const void* x, int ldx, const void* W, int ldw, int M, 
 
 using namespace inv;
 
-// ldx and ldw are multiples of 8 and at least K rounded up to 8; M <= 64. silu_half > 0: the gated form above.
+// ldx and ldw are multiples of 8 and at least K rounded up to 8; M <= 64. silu_half > 0: the gated form above. early: W is resident
+// (launch_step).
 extern "C" int inv_skinny_gemm(const void* x, int ldx, const void* W, int ldw, int M, int N, int K, int silu_half, void* out, int ldo, int out_f32,
-                               float cap, void* stream) {
+                               float cap, int early, void* stream) {
   const int k8 = (K + 7) & ~7;
   if (M > 64 || (ldx % 8) || (ldw % 8) || ldx < k8 || ldw < k8 || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(W) & 15))
     return -ERR_BAD_ARG;
@@ -167,8 +169,8 @@ extern "C" int inv_skinny_gemm(const void* x, int ldx, const void* W, int ldw, i
   cudaStream_t st = (cudaStream_t)stream;
   const bool pairs = K % 16 == 0 && ldw % 16 == 0 && (reinterpret_cast<uintptr_t>(W) & 31) == 0;   // 32-byte pieces of weight rows
 #define INV_SGP(MT, P)                                                                                                                \
-  (silu_half > 0 ? launch_skinny<MT, P, true>(x, ldx, W, ldw, M, N, K, silu_half, out, ldo, out_f32, cap, st)                             \
-                 : launch_skinny<MT, P, false>(x, ldx, W, ldw, M, N, K, 0, out, ldo, out_f32, cap, st))
+  (silu_half > 0 ? launch_skinny<MT, P, true>(x, ldx, W, ldw, M, N, K, silu_half, out, ldo, out_f32, cap, early != 0, st)                             \
+                 : launch_skinny<MT, P, false>(x, ldx, W, ldw, M, N, K, 0, out, ldo, out_f32, cap, early != 0, st))
 #define INV_SG(MT) (pairs ? INV_SGP(MT, 2) : INV_SGP(MT, 1))
   if (M <= 16) return INV_SG(1);
   if (M <= 32) return INV_SG(2);

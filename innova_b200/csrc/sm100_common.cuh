@@ -341,13 +341,15 @@ static inline void bind_context() {
 }
 
 // ---------------------------------------------------------------- programmatic dependent launch
-// Kernels of a decode step take a few microseconds each. One launched by launch_early may start while the kernel before it drains;
-// all of its threads pass wait_previous() before they touch anything an earlier kernel reads or writes (what comes before may only
-// read weights). release_next() lets the next kernel do the same.
+// Kernels of a decode step take a few microseconds each. One launched early may start while the kernel before it drains; all of its
+// threads pass wait_previous() before they touch anything an earlier kernel reads or writes. release_next() lets the next kernel do
+// the same. Some kernels read their weights in front of the wait: these must then be resident, that is written by nothing since the
+// last kernel that was launched plainly (which starts only after everything in front of it is complete and visible). Their entries take
+// that as a flag, and without it launch plainly, as launch_step does with early = false: the wait returns at once.
 __device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... Params, typename... Args>
-static inline void launch_early(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+static inline void launch_step(bool early, void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
@@ -357,8 +359,12 @@ static inline void launch_early(void (*kernel)(Params...), dim3 grid, int thread
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+template <typename... Params, typename... Args>
+static inline void launch_early(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+  launch_step(true, kernel, grid, threads, smem, st, args...);
 }
 
 }  // namespace inv

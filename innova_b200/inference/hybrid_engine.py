@@ -149,7 +149,7 @@ class HybridEngine:
     def _lin(self, x: torch.Tensor, name: str) -> torch.Tensor:
         if name in self.qw:
             from ..ops.oil_linear import oil_linear
-            return oil_linear(x.to(torch.bfloat16), self.qw[name]).to(self.dtype)
+            return oil_linear(x.to(torch.bfloat16), self.qw[name], resident=True).to(self.dtype)     # every pass starts with a lookup of PyTorch's
         return F.linear(x, self.w[name])
 
     # ------------------------------------------------------------------ state

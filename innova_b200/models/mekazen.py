@@ -128,18 +128,19 @@ class MekazenModel(SteppedDecoder):
         todo = dict(ids=batch.ids, table=self.embed.weight)       # what the residual takes in at the next step between sublayers
         for i, index in self.runs:
             for q, sub in enumerate(self.layers[i]):
-                h = sandwich_step(x, self.dtype, eps, NORM_OFFSET, norm_w=sub.norm, **todo)
+                # the step's first kernel is launched plainly: behind it all weights are resident, whoever wrote them just before
+                h = sandwich_step(x, self.dtype, eps, NORM_OFFSET, norm_w=sub.norm, resident="ids" not in todo, **todo)
                 if residuals is not None and q == 0 and i > 0:
                     residuals.append(x.clone())
                 todo = dict(y=sub.body.run(ctx, h, index), post_w=sub.post)
         if residuals is not None:
-            sandwich_step(x, self.dtype, eps, NORM_OFFSET, **todo)
+            sandwich_step(x, self.dtype, eps, NORM_OFFSET, resident="ids" not in todo, **todo)
             residuals.append(x.clone())
             todo = {}
         if batch.n_want == 0:
             return None
         rows = None if batch.want_all else batch.want
-        h = sandwich_step(x, self.dtype, eps, NORM_OFFSET, norm_w=self.final, rows=rows, **todo)
+        h = sandwich_step(x, self.dtype, eps, NORM_OFFSET, norm_w=self.final, rows=rows, resident="ids" not in todo, **todo)
         if hidden:
             return h
         return ctx.logits(h, self.head, cfg.vocab_size, cfg.logit_softcap)

@@ -48,7 +48,9 @@ def put(p: Proj, w: torch.Tensor, row: int = 0):
 class StepContext:
     """Precision of one forward step. bf16 steps of one token per sequence, at most 64 of them, hand fp32 projections to the
     consuming kernels: up to 32 rows from the skinny product, more from the tiled tcgen05 product split over K. Larger steps run
-    the tiled product and write bf16."""
+    the tiled product and write bf16.
+
+    Its projections take their weights as resident (``skinny_gemm``): a model's step starts with a plainly launched kernel."""
 
     SPLIT_ROWS = 64
 
@@ -65,7 +67,7 @@ class StepContext:
             return F.linear(x, w).to(out_dtype or self.dtype)
         rows, n = x.shape[0], w.shape[0]
         if self.skinny or (rows <= SKINNY_ROWS and out_dtype == torch.float32):
-            return skinny_gemm(x, w)
+            return skinny_gemm(x, w, resident=True)
         if self.small and (n + 255) // 256 <= NUM_SMS // 2:
             out = torch.zeros(rows, n, dtype=torch.float32, device=x.device)
             return gemm(x, w, out=out, epilogue=EPI_ATOMIC, split_k=max(1, NUM_SMS // ((n + 255) // 256)))
@@ -74,14 +76,14 @@ class StepContext:
     def gated(self, x: torch.Tensor, p: Proj, ff: int) -> torch.Tensor:
         """silu(gate x) * (up x) for a projection that holds the gate rows, then (from the middle) the up rows."""
         if self.skinny:
-            return skinny_gemm(x[:, : p.k], p.weight[:, : p.k], n=ff, silu_half=p.n // 2, out_dtype=torch.bfloat16)
+            return skinny_gemm(x[:, : p.k], p.weight[:, : p.k], n=ff, silu_half=p.n // 2, out_dtype=torch.bfloat16, resident=True)
         return gated_silu(self.project(x, p), ff, self.dtype)
 
 
     def logits(self, h: torch.Tensor, p: Proj, vocab: int, softcap=None) -> torch.Tensor:
         """fp32 [rows, vocab] of the output head, through the soft limit softcap * tanh(z / softcap) if there is one."""
         if self.bf16 and h.shape[0] <= SKINNY_ROWS:
-            return skinny_gemm(h[:, : p.k], p.weight[:, : p.k], softcap=softcap or 0.0)[:, :vocab]
+            return skinny_gemm(h[:, : p.k], p.weight[:, : p.k], softcap=softcap or 0.0, resident=True)[:, :vocab]
         z = self.project(h, p, torch.float32)[:, :vocab]
         return softcap_(z, softcap) if softcap else z
 

@@ -101,19 +101,23 @@ def gemm(a, b, out=None, *, a_mn=False, b_mn=False, M=None, N=None, K=None, epil
 
 
 _native.register_cuda_sigs({"inv_skinny_gemm": [_native.vp, _native.i32, _native.vp] + [_native.i32] * 5 +
-                                [_native.vp, _native.i32, _native.i32, _native.f32, _native.vp]})
+                                [_native.vp, _native.i32, _native.i32, _native.f32, _native.i32, _native.vp]})
 SKINNY_ROWS = 32          # the kernel takes 64; beyond 32 the split-K tiled product is faster
 
 
-def skinny_gemm(x, w, n=None, silu_half: int = 0, out_dtype=torch.float32, softcap: float = 0.0):
+def skinny_gemm(x, w, n=None, silu_half: int = 0, out_dtype=torch.float32, softcap: float = 0.0, resident: bool = False):
     """x [M <= 64, K] times w [N, K]^T for decode steps (csrc/skinny_gemm.cu): weights straight from memory into MMA fragments,
     no tile set-up. Rows of both operands start on 16-byte boundaries. ``silu_half``: w holds gate rows [0, n) and up rows
-    [silu_half, silu_half + n) and the result is silu(gate) * up. ``softcap``: the result is softcap * tanh(result / softcap)."""
+    [silu_half, silu_half + n) and the result is silu(gate) * up. ``softcap``: the result is softcap * tanh(result / softcap).
+
+    ``resident``: w is a weight that nothing has written on this stream since the last ordinary kernel (a kernel of PyTorch's, say), so
+    that its first rows may be read while the kernels in front are still running, as in a decode step. Never for a w that a kernel
+    of this package has just computed: it would be read too early."""
     M, K = x.shape
     n = w.shape[0] if n is None else n
     out = torch.empty((M, (n + 7) // 8 * 8), dtype=out_dtype, device=x.device)
     rt.check(rt.lib().inv_skinny_gemm(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), M, n, K, silu_half, out.data_ptr(), out.stride(0),
-                                      int(out_dtype == torch.float32), float(softcap), rt.stream_ptr()), "inv_skinny_gemm")
+                                      int(out_dtype == torch.float32), float(softcap), int(resident), rt.stream_ptr()), "inv_skinny_gemm")
     return out[:, :n]
 
 

@@ -6,6 +6,10 @@ through ``csrc/oil_gemm.cu`` on CUDA and through dequantise + matmul on the CPU.
 behaviour covered: OIL8Engine / OIL4Engine ``quant_gemm`` (src/oil_engines_core.cpp:51-160),
 ``oil4_gemm`` / ``oil8_gemm`` (src/kernel_oil4.cpp:31-128, src/kernel_oil8.cpp:14-79) and the
 production GEMVs (src/kernel_production.cpp:95-166).
+
+``resident``, in all of these: nothing has written the packed weights on this stream since the last ordinary kernel (a kernel of
+PyTorch's, say). They are then fetched and expanded while the kernels in front are still running, as in a decode step; a matrix that
+was quantised just before is not resident.
 """
 from __future__ import annotations
 
@@ -21,15 +25,15 @@ from . import runtime as rt
 
 _native.register_cuda_sigs({
     "inv_oil_gemm": [_native.vp, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp, _native.i32, _native.i32, _native.i32,
-                     _native.i32, _native.i32, _native.vp, _native.vp, _native.i32],
+                     _native.i32, _native.i32, _native.vp, _native.vp, _native.i32, _native.i32],
     "inv_oil_gemm_finish": [_native.vp, _native.vp, _native.vp, _native.vp, _native.i64, _native.i32, _native.i32, _native.i32, _native.i32,
                             _native.i32, _native.vp],
     "inv_oil_skinny": [_native.vp, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp, _native.f32, _native.vp, _native.vp,
-                       _native.i32, _native.vp, _native.i32, _native.i32, _native.i32, _native.i32, _native.i32, _native.vp],
+                       _native.i32, _native.vp, _native.i32, _native.i32, _native.i32, _native.i32, _native.i32, _native.i32, _native.vp],
     "inv_oil_gemm_peers": [_native.vp, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp, _native.i32, _native.i32, _native.i32,
-                           _native.i32, _native.i32, _native.vp, _native.vp],
+                           _native.i32, _native.i32, _native.vp, _native.i32, _native.vp],
     "inv_oil_gemm_rs": [_native.vp, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp, _native.i32, _native.i32, _native.i32,
-                        _native.i32, _native.i32, _native.i32, _native.vp, _native.vp],
+                        _native.i32, _native.i32, _native.i32, _native.vp, _native.i32, _native.vp],
     "inv_tp_slice_finish_push": [_native.vp, _native.i32, _native.vp, _native.vp, _native.i32, _native.vp, _native.vp, _native.i32, _native.i32,
                                  _native.i32, _native.i32, _native.i32, _native.i32, _native.vp, _native.vp, _native.vp, _native.vp, _native.vp],
     "inv_tp_norm_apply": [_native.vp, _native.i32, _native.vp, _native.i32, _native.i32, _native.vp, _native.f32, _native.vp, _native.i32, _native.i32,
@@ -131,10 +135,10 @@ def _acc_for(x: torch.Tensor, qw: QuantWeight, M: int) -> torch.Tensor:
     return acc
 
 
-def _gemm_into_acc(xs: torch.Tensor, qw: QuantWeight, acc: torch.Tensor):
+def _gemm_into_acc(xs: torch.Tensor, qw: QuantWeight, acc: torch.Tensor, resident: bool):
     status = rt.status_tensor(xs.device).data_ptr()
     rt.check(rt.lib().inv_oil_gemm(xs.data_ptr(), xs.stride(0), qw.idx.data_ptr(), qw.scales.data_ptr(), qw.codebook.data_ptr(), qw.bits,
-                                   acc.data_ptr(), acc.stride(0), xs.shape[0], qw.N, qw.K, 0, status, rt.stream_ptr(), 0), "inv_oil_gemm")
+                                   acc.data_ptr(), acc.stride(0), xs.shape[0], qw.N, qw.K, 0, status, rt.stream_ptr(), 0, int(resident)), "inv_oil_gemm")
 
 
 SKINNY_TOKENS = 16        # up to here one launch without tensor memory, accumulator and finish pass is faster
@@ -151,16 +155,18 @@ def skinny_fits(x2: torch.Tensor, qw: QuantWeight) -> bool:
     return skinny_takes(qw, x2.shape[0]) and x2.data_ptr() % 16 == 0 and x2.stride(0) % 8 == 0 and x2.stride(1) == 1
 
 
-def _skinny(x2: torch.Tensor, qw: QuantWeight, out: torch.Tensor, mode: int = SKINNY_PLAIN, residual: Optional[torch.Tensor] = None, norm=None):
+def _skinny(x2: torch.Tensor, qw: QuantWeight, out: torch.Tensor, mode: int = SKINNY_PLAIN, residual: Optional[torch.Tensor] = None, norm=None,
+            resident: bool = False):
     """One launch for ``out`` [M, N] (or [M, N / 2], or fp32 sums) from x2 [M, K]; ``norm = (weight, eps)``: of rms_norm(x2) * weight."""
     rt.check(rt.lib().inv_oil_skinny(x2.data_ptr(), x2.stride(0), qw.idx.data_ptr(), qw.scales.data_ptr(), qw.codebook.data_ptr(), qw.bits,
                                      None if norm is None else norm[0].data_ptr(), 0.0 if norm is None else float(norm[1]), rt.ptr(qw.bias),
                                      rt.ptr(residual), 0 if residual is None else residual.stride(0), out.data_ptr(), out.stride(0), x2.shape[0],
-                                     qw.N, qw.K, mode, rt.stream_ptr()), "inv_oil_skinny")
+                                     qw.N, qw.K, mode, int(resident), rt.stream_ptr()), "inv_oil_skinny")
     return out
 
 
-def oil_linear(x: torch.Tensor, qw: QuantWeight, residual: Optional[torch.Tensor] = None, split_k: int = 0) -> torch.Tensor:
+def oil_linear(x: torch.Tensor, qw: QuantWeight, residual: Optional[torch.Tensor] = None, split_k: int = 0,
+               resident: bool = False) -> torch.Tensor:
     """x [..., K] bf16 -> [..., N] bf16."""
     shp = x.shape
     x2 = x.reshape(-1, qw.K)
@@ -175,18 +181,18 @@ def oil_linear(x: torch.Tensor, qw: QuantWeight, residual: Optional[torch.Tensor
     out = torch.empty((M, qw.N), dtype=torch.bfloat16, device=x.device)
     res2 = None if residual is None else residual.reshape(-1, qw.N)
     if skinny_fits(x2, qw):
-        return _skinny(x2, qw, out, residual=res2).view(*shp[:-1], qw.N)
+        return _skinny(x2, qw, out, residual=res2, resident=resident).view(*shp[:-1], qw.N)
     acc = _acc_for(x, qw, M)
     for m0 in range(0, M, 256):
         m1 = min(M, m0 + 256)
-        _gemm_into_acc(x2[m0:m1], qw, acc)
+        _gemm_into_acc(x2[m0:m1], qw, acc, resident)
         rs = None if res2 is None else res2[m0:m1]
         rt.check(rt.lib().inv_oil_gemm_finish(acc.data_ptr(), rt.ptr(qw.bias), rt.ptr(rs), out[m0:m1].data_ptr(), m1 - m0, qw.N, acc.stride(0),
                                               out.stride(0), 0 if rs is None else rs.stride(0), 1, rt.stream_ptr()), "inv_oil_gemm_finish")
     return out.view(*shp[:-1], qw.N)
 
 
-def oil_linear_swiglu(x: torch.Tensor, qw: QuantWeight) -> torch.Tensor:
+def oil_linear_swiglu(x: torch.Tensor, qw: QuantWeight, resident: bool = False) -> torch.Tensor:
     """silu(g) * u with [g | u] = x W^T (+ b): the gate / up projection, its finish and the activation in two kernels
     (the GEMM, and one pass over the fp32 accumulator). x [..., K] -> [..., N / 2]."""
     shp = x.shape
@@ -194,17 +200,17 @@ def oil_linear_swiglu(x: torch.Tensor, qw: QuantWeight) -> torch.Tensor:
     Fh = qw.N // 2
     if not x2.is_cuda or Fh % 4:
         from .functional import swiglu
-        return swiglu(oil_linear(x, qw))
+        return swiglu(oil_linear(x, qw, resident=resident))
     if not x2.is_contiguous():
         x2 = x2.contiguous()
     M = x2.shape[0]
     out = torch.empty((M, Fh), dtype=torch.bfloat16, device=x.device)
     if skinny_fits(x2, qw):
-        return _skinny(x2, qw, out, SKINNY_SWIGLU).view(*shp[:-1], Fh)
+        return _skinny(x2, qw, out, SKINNY_SWIGLU, resident=resident).view(*shp[:-1], Fh)
     acc = _acc_for(x, qw, M)
     for m0 in range(0, M, 256):
         m1 = min(M, m0 + 256)
-        _gemm_into_acc(x2[m0:m1], qw, acc)
+        _gemm_into_acc(x2[m0:m1], qw, acc, resident)
         rt.check(rt.lib().inv_oil_gemm_finish_swiglu(acc.data_ptr(), rt.ptr(qw.bias), out[m0:m1].data_ptr(), m1 - m0, Fh, acc.stride(0),
                                                      out.stride(0), rt.stream_ptr()), "inv_oil_gemm_finish_swiglu")
     return out.view(*shp[:-1], Fh)
@@ -229,21 +235,22 @@ def finish_norm(acc: torch.Tensor, M: int, N: int, bias, residual, norm_w: torch
     return x_out, h_out
 
 
-def oil_linear_norm(x: torch.Tensor, qw: QuantWeight, residual: torch.Tensor, norm_w: torch.Tensor, eps: float):
+def oil_linear_norm(x: torch.Tensor, qw: QuantWeight, residual: torch.Tensor, norm_w: torch.Tensor, eps: float,
+                    resident: bool = False):
     """(y, rms_norm(y) * norm_w) with y = x W^T (+ b) + residual: a block's closing projection fused with the next
     block's RMSNorm. x [M, K], residual [M, N] -> two [M, N] bf16 tensors."""
     x2 = x.reshape(-1, qw.K)
     M = x2.shape[0]
     if not x2.is_cuda or qw.N % 4 or qw.N > 16384 or M > 256:
         from .functional import rms_norm
-        y = oil_linear(x2, qw, residual)
+        y = oil_linear(x2, qw, residual, resident=resident)
         return y, rms_norm(y, norm_w, eps)
     if not x2.is_contiguous():
         x2 = x2.contiguous()
     if skinny_fits(x2, qw):
         from .functional import rms_norm
-        y = _skinny(x2, qw, torch.empty((M, qw.N), dtype=torch.bfloat16, device=x.device), residual=residual.reshape(M, qw.N))
+        y = _skinny(x2, qw, torch.empty((M, qw.N), dtype=torch.bfloat16, device=x.device), residual=residual.reshape(M, qw.N), resident=resident)
         return y, rms_norm(y, norm_w, eps)
     acc = _acc_for(x, qw, M)
-    _gemm_into_acc(x2, qw, acc)
+    _gemm_into_acc(x2, qw, acc, resident)
     return finish_norm(acc, M, qw.N, qw.bias, residual.reshape(M, qw.N), norm_w, eps)

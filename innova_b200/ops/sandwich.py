@@ -15,16 +15,18 @@ from .hyper import row_buffer
 
 _vp, _i, _f = _native.vp, _native.i32, _native.f32
 _native.register_cuda_sigs({
-    "inv_sandwich_step": [_vp, _vp, _vp, _i, _f, _vp, _i, _i, _vp, _vp, _f, _f, _vp, _i, _i, _vp, _i, _i, _i, _vp],
+    "inv_sandwich_step": [_vp, _vp, _vp, _i, _f, _vp, _i, _i, _vp, _vp, _f, _f, _vp, _i, _i, _vp, _i, _i, _i, _i, _vp],
     "inv_softcap": [_vp, _i, _i, _i, _f, _vp],
 })
 
 
 def sandwich_step(x: torch.Tensor, dtype, eps: float, offset: float, y: Optional[torch.Tensor] = None, post_w: Optional[torch.Tensor] = None,
                   norm_w: Optional[torch.Tensor] = None, ids: Optional[torch.Tensor] = None, table: Optional[torch.Tensor] = None, scale: float = 1.0,
-                  rows: Optional[torch.Tensor] = None):
+                  rows: Optional[torch.Tensor] = None, resident: bool = False):
     """x [T, E] fp32, updated in place; y [T, >= E]. Returns the normed row [T (or len(rows)), E] in ``dtype`` if ``norm_w``. ``rows``
-    (int32) restricts the result to those tokens and leaves x as it is."""
+    (int32) restricts the result to those tokens and leaves x as it is. ``resident``: post_w and norm_w are weights that nothing has
+    written on this stream since the last ordinary kernel; they may then be read while the kernels in front are still running
+    (``skinny_gemm``)."""
     T, E = x.shape
     if not x.is_cuda:
         return _sandwich_cpu(x, dtype, eps, offset, y, post_w, norm_w, ids, table, scale, rows)
@@ -34,7 +36,7 @@ def sandwich_step(x: torch.Tensor, dtype, eps: float, offset: float, y: Optional
                                     float(scale), rt.ptr(y), 0 if y is None else y.stride(0),
                                     int(dtype == torch.float32 if y is None else y.dtype == torch.float32), rt.ptr(post_w), rt.ptr(norm_w),
                                     float(offset), float(eps), rt.ptr(h), 0 if h is None else h.stride(0), int(dtype == torch.float32),
-                                    rt.ptr(rows), n, int(rows is None), E, rt.stream_ptr())
+                                    rt.ptr(rows), n, int(rows is None), E, int(resident), rt.stream_ptr())
     rt.check(rc, "inv_sandwich_step")
     return h
 

@@ -72,16 +72,17 @@ class TPContext:
 
 
 def tp_reduce_linear(x: torch.Tensor, qw: QuantWeight, ctx: Optional[TPContext], residual=None, n_total: Optional[int] = None,
-                     n_offset: int = 0, out_fp32: bool = False, norm=None):
+                     n_offset: int = 0, out_fp32: bool = False, norm=None, resident: bool = False):
     """y[M, n_total] = sum over ranks of x_local @ W_local^T, every rank receiving the full result.
 
     Row-parallel layers pass n_offset = 0 and n_total = qw.N (true reduction); the vocabulary-parallel
     head passes its column offset, so that the "reduction" is an all-gather into disjoint columns.
-    With ``norm = (weight, eps)`` the finish pass also applies the next RMSNorm and the call returns (y, normed y)."""
+    With ``norm = (weight, eps)`` the finish pass also applies the next RMSNorm and the call returns (y, normed y).
+    ``resident``: as for ``oil_linear``."""
     if ctx is None or ctx.world == 1:
         if norm is not None:
-            return oil_linear_norm(x, qw, residual, norm[0], norm[1])
-        y = oil_linear(x, qw, residual)
+            return oil_linear_norm(x, qw, residual, norm[0], norm[1], resident)
+        y = oil_linear(x, qw, residual, resident=resident)
         return y.float() if out_fp32 else y
     x2 = x.reshape(-1, qw.K)
     if not x2.is_contiguous():
@@ -101,7 +102,7 @@ def tp_reduce_linear(x: torch.Tensor, qw: QuantWeight, ctx: Optional[TPContext],
         # the residual stream; after a second barrier every rank applies the RMSNorm to the full rows.
         oc = n_total // W
         rt.check(lib.inv_oil_gemm_rs(x2.data_ptr(), x2.stride(0), qw.idx.data_ptr(), qw.scales.data_ptr(), qw.codebook.data_ptr(), qw.bits,
-                                     buf.peers(), W, oc, n_total, M, qw.N, qw.K, status, st), "inv_oil_gemm_rs")
+                                     buf.peers(), W, oc, n_total, M, qw.N, qw.K, status, int(resident), st), "inv_oil_gemm_rs")
         # both barriers sit at the head of the kernel that needs them (flag sets 1 and 2): no launches of their own
         xb, sq = ctx.next_xbuf()
         res2 = residual.reshape(M, n_total)
@@ -117,13 +118,13 @@ def tp_reduce_linear(x: torch.Tensor, qw: QuantWeight, ctx: Optional[TPContext],
         return x_out, h_out
     if ctx.multimem:
         rt.check(lib.inv_oil_gemm(x2.data_ptr(), x2.stride(0), qw.idx.data_ptr(), qw.scales.data_ptr(), qw.codebook.data_ptr(), qw.bits,
-                                  buf.multicast_ptr + n_offset * 4, n_total, M, qw.N, qw.K, 0, status, st, 1), "inv_oil_gemm")
+                                  buf.multicast_ptr + n_offset * 4, n_total, M, qw.N, qw.K, 0, status, st, 1, int(resident)), "inv_oil_gemm")
     else:
         # no multicast object on this machine: one launch whose epilogue adds every tile into each rank's copy
         from .symm import ptr_array
         peers = ptr_array([buf.peer_ptrs[(ctx.rank + k) % ctx.world] + n_offset * 4 for k in range(ctx.world)])
         rt.check(lib.inv_oil_gemm_peers(x2.data_ptr(), x2.stride(0), qw.idx.data_ptr(), qw.scales.data_ptr(), qw.codebook.data_ptr(), qw.bits,
-                                        peers, ctx.world, n_total, M, qw.N, qw.K, status, st), "inv_oil_gemm_peers")
+                                        peers, ctx.world, n_total, M, qw.N, qw.K, status, int(resident), st), "inv_oil_gemm_peers")
     acc = buf.tensor
     res2 = None if residual is None else residual.reshape(M, n_total)
     if norm is not None and not out_fp32 and n_total % 4 == 0 and n_total <= 16384:
@@ -221,19 +222,19 @@ class TPDecoder:
         few = self.world == 1 and B * S <= FEW_PROMPT_TOKENS
         h = ops.rms_norm(x, self.layers[0]["n1"], cfg.norm_eps)
         for li, l in enumerate(self.layers):
-            qkv = oil_linear(h, l["qkv"]) if few else ops.linear(h, l["qkv"].dequantize())
+            qkv = oil_linear(h, l["qkv"], resident=True) if few else ops.linear(h, l["qkv"].dequantize())
             qkv = ops.rope_qk(qkv, self.rope[0], self.rope[1], H, Hkv, D)
             c.append(li, qkv[..., H * D:(H + Hkv) * D], qkv[..., (H + Hkv) * D:], rows, start)
             a = ops.flash_attention(qkv, H, Hkv, D, causal=True)
             nxt = self.layers[li + 1]["n1"] if li + 1 < len(self.layers) else None   # the last norm is taken of the last tokens only
             if few:
-                x2, h = oil_linear_norm(a.view(B * S, -1), l["o"], x.view(B * S, -1), l["n2"], cfg.norm_eps)
-                act = oil_linear_swiglu(h, l["gu"])
+                x2, h = oil_linear_norm(a.view(B * S, -1), l["o"], x.view(B * S, -1), l["n2"], cfg.norm_eps, resident=True)
+                act = oil_linear_swiglu(h, l["gu"], resident=True)
                 if nxt is not None:
-                    x2, h = oil_linear_norm(act, l["down"], x2, nxt, cfg.norm_eps)
+                    x2, h = oil_linear_norm(act, l["down"], x2, nxt, cfg.norm_eps, resident=True)
                     h = h.view(B, S, -1)
                 else:
-                    x2 = oil_linear(act, l["down"], x2)
+                    x2 = oil_linear(act, l["down"], x2, resident=True)
                 x = x2.view(B, S, -1)
                 continue
             if self.world > 1:
@@ -258,7 +259,7 @@ class TPDecoder:
     def _logits(self, last: torch.Tensor, normed: bool = False) -> torch.Tensor:
         h = last if normed else ops.rms_norm(last, self.norm_w, self.cfg.norm_eps)
         Vs = self.cfg.padded_vocab // self.world
-        lg = tp_reduce_linear(h, self.head, self.ctx, n_total=self.cfg.padded_vocab, n_offset=self.rank * Vs, out_fp32=True)
+        lg = tp_reduce_linear(h, self.head, self.ctx, n_total=self.cfg.padded_vocab, n_offset=self.rank * Vs, out_fp32=True, resident=True)
         if self.ctx is not None:
             # a step uses the two accumulators an odd number of times, so the next step starts on the
             # buffer this one just read: nobody may add into it before every rank has taken its logits
@@ -285,7 +286,8 @@ class TPDecoder:
 
     @torch.no_grad()
     def _decode_step(self, tokens: torch.Tensor) -> torch.Tensor:
-        """tokens [B] -> logits [B, vocab]. Uses and advances the device-side sequence lengths."""
+        """tokens [B] -> logits [B, vocab]. Uses and advances the device-side sequence lengths. The lookups in front of the first
+        projection are ordinary kernels, so all weights are resident."""
         cfg, c = self.cfg, self.cache
         B = tokens.shape[0]
         lens = c.seq_lens[:B]
@@ -302,24 +304,24 @@ class TPDecoder:
                 return torch.empty(B, n, dtype=dtype, device=self.dev)
 
             for li, l in enumerate(self.layers):
-                sums = _skinny(x, l["qkv"], rows(l["qkv"].N, torch.float32), SKINNY_SUMS, norm=(l["n1"], eps))
-                x = _skinny(self._attend(li, sums, pos), l["o"], rows(cfg.hidden_size), residual=x)
-                act = _skinny(x, l["gu"], rows(l["gu"].N // 2), SKINNY_SWIGLU, norm=(l["n2"], eps))
-                x = _skinny(act, l["down"], rows(cfg.hidden_size), residual=x)
-            return _skinny(x, self.head, rows(self.head.N), norm=(self.norm_w, eps)).float()[:, : cfg.vocab_size]
+                sums = _skinny(x, l["qkv"], rows(l["qkv"].N, torch.float32), SKINNY_SUMS, norm=(l["n1"], eps), resident=True)
+                x = _skinny(self._attend(li, sums, pos), l["o"], rows(cfg.hidden_size), residual=x, resident=True)
+                act = _skinny(x, l["gu"], rows(l["gu"].N // 2), SKINNY_SWIGLU, norm=(l["n2"], eps), resident=True)
+                x = _skinny(act, l["down"], rows(cfg.hidden_size), residual=x, resident=True)
+            return _skinny(x, self.head, rows(self.head.N), norm=(self.norm_w, eps), resident=True).float()[:, : cfg.vocab_size]
         h = ops.rms_norm(x, self.layers[0]["n1"], cfg.norm_eps)
         for li, l in enumerate(self.layers):
             # QKV projection: the GEMM leaves fp32 sums, one finish kernel adds the bias, applies RoPE, writes the queries
             # and appends the new keys / values to the paged cache (quantised)
             qw = l["qkv"]
             acc = _acc_for(h, qw, B)
-            _gemm_into_acc(h.reshape(B, -1), qw, acc)
+            _gemm_into_acc(h.reshape(B, -1), qw, acc, True)
             a = self._attend(li, acc, pos)
             # every projection's finish pass carries what follows it: the residual add and the next RMSNorm, or SwiGLU
-            x, h = tp_reduce_linear(a, l["o"], self.ctx, residual=x, norm=(l["n2"], cfg.norm_eps))
-            act = oil_linear_swiglu(h, l["gu"])
+            x, h = tp_reduce_linear(a, l["o"], self.ctx, residual=x, norm=(l["n2"], cfg.norm_eps), resident=True)
+            act = oil_linear_swiglu(h, l["gu"], resident=True)
             nxt = self.layers[li + 1]["n1"] if li + 1 < len(self.layers) else self.norm_w
-            x, h = tp_reduce_linear(act, l["down"], self.ctx, residual=x, norm=(nxt, cfg.norm_eps))
+            x, h = tp_reduce_linear(act, l["down"], self.ctx, residual=x, norm=(nxt, cfg.norm_eps), resident=True)
         return self._logits(h, normed=True)
 
     @torch.no_grad()

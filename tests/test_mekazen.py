@@ -121,6 +121,76 @@ def test_skinny_product_with_softcap(M, N, K):
     assert torch.allclose(skinny_gemm(x, w, softcap=2.0).double(), oracle.softcap(x.double() @ w.double().t(), 2.0), atol=5e-4, rtol=1e-3)
 
 
+def test_only_the_kernels_behind_a_plain_launch_take_weights_as_resident(monkeypatch):
+    """A weight may be read in front of the wait for earlier kernels only where a model's step says so; a call of the exported product
+    without the flag, and the first kernel of a step, are launched plainly."""
+    from types import SimpleNamespace
+    from innova_b200.models import mekazen
+    from innova_b200.models.mixers import Proj, StepContext
+    from innova_b200.ops import runtime as rt
+    from innova_b200.ops import skinny_gemm
+    flags = []
+
+    class Lib:
+        def inv_skinny_gemm(self, *args):
+            flags.append(args[-2])
+            return 0
+
+    monkeypatch.setattr(rt, "lib", Lib)
+    monkeypatch.setattr(rt, "stream_ptr", lambda: 0)
+    x, p = torch.zeros(2, 16, dtype=torch.bfloat16), Proj(24, 16, torch.bfloat16)
+    skinny_gemm(x, p.weight)
+    ctx = StepContext(SimpleNamespace(dtype=torch.bfloat16), SimpleNamespace(device=SimpleNamespace(type="cuda")), SimpleNamespace(single=True, T=2))
+    ctx.project(x, p), ctx.gated(x, p, 12), ctx.logits(x, p, 24)
+    assert flags == [0, 1, 1, 1]
+    seen = []
+
+    def record(*args, resident=False, **kw):
+        seen.append(resident)
+        return sandwich_step(*args, resident=resident, **kw)
+
+    monkeypatch.setattr(mekazen, "sandwich_step", record)
+    cfg = CONFIGS["mixed"]
+    model = MekazenModel.from_tensors(cfg, oracle.random_weights(cfg, 0), dtype=torch.float32, device=torch.device("cpu"))
+    model(torch.zeros(1, 3, dtype=torch.int64))
+    assert seen == [False] + [True] * (len(seen) - 1) and len(seen) == sum(1 + (l["mlp"] is not None) for l in cfg["layers"]) + 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [64, 2048])
+def test_weights_computed_just_before(K):
+    """Products and norms whose weight is what the kernel in front wrote, into memory that held another one: the same bits as with a wait
+    of the host in between."""
+    from innova_b200.ops import skinny_gemm
+    from innova_b200.ops.oil_linear import oil_linear, quantize_weight
+    g = torch.Generator(device="cuda").manual_seed(K)
+
+    def rand(*s):
+        return torch.randn(*s, device="cuda", generator=g)
+
+    def chain(a, b, x, r, between):
+        out = []
+        w = skinny_gemm(a, b, out_dtype=torch.bfloat16)                 # [24, K], the weight of the next
+        between()
+        out.append(skinny_gemm(x, w))
+        h = sandwich_step(r.clone(), torch.bfloat16, 1e-5, 1.0, norm_w=b[:, 0].float().contiguous())
+        between()
+        out.append(skinny_gemm(x, h))
+        post = skinny_gemm(a[:1], b)[0]                                 # fp32 [K]: a norm's weight
+        between()
+        out.append(sandwich_step(r.clone(), torch.bfloat16, 1e-5, 1.0, y=x[:1].expand(r.shape[0], K).contiguous(), post_w=post, norm_w=post))
+        qw = quantize_weight(w, "oil4")
+        between()
+        out.append(oil_linear(x, qw))
+        return out
+
+    torch.cuda.synchronize()
+    for _ in range(30):
+        a, b, x, r = rand(24, 64).bfloat16(), (rand(K, 64) / 8).bfloat16(), rand(3, K).bfloat16(), rand(16, K)
+        for got, want in zip(chain(a, b, x, r, lambda: None), chain(a, b, x, r, torch.cuda.synchronize)):
+            assert torch.equal(got, want)
+
+
 def test_frequencies():
     for r in (rot(32, 1e6, SCALED), rot(64, 500.0, SCALED), rot(10), rot(8, 100.0, {"factor": 2.0, "low": 1.0, "high": 1.0, "original": 50})):
         got = ka.rope_frequencies(r["dims"], r["base"], r["scaling"])
