@@ -11,7 +11,7 @@ import torch
 import torch.nn.functional as F
 
 from . import runtime as rt
-from .gemm import EPI_ATOMIC, gemm, main_grads
+from .gemm import EPI_ATOMIC, gemm, main_grad_of, main_grads
 
 
 def _acc_grad(param, g32):
@@ -68,8 +68,8 @@ def _norm_backward(ctx, dy, dres):
     dx = torch.empty_like(x2)
     grid = rt.lib().inv_norm_bwd_grid(T)
     scr = rt.scratch("norm_bwd", grid * 3 * D * 4, x2.device)
-    mg_g = getattr(gamma, "main_grad", ctx.main_grads[0])
-    mg_b = getattr(beta, "main_grad", ctx.main_grads[1]) if beta is not None else None
+    mg_g = main_grad_of(gamma, ctx.main_grads[0])
+    mg_b = main_grad_of(beta, ctx.main_grads[1]) if beta is not None else None
     dg = mg_g if mg_g is not None else torch.zeros(D, dtype=torch.float32, device=x2.device)
     db = None
     if beta is not None:

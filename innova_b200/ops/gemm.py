@@ -11,6 +11,7 @@ src/autograd_functions.cpp:226-239), gemm_tiled_bias_act (src/math_avx2_tiled.cp
 from __future__ import annotations
 
 import contextlib
+import weakref
 
 import torch
 import torch.nn.functional as F
@@ -122,16 +123,26 @@ def skinny_gemm(x, w, n=None, silu_half: int = 0, out_dtype=torch.float32, softc
 
 
 def main_grads(*params):
-    """The ``main_grad`` of each parameter, for a forward pass to keep: a saved tensor that comes back through saved-tensor hooks
-    (gradient checkpointing recomputes it) is another object without the attribute."""
-    return tuple(getattr(p, "main_grad", None) for p in params)
+    """For a forward pass to keep: each parameter, weakly, and its ``main_grad`` as it is now (``main_grad_of``)."""
+    return tuple(None if p is None else (weakref.ref(p), getattr(p, "main_grad", None)) for p in params)
+
+
+def main_grad_of(saved, kept):
+    """The ``main_grad`` of a saved parameter in the backward pass. A tensor that comes back through saved-tensor hooks (gradient
+    checkpointing recomputes it) is another object without the attribute: then what the forward's parameter has now counts, None if it
+    was taken away since, and only where that object is gone (a quantised copy of the first pass) what the forward saw."""
+    mg = getattr(saved, "main_grad", None)
+    if mg is None and kept is not None:
+        p = kept[0]()
+        mg = kept[1] if p is None else getattr(p, "main_grad", None)
+    return mg
 
 
 def _accumulate_wgrad(weight, dy2, x2, kept=None):
-    """weight.main_grad[N,K] += dy2[T,N]^T @ x2[T,K]; returns a grad tensor only when there is no main_grad (nor ``kept``, the one that
-    the forward pass saw)."""
+    """weight.main_grad[N,K] += dy2[T,N]^T @ x2[T,K]; returns a grad tensor only when there is no main_grad (``kept``: of
+    ``main_grads``)."""
     N, K = weight.shape
-    mg = getattr(weight, "main_grad", kept)
+    mg = main_grad_of(weight, kept)
     if mg is not None:
         gemm(dy2, x2, out=mg.view(N, K), a_mn=True, b_mn=True, epilogue=EPI_ATOMIC)
         return None
@@ -142,7 +153,7 @@ def _accumulate_wgrad(weight, dy2, x2, kept=None):
 
 def _accumulate_bgrad(bias, dy2, colsum=None, kept=None):
     """``colsum``: fp32 column sums of ``dy2`` when its producer already computed them (``rt.take_colsum``)."""
-    mg = getattr(bias, "main_grad", kept)
+    mg = main_grad_of(bias, kept)
     T, N = dy2.shape
     if colsum is not None:
         if mg is not None:

@@ -83,3 +83,22 @@ def test_token_loader_next_token_labels():
     assert len(dl) == 5
     ids, labels = next(iter(dl))
     assert torch.equal(labels, ids + 1)
+
+
+def test_main_grad_that_a_backward_pass_uses():
+    """The saved object's own buffer, else what the forward's parameter has by then, else (the object is gone) what the forward saw."""
+    from innova_b200.ops.gemm import main_grad_of, main_grads
+    p, buf, other = torch.nn.Parameter(torch.zeros(2)), torch.zeros(2), torch.ones(2)
+    p.main_grad = buf
+    kept, none = main_grads(p, None)
+    assert none is None and main_grad_of(torch.zeros(2), none) is None
+    assert main_grad_of(p, kept) is buf and main_grad_of(p.detach(), kept) is buf
+    p.main_grad = other
+    assert main_grad_of(p.detach(), kept) is other
+    del p.main_grad
+    assert main_grad_of(p, kept) is None and main_grad_of(p.detach(), kept) is None
+    copy = p.detach().clone()
+    copy.main_grad = buf
+    kept = main_grads(copy)[0]
+    del copy
+    assert main_grad_of(p.detach(), kept) is buf

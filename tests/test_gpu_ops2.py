@@ -521,3 +521,30 @@ def test_gpu_checkpointed_layers_accumulate_in_place():
             assert all(p.grad is None for p in m.parameters())
             grads.append(torch.cat([p.main_grad.reshape(-1) for p in m.parameters()]).double())
         assert float((grads[0] - grads[1]).norm() / grads[0].norm()) < 2.0 ** -8    # fp32 sums in another order, a bf16 rounding apart
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hooks", [False, True])
+@pytest.mark.parametrize("removed", [False, True])
+def test_gpu_gradients_follow_main_grad_as_it_is_in_the_backward_pass(hooks, removed):
+    """A main_grad that is taken away between the passes: gradients go to .grad and leave the old buffer alone."""
+    import contextlib
+    from innova_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(3)
+
+    def param(*s):
+        p = torch.nn.Parameter((torch.randn(*s, device="cuda", generator=g) * 0.1).bfloat16())
+        p.main_grad = torch.zeros(*s, device="cuda")
+        return p
+
+    ps = [param(128), param(128), param(192, 128), param(192), param(256, 192), param(256), param(192, 256), param(192)]
+    x = torch.randn(64, 128, device="cuda", generator=g).bfloat16()
+    with (torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach(), lambda t: t) if hooks else contextlib.nullcontext()):
+        y = ops.mlp_gelu(ops.linear(ops.layer_norm(x, ps[0], ps[1]), ps[2], ps[3]), ps[4], ps[5], ps[6], ps[7])
+    buffers = [p.main_grad for p in ps]
+    if removed:
+        for p in ps:
+            del p.main_grad
+    y.backward(torch.ones_like(y))
+    for p, b in zip(ps, buffers):
+        assert (p.grad is not None and bool(p.grad.any()) and not b.any()) if removed else (p.grad is None and bool(b.any()))
