@@ -247,10 +247,11 @@ def oil_linear_norm(x: torch.Tensor, qw: QuantWeight, residual: torch.Tensor, no
         return y, rms_norm(y, norm_w, eps)
     if not x2.is_contiguous():
         x2 = x2.contiguous()
-    if skinny_fits(x2, qw):
+    if skinny_fits(x2, qw) and qw.N % 8 == 0 and norm_w.data_ptr() % 16 == 0:      # what the norm's own kernel reads in 16-byte pieces
         from .functional import rms_norm
         y = _skinny(x2, qw, torch.empty((M, qw.N), dtype=torch.bfloat16, device=x.device), residual=residual.reshape(M, qw.N), resident=resident)
-        return y, rms_norm(y, norm_w, eps)
+        with torch.no_grad():
+            return y, rms_norm(y, norm_w, eps)
     acc = _acc_for(x, qw, M)
     _gemm_into_acc(x2, qw, acc, resident)
     return finish_norm(acc, M, qw.N, qw.bias, residual.reshape(M, qw.N), norm_w, eps)

@@ -267,3 +267,20 @@ def test_gpu_few_tokens_one_launch(fmt, M, N, K):
     assert off(oil_linear(x, qw, residual=res), plain) < 2.0 ** -8 and off(oil_linear_swiglu(x, qw), glu) < 2.0 ** -7
     y, hn = oil_linear_norm(x, qw, res, nwo, 1e-5)
     assert off(y, plain) < 2.0 ** -8 and off(hn, rms_norm(y, nwo, 1e-5).double()) < 2.0 ** -8
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [1, 5, 16, 17])
+@pytest.mark.parametrize("N,offset", [(20, 0), (100, 4), (256, 4), (256, 0)])
+def test_gpu_projection_and_norm_of_widths_and_weights_off_16_bytes(M, N, offset):
+    """Widths that are a multiple of four only, and norm weights on 8 bytes, with few tokens as with more; the results carry no graph."""
+    from innova_b200.ops.oil_linear import oil_linear_norm, quantize_weight
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    qw = quantize_weight(torch.randn(N, 128, device="cuda", generator=g) * 0.1, "oil4")
+    x, res = (torch.randn(M, n, device="cuda", generator=g).bfloat16() for n in (128, N))
+    nw = torch.nn.Parameter(torch.randn(N + offset, device="cuda", generator=g).bfloat16()[offset:])
+    y, h = oil_linear_norm(x, qw, res, nw, 1e-5)
+    want = x.double() @ qw.dequantize().double().t() + res.double()
+    normed = y.double() * torch.rsqrt(y.double().square().mean(-1, keepdim=True) + 1e-5) * nw.detach().double()
+    assert not y.requires_grad and not h.requires_grad
+    assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -8 and float((h.double() - normed).norm() / normed.norm()) < 2.0 ** -8
