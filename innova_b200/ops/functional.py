@@ -319,8 +319,8 @@ def cross_entropy(logits, labels, vocab=None, smoothing=0.0):
 
 
 def _scaled(x, factor):
-    """bf16(x * factor), the fp32 factor on the device; x [T, D] bf16, dense."""
-    if x.data_ptr() % 16:
+    """bf16(x * factor), the fp32 factor on the device; x [T, D] bf16, dense. A factor of several values spreads over x."""
+    if x.data_ptr() % 16 or factor.numel() != 1:
         return (x.float() * factor).to(torch.bfloat16)
     out = torch.empty_like(x)
     rt.check(rt.lib().inv_scale_bf16(x.data_ptr(), factor.data_ptr(), out.data_ptr(), x.numel(), rt.stream_ptr()), "inv_scale_bf16")

@@ -548,3 +548,21 @@ def test_gpu_gradients_follow_main_grad_as_it_is_in_the_backward_pass(hooks, rem
     y.backward(torch.ones_like(y))
     for p, b in zip(ps, buffers):
         assert (p.grad is not None and bool(p.grad.any()) and not b.any()) if removed else (p.grad is None and bool(b.any()))
+
+
+@pytest.mark.gpu
+def test_gpu_head_loss_with_a_scale_per_token():
+    """``grad_scale`` as a tensor of one value, or of one per token: the gradients of the weighted sum. bf16 products and roundings."""
+    from innova_b200 import ops
+    T, D, V = 48, 64, 128
+    g = torch.Generator(device="cuda").manual_seed(8)
+    x0, w0 = torch.randn(T, D, device="cuda", generator=g).bfloat16(), (torch.randn(V, D, device="cuda", generator=g) * 0.2).bfloat16()
+    labels = torch.randint(0, V, (T,), device="cuda", generator=g)
+    for scale in (torch.tensor([3.0], device="cuda"), torch.rand(T, 1, device="cuda", generator=g) + 0.5):
+        x, w = x0.clone().requires_grad_(), w0.clone().requires_grad_()
+        ops.lm_head_cross_entropy(x, w, labels, grad_scale=scale).backward()
+        xr, wr = x0.double().requires_grad_(), w0.double().requires_grad_()
+        nll = torch.nn.functional.cross_entropy(xr @ wr.t(), labels, reduction="none")
+        (nll * scale.double().expand(T, 1).view(-1)).sum().div(T).backward()
+        for a, b in ((x, xr), (w, wr)):
+            assert float((a.grad.double() - b.grad).norm() / b.grad.norm()) < 2e-2
