@@ -342,7 +342,9 @@ class TPDecoder:
         if use_graph:
             # The first time, a step runs on a side stream (allocations, lazy kernel attributes) and the state is restored. A capture takes
             # its buffers, one step's worth, from the pool of the one before it, which is never replayed again (torch.cuda.graph
-            # empties the allocator's cache instead: 10 ms and more of a call in allocations).
+            # empties the allocator's cache instead: 10 ms and more of a call in allocations). The pool stays with the decoder, except
+            # with ranks, whose graphs end before their process group does. "relaxed": a garbage collection may free CUDA objects in
+            # the middle of the capture, here or on another thread, and must not end it.
             saved = self.cache.seq_lens.clone()
             if self._side is None:
                 self._side = torch.cuda.Stream()
@@ -357,13 +359,13 @@ class TPDecoder:
                     self.ctx.turn = 0
                     self.ctx.xturn = 0
                 graph = torch.cuda.CUDAGraph()
-                graph.capture_begin(pool=None if self._graph is None else self._graph.pool())
+                graph.capture_begin(pool=None if self._graph is None else self._graph.pool(), capture_error_mode="relaxed")
                 try:
                     static_logits = self._decode_step(static_tok)
                     static_next = static_logits.argmax(-1)
                 finally:
                     graph.capture_end()
-            self._graph = graph
+            self._graph = graph if self.ctx is None else None
             torch.cuda.current_stream().wait_stream(s)
             self.cache.seq_lens.copy_(saved)
             e[1].record()

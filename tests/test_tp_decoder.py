@@ -1,5 +1,7 @@
 """``TPDecoder`` on one GPU against an fp64 forward over its own packed weights: prompts on either side of the packed route, steps of a few
 tokens and of more, captured and eager, one decoder through calls of changing sizes."""
+import gc
+
 import pytest
 import torch
 
@@ -106,3 +108,30 @@ def test_generation_through_changing_sizes(kv):
             z = reference(dec, torch.cat([ids, out], 1))[:, S - 1:-1]
             behind = z.amax(-1) - z.gather(-1, out.unsqueeze(-1)).squeeze(-1)
             assert float(behind.max()) < 4 * LOGITS[kv] * float(z.std())
+
+
+def test_a_collection_in_the_middle_of_a_capture():
+    dec = decoder("bf16")
+    ids = tokens(2, 20, 5)
+    want, _, _ = dec.generate(ids, 8)
+    step = dec._decode_step
+
+    def collecting(tok):
+        out = step(tok)
+        if torch.cuda.is_current_stream_capturing():
+            gc.collect()
+        return out
+
+    class Ring:
+        pass
+
+    ring, graph = Ring(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = torch.zeros(4, device="cuda") + 1
+    ring.me, ring.held = ring, (graph, y, torch.cuda.Event(), torch.empty(1 << 20, device="cuda"), torch.empty(1 << 16, pin_memory=True))
+    ring.held[2].record()
+    torch.cuda.synchronize()
+    del ring, graph, y
+    dec._decode_step = collecting
+    got, _, _ = dec.generate(ids, 8)
+    assert torch.equal(got, want)
