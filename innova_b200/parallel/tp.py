@@ -284,6 +284,14 @@ class TPDecoder:
                                       self._splits, st), "inv_paged_decode")
         return a
 
+    def _few(self, B: int) -> bool:
+        """Whether a step of B tokens runs on the skinny products: one rank, and every matrix and norm as they take them. Looked at anew in
+        every step, since weights may be replaced; a batch that is too large is told from the head alone."""
+        if self.ctx is not None or not skinny_takes(self.head, B) or self.norm_w.data_ptr() % 16:
+            return False
+        return all((l["n1"].data_ptr() | l["n2"].data_ptr()) % 16 == 0 and skinny_takes(l["qkv"], B) and skinny_takes(l["o"], B)
+                   and skinny_takes(l["gu"], B) and skinny_takes(l["down"], B) for l in self.layers)
+
     @torch.no_grad()
     def _decode_step(self, tokens: torch.Tensor) -> torch.Tensor:
         """tokens [B] -> logits [B, vocab]. Uses and advances the device-side sequence lengths. The lookups in front of the first
@@ -294,9 +302,7 @@ class TPDecoder:
         pos = lens.clone()                      # position of the new token
         lens.add_(1)
         x = self.emb[tokens]
-        mats = [self.head] + [l[k] for l in self.layers for k in ("qkv", "o", "gu", "down")]
-        norms = [self.norm_w] + [l[k] for l in self.layers for k in ("n1", "n2")]
-        if self.ctx is None and all(skinny_takes(qw, B) for qw in mats) and all(w.data_ptr() % 16 == 0 for w in norms):
+        if self._few(B):
             # A few tokens: every projection is one launch that takes the norm in front of it and the residual or SwiGLU behind it
             eps = cfg.norm_eps
 

@@ -110,9 +110,27 @@ def test_generation_through_changing_sizes(kv):
             assert float(behind.max()) < 4 * LOGITS[kv] * float(z.std())
 
 
+def test_the_route_of_a_step_follows_its_weights():
+    """Too many tokens are told from the head alone; a matrix or norm off its alignment takes the whole step to the tile product."""
+    from innova_b200.parallel import tp
+    dec, asked = decoder("bf16"), []
+    takes = tp.skinny_takes
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(tp, "skinny_takes", lambda qw, M: asked.append(qw) or takes(qw, M))
+        assert not dec._few(17) and asked == [dec.head] and dec._few(16)
+    down = dec.layers[1]["down"]
+    moved = torch.empty(down.idx.numel() + 16, dtype=torch.uint8, device="cuda")[16:].view_as(down.idx).copy_(down.idx)
+    ids = tokens(2, 30, 3)
+    down.idx = moved
+    assert not dec._few(2)
+    got, _, _ = dec.generate(ids, 6)
+    z = reference(dec, torch.cat([ids, got], 1))[:, 29:-1]
+    assert float((z.amax(-1) - z.gather(-1, got.unsqueeze(-1)).squeeze(-1)).max()) < 4 * LOGITS["bf16"] * float(z.std())
+
+
 def test_a_collection_in_the_middle_of_a_capture():
     dec = decoder("bf16")
-    ids = tokens(2, 20, 5)
+    ids = tokens(1, 12, 5)          # few enough for sums in a fixed order all the way
     want, _, _ = dec.generate(ids, 8)
     step = dec._decode_step
 
