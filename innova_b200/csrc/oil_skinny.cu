@@ -1,4 +1,4 @@
-// Products of a few tokens with packed block-32 weights: y[M, N] = x[M, K] dequant(W)[N, K]^T for M <= 32, in one kernel with what
+// Products of a few tokens with packed block-32 weights: y[M, N] = x[M, K] dequant(W)[N, K]^T for M <= 16, in one kernel with what
 // surrounds it: an RMSNorm of x in front, and bias, residual or SwiGLU behind.
 //
 // At a handful of tokens such a product is bound by latency: the weights of a layer of width 2048 are 25 MB, four microseconds. The
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(os::THREADS, 2) oil_skinny_kernel(const OilSki
   __shared__ float s_cb[BITS == 8 ? 256 : 16];
   __shared__ float s_red[WARPS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  release_next();
   if (tid < (BITS == 8 ? 256 : 1 << BITS)) s_cb[tid] = p.codebook[tid];
 
   const int half = p.N / 2;
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(os::THREADS, 2) oil_skinny_kernel(const OilSki
     if (warp + u * WARPS < slices) fetch(tile, warp + u * WARPS, raw[u], sc[u]);
   __syncthreads();
   if (BITS != 2) oil_lut_fill<BITS>(lut, s_cb, tid, THREADS);
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  wait_previous();
 
   // x into shared memory, P threads per token; what lies behind K is zero
   {
@@ -255,7 +255,7 @@ static int launch_oil_skinny(const OilSkinnyParams& p, bool early, cudaStream_t 
 
 using namespace inv;
 
-// M <= 32 tokens, K % 64 == 0, and x (M * K rounded up to 256, 2 bytes each, and a little) within 180 KB of shared memory. x and norm_w on 16
+// M <= 16 tokens, K % 64 == 0, and x (M * K rounded up to 256, 2 bytes each, and a little) within 180 KB of shared memory. x and norm_w on 16
 // bytes, the codes on 32, the scales on 4, ldx % 8 == 0. mode 0: out bf16 [M, N] = product + bias + residual. mode 1: out bf16
 // [M, N / 2] = silu(gate + bias) * (up + bias), gate rows [0, N / 2), up rows behind them. mode 2: out fp32 [M, N] = product. norm_w
 // (optional): x is rms_norm(x) * norm_w, as its own kernel would round it. early: codes, scales and codebook are
@@ -263,7 +263,7 @@ using namespace inv;
 extern "C" int inv_oil_skinny(const void* x, int ldx, const void* idx, const void* scales, const float* codebook, int bits, const void* norm_w,
                               float eps, const void* bias, const void* residual, int ld_res, void* out, int ldo, int M, int N, int K, int mode,
                               int early, void* stream) {
-  if ((bits != 2 && bits != 4 && bits != 8) || M < 1 || M > 32 || (K % 64) || K < 64 || (ldx % 8) || N < 1 || mode < 0 || mode > 2 ||
+  if ((bits != 2 && bits != 4 && bits != 8) || M < 1 || M > 16 || (K % 64) || K < 64 || (ldx % 8) || N < 1 || mode < 0 || mode > 2 ||
       (mode == 1 && (N % 2)) || ((uintptr_t)x | (uintptr_t)norm_w) % 16 || (uintptr_t)idx % 32 || (uintptr_t)scales % 4 ||
       (long)((K + 255) / 256) * 128 * (4 * M + 1) > 180 * 1024)
     return -ERR_BAD_ARG;
@@ -272,7 +272,7 @@ extern "C" int inv_oil_skinny(const void* x, int ldx, const void* idx, const voi
                     mode == 1 ? (N / 2 + 7) / 8 : (N + 15) / 16};
   cudaStream_t st = (cudaStream_t)stream;
   const bool pdl = early != 0;
-#define INV_OS(B) (M <= 8 ? launch_oil_skinny<B, 1>(p, pdl, st) : M <= 16 ? launch_oil_skinny<B, 2>(p, pdl, st) : launch_oil_skinny<B, 4>(p, pdl, st))
+#define INV_OS(B) (M <= 8 ? launch_oil_skinny<B, 1>(p, pdl, st) : launch_oil_skinny<B, 2>(p, pdl, st))
   return bits == 2 ? INV_OS(2) : bits == 4 ? INV_OS(4) : INV_OS(8);
 #undef INV_OS
 }

@@ -284,3 +284,21 @@ def test_gpu_projection_and_norm_of_widths_and_weights_off_16_bytes(M, N, offset
     normed = y.double() * torch.rsqrt(y.double().square().mean(-1, keepdim=True) + 1e-5) * nw.detach().double()
     assert not y.requires_grad and not h.requires_grad
     assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -8 and float((h.double() - normed).norm() / normed.norm()) < 2.0 ** -8
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,fits", [(1, 73728), (8, 11008), (9, 9728), (16, 5632)])
+def test_gpu_few_tokens_up_to_the_limit_of_shared_memory(M, fits):
+    """The longest rows that the skinny product takes at a token count, the next longer ones (the tile product's) and a token too many."""
+    from innova_b200.ops import runtime as rt
+    from innova_b200.ops.oil_linear import SKINNY_SUMS, _skinny, oil_linear, quantize_weight, skinny_takes
+    g = torch.Generator(device="cuda").manual_seed(M)
+    for K in (fits, fits + 256):
+        qw = quantize_weight(torch.randn(40, K, device="cuda", generator=g) * 0.05, "oil4")
+        x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+        want = x.double() @ qw.dequantize().double().t()
+        assert skinny_takes(qw, M) == (K == fits) and not skinny_takes(qw, 17)
+        assert float((oil_linear(x, qw).double() - want).norm() / want.norm()) < 2.0 ** -8
+    with pytest.raises(RuntimeError):
+        _skinny(x, qw, torch.empty(M, 40, device="cuda"), SKINNY_SUMS)
+    rt.check_status()
