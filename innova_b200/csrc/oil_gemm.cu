@@ -230,7 +230,7 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  release_next();
   if (threadIdx.x == 0) OG_STAMP(1);
   [[maybe_unused]] bool og_once = false, og_once2 = false;
 
@@ -251,7 +251,7 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
       // Everything that touches only the (then resident) weights runs ahead: index tiles are fetched and expanded
       // into tensor memory; the activation loads, and with them the MMAs and the epilogue, wait here for the
       // previous grid to complete.
-      asm volatile("griddepcontrol.wait;" ::: "memory");
+      wait_previous();
       OG_STAMP(3);
       int lb = 0;
       for (OgCursor c(n_tiles, nb, p.dp_rounds); c.valid; c.advance(), ++lb) {
@@ -735,20 +735,10 @@ static int oil_gemm_launch(const void* x, int ldx, const void* idx, const void* 
   int grid = (int)((total + 1) / 2);
   if (grid > num_sms) grid = num_sms;
   p.dp_rounds = n_tiles / grid;  // whole tiles while they fill rounds of the grid, the rest is the stream-K tail
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = early ? 1 : 0;
-  cudaError_t e;
-  if (bits == 2) e = cudaLaunchKernelEx(&cfg, oil_gemm_kernel<2>, ti, tx, p);
-  else if (bits == 4) e = cudaLaunchKernelEx(&cfg, oil_gemm_kernel<4>, ti, tx, p);
-  else e = cudaLaunchKernelEx(&cfg, oil_gemm_kernel<8>, ti, tx, p);
+  if (bits == 2) launch_step(early, oil_gemm_kernel<2>, dim3(grid), THREADS, smem, st, ti, tx, p);
+  else if (bits == 4) launch_step(early, oil_gemm_kernel<4>, dim3(grid), THREADS, smem, st, ti, tx, p);
+  else launch_step(early, oil_gemm_kernel<8>, dim3(grid), THREADS, smem, st, ti, tx, p);
+  const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
 

@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const __nv_bfloat16* 
   constexpr int EPL = D / 32;  // output elements per lane
   constexpr int HALF = D / 2;  // elements per lane in the QK phase (two lanes per token)
   using VRaw = typename std::conditional<EPL == 4, uint2, uint32_t>::type;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the output projection may start on its weights
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  release_next();  // the output projection may start on its weights
+  wait_previous();
   __shared__ float sq[MAXG][D];
   __shared__ float sm_m[4][MAXG], sm_l[4][MAXG];
   __shared__ float sm_o[4][MAXG][D];
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32)) paged_decode_oil4_mm
   constexpr int VCH = D / 8;        // d-values of a V row per lane (one eighth of the row)
   constexpr int VW = VCH / 8;       // ... as 32-bit words (2 for D = 128)
   constexpr int VMMA = VCH / 2;     // PV MMAs per page: 2 d-values per lane and MMA
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the output projection may start on its weights
+  release_next();  // the output projection may start on its weights
   __shared__ __align__(16) uint32_t lut[256 * 32];  // byte -> half2(level[low nibble], level[high nibble]); entry e of lane l at [e * 32 + l]
   __shared__ float sm_m[NW][MAXG], sm_l[NW][MAXG];
   float (*sm_o)[MAXG][D] = reinterpret_cast<float (*)[MAXG][D]>(lut);  // the per-warp outputs reuse the table once the loop is over
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32)) paged_decode_oil4_mm
     const uint32_t v = h2_as_u32(__floats2half2_rn(c_kv_levels[e & 15], c_kv_levels[e >> 4]));
     *reinterpret_cast<uint4*>(&lut[i4 * 4]) = make_uint4(v, v, v, v);
   }
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // the table is built while the queries are still being written
+  wait_previous();  // the table is built while the queries are still being written
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int G = H / Hkv;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -554,8 +554,8 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32)) paged_decode_oil4_mm
 // out[b, h*D + e] = sum_s o_s * 2^(m_s - m) / sum_s l_s * 2^(m_s - m)
 __global__ void attn_combine_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out, int ld_o, int B, int H, int Hkv, int D,
                                     int splits) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  release_next();
+  wait_previous();
   const int G = H / Hkv;
   const long total = (long)B * H * D;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
@@ -622,8 +622,8 @@ __global__ void __launch_bounds__(256) decode_qkv_finish_kernel(float* __restric
                                                                 uint8_t* __restrict__ k_pool, uint8_t* __restrict__ v_pool,
                                                                 __half* __restrict__ k_scale, __half* __restrict__ v_scale) {
   constexpr int NJ = D / 32, HALFJ = NJ / 2;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  release_next();
+  wait_previous();
   const int lane = threadIdx.x & 31;
   const long warp_id = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   const int slots = H + 2 * Hkv;
