@@ -4,7 +4,7 @@ import torch
 
 from innova_b200.formats import export, oil
 from innova_b200.inference.generator import Generator
-from innova_b200.inference.kv_cache import PagedKVCache
+from innova_b200.inference.kv_cache import KV_LEVELS, PagedKVCache
 from innova_b200.inference.sampler import Sampler, SamplingParams
 from innova_b200.models import DenseModel, TransformerConfig, tiny_dense
 
@@ -166,6 +166,51 @@ def test_gpu_kv_append_whole_rows_as_single_values(fmt, B, S, Hkv, D, start):
     for name in ("k_pool", "v_pool") + (("k_scale", "v_scale") if fmt == "oil4" else ()):
         a, b = (getattr(c, name)[0].view(torch.uint8) for c in caches)
         assert torch.equal(a, b), name
+
+
+def test_kv_thresholds_are_the_first_floats_nearer_to_the_next_level():
+    """The constants of the append kernels, in 32-bit arithmetic: each takes its level and the float below it does not."""
+    import pathlib
+    import re
+    import numpy as np
+    import innova_b200
+    text = (pathlib.Path(innova_b200.__file__).parent / "csrc" / "paged_attn.cu").read_text()
+
+    def table(name, parse):
+        return np.array([parse(v.strip().rstrip("f")) for v in re.search(name + r"\[\d+\] = \{([^}]*)\}", text).group(1).split(",")], dtype=np.float32)
+
+    levels, thr = table("c_kv_levels", float), table("KV_THRESHOLDS", float.fromhex)
+    assert len(levels) == 16 and len(thr) == 15 and np.allclose(levels, KV_LEVELS.numpy(), atol=1e-6)
+    for j in range(15):
+        for x, takes in ((thr[j], True), (np.nextafter(thr[j], np.float32(-2)), False)):
+            assert bool((levels[j + 1] - x) < (x - levels[j])) == takes, (j, x)
+
+
+@pytest.mark.gpu
+def test_gpu_kv_codes_beside_the_halfway_points():
+    """Codes of both append kernels against the level that the halfway points give in 64 bits: the bf16 values around each of them, in blocks
+    whose maximum is 1, so that the division is exact."""
+    dev = torch.device("cuda", 0)
+    mids = (KV_LEVELS.double()[1:] + KV_LEVELS.double()[:-1]) / 2
+    mids[7] = 0.0
+    bits = mids[mids != 0].bfloat16().view(torch.int16)
+    near = torch.cat([(bits + d).view(torch.bfloat16) for d in (-2, -1, 0, 1, 2)] + [torch.tensor([0.0, 2.0 ** -20, -2.0 ** -20]).bfloat16()])
+    rows = torch.zeros(-(-near.numel() // 31), 32, dtype=torch.bfloat16)
+    flat = torch.zeros(rows.shape[0] * 31, dtype=torch.bfloat16)
+    flat[: near.numel()] = near
+    rows[:, 0], rows[:, 1:] = 1.0, flat.view(-1, 31)
+    want = (rows.double().unsqueeze(-1) > mids).sum(-1)
+    S = rows.shape[0]
+    for pad in (0, 1):                                            # rows on 16 bytes, and off them
+        kv = torch.zeros(1, S, 64 + pad, dtype=torch.bfloat16, device=dev)
+        kv[0, :, :32] = kv[0, :, 32:64] = rows.to(dev)
+        c = PagedKVCache(1, 1, 32, 1, S + 16, dev, "oil4")
+        c.reserve(0, S)
+        c.append(0, kv[..., :32], kv[..., 32:64], [0], [0])
+        for pool, scale in ((c.k_pool, c.k_scale), (c.v_pool, c.v_scale)):
+            raw = pool[0][c._host_pages[0]].reshape(-1, 16)[:S].cpu()
+            assert torch.equal(torch.stack([raw & 15, raw >> 4], -1).view(S, 32).long(), want)
+            assert bool((scale[0][c._host_pages[0]].reshape(-1)[:S] == 1).all())
 
 
 def test_reserve_and_free_rows_as_one_by_one():
