@@ -5,9 +5,10 @@
 // warps take every eighth slice of K and meet in shared memory. Weights and activations go straight from global memory into
 // warp-level MMA fragments: a lane loads eight or sixteen consecutive k of a row and both operands read them in the same permuted
 // order, which a dot product does not notice. (A 128-row tcgen05 tile would be mostly padding here, and its tensor-memory set-up
-// and drain cost more than the whole product.) A warp keeps a ring of slices in registers, 64 KB per CTA and two CTAs per SM; the
-// ring is filled before the kernel waits for the previous one (resident weights; others are multiplied by a plainly launched kernel) and
-// refilled across tiles, so that the weights never stop flowing.
+// and drain cost more than the whole product.) A warp keeps a ring of slices in registers, 64 KB per CTA up to 32 rows and 32 KB above
+// (the accumulators of four row tiles take the rest), two CTAs per SM. It is filled before the kernel waits for the previous one
+// (resident weights; others are multiplied by a plainly launched kernel) and refilled across tiles, so that the weights never stop
+// flowing.
 //
 // SILU: W holds gate rows [0, N) and up rows [half, half + N); the output is silu(gate) * up.
 // cap > 0 (plain form): the output is cap * tanh(out / cap), the soft limit of logits.
