@@ -346,7 +346,8 @@ class TPDecoder:
         out = [tok]
         static_tok = tok.clone()
         if use_graph:
-            # The first time, a step runs on a side stream (allocations, lazy kernel attributes) and the state is restored. A capture takes
+            # The first time that a step has these sizes and this route, it runs on a side stream (lazy kernel attributes, accumulators that
+            # outlive the graph and must not come from its pool) and the state is restored. A capture takes
             # its buffers, one step's worth, from the pool of the one before it, which is never replayed again (torch.cuda.graph
             # empties the allocator's cache instead: 10 ms and more of a call in allocations). The pool stays with the decoder, except
             # with ranks, whose graphs end before their process group does. "relaxed": a garbage collection may free CUDA objects in
@@ -357,10 +358,11 @@ class TPDecoder:
             s = self._side
             s.wait_stream(torch.cuda.current_stream())
             with torch.cuda.stream(s):
-                if self.ctx is not None or (B, self._splits) not in self._warmed:
+                sizes = (B, self._splits, tuple(l[k].N for l in self.layers for k in ("qkv", "o", "gu", "down")), self.head.N, self._few(B))
+                if self.ctx is not None or sizes not in self._warmed:
                     self._decode_step(static_tok)
                     self.cache.seq_lens.copy_(saved)
-                    self._warmed.add((B, self._splits))
+                    self._warmed.add(sizes)
                 if self.ctx is not None:
                     self.ctx.turn = 0
                     self.ctx.xturn = 0

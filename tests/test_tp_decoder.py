@@ -128,6 +128,34 @@ def test_the_route_of_a_step_follows_its_weights():
     assert float((z.amax(-1) - z.gather(-1, got.unsqueeze(-1)).squeeze(-1)).max()) < 4 * LOGITS["bf16"] * float(z.std())
 
 
+@pytest.mark.parametrize("change", ["route", "width"])
+def test_no_accumulator_comes_from_a_capture(change, monkeypatch):
+    """A decoder whose step changes its route or a width after a call of the same batch: what the products keep for the process is
+    allocated before the capture, not in it."""
+    from innova_b200.ops import oil_linear as ol
+    from innova_b200.ops.oil_linear import quantize_weight
+    from innova_b200.parallel import tp
+    B, S = (2, 6) if change == "route" else (18, 10)       # prompts that do not allocate them either
+    dec, ids, taken = decoder("bf16"), tokens(B, S, 1), []
+    monkeypatch.setattr(ol, "_acc", {})
+
+    def spy(x, qw, M, make=ol._acc_for):
+        missing = (x.device.index, qw.N) not in ol._acc
+        taken.append(missing and torch.cuda.is_current_stream_capturing())
+        return make(x, qw, M)
+
+    monkeypatch.setattr(ol, "_acc_for", spy)
+    monkeypatch.setattr(tp, "_acc_for", spy)
+    dec.generate(ids, 2)
+    if change == "route":
+        q = dec.layers[0]["qkv"]
+        q.idx = torch.empty(q.idx.numel() + 16, dtype=torch.uint8, device="cuda")[16:].view_as(q.idx).copy_(q.idx)
+    else:
+        dec.layers[1]["gu"], dec.layers[1]["down"] = (quantize_weight(torch.randn(*s, device="cuda") / 16, "oil4") for s in ((1280, 256), (256, 640)))
+    dec.generate(ids, 1)
+    assert taken and not any(taken) and all(not a.any() for a in ol._acc.values())
+
+
 def test_a_collection_in_the_middle_of_a_capture():
     dec = decoder("bf16")
     ids = tokens(1, 12, 5)          # few enough for sums in a fixed order all the way
