@@ -222,7 +222,7 @@ class TPDecoder:
         few = self.world == 1 and B * S <= FEW_PROMPT_TOKENS
         h = ops.rms_norm(x, self.layers[0]["n1"], cfg.norm_eps)
         for li, l in enumerate(self.layers):
-            qkv = oil_linear(h, l["qkv"], resident=True) if few else ops.linear(h, l["qkv"].dequantize())
+            qkv = oil_linear(h, l["qkv"], resident=True) if few else ops.linear(h, l["qkv"].dequantize(), l["qkv"].bias)
             qkv = ops.rope_qk(qkv, self.rope[0], self.rope[1], H, Hkv, D)
             c.append(li, qkv[..., H * D:(H + Hkv) * D], qkv[..., (H + Hkv) * D:], rows, start)
             a = ops.flash_attention(qkv, H, Hkv, D, causal=True)
@@ -240,17 +240,17 @@ class TPDecoder:
             if self.world > 1:
                 o = ops.linear(a, l["o"].dequantize())
                 dist.all_reduce(o)
-                x = x + o
+                x = x + o if l["o"].bias is None else x + o + l["o"].bias
             else:
-                x = ops.linear(a, l["o"].dequantize(), residual=x, mode="add")
+                x = ops.linear(a, l["o"].dequantize(), l["o"].bias, residual=x, mode="add")
             h = ops.rms_norm(x, l["n2"], cfg.norm_eps)
-            act = ops.swiglu(ops.linear(h, l["gu"].dequantize()))
+            act = ops.swiglu(ops.linear(h, l["gu"].dequantize(), l["gu"].bias))
             if self.world > 1:
                 d = ops.linear(act, l["down"].dequantize())
                 dist.all_reduce(d)
-                x = x + d
+                x = x + d if l["down"].bias is None else x + d + l["down"].bias
             else:
-                x = ops.linear(act, l["down"].dequantize(), residual=x, mode="add")
+                x = ops.linear(act, l["down"].dequantize(), l["down"].bias, residual=x, mode="add")
             if nxt is not None:
                 h = ops.rms_norm(x, nxt, cfg.norm_eps)
         c.commit(rows, [S] * B)
