@@ -148,7 +148,7 @@ def test_no_accumulator_comes_from_a_capture(change, monkeypatch):
     monkeypatch.setattr(tp, "_acc_for", spy)
     dec.generate(ids, 2)
     if change == "route":
-        q = dec.layers[0]["qkv"]
+        q = dec.layers[0]["down"]
         q.idx = torch.empty(q.idx.numel() + 16, dtype=torch.uint8, device="cuda")[16:].view_as(q.idx).copy_(q.idx)
     else:
         dec.layers[1]["gu"], dec.layers[1]["down"] = (quantize_weight(torch.randn(*s, device="cuda") / 16, "oil4") for s in ((1280, 256), (256, 640)))
