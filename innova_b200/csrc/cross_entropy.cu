@@ -11,12 +11,13 @@
 namespace inv {
 
 constexpr int CE_THREADS = 512;
-constexpr float kL2E = 1.4426950408889634f, CE_LARGE = 1e38f;
+constexpr float kL2E = 1.4426950408889634f, CE_FLOOR = -131072.f, CE_LARGE = 91000.f;
 
+// The maximum in powers of two. No bf16 value lies within 300 of CE_FLOOR below it: what is held there adds nothing at all.
+__device__ __forceinline__ float ce_log2(float m) { return fmaxf(__fmul_rn(m, kL2E), CE_FLOOR); }
 // What a sum relative to the maximum m becomes relative to the maximum mn >= m.
 __device__ __forceinline__ float ce_ratio(float m, float mn) {
-  if (fmaxf(fabsf(m), fabsf(mn)) >= CE_LARGE) return exp2f((m - mn) * kL2E);
-  return exp2f(__fmul_rn(m, kL2E) - __fmul_rn(mn, kL2E));
+  return exp2f(ce_log2(m) - ce_log2(mn));
 }
 
 // logits: [T, ld] bf16, columns [V, ld) are padding. labels < 0 are ignored.
@@ -31,18 +32,18 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   const long label = labels[row];
   const int nvec = ld / 8, whole = V / 8;  // vectors of eight columns, those without padding
   // m is the maximum and mc = m * log2(e) as rounded: s sums 2^(x log2(e) - mc), and the logarithm below counts with the same mc.
-  // Above CE_LARGE in size (logits masked with their type's lowest value) the product is no longer finite, and s sums
-  // 2^((x - m) log2(e)) instead.
+  // Far from zero (masked logits) what the rounding takes is no longer small, nor the product finite: mc is held at CE_FLOOR, and
+  // columns below it add nothing. A row whose maximum is that large counts its maxima afterwards: bf16 values of that size lie at
+  // least 256 apart. (To sum them right as they come costs the loop its shape, with any test in it: 604 -> 624 us at the size below.)
   float m = -INFINITY, mc = 0.f, s = 0.f, sx = 0.f;
-  bool large = false;
   // A thread's vectors are read two at a time. Maximum on packed pairs, one fused multiply-add, one exponential and one addition per
-  // value: 16384 x 50257 in 674 us (a test per column and a sum of the logits nobody asked for: 740 us; the rows of the resident
+  // value: 16384 x 50257 in 604 us (a test per column and a sum of the logits nobody asked for: 740 us; the rows of the resident
   // CTAs stay in L2 for the second pass, so 500 us is what the bytes take).
   auto raise = [&](float to) {
-    s = m == -INFINITY ? 0.f : s * ce_ratio(m, to);
+    const float c = ce_log2(to);
+    s = m == -INFINITY ? 0.f : s * exp2f(mc - c);
     m = to;
-    mc = __fmul_rn(to, kL2E);
-    large = fabsf(to) >= CE_LARGE;
+    mc = c;
   };
   auto add = [&](const uint4& v) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -54,8 +55,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float lo = __uint_as_float(w[j] << 16), hi = __uint_as_float(w[j] & 0xffff0000u);
-      if (large) t += exp2f((lo - m) * kL2E) + exp2f((hi - m) * kL2E);
-      else t += exp2f(fmaf(lo, kL2E, -mc)) + exp2f(fmaf(hi, kL2E, -mc));
+      t += exp2f(fmaf(lo, kL2E, -mc)) + exp2f(fmaf(hi, kL2E, -mc));
       if (smoothing != 0.f) sx += lo + hi;
     }
     s += t;
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   if (threadIdx.x < V - whole * 8) {  // the columns before the padding, one per thread
     const float f = __bfloat162float(x[whole * 8 + threadIdx.x]);
     if (f > m) raise(f);
-    s += exp2f(large ? (f - m) * kL2E : fmaf(f, kL2E, -mc));
+    s += exp2f(fmaf(f, kL2E, -mc));
     if (smoothing != 0.f) sx += f;
   }
   // warp then block reduction of (m, s) pairs
@@ -114,9 +114,21 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   s = bc[1];
   sx = bc[2];
   mc = __fmul_rn(m, kL2E);
-  large = fabsf(m) >= CE_LARGE;
+  const bool large = fabsf(m) >= CE_LARGE;
+  if (large && fabsf(m) < INFINITY) {   // the same for all threads of the row
+    float n = 0.f;
+    for (int c = threadIdx.x; c < V; c += CE_THREADS) {
+      const float f = __bfloat162float(x[c]);
+      n += f == m ? 1.f : f < m ? 0.f : f;   // what is no number stays none
+    }
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    if (lane == 0) sm_s[warp] = n;
+    __syncthreads();
+    s = 0.f;
+    for (int w = 0; w < CE_THREADS / 32; ++w) s += sm_s[w];
+  }
   // the bracket gives back what the rounding of mc took, so that m is rounded once, in the last addition
-  const float lse = m + 0.6931471805599453f * (large ? __log2f(s) : __log2f(s) + fmaf(-m, kL2E, mc));
+  const float lse = m + 0.6931471805599453f * (__log2f(s) + (large ? 0.f : fmaf(-m, kL2E, mc)));
   const bool valid = label >= 0 && label < V;
   if (threadIdx.x == 0) {
     float l = 0.f;
@@ -159,7 +171,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   if (valid) {
     __syncthreads();
     if (threadIdx.x == 0) {
-      const float pl = exp2f(large ? (xl - m) * kL2E : fmaf(xl, kL2E, -mc)) / s;
+      const float pl = exp2f(large ? xl - m : fmaf(xl, kL2E, -mc)) / s;
       x[label] = __float2bfloat16((pl - smoothing / V - (1.f - smoothing)) * g);
     }
   }

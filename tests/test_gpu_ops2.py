@@ -445,17 +445,17 @@ def test_gpu_cross_entropy_rows(T, V, ld, smoothing):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("V,first", [(4099, 4096), (4096, 2048), (50257, 50000), (9, 8), (5, 4)])
-def test_gpu_cross_entropy_of_logits_masked_with_the_lowest_value(V, first):
-    """Columns at the type's lowest value count as masked, wherever a thread meets them (the product with log2(e) is not finite). The
-    bounds are those of the test above."""
+@pytest.mark.parametrize("mask", [torch.finfo(torch.bfloat16).min, -1e38, -1e20, -1e10, -1e9, -91136.0, -90624.0, -1e4])
+def test_gpu_cross_entropy_of_masked_logits(V, first, mask):
+    """Columns far below the others count as masked, wherever a thread meets them first: the type's lowest value, whose product with
+    log2(e) is not finite, and those whose product's rounding is large. The bounds are those of the test above."""
     from innova_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(V)
     lg = torch.zeros(3, (V + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)
-    low = torch.finfo(torch.bfloat16).min
     lg[:, :V] = torch.randn(3, V, device="cuda", generator=g) * 4
-    lg[0, :first] = low
-    lg[1, :V][torch.rand(V, device="cuda", generator=g) < 0.9] = low
-    lg[2, :V] = low
+    lg[0, :first] = mask
+    lg[1, :V][torch.rand(V, device="cuda", generator=g) < 0.9] = mask
+    lg[2, :V] = mask
     lg[:, V - 1] = 1.5
     labels = torch.full((3,), V - 1, device="cuda")
     ref = lg[:, :V].double().requires_grad_()
@@ -466,6 +466,26 @@ def test_gpu_cross_entropy_of_logits_masked_with_the_lowest_value(V, first):
     loss.backward()
     assert abs(float(loss.detach()) - float(want.detach())) < 1e-4
     assert float((x.grad[:, :V].double() - ref.grad).norm()) <= 4 * 2.0 ** -9 * float(ref.grad.norm()) + 2.0 ** -20
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("top", [torch.finfo(torch.bfloat16).min, -1e30, -1e10, -3e5, -91136.0, -90624.0, -65536.0, 65536.0, 90624.0, 91136.0, 1e10, 3e38])
+def test_gpu_cross_entropy_of_maxima_far_from_zero(top):
+    """log(sum exp) of rows that hold three values of a maximum far from zero and smaller ones, with and without what is no number; the
+    bound is one rounding (2^-24) and 2^-20 for the logarithm of small sums."""
+    from innova_b200.ops import runtime as rt
+    V = 4099
+    t = torch.tensor(top, device="cuda").bfloat16()
+    below = max(float(t) - max(abs(float(t)), 1e3), torch.finfo(torch.bfloat16).min) if top > -1e38 else float("-inf")
+    lg = torch.full((2, 4104), below, device="cuda").bfloat16()
+    lg[:, [0, 700, V - 1]] = t
+    lg[1, 900] = float("nan")
+    want = torch.logsumexp(lg[:, :V].double(), -1)
+    loss, lse = (torch.empty(2, device="cuda") for _ in range(2))
+    labels = torch.zeros(2, dtype=torch.int64, device="cuda")
+    rt.check(rt.lib().inv_cross_entropy(lg.data_ptr(), labels.data_ptr(), loss.data_ptr(), lse.data_ptr(), 2, V, 4104, 1.0, 0.0, 0, rt.stream_ptr()),
+             "inv_cross_entropy")
+    assert abs(float(lse[0].double() - want[0])) <= 2.0 ** -24 * abs(float(want[0])) + 2.0 ** -20 and bool(lse[1].isnan())
 
 
 @pytest.mark.gpu
