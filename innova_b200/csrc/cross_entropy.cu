@@ -34,10 +34,10 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   // m is the maximum and mc = m * log2(e) as rounded: s sums 2^(x log2(e) - mc), and the logarithm below counts with the same mc.
   // Far from zero (masked logits) what the rounding takes is no longer small, nor the product finite: mc is held at CE_FLOOR, and
   // columns below it add nothing. A row whose maximum is that large counts its maxima afterwards: bf16 values of that size lie at
-  // least 256 apart. (To sum them right as they come costs the loop its shape, with any test in it: 604 -> 624 us at the size below.)
+  // least 256 apart. (To sum them right as they come costs the loop its shape, with any test in it: 607 -> 625 us at the size below.)
   float m = -INFINITY, mc = 0.f, s = 0.f, sx = 0.f;
   // A thread's vectors are read two at a time. Maximum on packed pairs, one fused multiply-add, one exponential and one addition per
-  // value: 16384 x 50257 in 604 us (a test per column and a sum of the logits nobody asked for: 740 us; the rows of the resident
+  // value: 16384 x 50257 in 610 us (a test per column and a sum of the logits nobody asked for: 740 us; the rows of the resident
   // CTAs stay in L2 for the second pass, so 500 us is what the bytes take).
   auto raise = [&](float to) {
     const float c = ce_log2(to);
