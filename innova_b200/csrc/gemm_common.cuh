@@ -59,6 +59,8 @@ struct GemmParams {
 int make_tmap_2d_bf16(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner,
                       uint32_t box_outer);
 
+int make_tmap_2d_f32(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner, uint32_t box_outer);
+
 // One thread's 32 consecutive accumulator columns (row `row`, columns col0..col0+31) through the
 // fused epilogue and out to memory. `r` holds the raw fp32 bits read from TMEM.
 // bf16 results go either straight to global memory (stg_c == nullptr) or into this thread's 128-byte
@@ -67,17 +69,18 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_
 // `stg_in` (optional): this thread's 128-byte row of a box of the same shape and swizzle that a TMA load filled with
 // the epilogue's second operand (residual / pre-activation); it may be the same box as `stg_c` (each thread reads its
 // own 16-byte slots before it overwrites them).
-__device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& p, int row, bool row_ok, int col0, const uint32_t* r,
-                                                    uint8_t* stg_c = nullptr, uint8_t* stg_aux = nullptr, int sub = 0, int lane = 0,
-                                                    const uint8_t* stg_in = nullptr) {
+// `C` and `bias`: this unit's view of the output and the bias (grouped products shift them).
+__device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& p, void* C, const __nv_bfloat16* bias, int row, bool row_ok, int col0,
+                                                    const uint32_t* r, uint8_t* stg_c = nullptr, uint8_t* stg_aux = nullptr, int sub = 0,
+                                                    int lane = 0, const uint8_t* stg_in = nullptr) {
     float v[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
-    if (p.bias != nullptr) {
+    if (bias != nullptr) {
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
         if (col0 + g * 8 < p.N) {
-          uint4 bv = __ldg(reinterpret_cast<const uint4*>(p.bias + col0 + g * 8));
+          uint4 bv = __ldg(reinterpret_cast<const uint4*>(bias + col0 + g * 8));
           const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&bv);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -161,7 +164,7 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& p, int row
         }
       }
       if (p.c_f32) {
-        float* cp = reinterpret_cast<float*>(p.C) + (size_t)row * p.ldc + col0;
+        float* cp = reinterpret_cast<float*>(C) + (size_t)row * p.ldc + col0;
         if (p.epilogue == EPI_ATOMIC) {
 #pragma unroll
           for (int g = 0; g < 8; ++g) {
@@ -184,7 +187,7 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& p, int row
           }
         }
       } else {
-        __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)row * p.ldc + col0;
+        __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(C) + (size_t)row * p.ldc + col0;
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           if (col0 + g * 8 < p.N) {
@@ -201,6 +204,64 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& p, int row
     }
 }
 
+// The same for one fixed epilogue (EPI_NONE, EPI_GELU, EPI_ADD, EPI_GELU_DG, EPI_MUL; bf16 output through staging boxes): 32 columns from
+// registers into half `sub` of the box. Columns past N and rows past M are computed and clipped by the TMA store. `bv`: 32 columns of the
+// bias, or null. A tile with K = 256 has 2,050 cycles of products behind it; a box of 64 columns, two of which a warp writes per
+// tile, took 1,600 to 2,000 cycles with everything decided per chunk and the launch parameters copied to the stack, and takes 650 to
+// 800 in this form.
+template <int EPI>
+__device__ __forceinline__ void gemm_epilogue_fixed(float alpha, const uint4* bv, const uint32_t* r, uint8_t* stg_c, uint8_t* stg_aux, int sub,
+                                                    int lane) {
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[g * 8 + i]);
+    if (alpha != 1.f) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] *= alpha;
+    }
+    if (bv != nullptr) {
+      const uint32_t w[4] = {bv[g].x, bv[g].y, bv[g].z, bv[g].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v[2 * j] += __uint_as_float(w[j] << 16);
+        v[2 * j + 1] += __uint_as_float(w[j] & 0xffff0000u);
+      }
+    }
+    const uint32_t at = ((sub * 4 + g) ^ (lane & 7)) << 4;
+    if (EPI == EPI_GELU_DG) {
+      float d[8];
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) {
+        const float2 dd = gelu_tanh_grad_pair(v[i], v[i + 1]);
+        const float2 y = gelu_tanh_pair(v[i], v[i + 1]);   // the common subexpressions (clamp, cubic, tanh) are merged by the compiler
+        d[i] = dd.x; d[i + 1] = dd.y;
+        v[i] = y.x; v[i + 1] = y.y;
+      }
+      *reinterpret_cast<uint4*>(stg_aux + at) = make_uint4(pack_bf16x2(d[0], d[1]), pack_bf16x2(d[2], d[3]), pack_bf16x2(d[4], d[5]), pack_bf16x2(d[6], d[7]));
+    } else if (EPI == EPI_GELU) {
+      if (stg_aux)
+        *reinterpret_cast<uint4*>(stg_aux + at) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) {
+        const float2 y = gelu_tanh_pair(v[i], v[i + 1]);
+        v[i] = y.x; v[i + 1] = y.y;
+      }
+    } else if (EPI == EPI_ADD || EPI == EPI_MUL) {
+      const uint4 av = *reinterpret_cast<const uint4*>(stg_c + at);    // the second operand landed in the box the result leaves from
+      const uint32_t w[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float f0 = __uint_as_float(w[j] << 16), f1 = __uint_as_float(w[j] & 0xffff0000u);
+        v[2 * j] = EPI == EPI_ADD ? v[2 * j] + f0 : v[2 * j] * f0;
+        v[2 * j + 1] = EPI == EPI_ADD ? v[2 * j + 1] + f1 : v[2 * j + 1] * f1;
+      }
+    }
+    *reinterpret_cast<uint4*>(stg_c + at) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+  }
+}
+
 // TMA store of a shared-memory box (128B swizzle) into a 2-D bf16 tensor; rows / columns outside
 // the tensor are clipped by the hardware.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* smem_src, int c0, int c1) {
@@ -208,9 +269,16 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* s
                "r"(smem_u32(smem_src)), "r"(c0), "r"(c1)
                : "memory");
 }
+// The same box of fp32 values, added to what is there.
+__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* m, const void* smem_src, int c0, int c1) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(reinterpret_cast<uint64_t>(m)),
+               "r"(smem_u32(smem_src)), "r"(c0), "r"(c1)
+               : "memory");
+}
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Waits until the shared memory of every committed store group of this thread has been read.
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_read_but_one() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ----- fused all-gather: flags, bounded tile wait, copier CTAs (shared by the one- and two-CTA kernels) -----

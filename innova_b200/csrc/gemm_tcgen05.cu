@@ -93,7 +93,8 @@ __device__ __forceinline__ WorkUnit decode_work(int w, const GemmParams& p, int 
 
 template <bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                 const __grid_constant__ GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
@@ -146,7 +147,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one_sync()) {
       int it = 0;
       for (int w = bid; w < total_work; w += gdim) {
         WorkUnit u = decode_work(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
@@ -179,7 +180,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one_sync()) {
       const uint32_t idesc = make_idesc_bf16(BM, BN, A_MN ? 1u : 0u, B_MN ? 1u : 0u);
       // K-major, 128B swizzle: 8-row groups are 1024 B apart. MN-major (64-wide boxes of BK rows):
       // 64-element groups along MN are one box (8192 B) apart, 8-row groups along K 1024 B apart.
@@ -226,10 +227,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     for (int w = bid; w < total_work; w += gdim) {
       WorkUnit u = decode_work(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
       if (u.skip) continue;
-      GemmParams pe = p;  // this unit's view of the outputs (grouped modes shift bias / C)
+      void* C = p.C;                             // this unit's view of the outputs (grouped modes shift bias / C)
+      const __nv_bfloat16* bias = p.bias;
       if (p.group_mode) {
-        if (pe.bias) pe.bias += u.bias_off;
-        pe.C = p.c_f32 ? (void*)(reinterpret_cast<float*>(p.C) + u.c_off) : (void*)(reinterpret_cast<__nv_bfloat16*>(p.C) + u.c_off);
+        if (bias) bias += u.bias_off;
+        C = p.c_f32 ? (void*)(reinterpret_cast<float*>(p.C) + u.c_off) : (void*)(reinterpret_cast<__nv_bfloat16*>(p.C) + u.c_off);
       }
       const int acc = tile_i & 1;
       const uint32_t acc_ph = (tile_i >> 1) & 1;
@@ -239,7 +241,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       const bool row_ok = row < p.M;
       if (p.rs_world > 1) {  // this tile's rows belong to one owner: add into its buffer at the shard-relative row
         const int owner = u.m0 / p.rs_shard_rows;
-        pe.C = p.rs_dst[owner];
+        C = p.rs_dst[owner];
         row -= owner * p.rs_shard_rows;
       }
       const uint32_t t_row = tmem_base + acc * BN + (uint32_t(q * 32) << 16);
@@ -251,8 +253,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         tmem_ld_32x32(t_row + c * 32, r0);
         tmem_ld_32x32(t_row + c * 32 + 32, r1);
         tmem_ld_wait();
-        gemm_epilogue_chunk(pe, row, row_ok, col0, r0);
-        if (col0 + 32 < p.N) gemm_epilogue_chunk(pe, row, row_ok, col0 + 32, r1);
+        gemm_epilogue_chunk(p, C, bias, row, row_ok, col0, r0);
+        if (col0 + 32 < p.N) gemm_epilogue_chunk(p, C, bias, row, row_ok, col0 + 32, r1);
       }
       tc_fence_before();
       __syncwarp();
@@ -308,6 +310,19 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_
   CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -(int)r - 1000;
+}
+
+// The same over fp32 values.
+int make_tmap_2d_f32(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner, uint32_t box_outer) {
+  EncodeTiledFn enc = get_encode_fn();
+  if (!enc) return -1;
+  cuuint64_t dims[2] = {inner, outer};
+  cuuint64_t strides[1] = {ld * 4};
+  cuuint32_t box[2] = {box_inner, box_outer};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -(int)r - 1000;
 }
 

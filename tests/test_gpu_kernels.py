@@ -116,6 +116,41 @@ def test_gemm_second_operand_epilogues_tails(M, N, K):
     assert _rel_err(res, want) < 1e-2
 
 
+@pytest.mark.parametrize("M,N,K", [(129, 136, 72), (300, 264, 200), (2 * 74 * 256 + 33, 392, 64)])
+@pytest.mark.parametrize("a_mn,b_mn,epi", [(False, False, "NONE"), (False, False, "GELU"), (False, False, "ADD"), (False, False, "GELU_DG"),
+                                           (False, False, "ATOMIC"), (False, True, "NONE"), (False, True, "MUL"), (True, True, "ATOMIC")])
+def test_gemm_fixed_epilogues_stay_inside_their_view(a_mn, b_mn, epi, M, N, K):
+    """The CTA-pair kernels whose epilogue is compiled in: boxes that reach past the last row and column, outputs that are views of a wider
+    buffer (nothing around them is touched), bias, alpha, more tiles than pairs. bf16 results carry one rounding of 2^-9 (2^-8 with the
+    packed fp16 GELU); fp32 sums K * 2^-24."""
+    from innova_b200 import ops
+    torch.manual_seed(7)
+    dev = _dev()
+    Ma = (M + 7) // 8 * 8 if a_mn else M
+    A = (torch.randn(Ma, K, device=dev) * 0.5).bfloat16()
+    B = (torch.randn(N, K, device=dev) * 0.2).bfloat16()
+    bias = torch.randn(N, device=dev).bfloat16()
+    f32 = epi == "ATOMIC"
+    buf = torch.full((Ma + 3, N + 24), 3.0, device=dev, dtype=torch.float32 if f32 else torch.bfloat16)
+    out = buf[:Ma, 8:8 + N]
+    aux = torch.randn(Ma, N + 8, device=dev).bfloat16()[:, :N]
+    kw = dict(aux_in=aux) if epi in ("ADD", "MUL") else dict(aux_out=aux) if epi in ("GELU", "GELU_DG") else {}
+    aux_before = aux.float().clone()
+    use_bias = epi in ("NONE", "GELU", "ADD", "GELU_DG")
+    ops.gemm(A.t().contiguous() if a_mn else A, B.t().contiguous() if b_mn else B, out=out, a_mn=a_mn, b_mn=b_mn, epilogue=getattr(ops, "EPI_" + epi),
+             bias=bias if use_bias else None, alpha=0.5, **kw)
+    x = 0.5 * (A.double() @ B.double().t()) + (bias.double() if use_bias else 0.0)
+    xg = x.clone().requires_grad_(True)
+    y = F.gelu(xg, approximate="tanh")
+    y.sum().backward()
+    want = {"NONE": x, "ATOMIC": x + 3.0, "ADD": x + aux_before, "MUL": x * aux_before, "GELU": y.detach(), "GELU_DG": y.detach()}[epi]
+    assert _rel_err(out.double(), want) < (1e-5 if f32 else 4e-3)
+    if epi in ("GELU", "GELU_DG"):
+        assert _rel_err(aux.double(), x if epi == "GELU" else xg.grad) < 4e-3
+    buf[:Ma, 8:8 + N] = 3.0
+    assert (buf == 3.0).all()
+
+
 def test_gemm_wgrad_shape():
     """dW[N,K] += dY[T,N]^T X[T,K] with a long reduction and split-K chosen by the wrapper."""
     from innova_b200 import ops
