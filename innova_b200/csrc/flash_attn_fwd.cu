@@ -67,7 +67,7 @@ struct Fwd3Smem {
 template <int ND, bool EXT>
 __global__ void __launch_bounds__(FA_THREADS, ND == 1 ? 2 : 1)
 flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                  const __grid_constant__ CUtensorMap tmap_v, const FlashFwdParams p) {
+                  const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ FlashFwdParams p) {
   constexpr int D = 64 * ND;
   using L = Fwd3Smem<ND>;
   constexpr int SLOTS = L::SLOTS;
@@ -130,7 +130,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one_sync()) {
       mbar_expect_tx(q_full, L::TILE);
 #pragma unroll
       for (int a = 0; a < ND; ++a) tma_load_3d(sQ + a * 16384, &tmap_q, q_full, h * D + a * 64, row_base + q0, bz);
@@ -146,7 +146,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one_sync()) {
       const uint32_t idesc_qk = make_idesc_bf16(128, 128, 0, 0);
       const uint32_t idesc_pv = make_idesc_bf16(128, D, 0, 1);
       const uint32_t q_base = smem_u32(sQ);

@@ -43,7 +43,7 @@ constexpr int BK = 64;      // k-block: one A stage, one activation tile
 constexpr int STG_PITCH = 132;  // floats per token row of the epilogue staging tile (128 weight rows + 4: conflict-free both ways)
 constexpr int STG_TOK = 16;     // tokens per staging pass
 constexpr int MAX_IDX_STAGES = 6;
-constexpr int THREADS = 352;  // warp 0 TMA, warps 1 and 10 MMA issuers, warps 2-9 expand
+constexpr int THREADS = 384;  // warps 0 and 11 TMA, warps 1 and 10 MMA issuers, warps 2-9 expand
 constexpr int MAXM = 128;   // tokens per launch (MMA N); the host entry point splits larger M
 constexpr int A_COL0 = 256;  // TMEM: accumulators in [0,256) (per buffer and issuer), A slots in [256,512)
 }  // namespace og
@@ -166,7 +166,7 @@ __device__ long long og_trace_buf[16];
 
 template <int BITS>
 __global__ void __launch_bounds__(og::THREADS, 1)
-oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_constant__ CUtensorMap tmap_x, const OilGemmParams p) {
+oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ OilGemmParams p) {
   using namespace og;
   constexpr int KBB = BITS == 8 ? 2 : 4;           // k-blocks per index tile ("batch")
   constexpr int KB_BYTES = BK * BITS / 8;          // index bytes of one row in one k-block: 16, 32 or 64
@@ -235,8 +235,8 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
   [[maybe_unused]] bool og_once = false, og_once2 = false;
 
   if (warp == 0) {
-    // lane 0 streams index tiles, lane 1 streams activation tiles; each runs ahead on its own ring
-    if (lane == 0) {
+    // warp 0 streams index tiles, warp 11 activation tiles; each runs ahead on its own ring
+    if (elect_one_sync()) {
       int si = 0;
       uint32_t ph = 1;
       for (OgCursor c(n_tiles, nb, p.dp_rounds); c.valid; c.advance()) {
@@ -246,7 +246,9 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
         OG_STAMP_ONCE(2, og_once);
         if (++si == IDX_STAGES) { si = 0; ph ^= 1; }
       }
-    } else if (lane == 1) {
+    }
+  } else if (warp == 11) {
+    if (elect_one_sync()) {
       // Launched early, this grid may start while the kernel that produces the activations is still running.
       // Everything that touches only the (then resident) weights runs ahead: index tiles are fetched and expanded
       // into tensor memory; the activation loads, and with them the MMAs and the epilogue, wait here for the
@@ -264,12 +266,11 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
       }
     }
   } else if (warp == 1 || warp == 10) {
-    // Two MMA issuers, one per expanding group (a thread issues one tcgen05.mma per ~100 cycles whatever its size, so
-    // with 64 tokens per instruction a single issuer would be the bottleneck). Issuer g multiplies the batches of
-    // group g into its own accumulator; the epilogue adds the two. A thread runs at a few cycles per dependent
-    // instruction, so the loop is kept lean: one pair of waits and one commit per batch, descriptors advanced by
-    // additions.
-    if (lane == 0) {
+    // Two MMA issuers, one per expanding group: issuer g multiplies the batches of group g into its own accumulator, so that
+    // neither group waits for the other's tile; the epilogue adds the two. An elected thread issues (9 cycles per instruction with
+    // 16 tokens, where the branch "lane == 0" took 44: the compiler knows one thread and keeps descriptors in uniform registers).
+    // The loop is kept lean: one pair of waits and one commit per batch, descriptors advanced by additions.
+    if (elect_one_sync()) {
       const int g = warp == 1 ? 0 : 1;
       const uint32_t idesc = make_idesc_bf16(128, p.Mpad, 0, 0);
       const uint64_t xdesc0 = make_smem_desc(smem_u32(sX), 16, 1024, 2) + (uint64_t)(g * KBB) * (uint32_t)(X_TILE >> 4);
@@ -600,7 +601,7 @@ __global__ void __launch_bounds__(256) oil_gemm_finish_norm_kernel(float* __rest
                                                                    const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ x_out,
                                                                    const __nv_bfloat16* __restrict__ w, float eps, __nv_bfloat16* __restrict__ h_out,
                                                                    int N, int ld_acc, int ld_x, int ld_res, int ld_h, int W, int rank,
-                                                                   HeadBarrier hb) {
+                                                                   const __grid_constant__ HeadBarrier hb) {
   constexpr int MAXV = 16;  // float4 groups per thread: 256 * 16 * 4 = 16384 columns
   release_next();
   wait_previous();
@@ -800,7 +801,8 @@ struct SlicePeers {
 // slice's sum of squares per row, clear the accumulator slice. One CTA per row.
 __global__ void __launch_bounds__(256) tp_slice_finish_push_kernel(float* __restrict__ acc, int ld_acc, const __nv_bfloat16* __restrict__ bias,
                                                                    const __nv_bfloat16* __restrict__ residual, int ld_res, SlicePeers peers,
-                                                                   int ld_x, int W, int rank, int c0, int cols, int M, HeadBarrier hb) {
+                                                                   int ld_x, int W, int rank, int c0, int cols, int M,
+                                                                   const __grid_constant__ HeadBarrier hb) {
   const int m = blockIdx.x;
   uint32_t epoch = 1;
   if (hb.state != nullptr) {  // every rank's GEMM has added its partial sums into this rank's accumulator slice
@@ -854,7 +856,7 @@ __global__ void __launch_bounds__(256) tp_slice_finish_push_kernel(float* __rest
 // h[m, :] = x[m, :] * rsqrt(sum_r sumsq[r][m] / N + eps) * w   (rows of the gathered residual stream)
 __global__ void __launch_bounds__(256) tp_norm_apply_kernel(const __nv_bfloat16* __restrict__ x, int ld_x, const float* __restrict__ sumsq, int W,
                                                             int M, const __nv_bfloat16* __restrict__ w, float eps, __nv_bfloat16* __restrict__ h,
-                                                            int ld_h, int N, int rank, HeadBarrier hb) {
+                                                            int ld_h, int N, int rank, const __grid_constant__ HeadBarrier hb) {
   const int m = blockIdx.x;
   uint32_t epoch = 1;
   if (hb.state != nullptr) {  // every rank's slice and sums of squares have landed in this rank's copy
