@@ -4,7 +4,7 @@
 // At a handful of tokens such a product is bound by latency: the weights of a layer of width 2048 are 25 MB, four microseconds. The
 // tcgen05 kernel (oil_gemm.cu) pays for tensor memory, two barrier rings, reductions into a cleared accumulator and a finish
 // kernel of its own, 9 us a projection however small it is. Here a CTA owns 16 weight rows (8 gate and 8 up rows in the gated
-// form) and its eight warps take every eighth 256-wide slice of K straight from memory into registers: a lane loads two blocks of 32
+// form) and its eight or sixteen warps take every eighth or sixteenth 256-wide slice of K straight from memory into registers: a lane loads two blocks of 32
 // codes of a row (one whole 32-byte sector of the 4-bit format) with their scales, expands them through the lookup table and feeds
 // warp-level MMA fragments (weights are the 16-row side, tokens the 8-column side; both read k in the same permuted order, which a
 // dot product does not notice). Sums meet in shared memory, in one fixed order. Resident weights are requested before the
@@ -16,7 +16,7 @@
 namespace inv {
 
 namespace os {
-constexpr int WARPS = 8, THREADS = 32 * WARPS, ROWS = 16, SLICE = 256;
+constexpr int ROWS = 16, SLICE = 256;
 enum Mode { PLAIN = 0, SWIGLU = 1, SUMS = 2 };   // bf16 with bias and residual; silu(gate) * up; fp32 sums
 }  // namespace os
 
@@ -58,10 +58,11 @@ __device__ __forceinline__ void os_load(const uint8_t* p, uint32_t* w) {
   }
 }
 
-// MT: 8-token tiles.
-template <int BITS, int MT>
-__global__ void __launch_bounds__(os::THREADS, 2) oil_skinny_kernel(const OilSkinnyParams p) {
+// MT: 8-token tiles; WARPS: 8, two CTAs an SM, or 16.
+template <int BITS, int MT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) oil_skinny_kernel(const OilSkinnyParams p) {
   using namespace os;
+  constexpr int THREADS = 32 * WARPS;
   constexpr int UN = BITS == 8 ? 1 : 2;              // slices whose codes are in flight together
   constexpr int PL = MT * 8 + 1;                     // pitch of a row's partial sums
   extern __shared__ uint4 os_smem[];
@@ -233,22 +234,30 @@ __global__ void __launch_bounds__(os::THREADS, 2) oil_skinny_kernel(const OilSki
   }
 }
 
-template <int BITS, int MT>
-static int launch_oil_skinny(const OilSkinnyParams& p, bool early, cudaStream_t st) {
-  using namespace os;
-  const int slices = (p.K + SLICE - 1) / SLICE;
-  const int smem = slices * 128 * (4 * p.M + 1) + WARPS * ROWS * (MT * 8 + 1) * 4;
+template <int BITS, int MT, int WARPS>
+static int launch_oil_skinny(const OilSkinnyParams& p, bool early, int smem, cudaStream_t st) {
   static int limit = 0;
   if (limit == 0) {
-    const cudaError_t e = cudaFuncSetAttribute(oil_skinny_kernel<BITS, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 190 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(oil_skinny_kernel<BITS, MT, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 190 * 1024);
     if (e != cudaSuccess) return -(int)e;
     limit = 190 * 1024;
   }
   if (smem > limit) return -ERR_BAD_ARG;
-  const int per_sm = 2 * (smem + (BITS == 2 ? 3 : 35) * 1024) <= 226 * 1024 ? 2 : 1;
-  launch_step(early, oil_skinny_kernel<BITS, MT>, dim3(p.n_tiles < 148 * per_sm ? p.n_tiles : 148 * per_sm), THREADS, smem, st, p);
+  const int per_sm = WARPS == 8 && 2 * (smem + (BITS == 2 ? 3 : 35) * 1024) <= 226 * 1024 ? 2 : 1;
+  launch_step(early, oil_skinny_kernel<BITS, MT, WARPS>, dim3(p.n_tiles < 148 * per_sm ? p.n_tiles : 148 * per_sm), WARPS * 32, smem, st, p);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
+}
+// Sixteen warps where a tile has an SM to itself and more slices than eight warps: all of its weights are then in flight at once and the
+// expansion, which is bound by instruction issue, has four warps a scheduler (2048 x 5632: eight tokens 6.5 -> 5.5 us, one token alike, 4.3).
+// With several tiles an SM two CTAs of eight warps do the same and overlap their reductions.
+template <int BITS, int MT>
+static int launch_oil_skinny(const OilSkinnyParams& p, bool early, cudaStream_t st) {
+  using namespace os;
+  const int slices = (p.K + SLICE - 1) / SLICE;
+  const int x = slices * 128 * (4 * p.M + 1), sums = ROWS * (MT * 8 + 1) * 4;
+  if (p.n_tiles <= 148 && slices > 8 && x + 16 * sums <= 190 * 1024) return launch_oil_skinny<BITS, MT, 16>(p, early, x + 16 * sums, st);
+  return launch_oil_skinny<BITS, MT, 8>(p, early, x + 8 * sums, st);
 }
 
 }  // namespace inv

@@ -160,6 +160,93 @@ __global__ void __launch_bounds__(256) kv_append_rows_kernel(const __nv_bfloat16
   }
 }
 
+// What a decode step does with one head of a token's QKV projection (fp32 sums, a warp; lane l owns the elements l + 32 j, so that a rotation
+// pair (e, e + D / 2) sits in one thread): add the bias, round to bf16 as the stand-alone finish pass does, rotate query and key heads
+// (half-split RoPE at position `pos`). Queries stay with the caller; key and value heads go to their slot of the paged cache (OIL4: block-32
+// abs-max scale + nearest of the 16 levels; or bf16). `clear`: the sums are an accumulator that is zero between calls.
+struct QkvFinish {
+  float* acc;
+  int ld_acc;
+  const __nv_bfloat16* bias;
+  const float *cos_t, *sin_t;
+  int H, Hkv;
+  int clear;
+};
+template <int D>
+__device__ __forceinline__ void qkv_head(const QkvFinish& f, int b, int slot, int pos, int lane, float (&v)[D / 32]) {
+  constexpr int NJ = D / 32, HALFJ = NJ / 2;
+  float* arow = f.acc + (size_t)b * f.ld_acc + slot * D;
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) v[j] = arow[lane + 32 * j];
+  float cs[HALFJ], sn[HALFJ];
+  const bool turns = slot < f.H + f.Hkv;
+  if (turns) {
+#pragma unroll
+    for (int j = 0; j < HALFJ; ++j) {
+      cs[j] = f.cos_t[(size_t)pos * (D / 2) + lane + 32 * j];
+      sn[j] = f.sin_t[(size_t)pos * (D / 2) + lane + 32 * j];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    if (f.clear) arow[lane + 32 * j] = 0.f;
+    if (f.bias) v[j] += __bfloat162float(f.bias[slot * D + lane + 32 * j]);
+    v[j] = __bfloat162float(__float2bfloat16_rn(v[j]));
+  }
+  if (turns) {
+#pragma unroll
+    for (int j = 0; j < HALFJ; ++j) {
+      const float x1 = v[j], x2 = v[j + HALFJ];
+      v[j] = __bfloat162float(__float2bfloat16_rn(x1 * cs[j] - x2 * sn[j]));
+      v[j + HALFJ] = __bfloat162float(__float2bfloat16_rn(x1 * sn[j] + x2 * cs[j]));
+    }
+  }
+}
+template <bool OIL4, int D>
+__device__ __forceinline__ void kv_store_head(const float (&v)[D / 32], long row, uint8_t* pool, __half* scales, int lane) {
+  constexpr int NJ = D / 32;
+  if (!OIL4) {
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(pool) + row * D;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) dst[lane + 32 * j] = __float2bfloat16_rn(v[j]);
+    return;
+  }
+  __half* sc = scales + row * (D / 32);
+  uint8_t* dst = pool + row * (D / 2);
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    float amax = fabsf(v[j]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float scale = amax < 1e-10f ? 1.f : amax;
+    const int code = nearest_level16(v[j] / scale);
+    const int hi = __shfl_down_sync(0xffffffffu, code, 1);
+    if ((lane & 1) == 0) dst[j * 16 + (lane >> 1)] = (uint8_t)(code | (hi << 4));
+    if (lane == 0) sc[j] = __float2half_rn(scale);
+  }
+}
+// A CTA's share of it in front of its attention: the G query heads of key head hk of token b into `sq` (bf16 values in fp32, times
+// `mult`), the key and the value head into the cache, where the barrier behind it lets the CTA's own loads see them.
+template <bool OIL4, int D>
+__device__ __forceinline__ void qkv_heads_of_group(const QkvFinish& f, int b, int hk, int G, int pos, const int* page_table, int max_pages,
+                                                   uint8_t* k_pool, uint8_t* v_pool, __half* k_scale, __half* v_scale, float mult, float* sq) {
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  for (int i = threadIdx.x >> 5; i < G + 2; i += warps) {
+    const int which = G + 1 - i;                       // 0 value, 1 key, then the queries: the stores start first
+    const int slot = which == 0 ? f.H + f.Hkv + hk : which == 1 ? f.H + hk : hk * G + which - 2;
+    float v[D / 32];
+    qkv_head<D>(f, b, slot, pos, lane, v);
+    if (which >= 2) {
+#pragma unroll
+      for (int j = 0; j < D / 32; ++j) sq[(which - 2) * D + lane + 32 * j] = v[j] * mult;
+    } else {
+      const int page = page_table[(long)b * max_pages + pos / PAGE];
+      kv_store_head<OIL4, D>(v, ((long)page * f.Hkv + hk) * PAGE + pos % PAGE, which ? k_pool : v_pool, which ? k_scale : v_scale, lane);
+    }
+  }
+  __syncthreads();
+}
+
 // Rows of a token tree. Without it, query row b is the newest token of sequence b and sees seq_lens[b] cached tokens.
 // With it, query row b belongs to sequence row_seq[b] (several rows may share one), sees every cached token below
 // tail_start[b], and of the at most 64 tokens from tail_start[b] on only those whose bit is set in tail_mask[b]
@@ -173,51 +260,57 @@ __device__ __forceinline__ bool token_visible(int tok, int len, int tail0, unsig
   return tok < len && (tok < tail0 || ((tail_bits >> ((tok - tail0) & 63)) & 1ull));
 }
 
-// Decode attention over a bf16 cache: one query token per sequence. grid = (splits, Hkv, B), 128 threads, a warp per 16-token page.
-// With one split the result goes straight to `out_direct`, else partial (m, l, o[G][D]) per (b, hk, split) go to scratch and
-// attn_combine_kernel finishes. Short contexts are bound by the chain of loads, so a page's keys and values are all requested
-// before the scores are computed (a loop over the tokens with one load each took 17 us at one sequence of 32 to 96 tokens).
-template <int D>
-__global__ void __launch_bounds__(128) paged_decode_kernel(const __nv_bfloat16* __restrict__ q, int ld_q, const int* __restrict__ page_table,
-                                                           int max_pages, const int* __restrict__ seq_lens, int H, int Hkv,
-                                                           const uint8_t* __restrict__ k_pool, const uint8_t* __restrict__ v_pool, float scale,
-                                                           float* __restrict__ part, int splits, __nv_bfloat16* __restrict__ out_direct, int ld_o,
-                                                           TreeRows tree) {
-  constexpr int MAXG = 8;
+// Decode attention over a bf16 cache: one query token per sequence. grid = (splits, Hkv, B), a warp per 16-token page. With one split the
+// result goes straight to `out_direct`, else partial (m, l, o[G][D]) per (b, hk, split) go to scratch and attn_combine_kernel
+// finishes. Short contexts are bound by the chain of loads, so a page's keys and values are all requested before the scores are
+// computed, and sixteen warps take a page each where CTAs are few. GQ: the heads of a group that registers are kept for (1, 2, 4 or 8).
+// FUSED (one split, no tree): the kernel starts from the fp32 sums of the QKV projection and does that pass's finish itself
+// (qkv_heads_of_group). Finish and attention of 16 heads on 4, one sequence
+// of 64 tokens: 9.5 -> 6.6 us, of 190: 19.4 -> 8.6; 64 sequences of 544: 88 -> 53 us (before: four warps, sums indexed at run time and so on the stack).
+template <int D, int NW, int GQ, bool FUSED>
+__global__ void __launch_bounds__(NW * 32) paged_decode_kernel(const __nv_bfloat16* __restrict__ q, int ld_q, const int* __restrict__ page_table,
+                                                               int max_pages, const int* __restrict__ seq_lens, int H, int Hkv,
+                                                               uint8_t* k_pool, uint8_t* v_pool, float scale, float* __restrict__ part, int splits,
+                                                               __nv_bfloat16* __restrict__ out_direct, int ld_o,
+                                                               const __grid_constant__ TreeRows tree, const __grid_constant__ QkvFinish fin) {
   constexpr int EPL = D / 32;  // output elements per lane
   constexpr int HALF = D / 2;  // elements per lane in the QK phase (two lanes per token)
   using VRaw = typename std::conditional<EPL == 4, uint2, uint32_t>::type;
   release_next();  // the output projection may start on its weights
   wait_previous();
-  __shared__ float sq[MAXG][D];
-  __shared__ float sm_m[4][MAXG], sm_l[4][MAXG];
-  __shared__ float sm_o[4][MAXG][D];
+  __shared__ __align__(16) float sq[GQ][D];
+  __shared__ float sm_m[NW][GQ], sm_l[NW][GQ];
+  __shared__ float sm_o[NW][GQ][D];
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int G = H / Hkv;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int seq = tree.row_seq ? tree.row_seq[b] : b;
+  const int seq = !FUSED && tree.row_seq ? tree.row_seq[b] : b;
   const int len = seq_lens[seq];
-  const int tail0 = tree.tail_start ? tree.tail_start[b] : len;
-  const unsigned long long tail_bits = tree.tail_mask ? tree.tail_mask[b] : 0ull;
+  const int tail0 = !FUSED && tree.tail_start ? tree.tail_start[b] : len;
+  const unsigned long long tail_bits = !FUSED && tree.tail_mask ? tree.tail_mask[b] : 0ull;
   const int npages = (len + PAGE - 1) / PAGE;
   const int per = (npages + splits - 1) / splits;
   const int p0 = split * per, p1 = min(npages, p0 + per);
   const float c = scale * 1.4426950408889634f;
-  for (int i = threadIdx.x; i < G * D; i += blockDim.x) {
-    const int g = i / D, e = i % D;
-    sq[g][e] = __bfloat162float(q[(long)b * ld_q + (hk * G + g) * D + e]) * c;
+  if (FUSED) {
+    qkv_heads_of_group<false, D>(fin, b, hk, G, len - 1, page_table, max_pages, k_pool, v_pool, nullptr, nullptr, c, &sq[0][0]);
+  } else {
+    for (int i = threadIdx.x; i < G * D; i += blockDim.x) {
+      const int g = i / D, e = i % D;
+      sq[g][e] = __bfloat162float(q[(long)b * ld_q + (hk * G + g) * D + e]) * c;
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  float m[MAXG], l[MAXG], o[MAXG][EPL];
+  float m[GQ], l[GQ], o[GQ][EPL];
 #pragma unroll
-  for (int g = 0; g < MAXG; ++g) {
+  for (int g = 0; g < GQ; ++g) {
     m[g] = -INFINITY;
     l[g] = 0.f;
 #pragma unroll
     for (int e = 0; e < EPL; ++e) o[g][e] = 0.f;
   }
   const int t = lane & 15, hf = lane >> 4;
-  for (int pg = p0 + warp; pg < p1; pg += 4) {
+  for (int pg = p0 + warp; pg < p1; pg += NW) {
     const int page = page_table[(long)seq * max_pages + pg];
     const long row0 = ((long)page * Hkv + hk) * PAGE;
     // ---- loads: scores' lane = (token t, half hf); in the values a lane owns elements [lane * EPL, lane * EPL + EPL) ----
@@ -230,41 +323,43 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const __nv_bfloat16* 
 #pragma unroll
     for (int tt = 0; tt < PAGE; ++tt) vraw[tt] = *reinterpret_cast<const VRaw*>(vp + tt * D);
     const bool valid = token_visible(pg * PAGE + t, len, tail0, tail_bits);
-    float pr[MAXG], alpha[MAXG];
+    float pr[GQ];
 #pragma unroll
-    for (int g = 0; g < MAXG; ++g) {
+    for (int g = 0; g < GQ; ++g) {
+      pr[g] = 0.f;
       if (g < G) {
-        float s = 0.f;
-        const float* qg = &sq[g][hf * HALF];
+        float s0 = 0.f, s1 = 0.f;
+        const float4* qg = reinterpret_cast<const float4*>(&sq[g][hf * HALF]);
 #pragma unroll
         for (int j = 0; j < HALF / 8; ++j) {
-          const uint32_t w[4] = {kraw[j].x, kraw[j].y, kraw[j].z, kraw[j].w};
-#pragma unroll
-          for (int n = 0; n < 4; ++n) {
-            s += __uint_as_float(w[n] << 16) * qg[j * 8 + 2 * n];
-            s += __uint_as_float(w[n] & 0xffff0000u) * qg[j * 8 + 2 * n + 1];
-          }
+          const float4 q0 = qg[2 * j], q1 = qg[2 * j + 1];
+          s0 += __uint_as_float(kraw[j].x << 16) * q0.x;
+          s1 += __uint_as_float(kraw[j].x & 0xffff0000u) * q0.y;
+          s0 += __uint_as_float(kraw[j].y << 16) * q0.z;
+          s1 += __uint_as_float(kraw[j].y & 0xffff0000u) * q0.w;
+          s0 += __uint_as_float(kraw[j].z << 16) * q1.x;
+          s1 += __uint_as_float(kraw[j].z & 0xffff0000u) * q1.y;
+          s0 += __uint_as_float(kraw[j].w << 16) * q1.z;
+          s1 += __uint_as_float(kraw[j].w & 0xffff0000u) * q1.w;
         }
+        float s = s0 + s1;
         s += __shfl_xor_sync(0xffffffffu, s, 16);
         s = valid ? s : -INFINITY;
         float mx = s;
 #pragma unroll
         for (int off = 8; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
         const float m_new = fmaxf(m[g], mx);
-        alpha[g] = m[g] == -INFINITY ? 0.f : exp2f(m[g] - m_new);
+        const float alpha = m[g] == -INFINITY ? 0.f : exp2f(m[g] - m_new);
         pr[g] = (s == -INFINITY) ? 0.f : exp2f(s - m_new);
         float ps = pr[g];
 #pragma unroll
         for (int off = 8; off > 0; off >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, off);
-        l[g] = l[g] * alpha[g] + ps;
+        l[g] = l[g] * alpha + ps;
         m[g] = m_new;
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) o[g][e] *= alpha;
       }
     }
-#pragma unroll
-    for (int g = 0; g < MAXG; ++g)
-      if (g < G)
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) o[g][e] *= alpha[g];
     const int ntok = min(PAGE, len - pg * PAGE);  // slots past the sequence's end hold whatever was there
 #pragma unroll
     for (int tt = 0; tt < PAGE; ++tt) {
@@ -277,7 +372,7 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const __nv_bfloat16* 
           vf[e + 1] = __uint_as_float(w[e / 2] & 0xffff0000u);
         }
 #pragma unroll
-        for (int g = 0; g < MAXG; ++g)
+        for (int g = 0; g < GQ; ++g)
           if (g < G) {
             const float pt = __shfl_sync(0xffffffffu, pr[g], tt);
 #pragma unroll
@@ -286,23 +381,27 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const __nv_bfloat16* 
       }
     }
   }
-  // ---- fold the 4 warps ----
-  for (int g = 0; g < G; ++g) {
-    if (lane == 0) {
-      sm_m[warp][g] = m[g];
-      sm_l[warp][g] = l[g];
-    }
+  // ---- fold the warps ----
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) sm_o[warp][g][lane * EPL + e] = o[g][e];
+  for (int g = 0; g < GQ; ++g) {
+    if (g < G) {
+      if (lane == 0) {
+        sm_m[warp][g] = m[g];
+        sm_l[warp][g] = l[g];
+      }
+#pragma unroll
+      for (int e = 0; e < EPL; ++e) sm_o[warp][g][lane * EPL + e] = o[g][e];
+    }
   }
   __syncthreads();
+  const int used = min(NW, max(1, p1 - p0));         // warps that have seen a page (the first one in any case)
   float* out = part + (((long)b * Hkv + hk) * splits + split) * (long)G * (D + 2);
   for (int i = threadIdx.x; i < G * D; i += blockDim.x) {
     const int g = i / D, e = i % D;
     float mm = -INFINITY;
-    for (int w = 0; w < 4; ++w) mm = fmaxf(mm, sm_m[w][g]);
+    for (int w = 0; w < used; ++w) mm = fmaxf(mm, sm_m[w][g]);
     float acc = 0.f, ll = 0.f;
-    for (int w = 0; w < 4; ++w) {
+    for (int w = 0; w < used; ++w) {
       const float f = sm_m[w][g] == -INFINITY ? 0.f : exp2f(sm_m[w][g] - mm);
       acc += sm_o[w][g][e] * f;
       ll += sm_l[w][g] * f;
@@ -339,13 +438,15 @@ __device__ __forceinline__ void mma_16816(float* d, const uint32_t* a, uint32_t 
 __device__ __forceinline__ uint32_t h2_as_u32(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
 __device__ __forceinline__ __half2 u32_as_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
 
-template <int D, int NW>
+// FUSED: as in the kernel above, from the sums of the QKV projection (64 sequences of 544 tokens: finish and attention 19.7 -> 16.1 us).
+template <int D, int NW, bool FUSED>
 __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32)) paged_decode_oil4_mma_kernel(const __nv_bfloat16* __restrict__ q, int ld_q, const int* __restrict__ page_table,
                                                                     int max_pages, const int* __restrict__ seq_lens, int H, int Hkv,
-                                                                    const uint8_t* __restrict__ k_pool, const uint8_t* __restrict__ v_pool,
-                                                                    const __half* __restrict__ k_scale, const __half* __restrict__ v_scale,
+                                                                    uint8_t* k_pool, uint8_t* v_pool, __half* k_scale, __half* v_scale,
                                                                     float scale, float* __restrict__ part, int splits,
-                                                                    __nv_bfloat16* __restrict__ out_direct, int ld_o, TreeRows tree) {
+                                                                    __nv_bfloat16* __restrict__ out_direct, int ld_o,
+                                                                    const __grid_constant__ TreeRows tree,
+                                                                    const __grid_constant__ QkvFinish fin) {
   constexpr int MAXG = 8;
   constexpr int KCH = D / 4;        // d-values of a K row per lane (one quarter of the row)
   constexpr int KW = KCH / 8;       // ... as 32-bit words of indices (4 for D = 128)
@@ -362,33 +463,41 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32)) paged_decode_oil4_mm
     const uint32_t v = h2_as_u32(__floats2half2_rn(c_kv_levels[e & 15], c_kv_levels[e >> 4]));
     *reinterpret_cast<uint4*>(&lut[i4 * 4]) = make_uint4(v, v, v, v);
   }
+  __shared__ __align__(16) float sq[FUSED ? MAXG * D : 4];
   wait_previous();  // the table is built while the queries are still being written
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int G = H / Hkv;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gid = lane >> 2, tig = lane & 3;
-  const int seq = tree.row_seq ? tree.row_seq[b] : b;
+  const int seq = !FUSED && tree.row_seq ? tree.row_seq[b] : b;
   const int len = seq_lens[seq];
-  const int tail0 = tree.tail_start ? tree.tail_start[b] : len;
-  const unsigned long long tail_bits = tree.tail_mask ? tree.tail_mask[b] : 0ull;
+  const int tail0 = !FUSED && tree.tail_start ? tree.tail_start[b] : len;
+  const unsigned long long tail_bits = !FUSED && tree.tail_mask ? tree.tail_mask[b] : 0ull;
   const int npages = (len + PAGE - 1) / PAGE;
   const int per = (npages + splits - 1) / splits;
   const int p0 = split * per, p1 = min(npages, p0 + per);
   const float c = scale * 1.4426950408889634f;
+  if (FUSED) qkv_heads_of_group<true, D>(fin, b, hk, G, len - 1, page_table, max_pages, k_pool, v_pool, k_scale, v_scale, c, sq);
   // Q fragment: row gid = query head, this lane's d-quarter; rows 8..15 of the MMA are zero
   uint32_t qa[KSTEPS][2];
   {
-    const __nv_bfloat16* qrow = q + (long)b * ld_q + (hk * G + min(gid, G - 1)) * D + tig * KCH;
+    const int head = min(gid, G - 1);
+    const __nv_bfloat16* qrow = FUSED ? nullptr : q + (long)b * ld_q + (hk * G + head) * D + tig * KCH;
 #pragma unroll
     for (int st = 0; st < KSTEPS; ++st) {
-      const uint2 raw = *reinterpret_cast<const uint2*>(qrow + st * 4);
-      const float f0 = __uint_as_float(raw.x << 16) * c, f1 = __uint_as_float(raw.x & 0xffff0000u) * c;
-      const float f2 = __uint_as_float(raw.y << 16) * c, f3 = __uint_as_float(raw.y & 0xffff0000u) * c;
-      qa[st][0] = gid < G ? h2_as_u32(__floats2half2_rn(f0, f1)) : 0u;
-      qa[st][1] = gid < G ? h2_as_u32(__floats2half2_rn(f2, f3)) : 0u;
+      float4 f;
+      if (FUSED) {
+        f = *reinterpret_cast<const float4*>(sq + head * D + tig * KCH + st * 4);
+      } else {
+        const uint2 raw = *reinterpret_cast<const uint2*>(qrow + st * 4);
+        f = make_float4(__uint_as_float(raw.x << 16) * c, __uint_as_float(raw.x & 0xffff0000u) * c, __uint_as_float(raw.y << 16) * c,
+                        __uint_as_float(raw.y & 0xffff0000u) * c);
+      }
+      qa[st][0] = gid < G ? h2_as_u32(__floats2half2_rn(f.x, f.y)) : 0u;
+      qa[st][1] = gid < G ? h2_as_u32(__floats2half2_rn(f.z, f.w)) : 0u;
     }
   }
-  __syncthreads();
+  if (!FUSED) __syncthreads();
   float m_run = -INFINITY, l_run = 0.f;  // of head gid; l is this lane's share (its 4 tokens per page)
   float o[VMMA][4];
 #pragma unroll
@@ -609,77 +718,34 @@ extern "C" int inv_kv_append(const void* k_new, const void* v_new, int ld_k, int
 }
 
 namespace inv {
-// Decode-step finish of the QKV projection: one pass over the fp32 accumulator [B, (H + 2 Hkv) D] that adds the bias,
-// rounds to bf16 (as the stand-alone finish pass does), rotates the query and key heads (half-split RoPE at the token's
-// position), writes the queries as bf16 and appends the key / value heads to the paged cache (OIL4: block-32 abs-max
-// scale + nearest of the 16 levels; or bf16), and clears the accumulator. Replaces three launches per layer.
-// One warp per (token, head slot); lane l owns elements l + 32 j, so a rotation pair (e, e + D/2) sits in one thread.
+// Decode-step finish of the QKV projection where the attention is split over several CTAs a head: one pass over the fp32 accumulator
+// [B, (H + 2 Hkv) D], one warp per (token, head slot), that writes the queries as bf16, appends keys and values and clears the accumulator.
 template <bool OIL4, int D>
-__global__ void __launch_bounds__(256) decode_qkv_finish_kernel(float* __restrict__ acc, int ld_acc, const __nv_bfloat16* __restrict__ bias,
-                                                                const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                                                const int* __restrict__ pos, const int* __restrict__ page_table, int max_pages,
-                                                                int B, int H, int Hkv, __nv_bfloat16* __restrict__ q_out, int ld_q,
-                                                                uint8_t* __restrict__ k_pool, uint8_t* __restrict__ v_pool,
-                                                                __half* __restrict__ k_scale, __half* __restrict__ v_scale) {
-  constexpr int NJ = D / 32, HALFJ = NJ / 2;
+__global__ void __launch_bounds__(256) decode_qkv_finish_kernel(const __grid_constant__ QkvFinish fin, const int* __restrict__ pos,
+                                                                const int* __restrict__ page_table, int max_pages, int B,
+                                                                __nv_bfloat16* __restrict__ q_out, int ld_q, uint8_t* __restrict__ k_pool,
+                                                                uint8_t* __restrict__ v_pool, __half* __restrict__ k_scale,
+                                                                __half* __restrict__ v_scale) {
   release_next();
   wait_previous();
   const int lane = threadIdx.x & 31;
   const long warp_id = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int slots = H + 2 * Hkv;
+  const int slots = fin.H + 2 * fin.Hkv;
   if (warp_id >= (long)B * slots) return;
   const int slot = (int)(warp_id % slots), b = (int)(warp_id / slots);
-  float* arow = acc + (size_t)b * ld_acc + slot * D;
-  float v[NJ];
-#pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    const int e = lane + 32 * j;
-    float x = arow[e];
-    arow[e] = 0.f;
-    if (bias) x += __bfloat162float(bias[slot * D + e]);
-    v[j] = __bfloat162float(__float2bfloat16_rn(x));
-  }
   const int p = pos[b];
-  if (slot < H + Hkv) {  // query and key heads rotate
-#pragma unroll
-    for (int j = 0; j < HALFJ; ++j) {
-      const int i = lane + 32 * j;
-      const float c = cos_t[(size_t)p * (D / 2) + i], sn = sin_t[(size_t)p * (D / 2) + i];
-      const float x1 = v[j], x2 = v[j + HALFJ];
-      v[j] = __bfloat162float(__float2bfloat16_rn(x1 * c - x2 * sn));
-      v[j + HALFJ] = __bfloat162float(__float2bfloat16_rn(x1 * sn + x2 * c));
-    }
-  }
-  if (slot < H) {
+  float v[D / 32];
+  qkv_head<D>(fin, b, slot, p, lane, v);
+  if (slot < fin.H) {
     __nv_bfloat16* qo = q_out + (size_t)b * ld_q + slot * D;
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) qo[lane + 32 * j] = __float2bfloat16_rn(v[j]);
+    for (int j = 0; j < D / 32; ++j) qo[lane + 32 * j] = __float2bfloat16_rn(v[j]);
     return;
   }
-  const int which = slot >= H + Hkv;  // 0 = key, 1 = value
-  const int hk = slot - H - which * Hkv;
+  const int which = slot >= fin.H + fin.Hkv;  // 0 = key, 1 = value
+  const int hk = slot - fin.H - which * fin.Hkv;
   const int page = page_table[(long)b * max_pages + p / PAGE];
-  const long row = ((long)page * Hkv + hk) * PAGE + p % PAGE;
-  uint8_t* pool = which ? v_pool : k_pool;
-  if (!OIL4) {
-    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(pool) + row * D;
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) dst[lane + 32 * j] = __float2bfloat16_rn(v[j]);
-    return;
-  }
-  __half* sc = (which ? v_scale : k_scale) + row * (D / 32);
-  uint8_t* dst = pool + row * (D / 2);
-#pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    float amax = fabsf(v[j]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float scale = amax < 1e-10f ? 1.f : amax;
-    const int code = nearest_level16(v[j] / scale);
-    const int hi = __shfl_down_sync(0xffffffffu, code, 1);
-    if ((lane & 1) == 0) dst[j * 16 + (lane >> 1)] = (uint8_t)(code | (hi << 4));
-    if (lane == 0) sc[j] = __float2half_rn(scale);
-  }
+  kv_store_head<OIL4, D>(v, ((long)page * fin.Hkv + hk) * PAGE + p % PAGE, which ? v_pool : k_pool, which ? v_scale : k_scale, lane);
 }
 
 }  // namespace inv
@@ -692,10 +758,10 @@ extern "C" int inv_decode_qkv_finish(float* acc, int ld_acc, const void* bias, c
   const long warps = (long)B * (H + 2 * Hkv);
   const int grid = (int)((warps + 7) / 8);
   cudaStream_t st = (cudaStream_t)stream;
+  const QkvFinish fin{acc, ld_acc, (const __nv_bfloat16*)bias, cos_t, sin_t, H, Hkv, 1};
 #define INV_DQF(O, DD)                                                                                                                      \
-  launch_early(decode_qkv_finish_kernel<O, DD>, dim3(grid), 256, 0, st, acc, ld_acc, (const __nv_bfloat16*)bias, cos_t, sin_t, pos, page_table, max_pages, B, \
-                                                        H, Hkv, (__nv_bfloat16*)q_out, ld_q, (uint8_t*)k_pool, (uint8_t*)v_pool,             \
-                                                        (__half*)k_scale, (__half*)v_scale)
+  launch_early(decode_qkv_finish_kernel<O, DD>, dim3(grid), 256, 0, st, fin, pos, page_table, max_pages, B, (__nv_bfloat16*)q_out, ld_q,    \
+               (uint8_t*)k_pool, (uint8_t*)v_pool, (__half*)k_scale, (__half*)v_scale)
   if (oil4) {
     if (D == 64) INV_DQF(true, 64); else INV_DQF(true, 128);
   } else {
@@ -709,36 +775,52 @@ extern "C" int inv_decode_qkv_finish(float* acc, int ld_acc, const void* bias, c
 // Scratch floats needed by inv_paged_decode.
 extern "C" long inv_paged_decode_scratch_floats(int B, int H, int D, int splits) { return (long)B * H * splits * (D + 2); }
 
+// fin: the kernel finishes the QKV projection itself (one split, no tree), or null.
 static int paged_decode_impl(const void* q, int ld_q, const int* page_table, int max_pages, const int* seq_lens, int B, int H, int Hkv, int D,
-                             const void* k_pool, const void* v_pool, const void* k_scale, const void* v_scale, int oil4, float scale,
-                             void* out, int ld_o, float* scratch, int splits, TreeRows tree, void* stream) {
-  if ((D != 64 && D != 128) || H % Hkv || H / Hkv > 8 || splits < 1) return -ERR_BAD_ARG;
+                             void* k_pool, void* v_pool, void* k_scale, void* v_scale, int oil4, float scale, void* out, int ld_o, float* scratch,
+                             int splits, TreeRows tree, const QkvFinish* fin, void* stream) {
+  if ((D != 64 && D != 128) || Hkv < 1 || H % Hkv || H / Hkv > 8 || splits < 1) return -ERR_BAD_ARG;
   if (B <= 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
   dim3 grid(splits, Hkv, B);
-#define INV_PD(DD)                                                                                                                         \
-  launch_early(paged_decode_kernel<DD>, grid, 128, 0, st, (const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H, Hkv,                    \
-                                                (const uint8_t*)k_pool, (const uint8_t*)v_pool, scale, scratch, splits,                    \
-                                                splits == 1 ? (__nv_bfloat16*)out : nullptr, ld_o, tree)
+  const long ctas = (long)splits * Hkv * B;
+  const QkvFinish f = fin ? *fin : QkvFinish{};
+  const int G = H / Hkv;
   if (oil4) {
     // Four warps per CTA and four CTAs per SM, or, where all CTAs fit at two per SM, eight warps: half the chain of pages (64
     // sequences, 4 KV heads, 512 to 576 tokens). At batch 64, 8 KV heads, 640 tokens the two are alike, 35.7 us.
-    const bool few = (long)splits * Hkv * B <= 148 * 2;
-#define INV_PD4(DD, NW)                                                                                                                    \
-  launch_early(paged_decode_oil4_mma_kernel<DD, NW>, grid, NW * 32, 0, st, (const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H, Hkv,      \
-                                                             (const uint8_t*)k_pool, (const uint8_t*)v_pool, (const __half*)k_scale,       \
-                                                             (const __half*)v_scale, scale, scratch, splits,                                \
-                                                             splits == 1 ? (__nv_bfloat16*)out : nullptr, ld_o, tree)
-    if (few) {
-      if (D == 64) INV_PD4(64, 8); else INV_PD4(128, 8);
+#define INV_PD4(DD, NW, FU)                                                                                                                \
+  launch_early(paged_decode_oil4_mma_kernel<DD, NW, FU>, grid, NW * 32, 0, st, (const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H,  \
+               Hkv, (uint8_t*)k_pool, (uint8_t*)v_pool, (__half*)k_scale, (__half*)v_scale, scale, scratch, splits,                          \
+               splits == 1 ? (__nv_bfloat16*)out : nullptr, ld_o, tree, f)
+#define INV_PD4_D(NW, FU)                                                                                                                  \
+  if (D == 64) INV_PD4(64, NW, FU); else INV_PD4(128, NW, FU)
+    if (ctas <= 148 * 2) {
+      if (fin) { INV_PD4_D(8, true); } else { INV_PD4_D(8, false); }
     } else {
-      if (D == 64) INV_PD4(64, 4); else INV_PD4(128, 4);
+      if (fin) { INV_PD4_D(4, true); } else { INV_PD4_D(4, false); }
     }
+#undef INV_PD4_D
 #undef INV_PD4
   } else {
-    if (D == 64) INV_PD(64); else INV_PD(128);
+    // Sixteen warps (eight with more than four heads a group: their sums share 48 KB) where a CTA has an SM to itself, else four.
+#define INV_PD(DD, NW, GQ, FU)                                                                                                             \
+  launch_early(paged_decode_kernel<DD, NW, GQ, FU>, grid, NW * 32, 0, st, (const __nv_bfloat16*)q, ld_q, page_table, max_pages, seq_lens, H, Hkv,   \
+               (uint8_t*)k_pool, (uint8_t*)v_pool, scale, scratch, splits, splits == 1 ? (__nv_bfloat16*)out : nullptr, ld_o, tree, f)
+#define INV_PD_G(DD, FU)                                                                                                                   \
+  if (ctas <= 148) {                                                                                                                       \
+    if (G == 1) INV_PD(DD, 16, 1, FU); else if (G == 2) INV_PD(DD, 16, 2, FU); else if (G <= 4) INV_PD(DD, 16, 4, FU); else INV_PD(DD, 8, 8, FU); \
+  } else {                                                                                                                                 \
+    if (G == 1) INV_PD(DD, 4, 1, FU); else if (G == 2) INV_PD(DD, 4, 2, FU); else if (G <= 4) INV_PD(DD, 4, 4, FU); else INV_PD(DD, 4, 8, FU);    \
   }
+    if (fin) {
+      if (D == 64) { INV_PD_G(64, true) } else { INV_PD_G(128, true) }
+    } else {
+      if (D == 64) { INV_PD_G(64, false) } else { INV_PD_G(128, false) }
+    }
+#undef INV_PD_G
 #undef INV_PD
+  }
   if (splits == 1) {  // the kernel wrote the final output
     cudaError_t e1 = cudaGetLastError();
     return e1 == cudaSuccess ? 0 : -(int)e1;
@@ -754,8 +836,9 @@ static int paged_decode_impl(const void* q, int ld_q, const int* page_table, int
 extern "C" int inv_paged_decode(const void* q, int ld_q, const int* page_table, int max_pages, const int* seq_lens, int B, int H, int Hkv, int D,
                                 const void* k_pool, const void* v_pool, const void* k_scale, const void* v_scale, int oil4, float scale,
                                 void* out, int ld_o, float* scratch, int splits, void* stream) {
-  return paged_decode_impl(q, ld_q, page_table, max_pages, seq_lens, B, H, Hkv, D, k_pool, v_pool, k_scale, v_scale, oil4, scale, out, ld_o,
-                           scratch, splits, TreeRows{nullptr, nullptr, nullptr}, stream);
+  return paged_decode_impl(q, ld_q, page_table, max_pages, seq_lens, B, H, Hkv, D, const_cast<void*>(k_pool), const_cast<void*>(v_pool),
+                           const_cast<void*>(k_scale), const_cast<void*>(v_scale), oil4, scale, out, ld_o, scratch, splits,
+                           TreeRows{nullptr, nullptr, nullptr}, nullptr, stream);
 }
 
 // Attention of T query rows over shared sequences with a per-row visibility mask over the newest (at most 64) tokens:
@@ -767,6 +850,18 @@ extern "C" int inv_paged_decode_tree(const void* q, int ld_q, const int* page_ta
                                      const void* k_pool, const void* v_pool, const void* k_scale, const void* v_scale, int oil4, float scale,
                                      void* out, int ld_o, float* scratch, int splits, void* stream) {
   if (row_seq == nullptr || tail_start == nullptr || tail_mask == nullptr) return -ERR_BAD_ARG;
-  return paged_decode_impl(q, ld_q, page_table, max_pages, seq_lens, T, H, Hkv, D, k_pool, v_pool, k_scale, v_scale, oil4, scale, out, ld_o,
-                           scratch, splits, TreeRows{row_seq, tail_start, tail_mask}, stream);
+  return paged_decode_impl(q, ld_q, page_table, max_pages, seq_lens, T, H, Hkv, D, const_cast<void*>(k_pool), const_cast<void*>(v_pool),
+                           const_cast<void*>(k_scale), const_cast<void*>(v_scale), oil4, scale, out, ld_o, scratch, splits,
+                           TreeRows{row_seq, tail_start, tail_mask}, nullptr, stream);
+}
+
+// The finish of the QKV projection and the attention of a decode step in one launch, one CTA per (key head, sequence): sums fp32
+// [B, (H + 2 Hkv) D] (+ bias), the new token of sequence b at position seq_lens[b] - 1. clear: the sums are set to zero. Shapes as
+// for inv_paged_decode; each key head's keys and values are read by the CTA that wrote them.
+extern "C" int inv_decode_attend(float* sums, int ld_sums, const void* bias, const float* cos_t, const float* sin_t, int clear, const int* page_table,
+                                 int max_pages, const int* seq_lens, int B, int H, int Hkv, int D, void* k_pool, void* v_pool, void* k_scale,
+                                 void* v_scale, int oil4, float scale, void* out, int ld_o, void* stream) {
+  const QkvFinish fin{sums, ld_sums, (const __nv_bfloat16*)bias, cos_t, sin_t, H, Hkv, clear};
+  return paged_decode_impl(nullptr, 0, page_table, max_pages, seq_lens, B, H, Hkv, D, k_pool, v_pool, k_scale, v_scale, oil4, scale, out, ld_o, nullptr, 1,
+                           TreeRows{nullptr, nullptr, nullptr}, &fin, stream);
 }

@@ -272,6 +272,14 @@ class TPDecoder:
         c, B = self.cache, pos.shape[0]
         H, Hkv, D = self.H, self.Hkv, self.D
         lib, st = rt.lib(), rt.stream_ptr()
+        if self._splits == 1:
+            # one CTA walks a head's pages: it finishes the projection of its own heads too
+            a = torch.empty(B, H * D, dtype=torch.bfloat16, device=self.dev)
+            rt.check(lib.inv_decode_attend(sums.data_ptr(), sums.stride(0), rt.ptr(self.layers[li]["qkv"].bias), self.rope[0].data_ptr(),
+                                           self.rope[1].data_ptr(), 1, c.page_table.data_ptr(), c.max_pages, c.seq_lens.data_ptr(), B, H, Hkv, D,
+                                           c.k_pool[li].data_ptr(), c.v_pool[li].data_ptr(), rt.ptr(c.k_scale[li]), rt.ptr(c.v_scale[li]),
+                                           int(c.fmt == "oil4"), float(D ** -0.5), a.data_ptr(), a.stride(0), st), "inv_decode_attend")
+            return a
         q2 = torch.empty(B, H * D, dtype=torch.bfloat16, device=self.dev)
         rt.check(lib.inv_decode_qkv_finish(sums.data_ptr(), sums.stride(0), rt.ptr(self.layers[li]["qkv"].bias), self.rope[0].data_ptr(),
                                            self.rope[1].data_ptr(), pos.data_ptr(), c.page_table.data_ptr(), c.max_pages, B, H, Hkv, D, q2.data_ptr(),

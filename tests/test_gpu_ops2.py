@@ -586,3 +586,58 @@ def test_gpu_head_loss_with_a_scale_per_token():
         (nll * scale.double().expand(T, 1).view(-1)).sum().div(T).backward()
         for a, b in ((x, xr), (w, wr)):
             assert float((a.grad.double() - b.grad).norm() / b.grad.norm()) < 2e-2
+
+
+@pytest.mark.parametrize("fmt", ["bf16", "oil4"])
+@pytest.mark.parametrize("B,H,Hkv,D,lens", [(1, 16, 4, 128, [1]), (1, 16, 4, 128, [17]), (3, 4, 4, 64, [16, 33, 300]), (2, 24, 8, 64, [15, 190]),
+                                            (5, 8, 1, 128, [2, 31, 32, 48, 257]), (40, 8, 8, 64, None), (76, 8, 4, 128, None), (20, 14, 2, 128, None)])
+def test_projection_finish_and_attention_in_one_launch(fmt, B, H, Hkv, D, lens):
+    """``inv_decode_attend`` against the two launches it stands for (same queries, keys and values: the cache to the bit) and fp64 attention
+    over the cache as it is stored; groups of 1 to 8 heads, contexts around page edges, few and many CTAs, with and without a bias."""
+    from innova_b200.inference.kv_cache import PagedKVCache
+    from innova_b200.ops import rope_tables
+    from innova_b200.ops import runtime as rt
+    torch.manual_seed(B * 31 + H)
+    lens = lens or [1 + (37 * i) % 203 for i in range(B)]
+    W, scale = (H + 2 * Hkv) * D, D ** -0.5
+    cos, sin = rope_tables(512, D, 10000.0, torch.device(DEV))
+    sums = torch.randn(B, W, device=DEV)
+    bias = torch.randn(W, device=DEV).bfloat16() if B % 2 else None
+    old = torch.randn(B, max(lens), 2 * Hkv * D, device=DEV).bfloat16()
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV)
+    lib, st = rt.lib(), rt.stream_ptr()
+
+    def cache():
+        c = PagedKVCache(1, Hkv, D, B, 512, torch.device(DEV), fmt)
+        for p in (c.k_pool[0], c.v_pool[0]):
+            p.zero_()                                       # slots that nothing wrote compare equal
+        c.reserve_rows(range(B), 512)
+        c.append(0, old[..., :Hkv * D], old[..., Hkv * D:], list(range(B)), [0] * B)
+        for b, n in enumerate(lens):
+            c.commit([b], [n])
+        return c
+
+    a, b = cache(), cache()
+    q = torch.empty(B, H * D, dtype=torch.bfloat16, device=DEV)
+    two, one = torch.empty_like(q), torch.full_like(q, float("nan"))
+    s2, s1 = sums.clone(), sums.clone()
+    pools = [(c.k_pool[0].data_ptr(), c.v_pool[0].data_ptr(), rt.ptr(c.k_scale[0]), rt.ptr(c.v_scale[0]), int(fmt == "oil4")) for c in (a, b)]
+    rt.check(lib.inv_decode_qkv_finish(s2.data_ptr(), W, rt.ptr(bias), cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), a.page_table.data_ptr(), a.max_pages,
+                                       B, H, Hkv, D, q.data_ptr(), q.stride(0), *pools[0], st), "finish")
+    rt.check(lib.inv_paged_decode(q.data_ptr(), q.stride(0), a.page_table.data_ptr(), a.max_pages, a.seq_lens.data_ptr(), B, H, Hkv, D, *pools[0], scale,
+                                  two.data_ptr(), two.stride(0), 0, 1, st), "attend")
+    rt.check(lib.inv_decode_attend(s1.data_ptr(), W, rt.ptr(bias), cos.data_ptr(), sin.data_ptr(), 1, b.page_table.data_ptr(), b.max_pages,
+                                   b.seq_lens.data_ptr(), B, H, Hkv, D, *pools[1], scale, one.data_ptr(), one.stride(0), st), "both")
+    assert float(s1.abs().max()) == 0.0 and float(s2.abs().max()) == 0.0
+    assert torch.equal(a.k_pool[0], b.k_pool[0]) and torch.equal(a.v_pool[0], b.v_pool[0])
+    if fmt == "oil4":
+        assert torch.equal(a.k_scale[0], b.k_scale[0]) and torch.equal(a.v_scale[0], b.v_scale[0])
+    assert torch.equal(one, two)                            # the same arithmetic behind the same queries
+    if fmt == "bf16":
+        k, v = (p.view(torch.bfloat16).view(-1, Hkv, 16, D).double() for p in (b.k_pool[0], b.v_pool[0]))
+        for r, n in enumerate(lens):
+            pages = b.page_table[r, :(n + 15) // 16].long()
+            kk, vv = (t[pages].transpose(0, 1).reshape(Hkv, -1, D)[:, :n] for t in (k, v))
+            w = torch.softmax(torch.einsum("hgd,hnd->hgn", q[r].double().view(Hkv, H // Hkv, D), kk) * scale, -1)
+            want = torch.einsum("hgn,hnd->hgd", w, vv).reshape(-1)
+            assert float((one[r].double() - want).norm() / want.norm()) < 2.0 ** -8      # one rounding to bf16 of fp32 sums
