@@ -16,7 +16,7 @@
 //   warp 0    TMA: raw index tiles (128 rows x 256 k, swizzled) and activation tiles (M x 64 k, 128B swizzle)
 //   warp 1    MMA issuer: A operand from tensor memory, B (activations) from shared memory, two accumulators
 //             [128 weight rows x M tokens] fp32 in TMEM
-//   warps 2-9 dequantise, two groups of four warps on alternate index tiles: a thread owns a weight row, looks
+//   warps 2-17 dequantise, two groups of eight warps on alternate index tiles: a thread owns half of a weight row, looks
 //             the values up in a shared-memory table of bf16 pairs (OIL4: indexed by the byte, i.e. two weights
 //             per lookup), multiplies by the block scale with packed bf16 math and stores the row's 64 values
 //             per k-block into its lane of an A stage in tensor memory. The same warps run the epilogue.
@@ -41,9 +41,10 @@ namespace og {
 constexpr int BN = 128;     // weight rows per tile (MMA M)
 constexpr int BK = 64;      // k-block: one A stage, one activation tile
 constexpr int STG_PITCH = 132;  // floats per token row of the epilogue staging tile (128 weight rows + 4: conflict-free both ways)
-constexpr int STG_TOK = 16;     // tokens per staging pass
+constexpr int STG_TOK = 8;      // tokens per staging pass
 constexpr int MAX_IDX_STAGES = 6;
-constexpr int THREADS = 384;  // warps 0 and 11 TMA, warps 1 and 10 MMA issuers, warps 2-9 expand
+constexpr int EXPAND = 16;   // expanding warps, from warp 2 on: two groups of eight
+constexpr int THREADS = 32 * (EXPAND + 4);  // warps 0 and 19 TMA, warps 1 and 18 MMA issuers
 constexpr int MAXM = 128;   // tokens per launch (MMA N); the host entry point splits larger M
 constexpr int A_COL0 = 256;  // TMEM: accumulators in [0,256) (per buffer and issuer), A slots in [256,512)
 }  // namespace og
@@ -137,9 +138,10 @@ struct OgCursor {
   __device__ __forceinline__ OgCursor(int n_tiles, int nb_, int dp_rounds_) {
     nb = nb_; grid = gridDim.x; cta = blockIdx.x; dp_rounds = dp_rounds_;
     sk_tile0 = dp_rounds * grid;
-    const long long total = (long long)(n_tiles - sk_tile0) * nb;
-    sk_b = (int)(total * cta / grid);
-    sk_b1 = (int)(total * (cta + 1) / grid);
+    // the first `more` CTAs take one batch more (64-bit quotients total * cta / grid cost 1,500 cycles in front of every role's first action)
+    const unsigned total = (unsigned)(n_tiles - sk_tile0) * nb, each = total / (unsigned)grid, more = total - each * grid;
+    sk_b = (int)(cta * each + min((unsigned)cta, more));
+    sk_b1 = sk_b + (int)(each + (cta < (int)more ? 1 : 0));
     round = 0;
     next_segment();
   }
@@ -181,8 +183,8 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
   uint8_t* sX = smem;                                  // 2 slots x KBB activation tiles (X_TILE is a multiple of 2 KB)
   uint8_t* sIdx = sX + 2 * KBB * X_TILE;               // IDX_STAGES x IDX_TILE (swizzled by TMA: 1 KB aligned)
   __shared__ __align__(128) uint32_t lut[BITS == 2 ? 32 : 256 * 32];   // 256 entries x 32 bank copies, at a fixed address
-  float* stage = reinterpret_cast<float*>(sIdx + IDX_STAGES * IDX_TILE);  // epilogue staging: per group STG_TOK tokens x STG_PITCH
-  uint64_t* bars = reinterpret_cast<uint64_t*>(stage + 2 * STG_TOK * STG_PITCH);
+  float* stage = reinterpret_cast<float*>(sIdx + IDX_STAGES * IDX_TILE);  // epilogue staging: per half of a group STG_TOK tokens x STG_PITCH
+  uint64_t* bars = reinterpret_cast<uint64_t*>(stage + 4 * STG_TOK * STG_PITCH);
   uint64_t* idx_full = bars;
   uint64_t* idx_empty = idx_full + MAX_IDX_STAGES;
   uint64_t* a_full = idx_empty + MAX_IDX_STAGES;  // [2]: slot g holds the batch expanded by group g (KBB k-blocks, 32 TMEM columns each)
@@ -207,15 +209,15 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
   if (threadIdx.x == 0) {
     for (int s = 0; s < IDX_STAGES; ++s) {
       mbar_init(&idx_full[s], 1);
-      mbar_init(&idx_empty[s], 4);  // the four warps of the group that expanded the tile
+      mbar_init(&idx_empty[s], EXPAND / 2);  // the warps of the group that expanded the tile
     }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&a_full[s], 4);
+      mbar_init(&a_full[s], EXPAND / 2);
       mbar_init(&a_empty[s], 1);
       mbar_init(&x_full[s], 1);
       mbar_init(&acc_full[2 * s], 2);  // one commit per MMA issuer
       mbar_init(&acc_full[2 * s + 1], 2);
-      mbar_init(&acc_empty[s], 4);
+      mbar_init(&acc_empty[s], EXPAND / 2);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -235,7 +237,7 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
   [[maybe_unused]] bool og_once = false, og_once2 = false;
 
   if (warp == 0) {
-    // warp 0 streams index tiles, warp 11 activation tiles; each runs ahead on its own ring
+    // warp 0 streams index tiles, the last warp activation tiles; each runs ahead on its own ring
     if (elect_one_sync()) {
       int si = 0;
       uint32_t ph = 1;
@@ -247,7 +249,7 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
         if (++si == IDX_STAGES) { si = 0; ph ^= 1; }
       }
     }
-  } else if (warp == 11) {
+  } else if (warp == EXPAND + 3) {
     if (elect_one_sync()) {
       // Launched early, this grid may start while the kernel that produces the activations is still running.
       // Everything that touches only the (then resident) weights runs ahead: index tiles are fetched and expanded
@@ -265,7 +267,7 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
         for (int kk = 0; kk < nkb; ++kk) tma_load_2d(sX + (slot * KBB + kk) * X_TILE, &tmap_x, &x_full[slot], (kb0 + kk) * BK, 0);
       }
     }
-  } else if (warp == 1 || warp == 10) {
+  } else if (warp == 1 || warp == EXPAND + 2) {
     // Two MMA issuers, one per expanding group: issuer g multiplies the batches of group g into its own accumulator, so that
     // neither group waits for the other's tile; the epilogue adds the two. An elected thread issues (9 cycles per instruction with
     // 16 tokens, where the branch "lane == 0" took 44: the compiler knows one thread and keeps descriptors in uniform registers).
@@ -314,38 +316,41 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
       }
       if (g == 0) OG_STAMP(7);
     }
-  } else if (warp >= 2 && warp < 10) {
+  } else {
     // lookup table: OIL4 -> bf16 pair (codebook[low nibble], codebook[high nibble]) per byte; OIL8 -> one bf16
     // entry e for lane l lives at lut[e * 32 + l]: every lane reads its own bank, whatever the indices are
     const int q = warp & 3;
-    const int grp = (warp - 2) >> 2;
+    const int grp = (warp - 2) >> 3, sub = ((warp - 2) >> 2) & 1;   // group; which half of a tile's k-blocks and of the tokens
     const int r = q * 32 + lane;        // weight row inside the tile = TMEM lane
     const int nsb = p.K / 32;           // scale blocks per weight row
     const unsigned short* scales = reinterpret_cast<const unsigned short*>(p.scales);
     // block scales of a batch are fetched one own batch (two batches) ahead of their use
-    unsigned short sc_next[2 * KBB];
+    constexpr int KBS = KBB / 2;        // k-blocks of a batch that this thread expands, from sub * KBS on
+    unsigned short sc_next[2 * KBS];
     auto fetch_scales = [&](int t, int bbx) {
-      const int kb0 = bbx * KBB;
+      const int kb0 = bbx * KBB + sub * KBS;
       const unsigned short* row = scales + (size_t)min(t * BN + r, p.N - 1) * nsb + kb0 * 2;
 #pragma unroll
-      for (int j = 0; j < 2 * KBB; ++j) sc_next[j] = (kb0 * 2 + j < nsb) ? __ldg(row + j) : (unsigned short)0;
+      for (int j = 0; j < 2 * KBS; ++j) sc_next[j] = (kb0 * 2 + j < nsb) ? __ldg(row + j) : (unsigned short)0;
     };
     OgCursor pc(n_tiles, nb, p.dp_rounds);  // runs one own batch ahead of the main cursor
     if (grp == 1 && pc.valid) pc.advance();
     if (pc.valid) fetch_scales(pc.tile, pc.bb);  // in flight while the table is built
     if (BITS != 2) {
-      oil_lut_fill<BITS>(lut, cb, threadIdx.x - 64, 256);
-      asm volatile("bar.sync 1, 256;" ::: "memory");
+      oil_lut_fill<BITS>(lut, cb, threadIdx.x - 64, EXPAND * 32);
+      asm volatile("bar.sync 1, %0;" ::"n"(EXPAND * 32) : "memory");
     }
     if (threadIdx.x == 64) OG_STAMP(4);
     // ---------------- dequantise + epilogue ----------------
-    // Two groups of four warps take alternate batches, so that one group's waits and barrier traffic overlap the
-    // other group's table lookups. A thread owns weight row r of the tile: it reads the row's index bytes of the
-    // whole batch, expands one k-block at a time into 32 registers of packed bf16 and stores them into its lane
-    // of the A stage in tensor memory (the MMA reads A from there: no shared-memory round trip).
+    // Two groups of eight warps take alternate batches, so that one group's waits and barrier traffic overlap the
+    // other group's table lookups. A thread owns half of weight row r of the tile: it reads the row's index bytes of half of
+    // the batch's k-blocks, expands one k-block at a time into 32 registers of packed bf16 and stores them into its lane
+    // of the A stage in tensor memory (the MMA reads A from there: no shared-memory round trip). With four warps a group a scheduler
+    // had two, which table lookups left idle two cycles in three (issue slots 29 % used): 64 tokens, 11264 x 2048: 16.4 -> 12.6 us
+    // with the shorter set-up of OgCursor, 2048 x 5632 11.3 -> 8.6; 77 tokens, 22016 x 4096: 37.7 -> 32.5.
     const uint32_t t_lane = tmem_base + (uint32_t(q * 32) << 16);
-    float* stg = stage + grp * (STG_TOK * STG_PITCH);
-    [[maybe_unused]] const int gt = threadIdx.x - 64 - grp * 128;  // thread index inside the group
+    float* stg = stage + (grp * 2 + sub) * (STG_TOK * STG_PITCH);
+    [[maybe_unused]] const int gt = threadIdx.x - 64 - grp * (EXPAND * 16);  // thread index inside the group
     const bool vec_ok = ((p.ldo & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
     const int nbuf = p.Mpad <= 64 ? 2 : 1, accw = p.Mpad <= 64 ? 64 : 128;
     int seg = 0, lb = 0;
@@ -355,32 +360,32 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
       const int nkb = min(KBB, kb_total - c.bb * KBB);
       const bool seg_end = c.seg_last();
       if ((lb & 1) == grp) {
-        unsigned short sc[2 * KBB];
+        unsigned short sc[2 * KBS];
 #pragma unroll
-        for (int j = 0; j < 2 * KBB; ++j) sc[j] = sc_next[j];
+        for (int j = 0; j < 2 * KBS; ++j) sc[j] = sc_next[j];
         if (pc.valid) pc.advance();
         if (pc.valid) pc.advance();
         if (pc.valid) fetch_scales(pc.tile, pc.bb);
         const int si = lb % IDX_STAGES;
         if (!mbar_wait_warp(&idx_full[si], (lb / IDX_STAGES) & 1, abort_flag, p.status, ERR_WAIT_FULL)) { ok = false; break; }
         if (threadIdx.x == 64) OG_STAMP_ONCE(5, og_once);
-        uint4 raw[ROW_CHUNKS];
+        uint4 raw[ROW_CHUNKS / 2];
         {
           const uint8_t* src = sIdx + si * IDX_TILE + r * ROWB;
           const int swz = (ROWB == 128) ? (r & 7) : ((r >> 1) & 3);  // the TMA swizzle of a 128- / 64-byte row
 #pragma unroll
-          for (int ch = 0; ch < ROW_CHUNKS; ++ch) raw[ch] = *reinterpret_cast<const uint4*>(src + ((ch ^ swz) << 4));
+          for (int ch = 0; ch < ROW_CHUNKS / 2; ++ch) raw[ch] = *reinterpret_cast<const uint4*>(src + (((sub * (ROW_CHUNKS / 2) + ch) ^ swz) << 4));
         }
         // group g owns A slot g: free once the MMAs of this group's previous batch have completed
         if (!mbar_wait_warp(&a_empty[grp], ((lb >> 1) & 1) ^ 1, abort_flag, p.status, ERR_WAIT_EMPTY)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < KBB; ++kk) {
-          if (kk < nkb) {
+        for (int kk = 0; kk < KBS; ++kk) {
+          if (sub * KBS + kk < nkb) {
             uint32_t o[32];
             const __nv_bfloat16_raw r0{sc[2 * kk]}, r1{sc[2 * kk + 1]};
             expand_row<BITS>(raw + kk * KB_CHUNKS, __nv_bfloat16(r0), __nv_bfloat16(r1), lut, cb, lane, o);
-            tmem_st_32x32(t_lane + A_COL0 + (grp * KBB + kk) * 32, o);
+            tmem_st_32x32(t_lane + A_COL0 + (grp * KBB + sub * KBS + kk) * 32, o);
           }
         }
         // The tile is released only here: every index byte has been used as a table address by now. An arrival right after
@@ -393,7 +398,7 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
         if (lane == 0) mbar_arrive(&a_full[grp]);  // one arrival per warp
         if (seg_end) {
           // ---- segment end: accumulator [weight row (lane), token (column)] -> out[token][tile * 128 + row] ----
-          // The tile is transposed through shared memory 32 tokens at a time, so that a thread ends up with four
+          // The tile is transposed through shared memory eight tokens at a time, the halves of the group in turn, so that a thread ends up with four
           // consecutive weight rows of one token: one 16-byte store (whole tile) or vector reduction per thread.
           const bool full = c.seg_full() && p.multimem == 0;
           const int buf = nbuf == 2 ? (seg & 1) : 0, use = nbuf == 2 ? (seg >> 1) : seg;
@@ -404,16 +409,16 @@ oil_gemm_kernel(const __grid_constant__ CUtensorMap tmap_idx, const __grid_const
           if (gt == 0) OG_STAMP_ONCE(8, og_once2);
           const uint32_t t_acc = t_lane + (buf * 2 + grp) * accw, t_other = t_lane + (buf * 2 + (grp ^ 1)) * accw;
           const bool both = c.bb1 - c.bb0 >= 2;  // the other issuer contributed to this segment too
-          for (int mh = 0; mh < p.Mpad; mh += STG_TOK) {
-            uint32_t v[16], v2[16];
-            tmem_ld_32x16(t_acc + mh, v);
-            if (both) tmem_ld_32x16(t_other + mh, v2);
+          for (int mh = sub * STG_TOK; mh < p.Mpad; mh += 2 * STG_TOK) {
+            uint32_t v[8], v2[8];
+            tmem_ld_32x8(t_acc + mh, v);
+            if (both) tmem_ld_32x8(t_other + mh, v2);
             tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) stg[j * STG_PITCH + r] = __uint_as_float(v[j]) + (both ? __uint_as_float(v2[j]) : 0.f);
+            for (int j = 0; j < 8; ++j) stg[j * STG_PITCH + r] = __uint_as_float(v[j]) + (both ? __uint_as_float(v2[j]) : 0.f);
             __syncwarp();  // a warp reads back only the 32 weight rows it wrote: no barrier across the group
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
+            for (int k = 0; k < 2; ++k) {
               const int e = k * 32 + lane, m = e >> 3, n4 = q * 32 + (e & 7) * 4;
               const int gm = mh + m, n = c.tile * BN + n4;
               if (gm < p.M && n < p.N) {
@@ -716,7 +721,7 @@ static int oil_gemm_launch(const void* x, int ldx, const void* idx, const void* 
   if ((rc = make_tmap_2d_bf16(&tx, x, (uint64_t)K, (uint64_t)M, (uint64_t)ldx, BK, (uint32_t)p.Mpad))) return rc;
   const int idx_tile = BN * rowb;
   const int table = bits == 2 ? 128 : 256 * 32 * 4;   // static shared memory
-  const int fixed = 1024 + 2 * kbb * p.Mpad * BK * 2 + 2 * STG_TOK * STG_PITCH * 4 + (2 * MAX_IDX_STAGES + 12) * 8 + 16 + 1024 + 64;
+  const int fixed = 1024 + 2 * kbb * p.Mpad * BK * 2 + 4 * STG_TOK * STG_PITCH * 4 + (2 * MAX_IDX_STAGES + 12) * 8 + 16 + 1024 + 64;
   int stages = (227 * 1024 - table - fixed) / idx_tile;
   if (stages > MAX_IDX_STAGES) stages = MAX_IDX_STAGES;
   stages &= ~1;  // even: a ring stage is then always read by the same expanding group, which sees every phase of its barrier
