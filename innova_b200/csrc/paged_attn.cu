@@ -477,32 +477,6 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32)) paged_decode_oil4_mm
   const int per = (npages + splits - 1) / splits;
   const int p0 = split * per, p1 = min(npages, p0 + per);
   const float c = scale * 1.4426950408889634f;
-  if (FUSED) qkv_heads_of_group<true, D>(fin, b, hk, G, len - 1, page_table, max_pages, k_pool, v_pool, k_scale, v_scale, c, sq);
-  // Q fragment: row gid = query head, this lane's d-quarter; rows 8..15 of the MMA are zero
-  uint32_t qa[KSTEPS][2];
-  {
-    const int head = min(gid, G - 1);
-    const __nv_bfloat16* qrow = FUSED ? nullptr : q + (long)b * ld_q + (hk * G + head) * D + tig * KCH;
-#pragma unroll
-    for (int st = 0; st < KSTEPS; ++st) {
-      float4 f;
-      if (FUSED) {
-        f = *reinterpret_cast<const float4*>(sq + head * D + tig * KCH + st * 4);
-      } else {
-        const uint2 raw = *reinterpret_cast<const uint2*>(qrow + st * 4);
-        f = make_float4(__uint_as_float(raw.x << 16) * c, __uint_as_float(raw.x & 0xffff0000u) * c, __uint_as_float(raw.y << 16) * c,
-                        __uint_as_float(raw.y & 0xffff0000u) * c);
-      }
-      qa[st][0] = gid < G ? h2_as_u32(__floats2half2_rn(f.x, f.y)) : 0u;
-      qa[st][1] = gid < G ? h2_as_u32(__floats2half2_rn(f.z, f.w)) : 0u;
-    }
-  }
-  if (!FUSED) __syncthreads();
-  float m_run = -INFINITY, l_run = 0.f;  // of head gid; l is this lane's share (its 4 tokens per page)
-  float o[VMMA][4];
-#pragma unroll
-  for (int i = 0; i < VMMA; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-
   uint32_t kraw[2][KW], vraw[4][VW];
   __half ksc[2], vsc[4];
   auto fetch = [&](int pg) {
@@ -534,8 +508,37 @@ __global__ void __launch_bounds__(NW * 32, 512 / (NW * 32)) paged_decode_oil4_mm
       vsc[t] = v_scale[row * (D / 32) + (gid * VCH) / 32];
     }
   };
+  // the warp's first page is requested before the projection is finished, unless it is the one that the new token goes to
   int pg = p0 + warp;
-  if (pg < p1) fetch(pg);
+  const bool early = pg < p1 && (!FUSED || pg != npages - 1);
+  if (early) fetch(pg);
+  if (FUSED) qkv_heads_of_group<true, D>(fin, b, hk, G, len - 1, page_table, max_pages, k_pool, v_pool, k_scale, v_scale, c, sq);
+  // Q fragment: row gid = query head, this lane's d-quarter; rows 8..15 of the MMA are zero
+  uint32_t qa[KSTEPS][2];
+  {
+    const int head = min(gid, G - 1);
+    const __nv_bfloat16* qrow = FUSED ? nullptr : q + (long)b * ld_q + (hk * G + head) * D + tig * KCH;
+#pragma unroll
+    for (int st = 0; st < KSTEPS; ++st) {
+      float4 f;
+      if (FUSED) {
+        f = *reinterpret_cast<const float4*>(sq + head * D + tig * KCH + st * 4);
+      } else {
+        const uint2 raw = *reinterpret_cast<const uint2*>(qrow + st * 4);
+        f = make_float4(__uint_as_float(raw.x << 16) * c, __uint_as_float(raw.x & 0xffff0000u) * c, __uint_as_float(raw.y << 16) * c,
+                        __uint_as_float(raw.y & 0xffff0000u) * c);
+      }
+      qa[st][0] = gid < G ? h2_as_u32(__floats2half2_rn(f.x, f.y)) : 0u;
+      qa[st][1] = gid < G ? h2_as_u32(__floats2half2_rn(f.z, f.w)) : 0u;
+    }
+  }
+  if (!FUSED) __syncthreads();
+  float m_run = -INFINITY, l_run = 0.f;  // of head gid; l is this lane's share (its 4 tokens per page)
+  float o[VMMA][4];
+#pragma unroll
+  for (int i = 0; i < VMMA; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+
+  if (!early && pg < p1) fetch(pg);
   for (; pg < p1; pg += NW) {
     // ---- this page's registers; then start the next page's loads ----
     uint32_t kr[2][KW], vr[4][VW];
