@@ -87,6 +87,12 @@ def check(rc: int, what: str):
         raise RuntimeError(f"{what} failed with code {rc}")
 
 
+def count_launches(n: int):
+    """Counts ``n`` launches more than the one that ``check`` counted, for an entry point that issues several."""
+    global _launches
+    _launches += n
+
+
 def launch_count() -> int:
     """Number of native kernel-launching calls made so far (each launches at least one kernel)."""
     return _launches

@@ -71,6 +71,7 @@ class FlatParamEngine:
         self._hyper_slot = 0
         if self.device.type == "cuda":
             self._hyper_ring = self._hyper_ring.pin_memory()
+        self._hyper_rows = self._hyper_ring.numpy()      # the same memory: a row is written in one assignment
 
     def _pre_alloc(self):
         pass
@@ -97,10 +98,9 @@ class FlatParamEngine:
         bc1, bc2 = 1.0 - b1 ** t, 1.0 - b2 ** t
         lr_adj = lr * math.sqrt(bc2) / bc1 if self.reference_formula else lr / bc1
         self._hyper_slot = (self._hyper_slot + 1) % self._hyper_ring.shape[0]
-        h = self._hyper_ring[self._hyper_slot]
-        h[0], h[1], h[2], h[3], h[4], h[5] = lr_adj, b1, b2, self.eps, lr * wd, 1.0 / bc2
-        h[6], h[7], h[8] = self.max_grad_norm or 0.0, grad_scale, 1.0 if self.reference_formula else 0.0
-        return h
+        self._hyper_rows[self._hyper_slot, :9] = (lr_adj, b1, b2, self.eps, lr * wd, 1.0 / bc2, self.max_grad_norm or 0.0, grad_scale,
+                                                  1.0 if self.reference_formula else 0.0)
+        return self._hyper_ring[self._hyper_slot]
 
     def zero_grad(self):
         self.flat_grad.zero_()

@@ -100,7 +100,8 @@ class Trainer:
     # one optimizer step made of `grad_accum_steps` micro-batches; returns the mean loss (device tensor)
     def train_step(self, ids: torch.Tensor, labels: torch.Tensor) -> torch.Tensor:
         c = self.cfg
-        self.model.train()
+        if any(not m.training or type(m).train is not torch.nn.Module.train for m in self.model.modules()):
+            self.model.train()
         A = c.grad_accum_steps
         if A > 1:
             ids_m, lab_m = ids.chunk(A, dim=0), labels.chunk(A, dim=0)
