@@ -751,8 +751,56 @@ __global__ void __launch_bounds__(256) decode_qkv_finish_kernel(const __grid_con
   kv_store_head<OIL4, D>(v, ((long)page * fin.Hkv + hk) * PAGE + p % PAGE, which ? v_pool : k_pool, which ? v_scale : k_scale, lane);
 }
 
+// The same for prompts of a few tokens: token t of T is position t % S of sequence t / S, and all heads also go to qkv_out [T, ld_out] as bf16, where
+// flash attention reads them. Replaces the finish pass, the rotation and the append of a layer (14, 2.5 and 2.7 us at 77 tokens of 96 heads,
+// with a copy of the start positions from the host).
+template <bool OIL4, int D>
+__global__ void __launch_bounds__(256) prompt_qkv_finish_kernel(const __grid_constant__ QkvFinish fin, int S, const int* __restrict__ page_table,
+                                                                int max_pages, int T, __nv_bfloat16* __restrict__ qkv_out, int ld_out,
+                                                                uint8_t* __restrict__ k_pool, uint8_t* __restrict__ v_pool,
+                                                                __half* __restrict__ k_scale, __half* __restrict__ v_scale) {
+  release_next();
+  wait_previous();
+  const int lane = threadIdx.x & 31;
+  const long warp_id = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int slots = fin.H + 2 * fin.Hkv;
+  if (warp_id >= (long)T * slots) return;
+  const int slot = (int)(warp_id % slots), t = (int)(warp_id / slots), b = t / S, pos = t - b * S;
+  const int which = slot >= fin.H + fin.Hkv;  // of the cached heads: 0 = key, 1 = value
+  const int page = slot >= fin.H ? page_table[(long)b * max_pages + pos / PAGE] : 0;
+  float v[D / 32];
+  qkv_head<D>(fin, t, slot, pos, lane, v);
+  __nv_bfloat16* out = qkv_out + (size_t)t * ld_out + slot * D;
+#pragma unroll
+  for (int j = 0; j < D / 32; ++j) out[lane + 32 * j] = __float2bfloat16_rn(v[j]);
+  if (slot < fin.H) return;
+  const int hk = slot - fin.H - which * fin.Hkv;
+  kv_store_head<OIL4, D>(v, ((long)page * fin.Hkv + hk) * PAGE + pos % PAGE, which ? v_pool : k_pool, which ? v_scale : k_scale, lane);
+}
+
 }  // namespace inv
 using namespace inv;
+// sums: fp32 [T, (H + 2 Hkv) D], cleared; sequences of S tokens from position 0 in rows 0, 1, ... of the page table.
+extern "C" int inv_prompt_qkv_finish(float* sums, int ld_sums, const void* bias, const float* cos_t, const float* sin_t, int S, const int* page_table,
+                                     int max_pages, int T, int H, int Hkv, int D, void* qkv_out, int ld_out, void* k_pool, void* v_pool, void* k_scale,
+                                     void* v_scale, int oil4, void* stream) {
+  if ((D != 64 && D != 128) || S < 1) return -ERR_BAD_ARG;
+  if (T <= 0) return 0;
+  const int grid = (int)(((long)T * (H + 2 * Hkv) + 7) / 8);
+  cudaStream_t st = (cudaStream_t)stream;
+  const QkvFinish fin{sums, ld_sums, (const __nv_bfloat16*)bias, cos_t, sin_t, H, Hkv, 1};
+#define INV_PQF(O, DD)                                                                                                                    \
+  launch_early(prompt_qkv_finish_kernel<O, DD>, dim3(grid), 256, 0, st, fin, S, page_table, max_pages, T, (__nv_bfloat16*)qkv_out, ld_out,   \
+               (uint8_t*)k_pool, (uint8_t*)v_pool, (__half*)k_scale, (__half*)v_scale)
+  if (oil4) {
+    if (D == 64) INV_PQF(true, 64); else INV_PQF(true, 128);
+  } else {
+    if (D == 64) INV_PQF(false, 64); else INV_PQF(false, 128);
+  }
+#undef INV_PQF
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : -(int)e;
+}
 extern "C" int inv_decode_qkv_finish(float* acc, int ld_acc, const void* bias, const float* cos_t, const float* sin_t, const int* pos,
                                      const int* page_table, int max_pages, int B, int H, int Hkv, int D, void* q_out, int ld_q, void* k_pool,
                                      void* v_pool, void* k_scale, void* v_scale, int oil4, void* stream) {

@@ -22,6 +22,8 @@ _native.register_cuda_sigs({
                               _native.i32, _native.i32, _native.vp, _native.i32, _native.vp, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp],
     "inv_kv_append": [_native.vp, _native.vp, _native.i32, _native.i32, _native.vp, _native.i32, _native.vp, _native.i32, _native.i32, _native.i32,
                       _native.i32, _native.vp, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp],
+    "inv_prompt_qkv_finish": [_native.vp, _native.i32] + [_native.vp] * 3 + [_native.i32, _native.vp] + [_native.i32] * 5 +
+                             [_native.vp, _native.i32] + [_native.vp] * 4 + [_native.i32, _native.vp],
     "inv_decode_attend": [_native.vp, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp, _native.i32, _native.vp] +
                          [_native.i32] * 4 + [_native.vp] * 4 + [_native.i32, _native.f32, _native.vp, _native.i32, _native.vp],
     "inv_paged_decode": [_native.vp, _native.i32, _native.vp, _native.i32, _native.vp, _native.i32, _native.i32, _native.i32, _native.i32,

@@ -27,7 +27,7 @@ from ..inference.kv_cache import PagedKVCache, PAGE
 from ..models.config import TransformerConfig
 from ..ops import runtime as rt
 from ..ops.oil_linear import (SKINNY_SUMS, SKINNY_SWIGLU, QuantWeight, _acc_for, _gemm_into_acc, _skinny, finish_norm, oil_linear,
-                              oil_linear_norm, oil_linear_swiglu, quantize_weight, skinny_takes)
+                              oil_linear_norm, oil_linear_swiglu, quantize_weight, skinny_fits, skinny_takes)
 
 
 class TPContext:
@@ -219,24 +219,17 @@ class TPDecoder:
         c.reserve_rows(range(B), self.max_seq)  # every page a sequence can need, so that the decode graph never allocates
         x = self.emb[ids]
         rows, start = list(range(B)), [0] * B
-        few = self.world == 1 and B * S <= FEW_PROMPT_TOKENS
+        if self.world == 1 and 0 < B * S <= FEW_PROMPT_TOKENS:
+            x = self._few_prompt_tokens(x)
+            c.commit(rows, [S] * B)
+            return self._logits(x[:, -1].contiguous())
         h = ops.rms_norm(x, self.layers[0]["n1"], cfg.norm_eps)
         for li, l in enumerate(self.layers):
-            qkv = oil_linear(h, l["qkv"], resident=True) if few else ops.linear(h, l["qkv"].dequantize(), l["qkv"].bias)
+            qkv = ops.linear(h, l["qkv"].dequantize(), l["qkv"].bias)
             qkv = ops.rope_qk(qkv, self.rope[0], self.rope[1], H, Hkv, D)
             c.append(li, qkv[..., H * D:(H + Hkv) * D], qkv[..., (H + Hkv) * D:], rows, start)
             a = ops.flash_attention(qkv, H, Hkv, D, causal=True)
             nxt = self.layers[li + 1]["n1"] if li + 1 < len(self.layers) else None   # the last norm is taken of the last tokens only
-            if few:
-                x2, h = oil_linear_norm(a.view(B * S, -1), l["o"], x.view(B * S, -1), l["n2"], cfg.norm_eps, resident=True)
-                act = oil_linear_swiglu(h, l["gu"], resident=True)
-                if nxt is not None:
-                    x2, h = oil_linear_norm(act, l["down"], x2, nxt, cfg.norm_eps, resident=True)
-                    h = h.view(B, S, -1)
-                else:
-                    x2 = oil_linear(act, l["down"], x2, resident=True)
-                x = x2.view(B, S, -1)
-                continue
             if self.world > 1:
                 o = ops.linear(a, l["o"].dequantize())
                 dist.all_reduce(o)
@@ -255,6 +248,38 @@ class TPDecoder:
                 h = ops.rms_norm(x, nxt, cfg.norm_eps)
         c.commit(rows, [S] * B)
         return self._logits(x[:, -1].contiguous())
+
+    def _few_prompt_tokens(self, x: torch.Tensor) -> torch.Tensor:
+        """The layers over x [B, S, E], few tokens in all: products with the packed weights, seven launches a layer beside attention. Fills the
+        cache; the sequences are its first B rows."""
+        cfg, c, eps = self.cfg, self.cache, self.cfg.norm_eps
+        B, S, E = x.shape
+        T, H, Hkv, D = B * S, self.H, self.Hkv, self.D
+        lib, st, status = rt.lib(), rt.stream_ptr(), rt.status_tensor(self.dev).data_ptr()
+        h, x = ops.rms_norm(x, self.layers[0]["n1"], eps).view(T, E), x.view(T, E)
+        for li, l in enumerate(self.layers):
+            qw = l["qkv"]
+            if skinny_fits(h, qw):
+                sums = _skinny(h, qw, torch.empty(T, qw.N, dtype=torch.float32, device=self.dev), SKINNY_SUMS, resident=True)
+            else:
+                sums = _acc_for(h, qw, T)
+                _gemm_into_acc(h, qw, sums, True)
+            # one kernel adds the bias, rotates, lays the heads out for attention and appends the new keys / values to the cache
+            qkv = torch.empty(T, qw.N, dtype=torch.bfloat16, device=self.dev)
+            rt.check(lib.inv_prompt_qkv_finish(sums.data_ptr(), sums.stride(0), rt.ptr(qw.bias), self.rope[0].data_ptr(), self.rope[1].data_ptr(), S,
+                                               c.page_table.data_ptr(), c.max_pages, T, H, Hkv, D, qkv.data_ptr(), qkv.stride(0),
+                                               c.k_pool[li].data_ptr(), c.v_pool[li].data_ptr(), rt.ptr(c.k_scale[li]), rt.ptr(c.v_scale[li]),
+                                               int(c.fmt == "oil4"), st), "inv_prompt_qkv_finish")
+            a, q = torch.empty(T, H * D, dtype=torch.bfloat16, device=self.dev), qkv.data_ptr()
+            rt.check(lib.inv_flash_attn_fwd(q, q + H * D * 2, q + (H + Hkv) * D * 2, a.data_ptr(), 0, B, S, H, Hkv, D, qw.N, qw.N, qw.N, H * D,
+                                            float(D ** -0.5), 1, 0, status, st), "inv_flash_attn_fwd")
+            x, h = oil_linear_norm(a, l["o"], x, l["n2"], eps, resident=True)
+            act = oil_linear_swiglu(h, l["gu"], resident=True)
+            if li + 1 < len(self.layers):
+                x, h = oil_linear_norm(act, l["down"], x, self.layers[li + 1]["n1"], eps, resident=True)
+            else:                                  # the last norm is taken of the last tokens only
+                x = oil_linear(act, l["down"], x, resident=True)
+        return x.view(B, S, E)
 
     def _logits(self, last: torch.Tensor, normed: bool = False) -> torch.Tensor:
         h = last if normed else ops.rms_norm(last, self.norm_w, self.cfg.norm_eps)

@@ -641,3 +641,40 @@ def test_projection_finish_and_attention_in_one_launch(fmt, B, H, Hkv, D, lens):
             w = torch.softmax(torch.einsum("hgd,hnd->hgn", q[r].double().view(Hkv, H // Hkv, D), kk) * scale, -1)
             want = torch.einsum("hgn,hnd->hgd", w, vv).reshape(-1)
             assert float((one[r].double() - want).norm() / want.norm()) < 2.0 ** -8      # one rounding to bf16 of fp32 sums
+
+
+@pytest.mark.parametrize("fmt", ["bf16", "oil4"])
+@pytest.mark.parametrize("B,S,H,Hkv,D", [(1, 1, 4, 4, 64), (1, 77, 8, 2, 128), (3, 17, 6, 3, 64), (2, 64, 4, 1, 128)])
+def test_prompt_projection_finish_matches_its_three_passes(fmt, B, S, H, Hkv, D):
+    """``inv_prompt_qkv_finish`` against finish pass, rotation and append, to the bit: the heads that attention reads, the cache, cleared sums."""
+    from innova_b200.inference.kv_cache import PagedKVCache
+    from innova_b200.ops import rope_qk, rope_tables
+    from innova_b200.ops import runtime as rt
+    torch.manual_seed(S)
+    T, W = B * S, (H + 2 * Hkv) * D
+    cos, sin = rope_tables(128, D, 10000.0, torch.device(DEV))
+    sums = torch.randn(T, W, device=DEV)
+    bias = torch.randn(W, device=DEV).bfloat16() if B > 1 else None
+    a, b = (PagedKVCache(1, Hkv, D, B, 128, torch.device(DEV), fmt) for _ in range(2))
+    for c in (a, b):
+        c.k_pool[0].zero_()
+        c.v_pool[0].zero_()
+        c.reserve_rows(range(B), 128)
+    want = torch.empty(T, W, dtype=torch.bfloat16, device=DEV)
+    s1, s2 = sums.clone(), sums.clone()
+    lib, st = rt.lib(), rt.stream_ptr()
+    rt.check(lib.inv_oil_gemm_finish(s1.data_ptr(), rt.ptr(bias), 0, want.data_ptr(), T, W, W, W, 0, 1, st), "finish")
+    want = rope_qk(want.view(B, S, W), cos, sin, H, Hkv, D)
+    a.append(0, want[..., H * D:(H + Hkv) * D], want[..., (H + Hkv) * D:], list(range(B)), [0] * B)
+    got = torch.full((T, W), float("nan"), dtype=torch.bfloat16, device=DEV)
+    rt.check(lib.inv_prompt_qkv_finish(s2.data_ptr(), W, rt.ptr(bias), cos.data_ptr(), sin.data_ptr(), S, b.page_table.data_ptr(), b.max_pages, T, H, Hkv, D,
+                                       got.data_ptr(), W, b.k_pool[0].data_ptr(), b.v_pool[0].data_ptr(), rt.ptr(b.k_scale[0]), rt.ptr(b.v_scale[0]),
+                                       int(fmt == "oil4"), st), "prompt")
+    assert torch.equal(got.view(B, S, W), want) and float(s2.abs().max()) == 0.0
+    assert torch.equal(a.page_table, b.page_table) and torch.equal(a.k_pool[0], b.k_pool[0]) and torch.equal(a.v_pool[0], b.v_pool[0])
+    if fmt == "oil4":
+        for x, y in ((a.k_scale[0], b.k_scale[0]), (a.v_scale[0], b.v_scale[0])):
+            pages = a.page_table[:B, :(S + 15) // 16].reshape(-1).long()
+            seen = torch.arange(16, device=DEV).view(1, -1) < (S - 16 * torch.arange((S + 15) // 16, device=DEV).view(-1, 1))
+            keep = seen.repeat(B, 1).view(-1, 1, 16, 1).expand(-1, Hkv, 16, D // 32).reshape(len(pages), -1)
+            assert torch.equal(x.view(x.shape[0], -1)[pages][keep], y.view(y.shape[0], -1)[pages][keep])
