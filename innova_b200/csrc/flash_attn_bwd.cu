@@ -4,8 +4,8 @@
 // src/autograd_grad.cpp attention branch); the reference's memory-efficient backward is a
 // placeholder (src/zero_optimizer_mem.cpp:496-574), so the oracle is plain fp32 attention.
 //
-// One CTA per (batch, kv head, 128-key block). K and V tiles stay in shared memory; the CTA walks
-// the query blocks that can see its keys (and, for GQA, every query head of the group) and
+// One persistent CTA per SM; its work items are (batch, kv head, 128-key block). An item's K and V tiles stay in shared memory; the
+// CTA walks the query blocks that can see its keys (and, for GQA, every query head of the group) and
 // accumulates dK and dV in TMEM. Per query block, five MMAs:
 //   S^T  = K Q^T            dP^T = V dO^T            (both 128 keys x 128 queries, fp32 in TMEM)
 //   dV  += P^T dO           dK  += dS^T Q            dQ_blk = dS K
@@ -13,7 +13,15 @@
 // P^T = exp(S^T*scale - lse) and dS^T = P^T * (dP^T - D) as bf16 tiles in swizzled shared memory.
 // The same dS^T tile serves as a K-major A operand (dK) and as an MN-major A operand (dQ), and the
 // Q / dO / K tiles serve as K-major B operands (S^T, dP^T) and MN-major B operands (dK, dV, dQ), so
-// nothing is transposed in memory. dQ blocks are added to an fp32 buffer with vector reductions.
+// nothing is transposed in memory. dQ blocks are added to an fp32 buffer with TMA reductions.
+//
+// At 1024 tokens an item is 4.5 query blocks of 4,400 cycles on average (D = 64), and set-up, the first loads and the last read-outs of a CTA
+// of its own were 13,700 more, none of it under another CTA's work (tensor memory holds one). In a persistent CTA the next item's first
+// query and its K and V are loaded, and its first products run, while the softmax warps still write this item's dK and dV.
+// With delta, clearing and conversion: 64 x 1024, 12 heads of 64: 838 -> 721 us; 2 x 2048, 16 heads of 128: 269 -> 218 (of which the reductions in
+// place of 16-byte ones per lane are the larger part: a block took 10,500 cycles, now 9,000). A block is bound by its own chain: the
+// sixteen warps read S^T and dP^T, exponentiate (1,024 cycles of the special-function units), publish and read dQ one after the other, since
+// tensor memory holds one block's scores.
 // Every wait is bounded and reports through *status.
 #include "sm100_common.cuh"
 #include "inv_api.h"
@@ -63,19 +71,43 @@ struct BwdSmem {
   static constexpr int DO_OFF = Q_OFF + STAGES * TILE;
   static constexpr int PT_OFF = DO_OFF + STAGES * TILE;
   static constexpr int DST_OFF = PT_OFF + 32768;
-  static constexpr int DQS_OFF = DST_OFF + 32768;      // D = 64: the fp32 dQ block on its way to the reduce copies, one 32 x 16 box per softmax warp
-  static constexpr int STAT_OFF = DQS_OFF + (ND == 1 ? 32768 : 0);  // lse and delta of the current query block, two stages
+  // The fp32 dQ block on its way to the reduce copies, boxes of 32 x 16 per softmax warp: one with a place of its own for D = 64, two in the
+  // P^T and dS^T tiles for D = 128, which are free between the products of a block and the next block's tiles.
+  static constexpr int DQS_OFF = ND == 1 ? DST_OFF + 32768 : PT_OFF;
+  static constexpr int STAT_OFF = DST_OFF + 32768 + (ND == 1 ? 32768 : 0);  // lse and delta of the current query block, two stages
   static constexpr int BAR_OFF = STAT_OFF + 16 * 2 * 64 * 4;   // per softmax warp: two stages of 32 lse + 32 delta
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
-// Build with -DFB_TRACE to record the SM clock at the phases of CTA (0, 0, 0) of the most recent launch
+// Work item `round` of a CTA: items are numbered head by head (so that the SMs share a head's Q and dO in L2), key block by key block, and every
+// other round runs backwards over the CTAs, so that a CTA's long and short items (causal: key block j sees all later queries) even out.
+struct BwdItem {
+  int j, hk, b, k0, i0, nq_it, n_it;
+  bool valid;
+  __device__ __forceinline__ BwdItem(const FlashBwdParams& p, int round) {
+    const int nb = (p.S + 127) / 128, total = nb * p.Hkv * p.B, grid = gridDim.x, cta = blockIdx.x;
+    const int idx = round * grid + ((round & 1) ? grid - 1 - cta : cta);
+    valid = idx < total;
+    const int r = idx / nb;
+    j = idx - r * nb;
+    b = r / p.Hkv;
+    hk = r - b * p.Hkv;
+    k0 = j * 128;
+    i0 = p.causal ? j : 0;
+    // with a sliding window the last query that sees key k0 + 127 is row k0 + 126 + window
+    const int i_end = (p.causal && p.window > 0) ? min(nb, (k0 + 126 + p.window) / 128 + 1) : nb;
+    nq_it = i_end - i0;
+    n_it = (p.H / p.Hkv) * nq_it;
+  }
+};
+
+// Build with -DFB_TRACE to record the SM clock at the phases of the last item of CTA 0 of the most recent launch
 // (inv_fb_trace_read): 0 entry, 1 set-up done, 2 K/V landed (issuer), 3 exit, 4 dK/dV written, 8 + 3 it: S^T ready for
 // query block it, 9 + 3 it: P^T / dS^T published, 10 + 3 it: dQ of block it - 1 read out, 32 + 3 it: S^T / dP^T in registers,
 // 33 + 3 it: exponentials done, 34 + 3 it: the previous block's MMAs have released the P^T / dS^T tiles.
 #ifdef FB_TRACE
 __device__ long long fb_trace_buf[64];
-#define FB_STAMP(i) do { if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (i) < 64) fb_trace_buf[i] = clock64(); } while (0)
+#define FB_STAMP(i) do { if (blockIdx.x == 0 && (i) < 64) fb_trace_buf[i] = clock64(); } while (0)
 #else
 #define FB_STAMP(i) do {} while (0)
 #endif
@@ -86,7 +118,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                  const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
                  const __grid_constant__ CUtensorMap tmap_dq, const __grid_constant__ FlashBwdParams p) {
   constexpr int D = 64 * ND;
-  constexpr bool DQ_TMA = (ND == 1);  // dQ blocks leave through shared memory and one reduce copy per 32 columns, not per-thread reductions
   using L = BwdSmem<ND>;
   constexpr int STAGES = L::STAGES;
   constexpr bool OVERLAP = (ND == 1);  // D = 128 has no spare TMEM: dQ reuses the S^T columns
@@ -112,19 +143,13 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   uint64_t* pds_full = bars + 7;   // 256 arrivals: P^T and dS^T are in shared memory
   uint64_t* mma2_done = bars + 8;  // dV, dK, dQ MMAs of this block finished
   uint64_t* dq_empty = bars + 9;   // 256 arrivals: dQ has been read out of TMEM
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  uint64_t* kv_empty = bars + 10;  // the item's last MMAs have read K and V
+  uint64_t* dqs_free = bars + 11;  // D = 128: the reduce copies have read the boxes in the P^T / dS^T tiles
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int G = p.H / p.Hkv;
-  const int k0 = j * 128;
-  const int nqb = (p.S + 127) / 128;
-  const int i0 = p.causal ? j : 0;
-  // with a sliding window the last query that sees key k0 + 127 is row k0 + 126 + window
-  const int i_end = (p.causal && p.window > 0) ? min(nqb, (k0 + 126 + p.window) / 128 + 1) : nqb;
-  const int nq_it = i_end - i0;
-  const int n_it = G * nq_it;
   if (threadIdx.x == 0) FB_STAMP(0);
 
   if (threadIdx.x == 0) {
@@ -138,13 +163,15 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     mbar_init(pds_full, 16);
     mbar_init(mma2_done, 3);   // dV, dK and dQ have one issuer each
     mbar_init(dq_empty, 16);
+    mbar_init(kv_empty, 3);    // one commit per issuer
+    mbar_init(dqs_free, 16);
     *abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmap_q);
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
     tma_prefetch_desc(&tmap_do);
-    if (DQ_TMA) tma_prefetch_desc(&tmap_dq);
+    tma_prefetch_desc(&tmap_dq);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, TMEM_COLS);
@@ -158,23 +185,32 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 
   if (warp == 0) {
     if (elect_one_sync()) {
-      mbar_expect_tx(kv_full, 2 * L::TILE);
+      bool ok = true;
+      int g = 0;                       // query blocks over all items
+      for (int n = 0; ok; ++n) {
+        const BwdItem w(p, n);
+        if (!w.valid) break;
+        for (int it = 0; it < w.n_it; ++it, ++g) {
+          const int st = g % STAGES;
+          const uint32_t ph = (g / STAGES) & 1;
+          if (!mbar_wait(&q_empty[st], ph ^ 1, abort_flag, p.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+          const int h = w.hk * G + it / w.nq_it;
+          const int q0 = (w.i0 + it % w.nq_it) * 128;
+          mbar_expect_tx(&q_full[st], 2 * L::TILE);
 #pragma unroll
-      for (int a = 0; a < ND; ++a) {
-        tma_load_3d(sK + a * 16384, &tmap_k, kv_full, hk * D + a * 64, k0, b);
-        tma_load_3d(sV + a * 16384, &tmap_v, kv_full, hk * D + a * 64, k0, b);
-      }
-      for (int it = 0; it < n_it; ++it) {
-        const int st = it % STAGES;
-        const uint32_t ph = (it / STAGES) & 1;
-        if (!mbar_wait(&q_empty[st], ph ^ 1, abort_flag, p.status, ERR_WAIT_EMPTY)) break;
-        const int h = hk * G + it / nq_it;
-        const int q0 = (i0 + it % nq_it) * 128;
-        mbar_expect_tx(&q_full[st], 2 * L::TILE);
+          for (int a = 0; a < ND; ++a) {
+            tma_load_3d(sQ + st * L::TILE + a * 16384, &tmap_q, &q_full[st], h * D + a * 64, q0, w.b);
+            tma_load_3d(sdO + st * L::TILE + a * 16384, &tmap_do, &q_full[st], h * D + a * 64, q0, w.b);
+          }
+          if (it == 0) {               // behind the first query block, whose stage is free earlier
+            if (!mbar_wait(kv_empty, (n & 1) ^ 1, abort_flag, p.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+            mbar_expect_tx(kv_full, 2 * L::TILE);
 #pragma unroll
-        for (int a = 0; a < ND; ++a) {
-          tma_load_3d(sQ + st * L::TILE + a * 16384, &tmap_q, &q_full[st], h * D + a * 64, q0, b);
-          tma_load_3d(sdO + st * L::TILE + a * 16384, &tmap_do, &q_full[st], h * D + a * 64, q0, b);
+            for (int a = 0; a < ND; ++a) {
+              tma_load_3d(sK + a * 16384, &tmap_k, kv_full, w.hk * D + a * 64, w.k0, w.b);
+              tma_load_3d(sV + a * 16384, &tmap_v, kv_full, w.hk * D + a * 64, w.k0, w.b);
+            }
+          }
         }
       }
     }
@@ -192,13 +228,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       const uint32_t idesc_dq = make_idesc_bf16(128, D, 1, 1);    // MN-major A and B
       const uint32_t k_base = smem_u32(sK), v_base = smem_u32(sV);
       const uint32_t pt_base = smem_u32(sPt), dst_base = smem_u32(sdSt);
-      bool ok = mbar_wait(kv_full, 0, abort_flag, p.status, ERR_WAIT_FULL);
-      if (role == 0) FB_STAMP(2);
-      auto issue_s = [&](int it) -> bool {  // roles 0 and 1
-        const int st = it % STAGES;
-        if (!mbar_wait(&q_full[st], (it / STAGES) & 1, abort_flag, p.status, ERR_WAIT_FULL)) return false;
-        if (it > 0 && !mbar_wait(s_empty, (it - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) return false;
-        if (!OVERLAP && role == 0 && it > 0 && !mbar_wait(dq_empty, (it - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) return false;
+      auto issue_s = [&](int g) -> bool {  // roles 0 and 1
+        const int st = g % STAGES;
+        if (!mbar_wait(&q_full[st], (g / STAGES) & 1, abort_flag, p.status, ERR_WAIT_FULL)) return false;
+        if (g > 0 && !mbar_wait(s_empty, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) return false;
+        if (!OVERLAP && role == 0 && g > 0 && !mbar_wait(dq_empty, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) return false;
         tc_fence_after();
         const uint32_t a_base = role == 0 ? k_base : v_base;
         const uint32_t b_base = smem_u32((role == 0 ? sQ : sdO) + st * L::TILE);
@@ -211,40 +245,50 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         umma_commit(s_full);
         return true;
       };
-      if (ok && OVERLAP && role < 2) ok = issue_s(0);
-      for (int it = 0; ok && it < n_it; ++it) {
-        if (role < 2) {
-          if (OVERLAP) {
-            if (it + 1 < n_it && !issue_s(it + 1)) break;
+      bool ok = true;
+      int g = 0;
+      for (int n = 0; ok; ++n) {
+        const BwdItem w(p, n);
+        if (!w.valid) break;
+        if (!mbar_wait(kv_full, n & 1, abort_flag, p.status, ERR_WAIT_FULL)) break;
+        if (role == 0) FB_STAMP(2);
+        if (OVERLAP && role < 2 && !issue_s(g)) break;
+        for (int it = 0; it < w.n_it; ++it, ++g) {
+          if (role < 2) {
+            if (OVERLAP) {
+              if (it + 1 < w.n_it && !issue_s(g + 1)) { ok = false; break; }
+            } else {
+              if (!issue_s(g)) { ok = false; break; }
+            }
+          }
+          const int st = g % STAGES;
+          if (!mbar_wait(pds_full, g & 1, abort_flag, p.status, ERR_WAIT_MISC)) { ok = false; break; }
+          if (OVERLAP && role == 2 && g > 0 && !mbar_wait(dq_empty, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+          tc_fence_after();
+          if (role < 2) {
+            // dV += P^T dO ; dK += dS^T Q   (A: [keys x queries] K-major, B: [queries x d] MN-major). An item's first product overwrites:
+            // the softmax warps published its tiles after they had read the last item's sums.
+            const uint32_t a_base = role == 0 ? pt_base : dst_base;
+            const uint32_t b_base = smem_u32((role == 0 ? sdO : sQ) + st * L::TILE);
+            const uint32_t d_col = tmem_base + (role == 0 ? DV_COL : DK_COL);
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks) {
+              const uint32_t a_off = (ks / 4) * 16384 + (ks % 4) * 32;
+              umma_bf16(d_col, make_smem_desc(a_base + a_off, 16, 1024, 2), make_smem_desc(b_base + ks * 2048, 16384, 1024, 2), idesc_kv,
+                        (it > 0 || ks > 0) ? 1u : 0u);
+            }
+            umma_commit(mma2_done);
+            umma_commit(&q_empty[st]);  // both roles read Q and dO of this stage
           } else {
-            if (!issue_s(it)) break;
-          }
-        }
-        const int st = it % STAGES;
-        if (!mbar_wait(pds_full, it & 1, abort_flag, p.status, ERR_WAIT_MISC)) break;
-        if (OVERLAP && role == 2 && it > 0 && !mbar_wait(dq_empty, (it - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) break;
-        tc_fence_after();
-        if (role < 2) {
-          // dV += P^T dO ; dK += dS^T Q   (A: [keys x queries] K-major, B: [queries x d] MN-major)
-          const uint32_t a_base = role == 0 ? pt_base : dst_base;
-          const uint32_t b_base = smem_u32((role == 0 ? sdO : sQ) + st * L::TILE);
-          const uint32_t d_col = tmem_base + (role == 0 ? DV_COL : DK_COL);
+            // dQ_blk = dS K   (A: dS^T tile read MN-major, B: K tile read MN-major; reduction over keys)
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint32_t a_off = (ks / 4) * 16384 + (ks % 4) * 32;
-            umma_bf16(d_col, make_smem_desc(a_base + a_off, 16, 1024, 2), make_smem_desc(b_base + ks * 2048, 16384, 1024, 2), idesc_kv,
-                      (it > 0 || ks > 0) ? 1u : 0u);
+            for (int ks = 0; ks < 8; ++ks) {
+              umma_bf16(tmem_base + DQ_COL, make_smem_desc(dst_base + ks * 2048, 16384, 1024, 2), make_smem_desc(k_base + ks * 2048, 16384, 1024, 2),
+                        idesc_dq, ks > 0);
+            }
+            umma_commit(mma2_done);
           }
-          umma_commit(mma2_done);
-          umma_commit(&q_empty[st]);  // both roles read Q and dO of this stage
-        } else {
-          // dQ_blk = dS K   (A: dS^T tile read MN-major, B: K tile read MN-major; reduction over keys)
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            umma_bf16(tmem_base + DQ_COL, make_smem_desc(dst_base + ks * 2048, 16384, 1024, 2), make_smem_desc(k_base + ks * 2048, 16384, 1024, 2),
-                      idesc_dq, ks > 0);
-          }
-          umma_commit(mma2_done);
+          if (it + 1 == w.n_it) umma_commit(kv_empty);
         }
       }
     }
@@ -255,61 +299,42 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const int hf = cq >> 1;            // the 64-column half (shared-memory tile) it falls in
     constexpr int DC = D / 4;          // dQ / dK / dV columns per thread
     const int r = q * 32 + lane;       // row inside a tile
-    const int key = k0 + r;
     const uint32_t t_lane = tmem_base + (uint32_t(q * 32) << 16);
     const float c = p.scale * 1.4426950408889634f;
-    const bool vec_ok = (p.S & 3) == 0;  // rows of lse / delta start 16-byte aligned
     uint8_t* pt_row = sPt + hf * 16384 + (r >> 3) * 1024 + (r & 7) * 128;
     uint8_t* dst_row = sdSt + hf * 16384 + (r >> 3) * 1024 + (r & 7) * 128;
     bool ok = true;
-    // dQ block j: TMEM lanes are query rows now; this thread adds D/2 columns of row q0 + r into the fp32 buffer
-    auto dq_readout = [&](int j) {
-      const int hj = hk * G + j / nq_it;
-      const int qrow = (i0 + j % nq_it) * 128 + r;
-      if (DQ_TMA) {
-        // Every warp drains its own 32 rows x 16 columns: TMEM -> a private 2 KB box in shared memory (64-byte rows,
-        // 64-byte swizzle: chunk ^ ((row >> 1) & 3)) -> one reduce copy issued by the warp's first lane. No barrier
-        // across warps: a warp only waits for its own previous copy to have read its box.
-        uint32_t rr[16];
-        tmem_ld_32x16(t_lane + DQ_COL + cq * 16, rr);
-        if (lane == 0) bulk_wait_read();
-        __syncwarp();
-        tmem_ld_wait();
-        uint8_t* box = sDq + (warp - 2) * 2048;
-        uint8_t* row = box + lane * 64;
+    // dQ of block `it` of item w: TMEM lanes are query rows now. Every warp drains its own 32 rows x DC columns: TMEM -> private 2 KB boxes in
+    // shared memory (32 rows of 64 bytes, 64-byte swizzle: chunk ^ ((row >> 1) & 3)) -> reduce copies issued by the warp's first lane. No
+    // barrier across warps: a warp only waits for its own previous copies to have read its boxes.
+    auto dq_readout = [&](const BwdItem& w, int it) {
+      const int hj = w.hk * G + it / w.nq_it, row0 = (w.i0 + it % w.nq_it) * 128 + q * 32;
+      uint32_t rr[DC];
+      if (DC == 16) tmem_ld_32x16(t_lane + DQ_COL + cq * DC, rr);
+      else tmem_ld_32x32(t_lane + DQ_COL + cq * DC, rr);
+      if (lane == 0) bulk_wait_read();
+      __syncwarp();
+      tmem_ld_wait();
+      uint8_t* box = sDq + (warp - 2) * (DC * 128);
+#pragma unroll
+      for (int u = 0; u < DC / 16; ++u) {
+        uint8_t* row = box + u * 2048 + lane * 64;
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           const int chunk = g ^ ((lane >> 1) & 3);
-          *reinterpret_cast<uint4*>(row + chunk * 16) = make_uint4(rr[g * 4], rr[g * 4 + 1], rr[g * 4 + 2], rr[g * 4 + 3]);
-        }
-        tc_fence_before();
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(dq_empty);
-          tma_reduce_add_3d(&tmap_dq, box, hj * D + cq * 16, (i0 + j % nq_it) * 128 + q * 32, b);
-          bulk_commit();
-        }
-        return;
-      }
-      {
-        const int col0 = cq * DC;
-        uint32_t rr[DC];
-        if (DC == 16) tmem_ld_32x16(t_lane + DQ_COL + col0, rr);
-        else tmem_ld_32x32(t_lane + DQ_COL + col0, rr);
-        tmem_ld_wait();
-        if (qrow < p.S) {
-          float* dst = p.dq_acc + ((size_t)b * p.S + qrow) * ((size_t)p.H * D) + hj * D + col0;
-#pragma unroll
-          for (int g = 0; g < DC / 4; ++g)
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + g * 4), "f"(__uint_as_float(rr[g * 4])),
-                         "f"(__uint_as_float(rr[g * 4 + 1])), "f"(__uint_as_float(rr[g * 4 + 2])), "f"(__uint_as_float(rr[g * 4 + 3]))
-                         : "memory");
+          const uint32_t* v = rr + u * 16 + g * 4;
+          *reinterpret_cast<uint4*>(row + chunk * 16) = make_uint4(v[0], v[1], v[2], v[3]);
         }
       }
       tc_fence_before();
+      fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(dq_empty);
+      if (lane == 0) {
+        mbar_arrive(dq_empty);
+#pragma unroll
+        for (int u = 0; u < DC / 16; ++u) tma_reduce_add_3d(&tmap_dq, box + u * 2048, hj * D + cq * DC + u * 16, row0, w.b);
+        bulk_commit();
+      }
     };
     // The row statistics (lse, delta) of a query block go through shared memory, a private region per warp: lane i
     // fetches lse and delta of column cq * 32 + i (two global loads per thread and block; the four warps of a column
@@ -317,23 +342,28 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     // it + 1 are issued while block it is being computed and parked in registers, so that no warp waits on them, and
     // no barrier across warps is involved.
     float* wstat = sStat + (warp - 2) * 128;  // [stage][lse 32 | delta 32]
-    auto stat_load = [&](int it, float& l, float& d) {
-      const int h = hk * G + it / nq_it;
-      const int qi = min((i0 + it % nq_it) * 128 + cq * 32 + lane, p.S - 1);
-      const size_t o = ((size_t)b * p.H + h) * p.S + qi;
+    auto stat_load = [&](const BwdItem& w, int it, float& l, float& d) {
+      const int h = w.hk * G + it / w.nq_it;
+      const int qi = min((w.i0 + it % w.nq_it) * 128 + cq * 32 + lane, p.S - 1);
+      const size_t o = ((size_t)w.b * p.H + h) * p.S + qi;
       l = __ldg(p.lse + o);
       d = __ldg(p.delta + o);
     };
-    if (n_it > 0) {
+    BwdItem w(p, 0);
+    if (w.valid) {
       float l, d;
-      stat_load(0, l, d);
+      stat_load(w, 0, l, d);
       wstat[lane] = l;
       wstat[32 + lane] = d;
     }
-    for (int it = 0; it < n_it; ++it) {
-      const int q0 = (i0 + it % nq_it) * 128;
-      const float* stat = wstat + (it & 1) * 64;
-      if (!mbar_wait_warp(s_full, it & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+    int g = 0;                         // query blocks over all items: phase of the barriers, stage of the statistics
+    for (int n = 0; ok && w.valid; ++n) {
+    const BwdItem next(p, n + 1);
+    const int k0 = w.k0, key = k0 + r;
+    for (int it = 0; it < w.n_it; ++it, ++g) {
+      const int q0 = (w.i0 + it % w.nq_it) * 128;
+      const float* stat = wstat + (g & 1) * 64;
+      if (!mbar_wait_warp(s_full, g & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       if (threadIdx.x == 64) FB_STAMP(8 + 3 * it);
       __syncwarp();  // the statistics of this block are in place (written by this warp)
@@ -366,7 +396,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(s_empty);  // one arrival per warp: arrivals on one mbarrier are serialised
-          if (it + 1 < n_it) stat_load(it + 1, stat_next_l, stat_next_d);
+          if (it + 1 < w.n_it) stat_load(w, it + 1, stat_next_l, stat_next_d);
+          else if (next.valid) stat_load(next, 0, stat_next_l, stat_next_d);
         }
         // statistics as 16-byte broadcast loads; one MUFU op and half a conversion per element
         const float4* l4 = reinterpret_cast<const float4*>(stat + half * 16);
@@ -394,18 +425,23 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       };
       if (need_mask) softmax_block(std::true_type{});   // two copies of the loop: interior blocks carry no selects
       else softmax_block(std::false_type{});
-      // the warp's other statistics stage was last read in block it - 1
-      if (it + 1 < n_it) {
-        wstat[((it + 1) & 1) * 64 + lane] = stat_next_l;
-        wstat[((it + 1) & 1) * 64 + 32 + lane] = stat_next_d;
-      }
+      // the warp's other statistics stage was last read in the block before
+      wstat[((g + 1) & 1) * 64 + lane] = stat_next_l;
+      wstat[((g + 1) & 1) * 64 + 32 + lane] = stat_next_d;
       // Software pipeline (when dQ has its own TMEM columns): the arithmetic above ran while the MMAs of the previous
       // block were still reading its P^T / dS^T tiles; only now wait for them, publish this block's tiles, and read the
       // previous block's dQ out of TMEM while this block's MMAs run.
       if (threadIdx.x == 64) FB_STAMP(33 + 3 * it);
       if (OVERLAP && it > 0) {
-        if (!mbar_wait_warp(mma2_done, (it - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+        if (!mbar_wait_warp(mma2_done, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
         tc_fence_after();
+      }
+      if (!OVERLAP && g > 0) {         // every warp's dQ boxes of the block before, which lie in the tiles, have been read
+        if (lane == 0) {
+          bulk_wait_read();
+          mbar_arrive(dqs_free);
+        }
+        if (!mbar_wait_warp(dqs_free, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_MISC)) { ok = false; break; }
       }
       if (threadIdx.x == 64) FB_STAMP(34 + 3 * it);
 #pragma unroll
@@ -419,24 +455,24 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       if (lane == 0) mbar_arrive(pds_full);
       if (threadIdx.x == 64) FB_STAMP(9 + 3 * it);
       if (OVERLAP) {
-        if (it > 0) dq_readout(it - 1);
+        if (it > 0) dq_readout(w, it - 1);
         if (threadIdx.x == 64) FB_STAMP(10 + 3 * it);
       } else {
-        if (!mbar_wait_warp(mma2_done, it & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+        if (!mbar_wait_warp(mma2_done, g & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
         tc_fence_after();
-        dq_readout(it);
+        dq_readout(w, it);
       }
     }
-    if (OVERLAP && ok && n_it > 0) {
-      if (mbar_wait_warp(mma2_done, (n_it - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) {
+    if (OVERLAP && ok) {
+      if (mbar_wait_warp(mma2_done, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) {
         tc_fence_after();
-        dq_readout(n_it - 1);
+        dq_readout(w, w.n_it - 1);
       } else {
         ok = false;
       }
     }
     // dK, dV: the last mma2_done covers every accumulation. TMEM lanes are key rows.
-    if (ok && n_it > 0) {
+    if (ok) {
       tc_fence_after();
 #pragma unroll
       for (int which = 0; which < 2; ++which) {
@@ -451,7 +487,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           else tmem_ld_32x32(t_lane + colbase + col0, rr);
           tmem_ld_wait();
           if (key < p.S) {
-            __nv_bfloat16* dst = outp + ((size_t)b * p.S + key) * ld + hk * D + col0;
+            __nv_bfloat16* dst = outp + ((size_t)w.b * p.S + key) * ld + w.hk * D + col0;
 #pragma unroll
             for (int g = 0; g < DC / 8; ++g) {
               uint4 o;
@@ -467,7 +503,9 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       tc_fence_before();
       if (threadIdx.x == 64) FB_STAMP(4);
     }
-    if (DQ_TMA && lane == 0) bulk_wait_all();  // this warp's reduce copies must have landed before the grid ends
+    w = next;
+    }
+    if (lane == 0) bulk_wait_all();  // this warp's reduce copies must have landed before the grid ends
   }
 
   __syncthreads();
@@ -586,7 +624,8 @@ extern "C" int inv_flash_attn_bwd(const void* q, const void* k, const void* v, c
   p.lse = lse; p.delta = delta; p.dq_acc = dq_acc;
   p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv; p.ld_dk = ld_dk; p.ld_dv = ld_dv;
   p.B = B; p.S = S; p.H = H; p.Hkv = Hkv; p.scale = scale; p.causal = causal ? 1 : 0; p.window = window >= S ? 0 : window; p.status = status;
-  dim3 grid((S + 127) / 128, Hkv, B);
+  const long items = (long)((S + 127) / 128) * Hkv * B;
+  const dim3 grid((unsigned)(items < 148 ? items : 148));
   static bool configured = false;
   if (!configured) {
     cudaFuncSetAttribute(flash_bwd_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<1>::TOTAL);
