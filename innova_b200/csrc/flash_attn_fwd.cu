@@ -7,13 +7,21 @@
 // Layout: q, k, v are token-major views [B*S, ld] of one fused qkv buffer; head h of q occupies
 // columns [h*D, (h+1)*D). The output is token-major [B*S, H*D], ready for the o-projection GEMM.
 //
-// One CTA per (batch, head, 128-query block), 192 threads:
-//   warp 0    TMA producer: Q once, then K_j / V_j tiles through a ring of five (D = 64) or four slots (128B swizzle).
+// Two persistent CTAs per SM, 192 threads each; their work items are (batch, head, 128-query block):
+//   warp 0    TMA producer: Q, then K_j / V_j tiles through a ring of four (D = 64) or two slots (128B swizzle), on into the next item.
 //   warp 1    MMA issuer: S = Q K_j^T (128x128 fp32 in TMEM), then O += P_j V_j (128xD in TMEM, P read from TMEM).
 //   warps 2-5 softmax, one query row per thread: read S from TMEM, online max / exp2 / sum, write P_j back to
 //             tensor memory as packed bf16 (the A operand of the PV MMA); O and the row sums stay in TMEM with a lazy rescale.
-// For D = 64 two CTAs share an SM, so one CTA's softmax overlaps the other's MMAs. Every wait is bounded and
-// reports through *status.
+// One CTA's softmax overlaps the other's MMAs. Every wait is bounded and reports through *status.
+//
+// The loop over key blocks is bound by the exponentials (1,024 cycles of the special-function units for a block of an SM; a pair of CTAs takes
+// 1,400 a block). What was lost lay around it: an item of 4.5 blocks (1024 tokens, causal) paid for set-up, first loads and read-out
+// once more than the loop, with half an SM idle. In a persistent CTA the next item's operands are loaded and its first scores computed under this
+// item's last exponentials. For D = 128 the tiles and tensor memory of one CTA filled an SM: P now takes the place of the scores it was
+// computed from, and two ring slots do, since the other CTA covers the loads. 64 x 1024, 12 heads of 64: 278 -> 266 us; 2 x 2048, 16 heads of
+// 128: 62.5 -> 57.2; 64 x 512, 32 heads of 128 on 8: 442 -> 307. What is left between the loop and the read-out is a warp's own chain of a few
+// hundred instructions, and the mask of the diagonal blocks (without any mask code: 237 us; by pieces of 32 columns with dead pieces
+// skipped, in registers or in tensor memory, 335 to 344, since more of the scores leave the 168 registers).
 #include "sm100_common.cuh"
 #include "inv_api.h"
 
@@ -28,13 +36,14 @@ struct FlashFwdParams {
   __nv_bfloat16* out;
   int ld_o;
   float* lse;  // [B, H, S], log2 of the softmax denominator (scores scaled by scale*log2 e)
-  int B, S, H, Hkv;
+  int B, S, H, Hkv, group;
   float scale;
   int causal;
   int window;  // > 0 (causal only): a query sees the `window` most recent keys, its own position included
   int chunk;   // EXT; > 0 (causal only): a query sees the earlier keys of its own chunk of `chunk` positions (counted from position 0)
   const __nv_bfloat16* gate;  // EXT: the output is multiplied by sigmoid(gate), element by element; null: no gate
   int ld_gate;
+  uint32_t inv_per, inv_h, inv_group;  // of the divisors in FwdItems (fa_reciprocal)
   const int* cu;  // packed batch: sequence b is rows [cu[b], cu[b + 1]) of the token-major buffers; null: B sequences of S rows
   int* status;
 };
@@ -46,66 +55,99 @@ struct FlashFwdParams {
 // exponentials even started, ~1200 in the PV MMA plus a separate row-sum MMA, and ~1800 in the
 // exponential phase itself (MUFU-bound). This kernel
 //   * keeps P in tensor memory: the softmax threads write packed bf16 pairs with tcgen05.st and the PV MMA
-//     reads its A operand from TMEM, so the 32 KB shared-memory P tile, its stores and the proxy fence are
-//     gone and the K/V ring grows to five slots (loads run two key blocks ahead);
+//     reads its A operand from TMEM, so the 32 KB shared-memory P tile, its stores and the proxy fence are gone;
 //   * computes the exponentials into registers *before* it waits for the previous PV MMA, which is only
 //     needed for the TMEM store of P (and the rare rescale of O);
 //   * sums the exponentials on the FMA pipe: packed bf16 adds over groups of four, then fp32.
-// TMEM columns per CTA: S [0,128) fp32, O [128,128+D) fp32, P [128+D, 192+D) packed bf16.
+// TMEM columns per CTA: S [0,128) fp32, O [128,128+D) fp32, P packed bf16: [192,256) for D = 64, [0,64) for D = 128.
 // ------------------------------------------------------------------------------------------------
-template <int ND>
+// TWO: two CTAs share an SM.
+template <int ND, bool TWO>
 struct Fwd3Smem {
   static constexpr int TILE = ND * 16384;
-  static constexpr int SLOTS = ND == 1 ? 5 : 4;
+  static constexpr int QB = ND == 1 ? 2 : 1;     // Q tiles: the next item's is loaded ahead where there is room
+  static constexpr int SLOTS = TWO && ND == 2 ? 2 : 4;
   static constexpr int Q_OFF = 0;
-  static constexpr int KV_OFF = TILE;
+  static constexpr int KV_OFF = QB * TILE;
   static constexpr int BAR_OFF = KV_OFF + SLOTS * TILE;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
+// Walks a CTA's items: numbered head by head and query block by query block, the longest (causal) first; every other round runs backwards over the
+// CTAs, so that long and short items even out. Blocks past the end of a packed sequence are skipped.
+__host__ __device__ inline uint32_t fa_reciprocal(int d) { return d == 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d); }
+__device__ __forceinline__ int fa_divide(int n, int d, uint32_t inv) {
+  if (inv == 0) return n;
+  const int q = (int)__umulhi((uint32_t)n, inv);       // at most one too high for n < 2^31
+  return q * d > n ? q - 1 : q;
+}
+struct FwdItems {
+  int round = 0, b, h, hk, q0, q_blk, row_base, S, bz, jlo, nkb;
+  bool valid = false;
+  template <bool EXT>
+  __device__ __forceinline__ void next(const FlashFwdParams& p) {
+    const int per = (p.S + FA_BM - 1) / FA_BM, total = per * p.H * p.B, grid = gridDim.x, cta = blockIdx.x;
+    for (;;) {
+      const int idx = round * grid + ((round & 1) ? grid - 1 - cta : cta);
+      ++round;
+      if (idx >= total) {
+        valid = false;
+        return;
+      }
+      const int r = fa_divide(idx, per, p.inv_per), x = idx - r * per;
+      b = fa_divide(r, p.H, p.inv_h);
+      h = r - b * p.H;
+      row_base = p.cu ? p.cu[b] : 0;             // first row of the sequence in its tensor-map slice
+      S = p.cu ? p.cu[b + 1] - row_base : p.S;
+      q_blk = (S + FA_BM - 1) / FA_BM - 1 - x;
+      if (q_blk >= 0) break;
+    }
+    valid = true;
+    bz = p.cu ? 0 : b;
+    hk = fa_divide(h, p.group, p.inv_group);
+    q0 = q_blk * FA_BM;
+    const int nkb_all = (S + FA_BN - 1) / FA_BN;
+    // key blocks visited: [jlo, jlo + nkb). A sliding window skips the blocks that lie wholly before the first query's window, a
+    // chunked mask those before the first query's chunk.
+    jlo = !p.causal ? 0 : p.window > 0 ? max(0, q0 - p.window + 1) / FA_BN : EXT && p.chunk > 0 ? (q0 - q0 % p.chunk) / FA_BN : 0;
+    nkb = (p.causal ? min(nkb_all, q_blk + 1) : nkb_all) - jlo;
+  }
+};
+
 // EXT: with the chunked mask and the output gate (registers the plain form does not spend).
-template <int ND, bool EXT>
-__global__ void __launch_bounds__(FA_THREADS, ND == 1 ? 2 : 1)
+template <int ND, bool EXT, bool TWO>
+__global__ void __launch_bounds__(FA_THREADS, TWO ? 2 : 1)
 flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                   const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ FlashFwdParams p) {
   constexpr int D = 64 * ND;
-  using L = Fwd3Smem<ND>;
-  constexpr int SLOTS = L::SLOTS;
+  using L = Fwd3Smem<ND, TWO>;
+  constexpr int SLOTS = L::SLOTS, QB = L::QB;
+  constexpr bool ALIAS = TWO && ND == 2;      // P over the scores: the next scores wait for the values' product
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem + L::Q_OFF;
   uint8_t* sKV = smem + L::KV_OFF;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-  uint64_t* q_full = bars;              // 1
-  uint64_t* kv_full = bars + 1;         // SLOTS
-  uint64_t* kv_empty = bars + 1 + SLOTS;  // SLOTS
-  uint64_t* s_full = bars + 1 + 2 * SLOTS;
-  uint64_t* s_empty = s_full + 1;       // 128 arrivals
-  uint64_t* p_full = s_full + 2;        // 128 arrivals
+  uint64_t* q_full = bars;              // QB
+  uint64_t* q_empty = q_full + QB;      // QB: the item's last scores have been computed
+  uint64_t* kv_full = q_empty + QB;     // SLOTS
+  uint64_t* kv_empty = kv_full + SLOTS; // SLOTS
+  uint64_t* s_full = kv_empty + SLOTS;
+  uint64_t* s_empty = s_full + 1;       // one arrival per softmax warp
+  uint64_t* p_full = s_full + 2;        // one arrival per softmax warp
   uint64_t* o_full = s_full + 3;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int row_base = p.cu ? p.cu[b] : 0;      // first row of the sequence in its tensor-map slice
-  const int S = p.cu ? p.cu[b + 1] - row_base : p.S;
-  const int bz = p.cu ? 0 : b;
-  const int nqb = (S + FA_BM - 1) / FA_BM;
-  const int q_blk = nqb - 1 - (int)blockIdx.x;
-  if (q_blk < 0) return;                        // packed batches: the grid covers the longest sequence
-  const int hk = h / (p.H / p.Hkv);
-  const int q0 = q_blk * FA_BM;
-  const int nkb_all = (S + FA_BN - 1) / FA_BN;
-  // key blocks visited: [jlo, jlo + nkb). A sliding window skips the blocks that lie wholly before the first query's window, a
-  // chunked mask those before the first query's chunk.
-  const int jlo = !p.causal ? 0 : p.window > 0 ? max(0, q0 - p.window + 1) / FA_BN : EXT && p.chunk > 0 ? (q0 - q0 % p.chunk) / FA_BN : 0;
-  const int nkb = (p.causal ? min(nkb_all, q_blk + 1) : nkb_all) - jlo;
-  constexpr uint32_t TMEM_COLS = ND == 1 ? 256 : 512;
-  constexpr uint32_t O_COL = 128, P_COL = 128 + D;
+  constexpr uint32_t TMEM_COLS = TWO ? 256 : 512;
+  constexpr uint32_t O_COL = 128, P_COL = ALIAS ? 0 : 128 + D;
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
+    for (int i = 0; i < QB; ++i) {
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
+    }
     for (int i = 0; i < SLOTS; ++i) {
       mbar_init(&kv_full[i], 1);
       mbar_init(&kv_empty[i], 1);
@@ -131,18 +173,26 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 
   if (warp == 0) {
     if (elect_one_sync()) {
-      mbar_expect_tx(q_full, L::TILE);
+      bool ok = true;
+      int load = 0;                    // K and V tiles over all items
+      FwdItems w;
+      w.next<EXT>(p);
+      for (int n = 0; ok && w.valid; ++n, w.next<EXT>(p)) {
+        const int qb = n % QB;
+        if (!mbar_wait(&q_empty[qb], ((n / QB) & 1) ^ 1, abort_flag, p.status, ERR_WAIT_EMPTY)) break;
+        mbar_expect_tx(&q_full[qb], L::TILE);
 #pragma unroll
-      for (int a = 0; a < ND; ++a) tma_load_3d(sQ + a * 16384, &tmap_q, q_full, h * D + a * 64, row_base + q0, bz);
-      for (int n = 0; n < 2 * nkb; ++n) {
-        const int slot = n % SLOTS;
-        const uint32_t ph = (n / SLOTS) & 1;
-        if (!mbar_wait(&kv_empty[slot], ph ^ 1, abort_flag, p.status, ERR_WAIT_EMPTY)) break;
-        mbar_expect_tx(&kv_full[slot], L::TILE);
-        const int j = jlo + (n >> 1);
-        const CUtensorMap* tm = (n & 1) ? &tmap_v : &tmap_k;
+        for (int a = 0; a < ND; ++a) tma_load_3d(sQ + qb * L::TILE + a * 16384, &tmap_q, &q_full[qb], w.h * D + a * 64, w.row_base + w.q0, w.bz);
+        for (int i = 0; i < 2 * w.nkb; ++i, ++load) {
+          const int slot = load % SLOTS;
+          if (!mbar_wait(&kv_empty[slot], ((load / SLOTS) & 1) ^ 1, abort_flag, p.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+          mbar_expect_tx(&kv_full[slot], L::TILE);
+          const int j = w.jlo + (i >> 1);
+          const CUtensorMap* tm = (i & 1) ? &tmap_v : &tmap_k;
 #pragma unroll
-        for (int a = 0; a < ND; ++a) tma_load_3d(sKV + slot * L::TILE + a * 16384, tm, &kv_full[slot], hk * D + a * 64, row_base + j * FA_BN, bz);
+          for (int a = 0; a < ND; ++a)
+            tma_load_3d(sKV + slot * L::TILE + a * 16384, tm, &kv_full[slot], w.hk * D + a * 64, w.row_base + j * FA_BN, w.bz);
+        }
       }
     }
   } else if (warp == 1) {
@@ -150,51 +200,75 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const uint32_t idesc_qk = make_idesc_bf16(128, 128, 0, 0);
       const uint32_t idesc_pv = make_idesc_bf16(128, D, 0, 1);
       const uint32_t q_base = smem_u32(sQ);
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.status, ERR_WAIT_FULL);
-      auto issue_qk = [&](int j) -> bool {
-        const int n = 2 * j, slot = n % SLOTS;
-        if (!mbar_wait(&kv_full[slot], (n / SLOTS) & 1, abort_flag, p.status, ERR_WAIT_FULL)) return false;
-        if (j > 0 && !mbar_wait(s_empty, (j - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) return false;
+      // scores of block g over all items, whose keys are tile `load`: block j of nkb of the CTA's item n
+      auto issue_qk = [&](int g, int load, int n, int j, int nkb) -> bool {
+        const int slot = load % SLOTS, qb = n % QB;
+        if (j == 0 && !mbar_wait(&q_full[qb], (n / QB) & 1, abort_flag, p.status, ERR_WAIT_FULL)) return false;
+        if (!mbar_wait(&kv_full[slot], (load / SLOTS) & 1, abort_flag, p.status, ERR_WAIT_FULL)) return false;
+        if (!ALIAS && g > 0 && !mbar_wait(s_empty, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) return false;
         tc_fence_after();
-        const uint32_t k_base = smem_u32(sKV + slot * L::TILE);
+        const uint32_t k_base = smem_u32(sKV + slot * L::TILE), a_base = q_base + qb * L::TILE;
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
           const uint32_t off = (ks / 4) * 16384 + (ks % 4) * 32;
-          umma_bf16(tmem_base, make_smem_desc(q_base + off, 16, 1024, 2), make_smem_desc(k_base + off, 16, 1024, 2), idesc_qk, ks > 0);
+          umma_bf16(tmem_base, make_smem_desc(a_base + off, 16, 1024, 2), make_smem_desc(k_base + off, 16, 1024, 2), idesc_qk, ks > 0);
         }
         umma_commit(s_full);
         umma_commit(&kv_empty[slot]);
+        if (j + 1 == nkb) umma_commit(&q_empty[qb]);
         return true;
       };
-      if (ok) ok = issue_qk(0);
-      for (int j = 0; ok && j < nkb; ++j) {
-        if (j + 1 < nkb) {
-          if (!issue_qk(j + 1)) break;
-        }
-        const int n = 2 * j + 1, slot = n % SLOTS;
-        if (!mbar_wait(p_full, j & 1, abort_flag, p.status, ERR_WAIT_MISC)) break;
-        if (!mbar_wait(&kv_full[slot], (n / SLOTS) & 1, abort_flag, p.status, ERR_WAIT_FULL)) break;
-        tc_fence_after();
-        const uint32_t v_base = smem_u32(sKV + slot * L::TILE);
+      FwdItems w;
+      w.next<EXT>(p);
+      bool ok = w.valid && issue_qk(0, 0, 0, 0, w.nkb);
+      int g = 0, load = 0;             // load: the item's first K tile
+      for (int n = 0; ok && w.valid; ++n) {
+        FwdItems nx = w;
+        nx.next<EXT>(p);
+        for (int j = 0; j < w.nkb; ++j, ++g) {
+          // the scores behind these: this item's next block or the next item's first
+          auto ahead = [&]() {
+            if (j + 1 < w.nkb) return issue_qk(g + 1, load + 2 * (j + 1), n, j + 1, w.nkb);
+            return !nx.valid || issue_qk(g + 1, load + 2 * w.nkb, n + 1, 0, nx.nkb);
+          };
+          if (!ALIAS && !ahead()) { ok = false; break; }
+          const int v = load + 2 * j + 1, slot = v % SLOTS;
+          if (!mbar_wait(p_full, g & 1, abort_flag, p.status, ERR_WAIT_MISC)) { ok = false; break; }
+          if (!mbar_wait(&kv_full[slot], (v / SLOTS) & 1, abort_flag, p.status, ERR_WAIT_FULL)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t v_base = smem_u32(sKV + slot * L::TILE);
+          // An item's first product overwrites O: the softmax warps published its P after they had read the last item's O.
 #pragma unroll
-        for (int ks = 0; ks < FA_BN / 16; ++ks)  // 16 keys = 8 packed columns of P per step
-          umma_bf16_tmem_a(tmem_base + O_COL, tmem_base + P_COL + ks * 8, make_smem_desc(v_base + ks * 2048, 16384, 1024, 2), idesc_pv,
-                           (j > 0 || ks > 0) ? 1u : 0u);
-        umma_commit(o_full);
-        umma_commit(&kv_empty[slot]);
+          for (int ks = 0; ks < FA_BN / 16; ++ks)  // 16 keys = 8 packed columns of P per step
+            umma_bf16_tmem_a(tmem_base + O_COL, tmem_base + P_COL + ks * 8, make_smem_desc(v_base + ks * 2048, 16384, 1024, 2), idesc_pv,
+                             (j > 0 || ks > 0) ? 1u : 0u);
+          umma_commit(o_full);
+          umma_commit(&kv_empty[slot]);
+          if (ALIAS) {                 // P has been read: the next scores may take its place
+            if (!mbar_wait(o_full, g & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+            if (!ahead()) { ok = false; break; }
+          }
+        }
+        load += 2 * w.nkb;
+        w = nx;
       }
     }
   } else {
     // ---------------- softmax warps: thread <-> query row ----------------
     const int q = warp & 3;
     const int r = q * 32 + lane;
-    const int row = q0 + r;
     const uint32_t t_lane = tmem_base + (uint32_t(q * 32) << 16);
     const float c = p.scale * 1.4426950408889634f;
-    float m_used = -INFINITY, l = 0.f;
     bool ok = true;
-    for (int j = 0; j < nkb; ++j) {
-      if (!mbar_wait_warp(s_full, j & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+    int g = 0;                         // key blocks over all items
+    FwdItems w;
+    w.next<EXT>(p);
+    while (ok && w.valid) {
+    const int h = w.h, b = w.b, row_base = w.row_base, S = w.S, q0 = w.q0, jlo = w.jlo, nkb = w.nkb;
+    const int row = q0 + r;
+    float m_used = -INFINITY, l = 0.f;
+    for (int j = 0; j < nkb; ++j, ++g) {
+      if (!mbar_wait_warp(s_full, g & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const int k0 = (jlo + j) * FA_BN;
       const bool windowed = p.causal && p.window > 0, chunked = EXT && p.causal && p.chunk > 0;
@@ -210,8 +284,10 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       tmem_ld_32x32(t_lane + 96, sr + 96);
       tmem_ld_wait();
       tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(s_empty);  // the scores live in registers now: the next QK^T may start (one arrival per warp)
+      if (!ALIAS) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_empty);  // the scores live in registers now: the next QK^T may start (one arrival per warp)
+      }
       if (need_mask) {
 #pragma unroll
         for (int i = 0; i < 128; ++i)
@@ -246,7 +322,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       l = l * alpha + (rs0 + rs1);
       if (j > 0) {
         // PV of the previous block is complete: P may be overwritten, O is stable
-        if (!mbar_wait_warp(o_full, (j - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+        if (!mbar_wait_warp(o_full, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
         tc_fence_after();
         if (any_rescale) {
 #pragma unroll 1
@@ -267,6 +343,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
     }
+    w.next<EXT>(p);                    // while the last product runs
     uint4 gv[EXT ? D / 8 : 1];                    // the row's gate, requested while the last PV MMA runs
     const bool gated = EXT && p.gate != nullptr;
     if (gated && row < S) {
@@ -274,7 +351,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
       for (int i = 0; i < (EXT ? D / 8 : 1); ++i) gv[i] = *reinterpret_cast<const uint4*>(gate + i * 8);
     }
-    if (ok) ok = mbar_wait_warp(o_full, (nkb - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
+    if (ok) ok = mbar_wait_warp(o_full, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
     if (ok) {
       tc_fence_after();
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
@@ -311,6 +388,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       }
       if (p.lse && row < S) p.lse[((size_t)b * p.H + h) * S + row] = m_used * c + log2f(l);
       tc_fence_before();
+    }
     }
   }
 
@@ -390,21 +468,29 @@ static int flash_fwd_launch(const void* q, const void* k, const void* v, void* o
   p.window = window >= max_len ? 0 : window;
   p.chunk = chunk >= max_len ? 0 : chunk;
   p.gate = (const __nv_bfloat16*)gate; p.ld_gate = ld_gate;
-  dim3 grid((max_len + FA_BM - 1) / FA_BM, H, n_seq);
+  const int per = (max_len + FA_BM - 1) / FA_BM;
+  p.group = H / Hkv;
+  p.inv_per = fa_reciprocal(per); p.inv_h = fa_reciprocal(H); p.inv_group = fa_reciprocal(p.group);
+  const long items = (long)per * H * n_seq;
+  // 128-wide heads: while every item has an SM to itself, one CTA an SM with scores and P side by side (2 x 300 tokens, 16 heads on 4: 8.8 us
+  // against 12.5); beyond, two CTAs that overlap (64 x 512, 32 heads on 8: 442 -> 307 us).
+  const bool two = head_dim == 64 || items > 148;
+  const dim3 grid((unsigned)(items < (two ? 2 * 148 : 148) ? items : (two ? 2 * 148 : 148)));
   cudaStream_t st = (cudaStream_t)stream;
   static bool configured = false;
   if (!configured) {
-    cudaFuncSetAttribute(flash_fwd3_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd3Smem<1>::TOTAL);
-    cudaFuncSetAttribute(flash_fwd3_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd3Smem<2>::TOTAL);
-    cudaFuncSetAttribute(flash_fwd3_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd3Smem<1>::TOTAL);
-    cudaFuncSetAttribute(flash_fwd3_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd3Smem<2>::TOTAL);
+#define INV_FA(ND, EXT, TWO) \
+  cudaFuncSetAttribute(flash_fwd3_kernel<ND, EXT, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd3Smem<ND, TWO>::TOTAL)
+    INV_FA(1, false, true); INV_FA(1, true, true); INV_FA(2, false, true); INV_FA(2, true, true); INV_FA(2, false, false); INV_FA(2, true, false);
+#undef INV_FA
     configured = true;
   }
   const bool ext = p.gate || p.chunk;
-  if (head_dim == 64 && ext) flash_fwd3_kernel<1, true><<<grid, FA_THREADS, Fwd3Smem<1>::TOTAL, st>>>(tq, tk, tv, p);
-  else if (head_dim == 64) flash_fwd3_kernel<1, false><<<grid, FA_THREADS, Fwd3Smem<1>::TOTAL, st>>>(tq, tk, tv, p);
-  else if (ext) flash_fwd3_kernel<2, true><<<grid, FA_THREADS, Fwd3Smem<2>::TOTAL, st>>>(tq, tk, tv, p);
-  else flash_fwd3_kernel<2, false><<<grid, FA_THREADS, Fwd3Smem<2>::TOTAL, st>>>(tq, tk, tv, p);
+#define INV_FA(ND, EXT, TWO) flash_fwd3_kernel<ND, EXT, TWO><<<grid, FA_THREADS, Fwd3Smem<ND, TWO>::TOTAL, st>>>(tq, tk, tv, p)
+  if (head_dim == 64) { if (ext) INV_FA(1, true, true); else INV_FA(1, false, true); }
+  else if (two) { if (ext) INV_FA(2, true, true); else INV_FA(2, false, true); }
+  else { if (ext) INV_FA(2, true, false); else INV_FA(2, false, false); }
+#undef INV_FA
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
