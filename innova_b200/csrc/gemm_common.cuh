@@ -17,6 +17,7 @@ struct GemmParams {
   int ld_aux;
   __nv_bfloat16* aux_out;
   int epilogue;
+  int half = 0;  // EPI_SWIGLU: the up rows of B start this many rows below the gate rows
   float alpha;
   int* status;
   // Grouped (mixture-of-experts) operation, single-CTA kernel only. Rows of A are grouped in
@@ -259,6 +260,36 @@ __device__ __forceinline__ void gemm_epilogue_fixed(float alpha, const uint4* bv
       }
     }
     *reinterpret_cast<uint4*>(stg_c + at) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+  }
+}
+
+// silu(gate) * up of 32 columns from column `col` on, of N, into half `sub` of a box. Both are rounded to bf16 first, as the product of its own that a
+// separate activation reads. bias: of the gate columns, that of the up columns `half` further on, or null.
+__device__ __forceinline__ void gemm_epilogue_swiglu(float alpha, const __nv_bfloat16* bias, int half, int col, int N, const uint32_t* gate, const uint32_t* up,
+                                                     uint8_t* stg, int sub, int lane) {
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    uint4 bg = make_uint4(0, 0, 0, 0), bu = bg;
+    if (bias != nullptr && col + g * 8 < N) {
+      bg = __ldg(reinterpret_cast<const uint4*>(bias + col + g * 8));
+      bu = __ldg(reinterpret_cast<const uint4*>(bias + half + col + g * 8));
+    }
+    const uint32_t wg[4] = {bg.x, bg.y, bg.z, bg.w}, wu[4] = {bu.x, bu.y, bu.z, bu.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float y[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int i = g * 8 + 2 * j + e;
+        const float bgf = __uint_as_float(e ? wg[j] & 0xffff0000u : wg[j] << 16), buf = __uint_as_float(e ? wu[j] & 0xffff0000u : wu[j] << 16);
+        const float a = __bfloat162float(__float2bfloat16_rn(__uint_as_float(gate[i]) * alpha + bgf));
+        const float b = __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[i]) * alpha + buf));
+        y[e] = silu_f(a) * b;
+      }
+      o[j] = pack_bf16x2(y[0], y[1]);
+    }
+    *reinterpret_cast<uint4*>(stg + (((sub * 4 + g) ^ (lane & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 

@@ -579,6 +579,26 @@ extern "C" int inv_gemm_grouped(const void* A, const void* B, void* C, int M, in
   return launch_gemm<false, false>(ta, tb, p, grid, st);
 }
 
+// C[M, F] = silu(A Wg^T + bg) * (A Wu^T + bu): Wg rows [0, F) of B, Wu rows [half, half + F); bias (optional) laid out as B's rows. One CTA of a
+// pair loads gate rows, the other up rows, so that a tile's accumulator holds both halves of 128 output columns and the pair's product is never
+// stored: 32768 x 11008 x 4096 saves the write and the reading of 1.44 GB. M > 128, K-major operands, rows on 16 bytes, F % 8 == 0.
+extern "C" int inv_gemm_swiglu_bf16(const void* A, const void* B, void* C, int M, int F, int K, int lda, int ldb, int ldc, int half, const void* bias,
+                                    int* status, void* stream) {
+  if (M <= 0 || F <= 0 || K <= 0) return 0;
+  if (M <= 128 || (F % 8) || half < F || (half % 8) || (lda % 8) || (ldb % 8) || (ldc % 8) || ((uintptr_t)A | (uintptr_t)B | (uintptr_t)C | (uintptr_t)bias) % 16)
+    return -ERR_BAD_ARG;
+  if (g_num_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+    if (g_num_sms <= 0) g_num_sms = 148;
+  }
+  GemmParams p;
+  fill_plain(p, M, F, K, C, ldc, 0, bias, nullptr, 0, nullptr, EPI_SWIGLU, 1.0f, status);
+  p.half = half;
+  return gemm_2cta_dispatch(A, B, p, lda, ldb, 0, 0, g_num_sms, reinterpret_cast<cudaStream_t>(stream));
+}
+
 // GEMM fused with a reduce-scatter, push form: every rank computes the full [M, N] partial product of its K-slice in
 // bf16 and its epilogue stores the tile rows owned by rank r straight into this rank's slot of r's receive buffer
 // (peer_slots[r], [M / W, ldc] bf16, plain 16-byte stores: posted writes over NVLink, no atomics), visiting the

@@ -93,6 +93,8 @@ struct WorkUnit2 {
   int m0, n0, kb_begin, kb_end;
   int ag_tile;  // 256-row tile of the gathered operand this unit reads, -1 when it is local or nothing is gathered
 };
+// TN: output columns of a tile.
+template <int TN>
 __device__ __forceinline__ WorkUnit2 decode_work2(int w, const GemmParams& p, int m_tiles, int n_tiles, int kb_total, int kb_per_split) {
   WorkUnit2 u;
   u.ag_tile = -1;
@@ -102,7 +104,7 @@ __device__ __forceinline__ WorkUnit2 decode_work2(int w, const GemmParams& p, in
     const int rest = w / m_tiles;
     n_blk = rest % n_tiles;
     ks = rest / n_tiles;
-    const int per = p.ag_shard_rows / g2::BN;
+    const int per = p.ag_shard_rows / TN;
     n_blk = (n_blk + p.ag_rank * per) % n_tiles;
     if (n_blk / per != p.ag_rank) u.ag_tile = n_blk;
   } else {
@@ -119,7 +121,7 @@ __device__ __forceinline__ WorkUnit2 decode_work2(int w, const GemmParams& p, in
     }
   }
   u.m0 = m_blk * g2::BM;
-  u.n0 = n_blk * g2::BN;
+  u.n0 = n_blk * TN;
   u.kb_begin = ks * kb_per_split;
   u.kb_end = min(kb_total, u.kb_begin + kb_per_split);
   return u;
@@ -161,7 +163,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   const int pair = ((int)blockIdx.x - n_copy) >> 1, npairs = ((int)gridDim.x - n_copy) >> 1;
 
   const int m_tiles = (p.M + BM - 1) / BM;
-  const int n_tiles = (p.N + BN - 1) / BN;
+  constexpr int TN = EPI == EPI_SWIGLU ? BN / 2 : BN;   // SwiGLU: the tile's 256 columns are 128 of the gate and 128 of the up product
+  const int n_tiles = (p.N + TN - 1) / TN;
   const int kb_total = (p.K + BK - 1) / BK;
   const int kb_per_split = (kb_total + p.split_k - 1) / p.split_k;
   const int total_work = m_tiles * n_tiles * p.split_k;
@@ -199,9 +202,9 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       int it = 0;
       bool ok = true;
       for (int w = pair; ok && w < total_work; w += npairs) {
-        const WorkUnit2 u = decode_work2(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
+        const WorkUnit2 u = decode_work2<TN>(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
         const int my_m0 = u.m0 + (int)cta * 128;
-        const int my_n0 = u.n0 + (int)cta * 128;
+        const int my_n0 = EPI == EPI_SWIGLU ? u.n0 + (int)cta * p.half : u.n0 + (int)cta * 128;   // this CTA's 128 rows of B
         if (u.ag_tile >= 0 && !ag_wait_tile(p, u.ag_tile, abort_flag)) break;
         for (int kb = u.kb_begin; kb < u.kb_end; ++kb, ++it) {
           const int s = it % STAGES;
@@ -246,7 +249,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       uint32_t ph = 0;
       bool ok = true;
       for (int w = pair; ok && w < total_work; w += npairs, ++tile_i) {
-        const WorkUnit2 u = decode_work2(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
+        const WorkUnit2 u = decode_work2<TN>(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
         const int acc = tile_i & 1;
         const uint32_t acc_ph = (tile_i >> 1) & 1;
         if (!mbar_wait(&tmem_empty[acc], acc_ph ^ 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) break;
@@ -283,14 +286,16 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       const bool two_out = INV_EPI_WRITES_AUX(EPI) && p.aux_out != nullptr;
       uint8_t* my_stage = sStage + (warp - 2) * 8192;
       uint64_t* my_aux_bar = aux_bar + (warp - 2) * 2;
-      const int row_in_tile = (int)cta * 128 + q * 32, col_in_tile = half * 128;
+      const int row_in_tile = (int)cta * 128 + q * 32;
+      constexpr int CW = EPI == EPI_SWIGLU ? 64 : 128;   // output columns of a warp
+      const int col_in_tile = half * CW;
       const float alpha = p.alpha;
       const __nv_bfloat16* bias = p.bias;
       uint32_t box = 0;                          // boxes this warp has written
       int nw = pair, nj = 0;                     // READS: the next box to request, the nj-th of unit nw
       auto request = [&](uint32_t b) {           // one lane
         while (nw < total_work) {
-          const WorkUnit2 u = decode_work2(nw, p, m_tiles, n_tiles, kb_total, kb_per_split);
+          const WorkUnit2 u = decode_work2<TN>(nw, p, m_tiles, n_tiles, kb_total, kb_per_split);
           const int col0 = u.n0 + col_in_tile + nj * 64;
           if (col0 >= p.N) { nw += npairs; nj = 0; continue; }
           mbar_expect_tx(&my_aux_bar[b & 1], 4096);
@@ -303,7 +308,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       int tile_i = 0;
       bool ok = true;
       for (int w = pair; ok && w < total_work; w += npairs, ++tile_i) {
-        const WorkUnit2 u = decode_work2(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
+        const WorkUnit2 u = decode_work2<TN>(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
         const int acc = tile_i & 1;
         if (!mbar_wait_warp(&tmem_full[acc], (tile_i >> 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) break;
         tc_fence_after();
@@ -311,10 +316,30 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         const int row0 = u.m0 + row_in_tile;
         constexpr int STEP = SUMS ? 32 : 64;     // columns of a box
 #pragma unroll 1
-        for (int c = 0; c < 128; c += STEP) {
+        for (int c = 0; c < CW; c += STEP) {
           const int col0 = u.n0 + col_in_tile + c;
           if (col0 >= p.N) break;
           uint8_t* sc = my_stage + (two_out ? 0u : (box & 1) * 4096);
+          if constexpr (EPI == EPI_SWIGLU) {
+            if (lane == 0) tma_store_wait_read_but_one();
+            __syncwarp();
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {        // 32 columns of both products at a time
+              uint32_t g[32], v[32];
+              tmem_ld_32x32(t_row + x * 32, g);
+              tmem_ld_32x32(t_row + 128 + x * 32, v);
+              tmem_ld_wait();
+              gemm_epilogue_swiglu(alpha, bias, p.half, col0 + x * 32, p.N, g, v, sc + lane * 128, x, lane);
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(&tmap_c, sc, col0, row0);
+              tma_store_commit();
+            }
+            ++box;
+            continue;
+          }
           uint32_t r[STEP];
           tmem_ld_32x32(t_row + c, r);
           if (!SUMS) tmem_ld_32x32(t_row + c + 32, r + STEP - 32);
@@ -343,8 +368,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             const uint4* b8 = bias != nullptr ? bv : nullptr;
             uint8_t* my = sc + lane * 128;
             uint8_t* my_aux = two_out ? my + 4096 : nullptr;
-            gemm_epilogue_fixed<EPI>(alpha, b8, r, my, my_aux, 0, lane);
-            gemm_epilogue_fixed<EPI>(alpha, b8 == nullptr ? nullptr : b8 + 4, r + STEP - 32, my, my_aux, 1, lane);
+            if constexpr (EPI != EPI_SWIGLU) {
+              gemm_epilogue_fixed<EPI>(alpha, b8, r, my, my_aux, 0, lane);
+              gemm_epilogue_fixed<EPI>(alpha, b8 == nullptr ? nullptr : b8 + 4, r + STEP - 32, my, my_aux, 1, lane);
+            }
           }
           fence_proxy_async_smem();
           __syncwarp();
@@ -376,7 +403,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     // (w, j): j-th 64-column box of this warp in work unit w; false when the unit or the box does not exist
     auto box_of = [&](int w, int j, int& col0, int& row0) -> bool {
       if (w >= total_work) return false;
-      const WorkUnit2 u = decode_work2(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
+      const WorkUnit2 u = decode_work2<TN>(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
       col0 = u.n0 + (half * 4 + 2 * j) * 32;
       row0 = u.m0 + row_in_tile;
       return col0 < p.N;
@@ -396,7 +423,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     int tile_i = 0;
     bool ok = true;
     for (int w = pair; ok && w < total_work; w += npairs, ++tile_i) {
-      const WorkUnit2 u = decode_work2(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
+      const WorkUnit2 u = decode_work2<TN>(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
       const int acc = tile_i & 1;
       const uint32_t acc_ph = (tile_i >> 1) & 1;
       if (!mbar_wait_warp(&tmem_full[acc], acc_ph, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) break;
@@ -506,7 +533,7 @@ int gemm_2cta_dispatch(const void* A, const void* B, const GemmParams& p0, int l
   else rc = make_tmap_2d_bf16(&ta, A, (uint64_t)p.K, (uint64_t)p.M, (uint64_t)lda, BK, 128);
   if (rc) return rc;
   if (b_mn) rc = make_tmap_2d_bf16(&tb, B, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)ldb, 64, BK);
-  else rc = make_tmap_2d_bf16(&tb, B, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)ldb, BK, 128);
+  else rc = make_tmap_2d_bf16(&tb, B, (uint64_t)p.K, (uint64_t)(p.N + p.half), (uint64_t)ldb, BK, 128);
   if (rc) return rc;
   // output maps for the staged TMA-store epilogue (bf16 C and, for the GELU epilogue, the pre-activation)
   CUtensorMap tc = ta, tx = ta;
@@ -531,7 +558,8 @@ int gemm_2cta_dispatch(const void* A, const void* B, const GemmParams& p0, int l
     split_k = (kb_total + per - 1) / per;
   }
   p.split_k = split_k;
-  const long total = (long)((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * split_k;
+  const int tn = p.epilogue == EPI_SWIGLU ? BN / 2 : BN;
+  const long total = (long)((p.M + BM - 1) / BM) * ((p.N + tn - 1) / tn) * split_k;
   // helper CTAs come in whole clusters; the whole grid must be resident at once
   int n_copy = 0;
   if (p.ag_world > 1) {
@@ -571,6 +599,7 @@ int gemm_2cta_dispatch(const void* A, const void* B, const GemmParams& p0, int l
     case EPI_ADD: INV_G2(false, false, EPI_ADD);
     case EPI_GELU_DG: INV_G2(false, false, EPI_GELU_DG);
     case EPI_ATOMIC: INV_G2(false, false, EPI_ATOMIC);
+    case EPI_SWIGLU: INV_G2(false, false, EPI_SWIGLU);
     default: INV_G2(false, false, EPI_ANY);
   }
 #undef INV_G2

@@ -17,6 +17,7 @@ enum {
   EPI_ATOMIC = 4,  // C(fp32) += alpha*acc            (split-K / gradient accumulation)
   EPI_GELU_DG = 5, // x = alpha*acc + bias; aux_out = gelu'(x); C = gelu(x)   (the backward then needs one multiply: EPI_MUL)
   EPI_MUL = 6,     // C = alpha*acc * aux_in
+  EPI_SWIGLU = 7,  // C = silu(gate) * up of two products (inv_gemm_swiglu_bf16 only)
 };
 // epilogues that write a second bf16 output / read a second bf16 operand of C's shape
 #define INV_EPI_WRITES_AUX(e) ((e) == EPI_GELU || (e) == EPI_GELU_DG)

@@ -19,7 +19,7 @@ from ..inference.state_cache import KeyValues, Latents
 from ..ops import delta_rule as dr
 from ..ops import kv_attention as ka
 from ..ops import latent_attention as la
-from ..ops.gemm import EPI_ATOMIC, NUM_SMS, SKINNY_ROWS, gemm, skinny_gemm
+from ..ops.gemm import EPI_ATOMIC, NUM_SMS, SKINNY_ROWS, gemm, gemm_swiglu, skinny_gemm
 from ..ops.hyper import gated_silu
 from ..ops.sandwich import softcap_
 
@@ -77,8 +77,11 @@ class StepContext:
         """silu(gate x) * (up x) for a projection that holds the gate rows, then (from the middle) the up rows."""
         if self.skinny:
             return skinny_gemm(x[:, : p.k], p.weight[:, : p.k], n=ff, silu_half=p.n // 2, out_dtype=torch.bfloat16, resident=True)
+        if self.bf16 and not self.small:
+            y = gemm_swiglu(x[:, : p.k], p.weight[:, : p.k], ff, p.n // 2)
+            if y is not None:
+                return y
         return gated_silu(self.project(x, p), ff, self.dtype)
-
 
     def logits(self, h: torch.Tensor, p: Proj, vocab: int, softcap=None) -> torch.Tensor:
         """fp32 [rows, vocab] of the output head, through the soft limit softcap * tanh(z / softcap) if there is one."""

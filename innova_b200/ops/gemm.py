@@ -103,6 +103,24 @@ def gemm(a, b, out=None, *, a_mn=False, b_mn=False, M=None, N=None, K=None, epil
 
 _native.register_cuda_sigs({"inv_skinny_gemm": [_native.vp, _native.i32, _native.vp] + [_native.i32] * 5 +
                                 [_native.vp, _native.i32, _native.i32, _native.f32, _native.i32, _native.vp]})
+_native.register_cuda_sigs({"inv_gemm_swiglu_bf16": [_native.vp] * 3 + [_native.i32] * 7 + [_native.vp] * 3})
+
+
+def gemm_swiglu(x, w, n, half, bias=None):
+    """silu(x Wg^T + bg) * (x Wu^T + bu) for Wg = rows [0, n) of w and Wu = rows [half, half + n), in one product whose epilogue is the activation;
+    None where the kernel does not take these operands (few rows, other types, strides or alignments)."""
+    M, K = x.shape
+    if (not x.is_cuda or x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or M <= 128 or n < 8 or n % 8 or half < n or half % 8 or w.shape[0] < half + n
+            or w.shape[1] != K or K % 8 or x.stride(1) != 1 or w.stride(1) != 1 or x.stride(0) % 8 or w.stride(0) % 8 or (x.data_ptr() | w.data_ptr()) % 16
+            or (bias is not None and (bias.dtype != torch.bfloat16 or not bias.is_contiguous() or bias.numel() < half + n or bias.data_ptr() % 16))
+            or _kernel_select == 1 or _side_job_provider is not None):
+        return None
+    out = torch.empty((M, n), dtype=torch.bfloat16, device=x.device)
+    rt.check(rt.lib().inv_gemm_swiglu_bf16(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, n, K, x.stride(0), w.stride(0), out.stride(0), half, rt.ptr(bias),
+                                           rt.status_tensor(x.device).data_ptr(), rt.stream_ptr()), "inv_gemm_swiglu_bf16")
+    return out
+
+
 SKINNY_ROWS = 32          # the kernel takes 64; beyond 32 the split-K tiled product is faster
 
 

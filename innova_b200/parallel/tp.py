@@ -237,7 +237,10 @@ class TPDecoder:
             else:
                 x = ops.linear(a, l["o"].dequantize(), l["o"].bias, residual=x, mode="add")
             h = ops.rms_norm(x, l["n2"], cfg.norm_eps)
-            act = ops.swiglu(ops.linear(h, l["gu"].dequantize(), l["gu"].bias))
+            gu, F = l["gu"].dequantize(), l["gu"].N // 2
+            act = ops.gemm_swiglu(h.view(B * S, -1), gu, F, F, l["gu"].bias)
+            act = ops.swiglu(ops.linear(h, gu, l["gu"].bias)) if act is None else act.view(B, S, F)
+            del gu
             if self.world > 1:
                 d = ops.linear(act, l["down"].dequantize())
                 dist.all_reduce(d)

@@ -151,6 +151,29 @@ def test_gemm_fixed_epilogues_stay_inside_their_view(a_mn, b_mn, epi, M, N, K):
     assert (buf == 3.0).all()
 
 
+@pytest.mark.parametrize("M,F_,K,half,bias", [(129, 8, 64, 8, False), (300, 136, 72, 136, True), (257, 128, 200, 160, True), (1000, 1408, 512, 1408, False),
+                                             (2 * 74 * 256 + 9, 392, 64, 400, True)])
+def test_gemm_swiglu_matches_product_and_activation(M, F_, K, half, bias):
+    """The product whose epilogue is the gated activation: ragged tiles, up rows further down than the gate's count, more tiles than pairs. Against
+    fp64 of the projections rounded to bf16, which leaves the rounding of the result (2^-9) and projections that round the other way (2^-8)."""
+    from innova_b200 import ops
+    torch.manual_seed(11)
+    dev = _dev()
+    x = torch.randn(M, K + 8, device=dev).bfloat16()[:, :K]
+    w = (torch.randn(half + F_, K, device=dev) * 0.2).bfloat16()
+    b = torch.randn(half + F_, device=dev).bfloat16() if bias else None
+    y = ops.gemm_swiglu(x, w, F_, half, b)
+    z = x.double() @ w.double().t() + (0 if b is None else b.double())
+    z = z.bfloat16().double()
+    want = F.silu(z[:, :F_]) * z[:, half:]
+    assert y.shape == (M, F_) and _rel_err(y.double(), want) < 2.0 ** -7
+    if half == F_:
+        two = ops.swiglu(ops.linear(x.contiguous(), w, b))
+        assert _rel_err(y.double(), two.double()) < 2.0 ** -7
+    assert ops.gemm_swiglu(x[:128], w, F_, half, b) is None and ops.gemm_swiglu(x.float(), w, F_, half, b) is None
+    assert ops.gemm_swiglu(x[:, 1:], w[:, 1:], F_, half, b) is None
+
+
 def test_gemm_wgrad_shape():
     """dW[N,K] += dY[T,N]^T X[T,K] with a long reduction and split-K chosen by the wrapper."""
     from innova_b200 import ops
