@@ -22,12 +22,18 @@ from typing import List, Optional
 import torch
 import torch.distributed as dist
 
-from .. import ops
+from .. import _native, ops
 from ..inference.kv_cache import PagedKVCache, PAGE
 from ..models.config import TransformerConfig
 from ..ops import runtime as rt
 from ..ops.oil_linear import (SKINNY_SUMS, SKINNY_SWIGLU, QuantWeight, _acc_for, _gemm_into_acc, _skinny, finish_norm, oil_linear,
                               oil_linear_norm, oil_linear_swiglu, quantize_weight, skinny_fits, skinny_takes)
+
+
+_native.register_cuda_sigs({
+    "inv_step_begin": [_native.vp, _native.vp, _native.i32, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp],
+    "inv_step_next": [_native.vp, _native.i64, _native.i32, _native.vp, _native.vp, _native.i32, _native.vp, _native.i32, _native.i32, _native.vp],
+})
 
 
 class TPContext:
@@ -328,6 +334,12 @@ class TPDecoder:
         return all((l["n1"].data_ptr() | l["n2"].data_ptr()) % 16 == 0 and skinny_takes(l["qkv"], B) and skinny_takes(l["o"], B)
                    and skinny_takes(l["gu"], B) and skinny_takes(l["down"], B) for l in self.layers)
 
+    def _gathers(self, tokens: torch.Tensor) -> bool:
+        """Whether the step's own gather takes these tokens and this table: whole rows of 16-byte pieces."""
+        e = self.emb
+        return (e.is_contiguous() and e.data_ptr() % 16 == 0 and e.shape[1] * e.element_size() % 16 == 0 and tokens.dtype == torch.int64
+                and tokens.is_contiguous() and self.cache.seq_lens.dtype == torch.int32)
+
     @torch.no_grad()
     def _decode_step(self, tokens: torch.Tensor) -> torch.Tensor:
         """tokens [B] -> logits [B, vocab]. Uses and advances the device-side sequence lengths. The lookups in front of the first
@@ -335,9 +347,15 @@ class TPDecoder:
         cfg, c = self.cfg, self.cache
         B = tokens.shape[0]
         lens = c.seq_lens[:B]
-        pos = lens.clone()                      # position of the new token
-        lens.add_(1)
-        x = self.emb[tokens]
+        if self._gathers(tokens):               # x, the new tokens' positions and the advanced lengths in one launch
+            x = torch.empty(B, self.emb.shape[1], dtype=self.emb.dtype, device=self.dev)
+            pos = torch.empty(B, dtype=torch.int32, device=self.dev)
+            rt.check(rt.lib().inv_step_begin(tokens.data_ptr(), self.emb.data_ptr(), self.emb.shape[1] * self.emb.element_size(), self.emb.shape[0],
+                                             x.data_ptr(), lens.data_ptr(), pos.data_ptr(), B, rt.stream_ptr()), "inv_step_begin")
+        else:
+            pos = lens.clone()                  # position of the new token
+            lens.add_(1)
+            x = self.emb[tokens]
         if self._few(B):
             # A few tokens: every projection is one launch that takes the norm in front of it and the residual or SwiGLU behind it
             eps = cfg.norm_eps
@@ -379,7 +397,6 @@ class TPDecoder:
         logits = self.prefill(ids)
         tok = logits.argmax(-1)
         e[1].record()
-        out = [tok]
         static_tok = tok.clone()
         if use_graph:
             # The first time that a step has these sizes and this route, it runs on a side stream (lazy kernel attributes, accumulators that
@@ -389,6 +406,8 @@ class TPDecoder:
             # with ranks, whose graphs end before their process group does. "relaxed": a garbage collection may free CUDA objects in
             # the middle of the capture, here or on another thread, and must not end it.
             saved = self.cache.seq_lens.clone()
+            picked = torch.empty(B, max(1, max_new_tokens), dtype=torch.int64, device=self.dev)
+            picked[:, 0] = tok
             if self._side is None:
                 self._side = torch.cuda.Stream()
             s = self._side
@@ -405,8 +424,11 @@ class TPDecoder:
                 graph = torch.cuda.CUDAGraph()
                 graph.capture_begin(pool=None if self._graph is None else self._graph.pool(), capture_error_mode="relaxed")
                 try:
+                    # the step's last launch picks the next tokens, which the next replay starts from, and files them under the sequences' lengths
                     static_logits = self._decode_step(static_tok)
-                    static_next = static_logits.argmax(-1)
+                    assert static_logits.dtype == torch.float32 and static_logits.stride(1) == 1
+                    rt.check(rt.lib().inv_step_next(static_logits.data_ptr(), static_logits.stride(0), static_logits.shape[1], static_tok.data_ptr(),
+                                                    picked.data_ptr(), picked.shape[1], self.cache.seq_lens.data_ptr(), S, B, rt.stream_ptr()), "inv_step_next")
                 finally:
                     graph.capture_end()
             self._graph = graph if self.ctx is None else None
@@ -415,13 +437,12 @@ class TPDecoder:
             e[1].record()
             for _ in range(max_new_tokens - 1):
                 graph.replay()
-                static_tok.copy_(static_next)
-                out.append(static_next.clone())
         else:
+            out = [tok]
             for _ in range(max_new_tokens - 1):
                 tok = self._decode_step(tok).argmax(-1)
                 out.append(tok)
         e[2].record()
         torch.cuda.synchronize()
         rt.check_status()
-        return torch.stack(out, dim=1), e[0].elapsed_time(e[1]) / 1e3, e[1].elapsed_time(e[2]) / 1e3
+        return (picked if use_graph else torch.stack(out, dim=1)), e[0].elapsed_time(e[1]) / 1e3, e[1].elapsed_time(e[2]) / 1e3

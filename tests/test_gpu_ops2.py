@@ -678,3 +678,38 @@ def test_prompt_projection_finish_matches_its_three_passes(fmt, B, S, H, Hkv, D)
             seen = torch.arange(16, device=DEV).view(1, -1) < (S - 16 * torch.arange((S + 15) // 16, device=DEV).view(-1, 1))
             keep = seen.repeat(B, 1).view(-1, 1, 16, 1).expand(-1, Hkv, 16, D // 32).reshape(len(pages), -1)
             assert torch.equal(x.view(x.shape[0], -1)[pages][keep], y.view(y.shape[0], -1)[pages][keep])
+
+
+@pytest.mark.parametrize("B,V,ld", [(1, 1, 4), (3, 31, 40), (2, 1024, 1024), (64, 8192, 8192), (5, 50257, 50304), (1, 128256, 128256)])
+def test_ends_of_a_decode_step_match_torch(B, V, ld):
+    """The step's gather with lengths and positions, and its arg-max: ties (the first), infinities, NaN, rows wider than the vocabulary."""
+    from innova_b200.ops import runtime as rt
+    import innova_b200.parallel.tp  # noqa: F401  (binds the entry points)
+    torch.manual_seed(V)
+    lib, st = rt.lib(), rt.stream_ptr()
+    buf = torch.full((B, ld), float("inf"), device=DEV)
+    for kind in ("plain", "ties", "masked", "nan"):
+        z = torch.randn(B, V, device=DEV)
+        if kind == "ties":
+            z = z.round()
+        elif kind == "masked":
+            z[:] = float("-inf")
+        elif kind == "nan":
+            z[:, V // 2:] = float("nan")
+        buf[:, :V] = z
+        lens = torch.arange(B, dtype=torch.int32, device=DEV) + 7
+        nxt = torch.full((B,), -1, dtype=torch.int64, device=DEV)
+        out = torch.full((B, 4), -1, dtype=torch.int64, device=DEV)
+        rt.check(lib.inv_step_next(buf.data_ptr(), ld, V, nxt.data_ptr(), out.data_ptr(), 4, lens.data_ptr(), 7, B, st), "next")
+        assert torch.equal(nxt, z.argmax(-1)), kind
+        want = torch.full((B, 4), -1, dtype=torch.int64, device=DEV)          # row b to column b, the columns that there are
+        for b in range(min(B, 4)):
+            want[b, b] = nxt[b]
+        assert torch.equal(out, want)
+    for E, dt in ((8, torch.bfloat16), (2056, torch.bfloat16), (20, torch.float32)):
+        emb = torch.randn(max(V, 2), E, device=DEV).to(dt)
+        x, pos, before = torch.empty(B, E, dtype=dt, device=DEV), torch.empty(B, dtype=torch.int32, device=DEV), lens.clone()
+        tok = torch.randint(0, emb.shape[0], (B,), device=DEV)
+        rt.check(lib.inv_step_begin(tok.data_ptr(), emb.data_ptr(), E * emb.element_size(), emb.shape[0], x.data_ptr(), lens.data_ptr(), pos.data_ptr(), B, st),
+                 "begin")
+        assert torch.equal(x, emb[tok]) and torch.equal(pos, before) and torch.equal(lens, before + 1)
