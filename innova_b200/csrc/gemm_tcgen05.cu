@@ -26,7 +26,8 @@ constexpr int BM = 128, BN = 256, BK = 64, STAGES = 4, UMMA_K = 16;
 constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KB
 constexpr int B_STAGE_BYTES = BN * BK * 2;  // 32 KB
 constexpr int GEMM_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
-constexpr int GEMM_SMEM_BYTES = STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 1024 /*align*/ + 256 /*barriers*/;
+constexpr int GEMM_STAGING = 8 * 4096;  // a box of 32 rows x 128 bytes per epilogue warp
+constexpr int GEMM_SMEM_BYTES = STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + GEMM_STAGING + 1024 /*align*/ + 256 /*barriers*/;
 constexpr int TMEM_COLS = 512;
 
 
@@ -35,6 +36,7 @@ struct WorkUnit {
   int b_row_off;   // extra row offset into the stacked B (grouped mode 1)
   int bias_off;
   long c_off;      // element offset of this unit's C (grouped mode 2)
+  int group;       // (grouped mode 2)
   bool skip;
   int ag_tile;     // tile index of the gathered operand this unit reads, -1 when it is local or nothing is gathered
 };
@@ -43,6 +45,7 @@ __device__ __forceinline__ WorkUnit decode_work(int w, const GemmParams& p, int 
   u.b_row_off = 0;
   u.bias_off = 0;
   u.c_off = 0;
+  u.group = 0;
   u.skip = false;
   u.ag_tile = -1;
   int n_blk, m_blk, rest;
@@ -76,6 +79,7 @@ __device__ __forceinline__ WorkUnit decode_work(int w, const GemmParams& p, int 
     u.kb_begin = off / BK + ks * per;
     u.kb_end = min(off / BK + nkb, u.kb_begin + per);
     u.c_off = (long)e * p.group_stride_c;
+    u.group = e;
     u.skip = u.kb_begin >= u.kb_end;
     return u;
   }
@@ -91,15 +95,21 @@ __device__ __forceinline__ WorkUnit decode_work(int w, const GemmParams& p, int 
   return u;
 }
 
-template <bool A_MN, bool B_MN>
+// EPI: GEMM_ANY, or one epilogue compiled in whose results leave as boxes: EPI_NONE (bf16, TMA stores) and EPI_ATOMIC (fp32 sums, TMA reductions
+// into the group's matrix), both for grouped products. The general form writes sixteen bytes a lane in 32 rows. All products of 8 experts in a
+// training step (4096 tokens, top 2, widths 2048 and 5632): 1.52 -> 1.40 ms, of which the two weight gradients take 0.56.
+constexpr int GEMM_ANY = -1;
+
+template <bool A_MN, bool B_MN, int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_c,
                  const __grid_constant__ GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
   uint8_t* sB = smem + STAGES * A_STAGE_BYTES;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * (A_STAGE_BYTES + B_STAGE_BYTES));
+  uint8_t* sStage = smem + STAGES * (A_STAGE_BYTES + B_STAGE_BYTES);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sStage + GEMM_STAGING);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tmem_full = empty_bar + STAGES;
   uint64_t* tmem_empty = tmem_full + 2;
@@ -245,6 +255,43 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         row -= owner * p.rs_shard_rows;
       }
       const uint32_t t_row = tmem_base + acc * BN + (uint32_t(q * 32) << 16);
+      if constexpr (EPI != GEMM_ANY) {
+        constexpr int STEP = EPI == EPI_ATOMIC ? 32 : 64;     // columns of a box
+        uint8_t* box = sStage + (warp - 2) * 4096;
+#pragma unroll 1
+        for (int c = half * 128; c < half * 128 + 128; c += STEP) {
+          const int col0 = u.n0 + c;
+          if (col0 >= p.N) break;
+          uint32_t r[STEP];
+          tmem_ld_32x32(t_row + c, r);
+          if (EPI != EPI_ATOMIC) tmem_ld_32x32(t_row + c + 32, r + STEP - 32);
+          uint4 bv[8];
+          if (EPI != EPI_ATOMIC && bias != nullptr) {
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+              bv[g] = col0 + g * 8 < p.N ? __ldg(reinterpret_cast<const uint4*>(bias + col0) + g) : make_uint4(0, 0, 0, 0);
+          }
+          if (lane == 0) tma_store_wait_read();
+          __syncwarp();
+          tmem_ld_wait();
+          if constexpr (EPI == EPI_ATOMIC) {
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+              *reinterpret_cast<uint4*>(box + lane * 128 + ((g ^ (lane & 7)) << 4)) = make_uint4(r[g * 4], r[g * 4 + 1], r[g * 4 + 2], r[g * 4 + 3]);
+          } else {
+            const uint4* b8 = bias != nullptr ? bv : nullptr;
+            gemm_epilogue_fixed<EPI>(1.f, b8, r, box + lane * 128, nullptr, 0, lane);
+            gemm_epilogue_fixed<EPI>(1.f, b8 == nullptr ? nullptr : b8 + 4, r + STEP - 32, box + lane * 128, nullptr, 1, lane);
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if constexpr (EPI == EPI_ATOMIC) tma_reduce_add_3d_f32(&tmap_c, box, col0, u.m0 + q * 32, u.group);
+            else tma_store_2d(&tmap_c, box, col0, u.m0 + q * 32);
+            tma_store_commit();
+          }
+        }
+      } else {
 #pragma unroll 1
       for (int c = half * 4; c < half * 4 + 4; c += 2) {
         const int col0 = u.n0 + c * 32;
@@ -256,11 +303,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         gemm_epilogue_chunk(p, C, bias, row, row_ok, col0, r0);
         if (col0 + 32 < p.N) gemm_epilogue_chunk(p, C, bias, row, row_ok, col0 + 32, r1);
       }
+      }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[acc]);
       ++tile_i;
     }
+    if (EPI != GEMM_ANY && lane == 0) tma_store_wait_all();   // shared memory must outlive the stores that read it
   }
 
   // ---------------- teardown ----------------
@@ -326,15 +375,29 @@ int make_tmap_2d_f32(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t
   return r == CUDA_SUCCESS ? 0 : -(int)r - 1000;
 }
 
-template <bool A_MN, bool B_MN>
-static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream) {
+// Matrices of fp32 values `stride` apart.
+static int make_tmap_3d_f32(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t groups, uint64_t ld, uint64_t stride,
+                            uint32_t box_inner, uint32_t box_outer) {
+  EncodeTiledFn enc = get_encode_fn();
+  if (!enc) return -1;
+  cuuint64_t dims[3] = {inner, outer, groups};
+  cuuint64_t strides[2] = {ld * 4, stride * 4};
+  cuuint32_t box[3] = {box_inner, box_outer, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -(int)r - 1000;
+}
+
+template <bool A_MN, bool B_MN, int EPI = GEMM_ANY>
+static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream, const CUtensorMap* tc = nullptr) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<A_MN, B_MN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES);
     if (e != cudaSuccess) return -(int)e;
     configured = true;
   }
-  gemm_bf16_kernel<A_MN, B_MN><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, stream>>>(ta, tb, p);
+  gemm_bf16_kernel<A_MN, B_MN, EPI><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, stream>>>(ta, tb, tc ? *tc : ta, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
@@ -573,6 +636,17 @@ extern "C" int inv_gemm_grouped(const void* A, const void* B, void* C, int M, in
   const long total = (long)m_tiles * n_tiles * p.split_k * (group_mode == 2 ? num_groups : 1);
   const int grid = (int)(total < g_num_sms ? total : g_num_sms);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  // results through boxes where the epilogue is plain and the output's addresses are those of a tensor map
+  CUtensorMap tc;
+  if (group_mode == 1 && epilogue == EPI_NONE && !c_f32 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (reinterpret_cast<uintptr_t>(bias) & 15) == 0 &&
+      (bias == nullptr || group_stride_bias % 8 == 0)) {
+    if ((rc = make_tmap_2d_bf16(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)ldc, 64, 32))) return rc;
+    return b_mn ? launch_gemm<false, true, EPI_NONE>(ta, tb, p, grid, st, &tc) : launch_gemm<false, false, EPI_NONE>(ta, tb, p, grid, st, &tc);
+  }
+  if (group_mode == 2 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && group_stride_c > 0 && group_stride_c % 4 == 0) {
+    if ((rc = make_tmap_3d_f32(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)num_groups, (uint64_t)ldc, (uint64_t)group_stride_c, 32, 32))) return rc;
+    return launch_gemm<true, true, EPI_ATOMIC>(ta, tb, p, grid, st, &tc);
+  }
   if (a_mn && b_mn) return launch_gemm<true, true>(ta, tb, p, grid, st);
   if (!a_mn && b_mn) return launch_gemm<false, true>(ta, tb, p, grid, st);
   if (a_mn && !b_mn) return launch_gemm<true, false>(ta, tb, p, grid, st);

@@ -467,3 +467,35 @@ def test_llama_style_model_trains():
     for _ in range(10):
         last = float(tr.train_step(ids, labels))
     assert last < first - 0.5
+
+
+@pytest.mark.parametrize("N,K", [(136, 72), (264, 200), (520, 128)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_grouped_gemm_results_stay_in_their_groups(N, K, b_mn):
+    """Products of expert segments (rows in multiples of 128, one segment empty, an unused tile) and their weight gradients, whose ragged matrices
+    lie next to each other: every group's result, and nothing beside it. bf16 results carry one rounding; fp32 sums K or rows * 2^-24."""
+    from innova_b200.ops import moe
+    torch.manual_seed(5)
+    dev = _dev()
+    rows, E = [128, 0, 384, 256], 4
+    offs = [0, 128, 128, 512, 768]
+    R = 768 + 128                                                     # the last tile belongs to nobody
+    tile = torch.tensor([0, 2, 2, 2, 3, 3, -1], dtype=torch.int32, device=dev)
+    off = torch.tensor(offs, dtype=torch.int32, device=dev)
+    x = torch.randn(R, K, device=dev).bfloat16()
+    w = (torch.randn(E, N, K, device=dev) * 0.2).bfloat16()
+    stack = w.transpose(1, 2).contiguous() if b_mn else w             # [E, K, N] or [E, N, K]
+    buf = torch.full((R, N + 8), 7.0, dtype=torch.bfloat16, device=dev)
+    out = buf[:, :N]
+    moe._grouped(x, stack.view(-1, stack.shape[-1]), out, mode=1, E=E, tile_expert=tile, offsets=off, rows_b=stack.shape[1], b_mn=b_mn, M=R, N=N, K=K)
+    for e in range(E):
+        if rows[e]:
+            assert _rel_err(out[offs[e]:offs[e + 1]].double(), x[offs[e]:offs[e + 1]].double() @ w[e].double().t()) < 4e-3
+    assert (buf[768:] == 7.0).all() and (buf[:, N:] == 7.0).all()
+    # weight gradients: C_e[K, N] += x_e^T dy_e
+    dy = torch.randn(R, N, device=dev).bfloat16()
+    g = torch.full((E, K, N), 2.0, device=dev)
+    moe._grouped(x, dy, g, mode=2, E=E, tile_expert=None, offsets=off, rows_b=0, a_mn=True, b_mn=True, M=K, N=N, K=R, split_k=2, stride_c=K * N)
+    for e in range(E):
+        want = x[offs[e]:offs[e + 1]].double().t() @ dy[offs[e]:offs[e + 1]].double() + 2.0
+        assert _rel_err(g[e].double(), want) < 1e-5
