@@ -43,6 +43,16 @@ _CUDA_SIGS = {
 }
 
 
+class _CudaLib(C.CDLL):
+    """Only entry points whose signature is known: without one, ctypes would pass pointers as 32-bit integers and a kernel would
+    get an address that is not one. The module that owns an entry point registers it when it is imported."""
+
+    def __getattr__(self, name):
+        if name not in _CUDA_SIGS:
+            raise AttributeError(f"{name} has no registered signature: import the module that calls register_cuda_sigs for it")
+        return super().__getattr__(name)
+
+
 def _bind(lib, sigs):
     for name, args in sigs.items():
         try:
@@ -81,7 +91,7 @@ def cuda():
                         build.build_cuda()
                     else:
                         path = build.build_subset(_subset[0] + "_cuda", _subset[1])
-                _cuda = _bind(C.CDLL(str(path)), _CUDA_SIGS)
+                _cuda = _bind(_CudaLib(str(path)), _CUDA_SIGS)
     return _cuda
 
 

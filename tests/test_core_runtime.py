@@ -168,3 +168,13 @@ def test_rng_matches_the_reference_sources():
         assert n > 0 and bytes(out[:n]) == serialize_tensor(t)
         back, _ = deserialize_tensor(bytes(out[:n]))
         assert torch.equal(back, t)
+
+
+def test_cuda_entry_points_need_a_signature(monkeypatch):
+    """An entry point whose owner was not imported is an error, not a call with pointers cut to 32 bits."""
+    from innova_b200 import _native
+    monkeypatch.setattr(_native, "_CUDA_SIGS", {"getpid": []})
+    lib = _native._bind(_native._CudaLib(None), _native._CUDA_SIGS)
+    assert lib.getpid() > 0
+    with pytest.raises(AttributeError, match="no registered signature"):
+        lib.getppid

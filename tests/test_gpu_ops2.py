@@ -648,7 +648,7 @@ def test_projection_finish_and_attention_in_one_launch(fmt, B, H, Hkv, D, lens):
 def test_prompt_projection_finish_matches_its_three_passes(fmt, B, S, H, Hkv, D):
     """``inv_prompt_qkv_finish`` against finish pass, rotation and append, to the bit: the heads that attention reads, the cache, cleared sums."""
     from innova_b200.inference.kv_cache import PagedKVCache
-    from innova_b200.ops import rope_qk, rope_tables
+    from innova_b200.ops import oil_linear, rope_qk, rope_tables  # noqa: F401  (binds the finish pass)
     from innova_b200.ops import runtime as rt
     torch.manual_seed(S)
     T, W = B * S, (H + 2 * Hkv) * D
