@@ -2,13 +2,13 @@
 //
 // Such a product reads every weight once and does almost no arithmetic, so it is bound by weight bytes and, for the sizes of
 // one layer, by latency. A CTA owns eight weight rows per tile and two tiles (one gate and one up tile in the gated form); its eight
-// warps take every eighth slice of K and meet in shared memory. Weights and activations go straight from global memory into
-// warp-level MMA fragments: a lane loads eight or sixteen consecutive k of a row and both operands read them in the same permuted
+// or sixteen warps take every eighth or sixteenth slice of K and meet in shared memory. Weights and activations go straight from global
+// memory into warp-level MMA fragments: a lane loads eight or sixteen consecutive k of a row and both operands read them in the same permuted
 // order, which a dot product does not notice. (A 128-row tcgen05 tile would be mostly padding here, and its tensor-memory set-up
-// and drain cost more than the whole product.) A warp keeps a ring of slices in registers, 64 KB per CTA up to 32 rows and 32 KB above
-// (the accumulators of four row tiles take the rest), two CTAs per SM. It is filled before the kernel waits for the previous one
-// (resident weights; others are multiplied by a plainly launched kernel) and refilled across tiles, so that the weights never stop
-// flowing.
+// and drain cost more than the whole product.) A warp keeps a ring of slices in registers; a CTA of eight warps 64 KB up to 32 rows and
+// 32 KB above (the accumulators of four row tiles take the rest), two of them an SM; a CTA of sixteen 128 KB. It is filled before the
+// kernel waits for the previous one (resident weights; others are multiplied by a plainly launched kernel) and refilled across tiles, so
+// that the weights never stop flowing.
 //
 // SILU: W holds gate rows [0, N) and up rows [half, half + N); the output is silu(gate) * up.
 // cap > 0 (plain form): the output is cap * tanh(out / cap), the soft limit of logits.
@@ -16,8 +16,6 @@
 #include "inv_api.h"
 
 namespace inv {
-
-constexpr int SG_WARPS = 8, SG_THREADS = 32 * SG_WARPS;
 
 __device__ __forceinline__ void sg_mma(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -42,11 +40,13 @@ __device__ __forceinline__ uint4 sg_mask(uint4 v, int n) {
   return make_uint4(u[0], u[1], u[2], u[3]);
 }
 
-// MT: 16-row tiles of x. P: 16-byte pieces per lane and slice (two where rows allow it: whole lines instead of halves).
-template <int MT, int P, bool SILU>
-__global__ void __launch_bounds__(SG_THREADS, 2) skinny_gemm_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ W,
-                                                                    int ldw, int M, int N, int K, int half, void* __restrict__ out, int ldo,
-                                                                    int out_f32, float cap, int n_tiles) {
+// MT: 16-row tiles of x. P: 16-byte pieces per lane and slice (two where rows allow it: whole lines instead of halves). SG_WARPS: 8, two CTAs an
+// SM, or 16.
+template <int MT, int P, bool SILU, int SG_WARPS>
+__global__ void __launch_bounds__(SG_WARPS * 32, SG_WARPS == 8 ? 2 : 1)
+    skinny_gemm_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ W, int ldw, int M, int N, int K, int half,
+                       void* __restrict__ out, int ldo, int out_f32, float cap, int n_tiles) {
+  constexpr int SG_THREADS = 32 * SG_WARPS;
   constexpr int WT = 2;                      // weight tiles of eight rows: neighbours, or gate and up
   constexpr int COLS = SILU ? 8 : 16;        // output columns of a CTA's tile
   constexpr int SL = 32 * P;                 // k of a slice
@@ -144,15 +144,28 @@ __global__ void __launch_bounds__(SG_THREADS, 2) skinny_gemm_kernel(const __nv_b
   }
 }
 
-template <int MT, int P, bool SILU>
-static int launch_skinny(const void* x, int ldx, const void* W, int ldw, int M, int N, int K, int half, void* out, int ldo, int out_f32, float cap,
+template <int MT, int P, bool SILU, int SG_WARPS>
+static int launch_skinny(const void* x, int ldx, const void* W, int ldw, int M, int N, int K, int half, void* out, int ldo, int out_f32, float cap, int tiles,
                          bool early, cudaStream_t st) {
-  constexpr int bytes = SG_WARPS * MT * 16 * (2 * 8 + 4) * 4;
-  const int tiles = SILU ? (N + 7) / 8 : (N + 15) / 16;
-  launch_step(early, skinny_gemm_kernel<MT, P, SILU>, dim3(tiles < 148 * 2 ? tiles : 148 * 2), SG_THREADS, bytes, st, (const __nv_bfloat16*)x, ldx,
+  constexpr int bytes = SG_WARPS * MT * 16 * (2 * 8 + 4) * 4, ctas = 148 * (SG_WARPS == 8 ? 2 : 1);
+  launch_step(early, skinny_gemm_kernel<MT, P, SILU, SG_WARPS>, dim3(tiles < ctas ? tiles : ctas), SG_WARPS * 32, bytes, st, (const __nv_bfloat16*)x, ldx,
                (const __nv_bfloat16*)W, ldw, M, N, K, half, out, ldo, out_f32, cap, tiles);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
+}
+// Sixteen warps where every tile has an SM to itself and a row has more slices than eight warps keep in flight (K > 2048): a second CTA would find
+// no tile, so eight warps left half of the SM's loads unissued and walked a chain of slices twice as long. Back to back, 2048 x 5632: one row
+// 9.4 -> 6.3 us, 16 rows 9.9 -> 6.7, 32 rows 13.7 -> 9.6; 1024 x 2816, 16 rows: 3.8 -> 2.8. Shorter rows (2048 x 2048, 3.2 us) fit in the eight
+// warps' rings, and more tiles (6656 x 2048, 7.5 us) fill the SMs with two CTAs each. Above 32 rows the accumulators of four row tiles take the
+// registers.
+template <int MT, int P, bool SILU>
+static int launch_skinny(const void* x, int ldx, const void* W, int ldw, int M, int N, int K, int half, void* out, int ldo, int out_f32, float cap,
+                         bool early, cudaStream_t st) {
+  const int tiles = SILU ? (N + 7) / 8 : (N + 15) / 16, slices = (K + 32 * P - 1) / (32 * P);
+  if constexpr (MT <= 2) {
+    if (tiles <= 148 && slices > 8 * (8 / P)) return launch_skinny<MT, P, SILU, 16>(x, ldx, W, ldw, M, N, K, half, out, ldo, out_f32, cap, tiles, early, st);
+  }
+  return launch_skinny<MT, P, SILU, 8>(x, ldx, W, ldw, M, N, K, half, out, ldo, out_f32, cap, tiles, early, st);
 }
 
 }  // namespace inv

@@ -390,6 +390,23 @@ def test_gpu_decode_projection_over_tiles_and_pieces(M, N, K, pad):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,pad", [(1, 8, 2064, 0), (16, 2368, 2056, 0), (17, 1184, 2080, 8), (32, 2048, 5632, 0), (16, 2369, 4112, 0), (5, 100, 9000, 8)])
+def test_gpu_decode_projection_of_long_rows(M, N, K, pad):
+    """Rows of more than 2048 on both sides of one tile per SM (148 tiles: 2368 columns, 1184 gated), one slice behind the rings and many;
+    plain and gated, against fp64 on the same bf16 operands (fp32 sums)."""
+    from innova_b200.ops import skinny_gemm
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    x = torch.randn(M, K + pad, device="cuda", generator=g).bfloat16()[:, :K]
+    w = (torch.randn(2 * N, K + pad, device="cuda", generator=g) * K ** -0.5).bfloat16()[:, :K]
+    gate, up = (x.double() @ t.double().t() for t in (w[:N], w[N:]))
+    plain = skinny_gemm(x, w, n=N, resident=True)
+    assert float((plain.double() - gate).norm() / gate.norm()) < 1e-5
+    want = torch.nn.functional.silu(gate) * up
+    got = skinny_gemm(x, w, n=N, silu_half=N)
+    assert float((got.double() - want).norm() / want.norm()) < 1e-5
+
+
+@pytest.mark.gpu
 def test_gpu_first_call_of_a_thread_may_be_a_product():
     """A thread whose first CUDA work is a tensor-map product (a backward that starts with a weight gradient) has no context bound yet."""
     import threading
