@@ -43,14 +43,24 @@ _CUDA_SIGS = {
 }
 
 
+class _Unbound:
+    """First parameter of an entry point nobody has declared."""
+
+    @classmethod
+    def from_param(cls, _):
+        raise TypeError("no signature: import the module that registers this entry point, or set its argtypes")
+
+
 class _CudaLib(C.CDLL):
-    """Only entry points whose signature is known: without one, ctypes would pass pointers as 32-bit integers and a kernel would
-    get an address that is not one. The module that owns an entry point registers it when it is imported."""
+    """Entry points refuse to be called with arguments before their signature is known: without one, ctypes would pass pointers as
+    32-bit integers and a kernel would get an address that is not one. The module that owns an entry point registers it when it
+    is imported."""
 
     def __getattr__(self, name):
+        fn = super().__getattr__(name)
         if name not in _CUDA_SIGS:
-            raise AttributeError(f"{name} has no registered signature: import the module that calls register_cuda_sigs for it")
-        return super().__getattr__(name)
+            fn.argtypes = [_Unbound]
+        return fn
 
 
 def _bind(lib, sigs):

@@ -171,10 +171,13 @@ def test_rng_matches_the_reference_sources():
 
 
 def test_cuda_entry_points_need_a_signature(monkeypatch):
-    """An entry point whose owner was not imported is an error, not a call with pointers cut to 32 bits."""
+    """An entry point whose owner was not imported is an error, not a call with pointers cut to 32 bits; a caller may declare it too."""
+    import ctypes
     from innova_b200 import _native
-    monkeypatch.setattr(_native, "_CUDA_SIGS", {"getpid": []})
+    monkeypatch.setattr(_native, "_CUDA_SIGS", {"abs": [_native.i32]})
     lib = _native._bind(_native._CudaLib(None), _native._CUDA_SIGS)
-    assert lib.getpid() > 0
-    with pytest.raises(AttributeError, match="no registered signature"):
-        lib.getppid
+    assert lib.abs(-3) == 3
+    with pytest.raises(ctypes.ArgumentError, match="no signature"):
+        lib.labs(-3)
+    lib.labs.argtypes, lib.labs.restype = [ctypes.c_long], ctypes.c_long
+    assert lib.labs(-2 ** 40) == 2 ** 40
