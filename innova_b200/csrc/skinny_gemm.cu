@@ -153,17 +153,19 @@ static int launch_skinny(const void* x, int ldx, const void* W, int ldw, int M, 
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
-// Sixteen warps where every tile has an SM to itself and a row has more slices than eight warps keep in flight (K > 2048): a second CTA would find
+// Sixteen warps: where every tile has an SM to itself and a row has more slices than eight warps keep in flight (K > 2048): a second CTA would find
 // no tile, so eight warps left half of the SM's loads unissued and walked a chain of slices twice as long. Back to back, 2048 x 5632: one row
 // 9.4 -> 6.3 us, 16 rows 9.9 -> 6.7, 32 rows 13.7 -> 9.6; 1024 x 2816, 16 rows: 3.8 -> 2.8. Shorter rows (2048 x 2048, 3.2 us) fit in the eight
-// warps' rings, and more tiles (6656 x 2048, 7.5 us) fill the SMs with two CTAs each. Above 32 rows the accumulators of four row tiles take the
-// registers.
+// warps' rings. With more tiles than that, where it takes less than twice as many rounds as two CTAs an SM and every warp has two slices or more:
+// the last round is less empty (6656 x 2048, 3 rounds instead of 2 double ones: 7.5 -> 6.6 us; gated 5632 x 2048, 5 instead of 3: 10.1 -> 9.6).
+// Above 32 rows the accumulators of four row tiles take the registers.
 template <int MT, int P, bool SILU>
 static int launch_skinny(const void* x, int ldx, const void* W, int ldw, int M, int N, int K, int half, void* out, int ldo, int out_f32, float cap,
                          bool early, cudaStream_t st) {
   const int tiles = SILU ? (N + 7) / 8 : (N + 15) / 16, slices = (K + 32 * P - 1) / (32 * P);
   if constexpr (MT <= 2) {
-    if (tiles <= 148 && slices > 8 * (8 / P)) return launch_skinny<MT, P, SILU, 16>(x, ldx, W, ldw, M, N, K, half, out, ldo, out_f32, cap, tiles, early, st);
+    if (tiles <= 148 ? slices > 8 * (8 / P) : slices >= 32 && (tiles + 147) / 148 < 2 * ((tiles + 295) / 296))
+      return launch_skinny<MT, P, SILU, 16>(x, ldx, W, ldw, M, N, K, half, out, ldo, out_f32, cap, tiles, early, st);
   }
   return launch_skinny<MT, P, SILU, 8>(x, ldx, W, ldw, M, N, K, half, out, ldo, out_f32, cap, tiles, early, st);
 }

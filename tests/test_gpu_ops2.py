@@ -390,10 +390,11 @@ def test_gpu_decode_projection_over_tiles_and_pieces(M, N, K, pad):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("M,N,K,pad", [(1, 8, 2064, 0), (16, 2368, 2056, 0), (17, 1184, 2080, 8), (32, 2048, 5632, 0), (16, 2369, 4112, 0), (5, 100, 9000, 8)])
+@pytest.mark.parametrize("M,N,K,pad", [(1, 8, 2064, 0), (16, 2368, 2056, 0), (17, 1184, 2080, 8), (32, 2048, 5632, 0), (16, 2369, 4112, 0), (5, 100, 9000, 8),
+                                       (16, 6656, 2048, 0), (32, 4737, 1032, 0), (1, 5632, 1024, 8)])
 def test_gpu_decode_projection_of_long_rows(M, N, K, pad):
     """Rows of more than 2048 on both sides of one tile per SM (148 tiles: 2368 columns, 1184 gated), one slice behind the rings and many;
-    plain and gated, against fp64 on the same bf16 operands (fp32 sums)."""
+    tiles in an odd number of rounds; plain and gated, against fp64 on the same bf16 operands (fp32 sums)."""
     from innova_b200.ops import skinny_gemm
     g = torch.Generator(device="cuda").manual_seed(N + K)
     x = torch.randn(M, K + pad, device="cuda", generator=g).bfloat16()[:, :K]
