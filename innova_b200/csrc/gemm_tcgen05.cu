@@ -636,14 +636,14 @@ extern "C" int inv_gemm_grouped(const void* A, const void* B, void* C, int M, in
   const long total = (long)m_tiles * n_tiles * p.split_k * (group_mode == 2 ? num_groups : 1);
   const int grid = (int)(total < g_num_sms ? total : g_num_sms);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  // results through boxes where the epilogue is plain and the output's addresses are those of a tensor map
+  // results through boxes where the epilogue is plain (sums: without a bias) and the output's addresses are those of a tensor map
   CUtensorMap tc;
   if (group_mode == 1 && epilogue == EPI_NONE && !c_f32 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (reinterpret_cast<uintptr_t>(bias) & 15) == 0 &&
       (bias == nullptr || group_stride_bias % 8 == 0)) {
     if ((rc = make_tmap_2d_bf16(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)ldc, 64, 32))) return rc;
     return b_mn ? launch_gemm<false, true, EPI_NONE>(ta, tb, p, grid, st, &tc) : launch_gemm<false, false, EPI_NONE>(ta, tb, p, grid, st, &tc);
   }
-  if (group_mode == 2 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && group_stride_c > 0 && group_stride_c % 4 == 0) {
+  if (group_mode == 2 && bias == nullptr && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && group_stride_c > 0 && group_stride_c % 4 == 0) {
     if ((rc = make_tmap_3d_f32(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)num_groups, (uint64_t)ldc, (uint64_t)group_stride_c, 32, 32))) return rc;
     return launch_gemm<true, true, EPI_ATOMIC>(ta, tb, p, grid, st, &tc);
   }

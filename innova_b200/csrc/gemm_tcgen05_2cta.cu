@@ -580,8 +580,10 @@ int gemm_2cta_dispatch(const void* A, const void* B, const GemmParams& p0, int l
     for (int r = 0; r < p.rs_world; ++r)
       if ((rc = make_tmap_2d_bf16(&rs.m[r], p.rs_dst[r], (uint64_t)p.N, (uint64_t)p.rs_shard_rows, (uint64_t)p.ldc, 64, 32))) return rc;
   }
-  // The combinations of a training step and of prompts have kernels of their own; the rest decides per chunk.
-  const int epi = p.ag_world > 1 || p.rs_world > 1 || (p.c_f32 != 0) != (p.epilogue == EPI_ATOMIC) ? EPI_ANY : p.epilogue;
+  // The combinations of a training step and of prompts have kernels of their own; the rest decides per chunk (sums with a bias too: the kernel
+  // whose sums leave through TMA reductions adds none).
+  const bool any = p.ag_world > 1 || p.rs_world > 1 || (p.c_f32 != 0) != (p.epilogue == EPI_ATOMIC) || (p.epilogue == EPI_ATOMIC && p.bias != nullptr);
+  const int epi = any ? EPI_ANY : p.epilogue;
 #define INV_G2(A, B, E) return launch_gemm_2cta<A, B, E>(ta, tb, tc, tx, rs, p, grid, stream)
   if (a_mn && b_mn) {
     if (epi == EPI_ATOMIC) INV_G2(true, true, EPI_ATOMIC);

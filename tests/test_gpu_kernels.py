@@ -151,6 +151,30 @@ def test_gemm_fixed_epilogues_stay_inside_their_view(a_mn, b_mn, epi, M, N, K):
     assert (buf == 3.0).all()
 
 
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (True, True), (True, False)])
+@pytest.mark.parametrize("M,N", [(128, 136), (256, 264), (304, 136)])
+def test_gemm_sums_take_a_bias(a_mn, b_mn, M, N):
+    """C += A B^T + bias, on both kernels and whatever the layout; grouped sums too. fp32 sums: K * 2^-24."""
+    from innova_b200 import ops
+    from innova_b200.ops import moe  # noqa: F401  (binds the grouped product)
+    from innova_b200.ops import runtime as rt
+    torch.manual_seed(3)
+    dev, K = _dev(), 128
+    A, B = torch.randn(M, K, device=dev).bfloat16(), torch.randn(N, K, device=dev).bfloat16()
+    bias = torch.randn(N, device=dev).bfloat16() * 8
+    out = torch.full((M, N), 2.0, device=dev)
+    ops.gemm(A.t().contiguous() if a_mn else A, B.t().contiguous() if b_mn else B, out=out, a_mn=a_mn, b_mn=b_mn, epilogue=ops.EPI_ATOMIC, bias=bias, split_k=1)
+    want = A.double() @ B.double().t() + bias.double() + 2.0
+    assert _rel_err(out.double(), want) < 1e-5
+    if a_mn and b_mn:
+        off = torch.tensor([0, K], dtype=torch.int32, device=dev)
+        out = torch.full((1, M, N), 2.0, device=dev)
+        At, Bt = A.t().contiguous(), B.t().contiguous()
+        rt.check(rt.lib().inv_gemm_grouped(At.data_ptr(), Bt.data_ptr(), out.data_ptr(), M, N, K, M, N, N, 1, 1, ops.EPI_ATOMIC, bias.data_ptr(), 0, 0, 0, 1, 1, 2,
+                                           1, 0, off.data_ptr(), 0, 0, M * N, rt.status_tensor(dev).data_ptr(), rt.stream_ptr()), "inv_gemm_grouped")
+        assert _rel_err(out[0].double(), want) < 1e-5
+
+
 @pytest.mark.parametrize("M,F_,K,half,bias", [(129, 8, 64, 8, False), (300, 136, 72, 136, True), (257, 128, 200, 160, True), (1000, 1408, 512, 1408, False),
                                              (2 * 74 * 256 + 9, 392, 64, 400, True)])
 def test_gemm_swiglu_matches_product_and_activation(M, F_, K, half, bias):
