@@ -97,6 +97,13 @@ class FFN(nn.Module):
         return ops.linear(act, _ste(self.down_proj.weight, cfg), self.down_proj.bias, residual=residual, mode="add")
 
 
+def _steps(cls):
+    return cls.forward, getattr(cls, "with_residual", None)
+
+
+_AS_WRITTEN = {cls: _steps(cls) for cls in (Attention, FFN, Norm)}     # a class whose steps were replaced since (by a profiler, say) is called itself
+
+
 class TransformerBlock(nn.Module):
     def __init__(self, cfg: TransformerConfig, dtype):
         super().__init__()
@@ -107,10 +114,12 @@ class TransformerBlock(nn.Module):
         self.ffn = FFN(cfg, dtype)
 
     def _whole(self):
-        """Whether nothing inside the block was hooked or replaced, so that its launches may be issued together."""
+        """Whether nothing inside the block was hooked, replaced or configured on its own, so that its launches may be issued together."""
+        if self.attention.cfg is not self.cfg or self.ffn.cfg is not self.cfg:
+            return False
         for m, cls in ((self.attention, Attention), (self.ffn, FFN), (self.attention_norm, Norm), (self.ffn_norm, Norm)):
             if (type(m) is not cls or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__
-                    or "with_residual" in m.__dict__):
+                    or "with_residual" in m.__dict__ or _steps(cls) != _AS_WRITTEN[cls]):
                 return False
         return True
 

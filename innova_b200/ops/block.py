@@ -133,8 +133,9 @@ def block_forward(blk, x, rope, positions):
     if torch.compiler.is_compiling() or torch.jit.is_tracing() or torch.nn.modules.module._has_any_global_hook():
         return None
     first = ffn.gate_up_proj if gated else ffn.up_proj
-    params = (n1.weight, n1.bias, att.qkv_proj.weight, att.qkv_proj.bias, att.o_proj.weight, att.o_proj.bias, n2.weight, n2.bias,
-              first.weight, first.bias, ffn.down_proj.weight, ffn.down_proj.bias)
+    shifts = n1.kind == "layernorm"                     # an RMS norm has no use for a bias
+    params = (n1.weight, n1.bias if shifts else None, att.qkv_proj.weight, att.qkv_proj.bias, att.o_proj.weight, att.o_proj.bias, n2.weight,
+              n2.bias if shifts else None, first.weight, first.bias, ffn.down_proj.weight, ffn.down_proj.bias)
     grad = torch.is_grad_enabled()
     for p in params:
         if not _plain(p) or (grad and p is not None and not p.requires_grad):

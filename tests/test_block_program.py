@@ -109,6 +109,33 @@ def test_block_follows_what_changes_between_and_within_passes(monkeypatch):
     assert real(m.layers[0], x, None, None) is None and m.layers[0](x, None).shape == x.shape
 
 
+@pytest.mark.gpu
+def test_block_asks_parts_that_were_set_up_on_their_own(monkeypatch):
+    """Another format for one part of a block, and steps that were replaced in their class, count as they do layer by layer."""
+    import copy
+    m = _model(**GELU)
+    x = torch.randn(2, 64, 256, device=DEV).bfloat16()
+    plain = m.layers[0](x, None)
+    own = copy.copy(m.cfg)
+    own.ste_format = "spark"
+    m.layers[0].ffn.cfg = own
+    got = m.layers[0](x, None)
+    with monkeypatch.context() as mp:
+        mp.setattr(dense.ops, "block_forward", lambda *a: None)
+        want = m.layers[0](x, None)
+    assert torch.equal(got, want) and not torch.equal(got, plain)
+    m.layers[0].ffn.cfg = m.cfg
+    calls, real = [], dense.Attention.forward
+    monkeypatch.setattr(dense.Attention, "forward", lambda self, *a: calls.append(1) or real(self, *a))
+    assert torch.equal(m.layers[0](x, None), plain) and calls == [1]
+    monkeypatch.undo()
+    m = _model(norm="rmsnorm")
+    rope = m.rope(x.device)
+    want = m.layers[0](x, rope)
+    m.layers[0].ffn_norm.bias = torch.nn.Parameter(torch.ones_like(m.layers[0].ffn_norm.weight))     # nothing that an RMS norm reads
+    assert torch.equal(m.layers[0](x, rope), want)
+
+
 def test_train_step_puts_parts_in_eval_mode_back():
     from innova_b200.training.trainer import Trainer
     m = DenseModel(PRESETS["tiny"](num_layers=1, vocab_size=64, max_seq_len=16, hidden_size=32, num_heads=1, head_dim=32, ffn_hidden_size=32), dtype=torch.float32)
