@@ -219,8 +219,14 @@ struct BlockRun {
 
 using namespace inv;
 
-// Bytes of `saved` (which = 0) and of the backward pass's scratch (which = 1).
-extern "C" long inv_block_bytes(const BlockDesc* d, int which) { return which ? BlockScratch(*d).total : BlockSaved(*d).total; }
+// Bytes of the caller's buffers: `saved` (which = 0), the backward pass's scratch (1).
+extern "C" int inv_block_bytes(int which, long B, long S, long E, long H, long Hkv, long D, long F, long gated, long quantised, long* bytes) {
+  if (which < 0 || which > 1 || B < 1 || S < 1 || E < 1 || H < 1 || Hkv < 1 || D < 1 || F < 1) return -ERR_BAD_ARG;
+  BlockDesc d{};
+  d.B = B; d.S = S; d.E = E; d.H = H; d.Hkv = Hkv; d.D = D; d.F = F; d.gated = gated; d.quantised = quantised;
+  *bytes = which == 1 ? BlockScratch(d).total : BlockSaved(d).total;
+  return 0;
+}
 
 // Pre-norm block: y = x2 + MLP(norm2(x2)), x2 = x + attention(norm1(x)); causal. Returns the number of launches, or a negative code.
 extern "C" int inv_block_fwd(const BlockDesc* d) {

@@ -7,6 +7,8 @@ Reference behaviour covered: TransformerBlock::forward (src/transformer.cpp:380-
 """
 from __future__ import annotations
 
+import ctypes as C
+import functools
 import importlib
 import struct
 
@@ -19,7 +21,7 @@ from .quant import BLOCK, MODES, default_codebook
 
 _gemm = importlib.import_module(".gemm", __package__)      # the module: the package exports the function under this name
 
-_native.register_cuda_sigs({"inv_block_fwd": [_native.vp], "inv_block_bwd": [_native.vp]})
+_native.register_cuda_sigs({"inv_block_fwd": [_native.vp], "inv_block_bwd": [_native.vp], "inv_block_bytes": [_native.i32] + [_native.i64] * 9 + [_native.vp]})
 
 # BlockDesc: 12 parameters, tables, positions, codebook, x, y, saved, status, stream | dy, dx, two column sums, 12 gradients, scratch | 13 sizes |
 # eps1, eps2, scale
@@ -27,24 +29,16 @@ _PACK = struct.Struct("=12Q 9Q 17Q 13q 3d").pack
 _FORWARD_ONLY = (0,) * 17
 
 
-def _up(n):
-    return (n + 255) // 256 * 256
+SAVED, SCRATCH = 0, 1
 
 
-def _saved_bytes(T, E, H, Hkv, D, F, gated, quantised):
-    W, O, mid = (H + 2 * Hkv) * D, H * D, 2 * F if gated else F
-    q = 2 if quantised else 0
-    sizes = (q * W * E, q * E * O, q * mid * E, q * E * F, 2 * T * E, 2 * T * W, 2 * T * O, 2 * T * E, 2 * T * E, 2 * T * mid, 2 * T * F, 4 * T * H,
-             4 * T, 4 * T, 4 * T, 4 * T)
-    return sum(map(_up, sizes))
-
-
-def _scratch_bytes(B, S, E, H, Hkv, D, F, gated):
-    T, W, O, mid = B * S, (H + 2 * Hkv) * D, H * D, 2 * F if gated else F
-    mlp = _up(2 * T * mid) + (_up(2 * T * F) if gated else 0)
-    norm = min(max(rt.lib().inv_norm_bwd_grid(T), 1), 148) * 3 * E * 4
-    attn = _up(4 * B * H * S) + 4 * T * O
-    return _up(max(mlp, _up(2 * T * W))) + sum(map(_up, (2 * T * E, 2 * T * E, 2 * T * O, 4 * E, norm, attn)))
+@functools.lru_cache(maxsize=256)
+def _bytes(which, B, S, E, H, Hkv, D, F, gated, quantised):
+    """What the native side lays out: what the forward pass leaves for the backward pass, and that pass's scratch."""
+    n = C.c_long()
+    if rt.lib().inv_block_bytes(which, B, S, E, H, Hkv, D, F, gated, quantised, C.addressof(n)) != 0:
+        raise ValueError("block sizes")
+    return n.value
 
 
 def _ptr(t):
@@ -60,7 +54,7 @@ class _BlockFn(torch.autograd.Function):
         H, Hkv, D, F, gated, rms, eps1, eps2, mode = cfg
         B, S, E = x.shape
         dev = x.device
-        saved = torch.empty(_saved_bytes(B * S, E, H, Hkv, D, F, gated, codebook is not None), dtype=torch.uint8, device=dev)
+        saved = torch.empty(_bytes(SAVED, B, S, E, H, Hkv, D, F, gated, int(codebook is not None)), dtype=torch.uint8, device=dev)
         y = torch.empty_like(x)
         _issue("inv_block_fwd", cfg, (B, S, E), params, cos, sin, positions, codebook, x, y.data_ptr(), saved, _FORWARD_ONLY)
         ctx.cfg = cfg
@@ -92,7 +86,7 @@ class _BlockFn(torch.autograd.Function):
             ptrs.append(g.data_ptr())
         dx = torch.empty_like(x)
         dx_colsum = torch.empty(E, dtype=torch.float32, device=dev) if E <= 1024 else None
-        scratch = torch.empty(_scratch_bytes(B, S, E, H, Hkv, D, F, gated), dtype=torch.uint8, device=dev)
+        scratch = torch.empty(_bytes(SCRATCH, B, S, E, H, Hkv, D, F, gated, int(codebook is not None)), dtype=torch.uint8, device=dev)
         _issue("inv_block_bwd", ctx.cfg, (B, S, E), params, cos, sin, positions, codebook, x, 0, saved,
                (dy.data_ptr(), dx.data_ptr(), _ptr(colsum), _ptr(dx_colsum), *ptrs, scratch.data_ptr()))
         if dx_colsum is not None:

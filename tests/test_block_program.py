@@ -136,6 +136,24 @@ def test_block_asks_parts_that_were_set_up_on_their_own(monkeypatch):
     assert torch.equal(m.layers[0](x, rope), want)
 
 
+def test_block_buffers_are_sized_by_their_layout():
+    """The bytes that the native side asks for, stated once more by hand, at sizes off the 256 bytes that buffers start on."""
+    from innova_b200.ops import block
+    up = lambda *n: sum((x + 255) // 256 * 256 for x in n)
+    for B, S, E, H, Hkv, D, F, gated, q in ((1, 1, 64, 1, 1, 64, 8, 0, 0), (3, 77, 200, 4, 2, 64, 136, 1, 1), (2, 129, 1280, 5, 1, 128, 200, 0, 1)):
+        T, W, O, mid = B * S, (H + 2 * Hkv) * D, H * D, 2 * F if gated else F
+        weights = up(*(2 * q * n for n in (W * E, E * O, mid * E, E * F)))
+        stats = up(4 * T * H) + 4 * up(4 * T)
+        args = (B, S, E, H, Hkv, D, F, gated, q)
+        assert block._bytes(block.SAVED, *args) == weights + up(2 * T * E, 2 * T * W, 2 * T * O, 2 * T * E, 2 * T * E, 2 * T * mid, 2 * T * F) + stats
+        mlp = up(2 * T * mid) + (up(2 * T * F) if gated else 0)
+        attn = up(up(4 * B * H * S) + 4 * T * O)
+        grid = max(1, min(148, (T + 7) // 8))
+        assert block._bytes(block.SCRATCH, *args) == max(mlp, up(2 * T * W)) + up(2 * T * E, 2 * T * E, 2 * T * O, 4 * E, grid * 3 * E * 4) + attn
+    with pytest.raises(ValueError):
+        block._bytes(block.SAVED, 0, 1, 64, 1, 1, 64, 8, 0, 0)
+
+
 def test_train_step_puts_parts_in_eval_mode_back():
     from innova_b200.training.trainer import Trainer
     m = DenseModel(PRESETS["tiny"](num_layers=1, vocab_size=64, max_seq_len=16, hidden_size=32, num_heads=1, head_dim=32, ffn_hidden_size=32), dtype=torch.float32)
