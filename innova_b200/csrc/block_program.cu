@@ -56,23 +56,37 @@ struct BlockDesc {
   float *dg1, *db1, *dwqkv, *dbqkv, *dwo, *dbo, *dg2, *db2, *dw1, *dbias1, *dw2, *dbias2;   // fp32, added to
   void* scratch;
   long B, S, E, H, Hkv, D, F, gated, rms, n_codebook, quant_mode, quantised, kernel_select;
+  long keep;                       // a backward pass follows
   double eps1, eps2, scale;
+  bool in_y() const { return !keep && H * D <= E; }      // y holds what is dead before it is written
 };
 
 constexpr long AT = 256;           // every buffer starts on 256 bytes
 static long up(long bytes) { return (bytes + AT - 1) / AT * AT; }
 
-// Offsets into `saved`: the quantised weights, the activations and the statistics.
+// Offsets into `saved`: the quantised weights, the activations and the statistics. Where no backward pass follows (keep = 0) buffers whose lives
+// do not overlap share their place, as they do where the layers run one by one and free each result behind its last use, and what is dead before
+// the last product lies in its output y: a layer of width 2048 (gated MLP of 5632, 16 heads on 4) over 16 x 4096 tokens 2.49 GB instead of 3.70.
 struct BlockSaved {
   long qkv_w, o_w, w1, w2, h1, qkv, a, x2, h2, mid, act, lse, mean1, rstd1, mean2, rstd2, total;
   BlockSaved(const BlockDesc& d) {
     const long T = d.B * d.S, W = (d.H + 2 * d.Hkv) * d.D, mid_cols = d.gated ? 2 * d.F : d.F, O = d.H * d.D, q = d.quantised ? 2 : 0;
     long at = 0;
     auto take = [&](long bytes) { const long here = at; at += up(bytes); return here; };
-    qkv_w = take(q * W * d.E); o_w = take(q * d.E * O); w1 = take(q * mid_cols * d.E); w2 = take(q * d.E * d.F);
-    h1 = take(2 * T * d.E); qkv = take(2 * T * W); a = take(2 * T * O); x2 = take(2 * T * d.E); h2 = take(2 * T * d.E);
-    mid = take(2 * T * mid_cols); act = take(2 * T * d.F);
-    lse = take(4 * T * d.H); mean1 = take(4 * T); rstd1 = take(4 * T); mean2 = take(4 * T); rstd2 = take(4 * T);
+    auto max2 = [](long a, long b) { return a > b ? a : b; };
+    if (d.keep) {
+      qkv_w = take(q * W * d.E); o_w = take(q * d.E * O); w1 = take(q * mid_cols * d.E); w2 = take(q * d.E * d.F);
+      h1 = take(2 * T * d.E); qkv = take(2 * T * W); a = take(2 * T * O); x2 = take(2 * T * d.E); h2 = take(2 * T * d.E);
+      mid = take(2 * T * mid_cols); act = take(2 * T * d.F);
+      lse = take(4 * T * d.H); mean1 = take(4 * T); rstd1 = take(4 * T); mean2 = take(4 * T); rstd2 = take(4 * T);
+    } else {
+      qkv_w = o_w = w1 = w2 = take(q * max2(max2(W * d.E, d.E * O), max2(mid_cols * d.E, d.E * d.F)));   // each is quantised in front of its product
+      h1 = a = h2 = take(d.in_y() ? 0 : 2 * T * max2(d.E, O));             // norm 1, attention, norm 2: each dead before the next is written
+      const long mlp = up(2 * T * d.E) + up(2 * T * d.F) + up(2 * T * mid_cols);
+      qkv = x2 = take(max2(up(2 * T * W), mlp));                           // q, k, v are dead behind attention; then x2 and the MLP's activations
+      act = x2 + up(2 * T * d.E); mid = act + up(2 * T * d.F);
+      lse = take(4 * T * d.H); mean1 = mean2 = take(4 * T); rstd1 = rstd2 = take(4 * T);
+    }
     total = at;
   }
 };
@@ -111,6 +125,7 @@ struct BlockRun {
       : d(desc), s(desc), saved((char*)desc.saved), T((int)(desc.B * desc.S)), E((int)desc.E), W((int)((desc.H + 2 * desc.Hkv) * desc.D)),
         O((int)(desc.H * desc.D)), F((int)desc.F), mid_cols((int)(desc.gated ? 2 * desc.F : desc.F)) {}
   void* at(long o) const { return saved + o; }
+  void* early(long o) const { return d.in_y() ? (char*)d.y : saved + o; }     // norm 1, attention, norm 2 in the forward pass
   float* f32(long o) const { return (float*)(saved + o); }
   const void* weight(const void* w, long o) const { return d.quantised ? saved + o : w; }
   // runs a launch unless one before it failed
@@ -142,30 +157,29 @@ struct BlockRun {
       INV_RUN(inv_rope(buf, d.positions, d.cos_t, d.sin_t, T, (int)d.S, W, 0, (int)(d.H + d.Hkv), (int)d.D, inverse, d.stream));
   }
   void quantise(const void* w, long o, long n) {
-    INV_RUN(inv_block_quant(w, 1, at(o), 1, nullptr, nullptr, d.codebook, (int)d.n_codebook, n, (int)d.quant_mode, d.stream));
+    if (d.quantised)
+      INV_RUN(inv_block_quant(w, 1, at(o), 1, nullptr, nullptr, d.codebook, (int)d.n_codebook, n, (int)d.quant_mode, d.stream));
   }
 
   void forward() {
-    if (d.quantised) {
-      quantise(d.wqkv, s.qkv_w, (long)W * E);
-      quantise(d.wo, s.o_w, (long)E * O);
-      quantise(d.w1, s.w1, (long)mid_cols * E);
-      quantise(d.w2, s.w2, (long)E * F);
-    }
-    INV_RUN(inv_norm_fwd(d.x, nullptr, d.g1, d.b1, at(s.h1), nullptr, f32(s.mean1), f32(s.rstd1), T, E, (float)d.eps1, (int)d.rms, d.stream));
-    product(at(s.h1), weight(d.wqkv, s.qkv_w), at(s.qkv), T, W, E, 0, EPI_NONE, d.bqkv, nullptr, nullptr);
+    INV_RUN(inv_norm_fwd(d.x, nullptr, d.g1, d.b1, early(s.h1), nullptr, f32(s.mean1), f32(s.rstd1), T, E, (float)d.eps1, (int)d.rms, d.stream));
+    quantise(d.wqkv, s.qkv_w, (long)W * E);
+    product(early(s.h1), weight(d.wqkv, s.qkv_w), at(s.qkv), T, W, E, 0, EPI_NONE, d.bqkv, nullptr, nullptr);
     rotate(at(s.qkv), 0);
     const char* q = (const char*)at(s.qkv);
-    INV_RUN(inv_flash_attn_fwd(q, q + O * 2, q + (O + d.Hkv * d.D) * 2, at(s.a), f32(s.lse), (int)d.B, (int)d.S, (int)d.H, (int)d.Hkv, (int)d.D, W, W, W, O,
+    INV_RUN(inv_flash_attn_fwd(q, q + O * 2, q + (O + d.Hkv * d.D) * 2, early(s.a), f32(s.lse), (int)d.B, (int)d.S, (int)d.H, (int)d.Hkv, (int)d.D, W, W, W, O,
                                (float)d.scale, 1, 0, d.status, d.stream));
-    product(at(s.a), weight(d.wo, s.o_w), at(s.x2), T, E, O, 0, EPI_ADD, d.bo, d.x, nullptr);
-    INV_RUN(inv_norm_fwd(at(s.x2), nullptr, d.g2, d.b2, at(s.h2), nullptr, f32(s.mean2), f32(s.rstd2), T, E, (float)d.eps2, (int)d.rms, d.stream));
+    quantise(d.wo, s.o_w, (long)E * O);
+    product(early(s.a), weight(d.wo, s.o_w), at(s.x2), T, E, O, 0, EPI_ADD, d.bo, d.x, nullptr);
+    INV_RUN(inv_norm_fwd(at(s.x2), nullptr, d.g2, d.b2, early(s.h2), nullptr, f32(s.mean2), f32(s.rstd2), T, E, (float)d.eps2, (int)d.rms, d.stream));
+    quantise(d.w1, s.w1, (long)mid_cols * E);
     if (d.gated) {
-      product(at(s.h2), weight(d.w1, s.w1), at(s.mid), T, mid_cols, E, 0, EPI_NONE, d.bias1, nullptr, nullptr);
+      product(early(s.h2), weight(d.w1, s.w1), at(s.mid), T, mid_cols, E, 0, EPI_NONE, d.bias1, nullptr, nullptr);
       INV_RUN(inv_act(at(s.mid), nullptr, at(s.act), T, F, 2, d.stream));
     } else {
-      product(at(s.h2), weight(d.w1, s.w1), at(s.act), T, F, E, 0, EPI_GELU_DG, d.bias1, nullptr, at(s.mid));
+      product(early(s.h2), weight(d.w1, s.w1), at(s.act), T, F, E, 0, EPI_GELU_DG, d.bias1, nullptr, at(s.mid));
     }
+    quantise(d.w2, s.w2, (long)E * F);
     product(at(s.act), weight(d.w2, s.w2), d.y, T, E, F, 0, EPI_ADD, d.bias2, at(s.x2), nullptr);
   }
 
@@ -219,11 +233,12 @@ struct BlockRun {
 
 using namespace inv;
 
-// Bytes of the caller's buffers: `saved` (which = 0), the backward pass's scratch (1).
+// Bytes of the caller's buffer: `saved` of a forward pass that a backward pass follows (which = 0), the backward pass's scratch (1), `saved` of a
+// forward pass alone (2).
 extern "C" int inv_block_bytes(int which, long B, long S, long E, long H, long Hkv, long D, long F, long gated, long quantised, long* bytes) {
-  if (which < 0 || which > 1 || B < 1 || S < 1 || E < 1 || H < 1 || Hkv < 1 || D < 1 || F < 1) return -ERR_BAD_ARG;
+  if (which < 0 || which > 2 || B < 1 || S < 1 || E < 1 || H < 1 || Hkv < 1 || D < 1 || F < 1) return -ERR_BAD_ARG;
   BlockDesc d{};
-  d.B = B; d.S = S; d.E = E; d.H = H; d.Hkv = Hkv; d.D = D; d.F = F; d.gated = gated; d.quantised = quantised;
+  d.B = B; d.S = S; d.E = E; d.H = H; d.Hkv = Hkv; d.D = D; d.F = F; d.gated = gated; d.quantised = quantised; d.keep = which != 2;
   *bytes = which == 1 ? BlockScratch(d).total : BlockSaved(d).total;
   return 0;
 }

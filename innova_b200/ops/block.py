@@ -23,18 +23,18 @@ _gemm = importlib.import_module(".gemm", __package__)      # the module: the pac
 
 _native.register_cuda_sigs({"inv_block_fwd": [_native.vp], "inv_block_bwd": [_native.vp], "inv_block_bytes": [_native.i32] + [_native.i64] * 9 + [_native.vp]})
 
-# BlockDesc: 12 parameters, tables, positions, codebook, x, y, saved, status, stream | dy, dx, two column sums, 12 gradients, scratch | 13 sizes |
+# BlockDesc: 12 parameters, tables, positions, codebook, x, y, saved, status, stream | dy, dx, two column sums, 12 gradients, scratch | 14 sizes |
 # eps1, eps2, scale
-_PACK = struct.Struct("=12Q 9Q 17Q 13q 3d").pack
+_PACK = struct.Struct("=12Q 9Q 17Q 14q 3d").pack
 _FORWARD_ONLY = (0,) * 17
 
 
-SAVED, SCRATCH = 0, 1
+SAVED, SCRATCH, FORWARD = 0, 1, 2
 
 
 @functools.lru_cache(maxsize=256)
 def _bytes(which, B, S, E, H, Hkv, D, F, gated, quantised):
-    """What the native side lays out: what the forward pass leaves for the backward pass, and that pass's scratch."""
+    """What the native side lays out: the forward pass's buffer when a backward pass follows, that pass's scratch, a forward pass's alone."""
     n = C.c_long()
     if rt.lib().inv_block_bytes(which, B, S, E, H, Hkv, D, F, gated, quantised, C.addressof(n)) != 0:
         raise ValueError("block sizes")
@@ -50,13 +50,16 @@ class _BlockFn(torch.autograd.Function):
     be None."""
 
     @staticmethod
-    def forward(ctx, x, cfg, cos, sin, positions, codebook, *params):
+    def forward(ctx, x, cfg, keep, cos, sin, positions, codebook, *params):
         H, Hkv, D, F, gated, rms, eps1, eps2, mode = cfg
         B, S, E = x.shape
         dev = x.device
-        saved = torch.empty(_bytes(SAVED, B, S, E, H, Hkv, D, F, gated, int(codebook is not None)), dtype=torch.uint8, device=dev)
+        # without gradients nothing is left for a backward pass, and buffers share their places
+        saved = torch.empty(_bytes(SAVED if keep else FORWARD, B, S, E, H, Hkv, D, F, gated, int(codebook is not None)), dtype=torch.uint8, device=dev)
         y = torch.empty_like(x)
-        _issue("inv_block_fwd", cfg, (B, S, E), params, cos, sin, positions, codebook, x, y.data_ptr(), saved, _FORWARD_ONLY)
+        _issue("inv_block_fwd", cfg, (B, S, E), params, cos, sin, positions, codebook, x, y.data_ptr(), saved, _FORWARD_ONLY, int(keep))
+        if not keep:
+            return y
         ctx.cfg = cfg
         ctx.main_grads = main_grads(*params)
         ctx.save_for_backward(x, saved, cos, sin, positions, codebook, *params)
@@ -96,14 +99,14 @@ class _BlockFn(torch.autograd.Function):
                 mg.add_(g.view(mg.shape))
             else:
                 out[i] = g.to(p.dtype)
-        return (dx, None, None, None, None, None, *out)
+        return (dx, None, None, None, None, None, None, *out)
 
 
-def _issue(what, cfg, shape, params, cos, sin, positions, codebook, x, y, saved, backward):
+def _issue(what, cfg, shape, params, cos, sin, positions, codebook, x, y, saved, backward, keep=1):
     H, Hkv, D, F, gated, rms, eps1, eps2, mode = cfg
     desc = _PACK(*[_ptr(p) for p in params], _ptr(cos), _ptr(sin), _ptr(positions), _ptr(codebook), x.data_ptr(), y, saved.data_ptr(),
                  rt.status_tensor(x.device).data_ptr(), rt.stream_ptr(), *backward,
-                 *shape, H, Hkv, D, F, gated, rms, 0 if codebook is None else codebook.numel(), mode, int(codebook is not None), _gemm._kernel_select,
+                 *shape, H, Hkv, D, F, gated, rms, 0 if codebook is None else codebook.numel(), mode, int(codebook is not None), _gemm._kernel_select, keep,
                  eps1, eps2, D ** -0.5)
     n = getattr(rt.lib(), what)(desc)
     rt.check(min(n, 0), what)
@@ -150,4 +153,4 @@ def block_forward(blk, x, rope, positions):
             codebook = default_codebook(cfg.ste_format, x.device)
         mode = MODES[cfg.ste_format]
     return _BlockFn.apply(x, (cfg.num_heads, cfg.kv_heads, cfg.head_dim, F, int(gated), int(n1.kind != "layernorm"), float(n1.eps), float(n2.eps), mode),
-                          cos, sin, positions, codebook, *params)
+                          grad, cos, sin, positions, codebook, *params)

@@ -140,6 +140,30 @@ def test_block_buffers_are_sized_by_their_layout():
     """The bytes that the native side asks for, stated once more by hand, at sizes off the 256 bytes that buffers start on."""
     from innova_b200.ops import block
     up = lambda *n: sum((x + 255) // 256 * 256 for x in n)
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw", [{}, GELU, dict(ste_format="oil8", num_kv_heads=2), dict(GELU, ste_format="oil4"), dict(hidden_size=128, num_heads=4, ffn_hidden_size=64)])
+def test_block_without_gradients(kw, monkeypatch):
+    """No graph: the same output, and no more memory at once than layer by layer (and the bytes by which buffers are rounded up)."""
+    m = _model(**kw)
+    x = torch.randn(4, 500, m.cfg.hidden_size, device=DEV).bfloat16()
+    rope = m.rope(x.device)
+    want = m.layers[0](x, rope)
+
+    def peak():
+        torch.cuda.synchronize()
+        base = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        with torch.no_grad():
+            y = m.layers[0](x, rope)
+        torch.cuda.synchronize()
+        assert torch.equal(y, want) and not y.requires_grad
+        return torch.cuda.max_memory_allocated() - base
+
+    once = peak()
+    monkeypatch.setattr(dense.ops, "block_forward", lambda *a: None)
+    assert once <= peak() + 64 * 1024
+
+
     for B, S, E, H, Hkv, D, F, gated, q in ((1, 1, 64, 1, 1, 64, 8, 0, 0), (3, 77, 200, 4, 2, 64, 136, 1, 1), (2, 129, 1280, 5, 1, 128, 200, 0, 1)):
         T, W, O, mid = B * S, (H + 2 * Hkv) * D, H * D, 2 * F if gated else F
         weights = up(*(2 * q * n for n in (W * E, E * O, mid * E, E * F)))
@@ -150,6 +174,8 @@ def test_block_buffers_are_sized_by_their_layout():
         attn = up(up(4 * B * H * S) + 4 * T * O)
         grid = max(1, min(148, (T + 7) // 8))
         assert block._bytes(block.SCRATCH, *args) == max(mlp, up(2 * T * W)) + up(2 * T * E, 2 * T * E, 2 * T * O, 4 * E, grid * 3 * E * 4) + attn
+        once = up(0 if O <= E else 2 * T * max(E, O)) + max(up(2 * T * W), up(2 * T * E, 2 * T * F, 2 * T * mid))
+        assert block._bytes(block.FORWARD, *args) == up(2 * q * max(W * E, E * O, mid * E, E * F)) + once + up(4 * T * H) + 2 * up(4 * T)
     with pytest.raises(ValueError):
         block._bytes(block.SAVED, 0, 1, 64, 1, 1, 64, 8, 0, 0)
 
