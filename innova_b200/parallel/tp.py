@@ -335,10 +335,12 @@ class TPDecoder:
                    and skinny_takes(l["gu"], B) and skinny_takes(l["down"], B) for l in self.layers)
 
     def _gathers(self, tokens: torch.Tensor) -> bool:
-        """Whether the step's own gather takes these tokens and this table: whole rows of 16-byte pieces."""
+        """Whether the step's own gather takes these tokens and this table: one token for each of the cache's first rows, on the table's
+        device; whole rows of 16-byte pieces."""
         e = self.emb
-        return (e.is_contiguous() and e.data_ptr() % 16 == 0 and e.shape[1] * e.element_size() % 16 == 0 and tokens.dtype == torch.int64
-                and tokens.is_contiguous() and self.cache.seq_lens.dtype == torch.int32)
+        return (tokens.device == e.device and tokens.dim() == 1 and tokens.shape[0] <= self.cache.seq_lens.shape[0] and e.is_contiguous()
+                and e.data_ptr() % 16 == 0 and e.shape[1] * e.element_size() % 16 == 0 and tokens.dtype == torch.int64 and tokens.is_contiguous()
+                and self.cache.seq_lens.dtype == torch.int32)
 
     @torch.no_grad()
     def _decode_step(self, tokens: torch.Tensor) -> torch.Tensor:

@@ -181,3 +181,13 @@ def test_cuda_entry_points_need_a_signature(monkeypatch):
         lib.labs(-3)
     lib.labs.argtypes, lib.labs.restype = [ctypes.c_long], ctypes.c_long
     assert lib.labs(-2 ** 40) == 2 ** 40
+
+
+def test_a_decode_step_gathers_only_tokens_on_its_device():
+    """Tokens elsewhere, of another shape or for more rows than the cache has are looked up by PyTorch, whose checks they get."""
+    from types import SimpleNamespace
+    from innova_b200.parallel.tp import TPDecoder
+    dec = SimpleNamespace(emb=torch.empty(50, 64, dtype=torch.bfloat16, device="meta"), cache=SimpleNamespace(seq_lens=torch.zeros(4, dtype=torch.int32)))
+    tok = lambda *s, **kw: torch.zeros(*s, **{"dtype": torch.int64, "device": "meta", **kw})
+    assert TPDecoder._gathers(dec, tok(4))
+    assert not any(TPDecoder._gathers(dec, t) for t in (tok(4, device="cpu"), tok(5), tok(2, 2), tok(4, dtype=torch.int32)))

@@ -110,6 +110,16 @@ def test_generation_through_changing_sizes(kv):
             assert float(behind.max()) < 4 * LOGITS[kv] * float(z.std())
 
 
+def test_a_step_takes_tokens_from_the_host():
+    dec = decoder("bf16")
+    dec._splits, dec._scratch = 1, torch.empty(1, device="cuda")
+    got = []
+    for dev in ("cuda", "cpu"):
+        dec.prefill(tokens(3, 7, 5))
+        got.append(dec._decode_step(tokens(3, 1, 6)[:, 0].contiguous().to(dev)))
+    assert float((got[0] - got[1]).norm() / got[0].norm()) < 2e-2
+
+
 def test_the_route_of_a_step_follows_its_weights():
     """Too many tokens are told from the head alone; a matrix or norm off its alignment takes the whole step to the tile product."""
     from innova_b200.parallel import tp
