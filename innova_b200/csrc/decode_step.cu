@@ -5,13 +5,18 @@
 
 namespace inv {
 
-// x[b, :] = emb[tokens[b], :], pos[b] = lens[b], lens[b] += 1. grid (pieces of a row, B); one thread a sequence moves its length.
+// x[b, :] = emb[tokens[b], :], pos[b] = lens[b], lens[b] += 1. A token below zero counts from the end of the table, one outside it reads row 0
+// and leaves ERR_BAD_ARG in *status. grid (pieces of a row, B); one thread a sequence moves its length.
 __global__ void __launch_bounds__(256) step_begin_kernel(const int64_t* __restrict__ tokens, const uint4* __restrict__ emb, int row, int rows,
-                                                         uint4* __restrict__ x, int* __restrict__ lens, int* __restrict__ pos) {
+                                                         uint4* __restrict__ x, int* __restrict__ lens, int* __restrict__ pos, int* status) {
   const int b = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x;
   if (i < row) {
     int64_t id = tokens[b];
-    if (id < 0 || id >= rows) id = 0;
+    if (id < 0) id += rows;
+    if (id < 0 || id >= rows) {
+      if (i == 0 && status) atomicCAS(status, 0, ERR_BAD_ARG);
+      id = 0;
+    }
     x[(size_t)b * row + i] = emb[(size_t)id * row + i];
   }
   if (i == 0) {
@@ -79,18 +84,22 @@ __global__ void __launch_bounds__(1024) step_next_kernel(const float* __restrict
 
 using namespace inv;
 
-// emb: rows of row_bytes bytes (a multiple of 16) on 16 bytes; tokens int64 [B]. Plainly launched.
-extern "C" int inv_step_begin(const void* tokens, const void* emb, int row_bytes, int rows, void* x, int* lens, int* pos, int B, void* stream) {
+// emb: rows of row_bytes bytes (a multiple of 16) on 16 bytes; tokens int64 [B]; status may be null. Plainly launched.
+extern "C" int inv_step_begin_checked(const void* tokens, const void* emb, int row_bytes, int rows, void* x, int* lens, int* pos, int B, int* status,
+                                      void* stream) {
   if (row_bytes < 16 || row_bytes % 16 || rows < 1 || ((uintptr_t)emb | (uintptr_t)x) % 16) return -ERR_BAD_ARG;
   if (B <= 0) return 0;
   const int row = row_bytes / 16;
   for (int b0 = 0; b0 < B; b0 += 65535) {
     const int n = B - b0 < 65535 ? B - b0 : 65535;
     step_begin_kernel<<<dim3((row + 255) / 256, n), 256, 0, (cudaStream_t)stream>>>((const int64_t*)tokens + b0, (const uint4*)emb, row, rows,
-                                                                                    (uint4*)x + (size_t)b0 * row, lens + b0, pos + b0);
+                                                                                    (uint4*)x + (size_t)b0 * row, lens + b0, pos + b0, status);
   }
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
+}
+extern "C" int inv_step_begin(const void* tokens, const void* emb, int row_bytes, int rows, void* x, int* lens, int* pos, int B, void* stream) {
+  return inv_step_begin_checked(tokens, emb, row_bytes, rows, x, lens, pos, B, nullptr, stream);
 }
 
 // logits fp32 [B, ld], V of each row; next int64 [B]; out int64 [B, ld_out] or null.

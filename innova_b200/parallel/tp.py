@@ -32,6 +32,7 @@ from ..ops.oil_linear import (SKINNY_SUMS, SKINNY_SWIGLU, QuantWeight, _acc_for,
 
 _native.register_cuda_sigs({
     "inv_step_begin": [_native.vp, _native.vp, _native.i32, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp],
+    "inv_step_begin_checked": [_native.vp, _native.vp, _native.i32, _native.i32, _native.vp, _native.vp, _native.vp, _native.i32, _native.vp, _native.vp],
     "inv_step_next": [_native.vp, _native.i64, _native.i32, _native.vp, _native.vp, _native.i32, _native.vp, _native.i32, _native.i32, _native.vp],
 })
 
@@ -345,15 +346,17 @@ class TPDecoder:
     @torch.no_grad()
     def _decode_step(self, tokens: torch.Tensor) -> torch.Tensor:
         """tokens [B] -> logits [B, vocab]. Uses and advances the device-side sequence lengths. The lookups in front of the first
-        projection are ordinary kernels, so all weights are resident."""
+        projection are ordinary kernels, so all weights are resident. A token that the table does not have is an error of the status word
+        (``check_status``)."""
         cfg, c = self.cfg, self.cache
         B = tokens.shape[0]
         lens = c.seq_lens[:B]
         if self._gathers(tokens):               # x, the new tokens' positions and the advanced lengths in one launch
             x = torch.empty(B, self.emb.shape[1], dtype=self.emb.dtype, device=self.dev)
             pos = torch.empty(B, dtype=torch.int32, device=self.dev)
-            rt.check(rt.lib().inv_step_begin(tokens.data_ptr(), self.emb.data_ptr(), self.emb.shape[1] * self.emb.element_size(), self.emb.shape[0],
-                                             x.data_ptr(), lens.data_ptr(), pos.data_ptr(), B, rt.stream_ptr()), "inv_step_begin")
+            rt.check(rt.lib().inv_step_begin_checked(tokens.data_ptr(), self.emb.data_ptr(), self.emb.shape[1] * self.emb.element_size(),
+                                                     self.emb.shape[0], x.data_ptr(), lens.data_ptr(), pos.data_ptr(), B,
+                                                     rt.status_tensor(self.dev).data_ptr(), rt.stream_ptr()), "inv_step_begin_checked")
         else:
             pos = lens.clone()                  # position of the new token
             lens.add_(1)

@@ -120,6 +120,28 @@ def test_a_step_takes_tokens_from_the_host():
     assert float((got[0] - got[1]).norm() / got[0].norm()) < 2e-2
 
 
+def test_a_step_counts_tokens_from_the_end_and_reports_others():
+    """As PyTorch's lookup: a negative token is a row from the end of the table, one outside it an error, here of the status word."""
+    from innova_b200.ops import runtime as rt
+    dec = decoder("bf16")
+    dec._splits, dec._scratch = 1, torch.empty(1, device="cuda")
+    rows = dec.emb.shape[0]
+
+    def step(*t):
+        dec.prefill(tokens(2, 5, 3))
+        return dec._decode_step(torch.tensor(t, device="cuda"))
+
+    want = step(rows - 1, 7)
+    got = step(-1, 7)
+    rt.check_status()
+    assert float((got - want).norm() / want.norm()) < 2e-2
+    for bad in (rows, -rows - 1, 2 ** 40):
+        step(3, bad)
+        with pytest.raises(RuntimeError, match="bad_arg"):
+            rt.check_status()
+    rt.check_status()
+
+
 def test_the_route_of_a_step_follows_its_weights():
     """Too many tokens are told from the head alone; a matrix or norm off its alignment takes the whole step to the tile product."""
     from innova_b200.parallel import tp
