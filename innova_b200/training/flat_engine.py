@@ -98,8 +98,8 @@ class FlatParamEngine:
         bc1, bc2 = 1.0 - b1 ** t, 1.0 - b2 ** t
         lr_adj = lr * math.sqrt(bc2) / bc1 if self.reference_formula else lr / bc1
         self._hyper_slot = (self._hyper_slot + 1) % self._hyper_ring.shape[0]
-        self._hyper_rows[self._hyper_slot, :9] = (lr_adj, b1, b2, self.eps, lr * wd, 1.0 / bc2, self.max_grad_norm or 0.0, grad_scale,
-                                                  1.0 if self.reference_formula else 0.0)
+        row = (lr_adj, b1, b2, self.eps, lr * wd, 1.0 / bc2, self.max_grad_norm or 0.0, grad_scale, 1.0 if self.reference_formula else 0.0)
+        self._hyper_rows[self._hyper_slot, :9] = [float(v) for v in row]      # any of them may be a tensor
         return self._hyper_ring[self._hyper_slot]
 
     def zero_grad(self):

@@ -102,3 +102,16 @@ def test_main_grad_that_a_backward_pass_uses():
     kept = main_grads(copy)[0]
     del copy
     assert main_grad_of(p.detach(), kept) is buf
+
+
+def test_hyperparameters_may_be_tensors():
+    from innova_b200.training.flat_engine import FlatParamEngine
+    out = []
+    for scale, lr in ((0.5, 1e-2), (torch.tensor([0.5], dtype=torch.bfloat16), torch.tensor(1e-2, dtype=torch.float64))):
+        torch.manual_seed(0)
+        lin = torch.nn.Linear(8, 8)
+        eng = FlatParamEngine(lin, lr=lr)
+        eng.flat_grad.copy_(torch.randn_like(eng.flat_grad))
+        eng.step(grad_scale=scale)
+        out.append(eng.master)
+    assert torch.equal(*out)
