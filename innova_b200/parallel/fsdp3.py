@@ -32,7 +32,7 @@ import torch
 import torch.distributed as dist
 
 from .. import _native, ops
-from ..training.flat_engine import _round_up
+from ..training.flat_engine import HyperRows, _round_up
 
 ALIGN = 64            # elements: every parameter starts 128-byte aligned inside its unit
 JOB_GATHER, JOB_REDUCE = 1, 2
@@ -182,10 +182,7 @@ class FSDP3Engine:
         self._prepared = set()
         self.gnorm_sq = torch.zeros(1, dtype=torch.float32, device=dev)
         self.hyper = torch.zeros(2, 16, dtype=torch.float32, device=dev)
-        self._hyper_ring = torch.zeros(64, 16, dtype=torch.float32)
-        self._hyper_slot = 0
-        if dev.type == "cuda":
-            self._hyper_ring = self._hyper_ring.pin_memory()
+        self._hyper_rows = HyperRows(64, dev)
         # one row of partial sums of squares per reduce piece (a piece = what one GEMM carries), one float per helper CTA
         self.MAX_PIECES, self.MAX_CTAS = 1024, 64
         self.sumsq_parts = torch.zeros(self.MAX_PIECES * self.MAX_CTAS, dtype=torch.float32, device=dev)
@@ -436,11 +433,8 @@ class FSDP3Engine:
         lr = self.current_lr()
         bc1, bc2 = 1.0 - b1 ** t, 1.0 - b2 ** t
         lr_adj = lr * math.sqrt(bc2) / bc1 if self.reference_formula else lr / bc1
-        self._hyper_slot = (self._hyper_slot + 1) % self._hyper_ring.shape[0]
-        h = self._hyper_ring[self._hyper_slot]
-        h[0], h[1], h[2], h[3], h[4], h[5] = lr_adj, b1, b2, self.eps, lr * wd, 1.0 / bc2
-        h[6], h[7], h[8] = self.max_grad_norm or 0.0, grad_scale, 1.0 if self.reference_formula else 0.0
-        return h
+        return self._hyper_rows.fill(lr_adj, b1, b2, self.eps, lr * wd, 1.0 / bc2, self.max_grad_norm or 0.0, grad_scale,
+                                     1.0 if self.reference_formula else 0.0)
 
     def micro_step_done(self):
         """Between micro-batches of one optimizer step (gradient accumulation); the next forward calls it by itself."""
@@ -489,8 +483,8 @@ class FSDP3Engine:
             dist.all_reduce(self.gnorm_sq, group=self.group)
         h0 = self._fill_hyper(self.weight_decay, grad_scale)
         h1 = self._fill_hyper(0.0, grad_scale)
-        self.hyper[0].copy_(h0, non_blocking=True)
-        self.hyper[1].copy_(h1, non_blocking=True)
+        self._hyper_rows.send(self.hyper[0], h0)
+        self._hyper_rows.send(self.hyper[1], h1)
         for u in self.units:
             lo, hi = self.rank * u.n, (self.rank + 1) * u.n      # this rank's range inside the unit
             d_hi = min(hi, max(lo, u.decay_end))

@@ -24,6 +24,40 @@ def _round_up(n, a):
     return (n + a - 1) // a * a
 
 
+class HyperRows:
+    """Rows of 16 hyperparameters in pinned memory on their way to the device. A copy is asynchronous: a row is written again only when the
+    stream has read it, which the host waits for when it is a whole ring of rows ahead."""
+
+    def __init__(self, rows: int, device, event=None):
+        self.rows = torch.zeros(rows, 16, dtype=torch.float32)
+        if device.type == "cuda":
+            self.rows = self.rows.pin_memory()
+        self._values = self.rows.numpy()        # the same memory: a row is written in one assignment
+        self._event = event or (torch.cuda.Event if device.type == "cuda" else None)
+        self._read = [None] * rows              # the event behind the last copy of each row ...
+        self._sent = [False] * rows             # ... where there was one since the row was written
+        self._slot = 0
+
+    def fill(self, *values) -> torch.Tensor:
+        """The next row, holding ``values`` (numbers, or tensors of one)."""
+        self._slot = slot = (self._slot + 1) % len(self._read)
+        if self._sent[slot]:
+            self._read[slot].synchronize()
+            self._sent[slot] = False
+        self._values[slot, :len(values)] = [float(v) for v in values]
+        return self.rows[slot]
+
+    def send(self, dst: torch.Tensor, row: torch.Tensor):
+        dst.copy_(row, non_blocking=True)
+        if self._event is None or (dst.is_cuda and torch.cuda.is_current_stream_capturing()):
+            return
+        slot = row.storage_offset() // 16
+        if self._read[slot] is None:
+            self._read[slot] = self._event()
+        self._read[slot].record(*((torch.cuda.current_stream(dst.device),) if dst.is_cuda else ()))
+        self._sent[slot] = True
+
+
 class FlatParamEngine:
     def __init__(self, model: torch.nn.Module, lr: float = 3e-4, betas=(0.9, 0.999), eps: float = 1e-8, weight_decay: float = 0.1,
                  max_grad_norm: float = 1.0, lr_schedule: Optional[Callable[[int], float]] = None, reference_formula: bool = False,
@@ -65,13 +99,7 @@ class FlatParamEngine:
         self._init_state(0, self.total)
         self.gnorm_sq = torch.zeros(1, dtype=torch.float32, device=self.device)
         self.hyper = torch.zeros(16, dtype=torch.float32, device=self.device)
-        # ring of pinned staging rows: the copy to the device is asynchronous, so a row must not be
-        # rewritten before the stream has consumed it (the host never runs more than a few steps ahead)
-        self._hyper_ring = torch.zeros(32, 16, dtype=torch.float32)
-        self._hyper_slot = 0
-        if self.device.type == "cuda":
-            self._hyper_ring = self._hyper_ring.pin_memory()
-        self._hyper_rows = self._hyper_ring.numpy()      # the same memory: a row is written in one assignment
+        self._hyper_rows = HyperRows(32, self.device)
 
     def _pre_alloc(self):
         pass
@@ -97,10 +125,8 @@ class FlatParamEngine:
         lr = self.current_lr()
         bc1, bc2 = 1.0 - b1 ** t, 1.0 - b2 ** t
         lr_adj = lr * math.sqrt(bc2) / bc1 if self.reference_formula else lr / bc1
-        self._hyper_slot = (self._hyper_slot + 1) % self._hyper_ring.shape[0]
-        row = (lr_adj, b1, b2, self.eps, lr * wd, 1.0 / bc2, self.max_grad_norm or 0.0, grad_scale, 1.0 if self.reference_formula else 0.0)
-        self._hyper_rows[self._hyper_slot, :9] = [float(v) for v in row]      # any of them may be a tensor
-        return self._hyper_ring[self._hyper_slot]
+        return self._hyper_rows.fill(lr_adj, b1, b2, self.eps, lr * wd, 1.0 / bc2, self.max_grad_norm or 0.0, grad_scale,
+                                     1.0 if self.reference_formula else 0.0)
 
     def zero_grad(self):
         self.flat_grad.zero_()
@@ -121,7 +147,7 @@ class FlatParamEngine:
             from ..ops import runtime as rt
             h = self._fill_hyper(wd, grad_scale)
             hyper = self.hyper if wd == self.weight_decay else self._hyper_nd
-            hyper.copy_(h, non_blocking=True)
+            self._hyper_rows.send(hyper, h)
             rt.check(rt.lib().inv_adamw(p.data_ptr(), m.data_ptr(), v.data_ptr(), g.data_ptr(),
                                         p16.data_ptr() if self.dtype == torch.bfloat16 else 0, n, hyper.data_ptr(), gnorm_sq.data_ptr(), 1,
                                         rt.stream_ptr()), "inv_adamw")

@@ -104,6 +104,34 @@ def test_main_grad_that_a_backward_pass_uses():
     assert main_grad_of(p.detach(), kept) is buf
 
 
+def test_a_row_of_hyperparameters_is_kept_until_it_was_read():
+    """The copy of a row is asynchronous: whatever the host's lead, its memory is written again only behind the event of that copy."""
+    from innova_b200.training.flat_engine import HyperRows
+    log = []
+
+    class Event:
+        def record(self):
+            self.row = rows.rows[rows._slot].clone()
+            log.append("sent")
+
+        def synchronize(self):
+            assert torch.equal(rows.rows[rows._slot], self.row)              # still what the copy has to read
+            log.append("waited")
+
+    rows = HyperRows(3, torch.device("cpu"), Event)
+    dst = torch.zeros(16)
+    for i in range(7):
+        row = rows.fill(i, 2.0, torch.tensor([0.5]))
+        rows.send(dst, row)
+        assert dst[:3].tolist() == [i, 2.0, 0.5]
+    assert log == ["sent"] * 3 + ["waited", "sent"] * 4
+    rows.fill(9.0)
+    rows.fill(9.0)
+    rows.fill(9.0)
+    rows.fill(9.0)                                                           # rows that were never sent need no wait
+    assert log[-3:] == ["waited"] * 3
+
+
 def test_hyperparameters_may_be_tensors():
     from innova_b200.training.flat_engine import FlatParamEngine
     out = []
