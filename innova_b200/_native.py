@@ -43,23 +43,29 @@ _CUDA_SIGS = {
 }
 
 
-class _Unbound:
-    """First parameter of an entry point nobody has declared."""
-
-    @classmethod
-    def from_param(cls, _):
-        raise TypeError("no signature: import the module that registers this entry point, or set its argtypes")
-
-
 class _CudaLib(C.CDLL):
-    """Entry points refuse to be called with arguments before their signature is known: without one, ctypes would pass pointers as
-    32-bit integers and a kernel would get an address that is not one. The module that owns an entry point registers it when it
-    is imported."""
+    """An entry point that nobody has declared yet refuses plain integers: ctypes would pass them as 32 bits, a pointer among them too, and a kernel
+    would get an address that is not one. The module that owns an entry point registers its signature when it is imported. Calls
+    without arguments, or with ctypes values, which say what they are, need none."""
+
+    def __init__(self, *args, **kw):
+        super().__init__(*args, **kw)
+
+        class Undeclared(self._FuncPtr):
+            _flags_, _restype_ = self._FuncPtr._flags_, self._FuncPtr._restype_
+
+            def __call__(self, *args):
+                if self.argtypes is None and any(type(a) is int for a in args):
+                    raise C.ArgumentError("no signature: import the module that registers this entry point, or set its argtypes")
+                return super().__call__(*args)
+
+        self._undeclared = Undeclared
 
     def __getattr__(self, name):
         fn = super().__getattr__(name)
         if name not in _CUDA_SIGS:
-            fn.argtypes = [_Unbound]
+            fn = self._undeclared((name, self))
+            setattr(self, name, fn)
         return fn
 
 

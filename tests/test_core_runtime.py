@@ -183,6 +183,19 @@ def test_cuda_entry_points_need_a_signature(monkeypatch):
     assert lib.labs(-2 ** 40) == 2 ** 40
 
 
+def test_cuda_entry_points_without_a_signature_take_what_says_its_type(monkeypatch):
+    import ctypes
+    import os
+    from innova_b200 import _native
+    monkeypatch.setattr(_native, "_CUDA_SIGS", {})
+    lib = _native._CudaLib(None)
+    assert lib.getpid() == os.getpid() and lib.labs(ctypes.c_long(-5)) == 5 and lib.strlen(b"four") == 4
+    with pytest.raises(ctypes.ArgumentError, match="no signature"):
+        lib.labs(-5)
+    _native._bind(lib, {"labs": [_native.i64]})                             # registered since
+    assert lib.labs(-5) == 5
+
+
 def test_a_decode_step_gathers_only_tokens_on_its_device():
     """Tokens elsewhere, of another shape or for more rows than the cache has are looked up by PyTorch, whose checks they get."""
     from types import SimpleNamespace
