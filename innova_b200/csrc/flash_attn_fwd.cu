@@ -43,7 +43,8 @@ struct FlashFwdParams {
   int chunk;   // EXT; > 0 (causal only): a query sees the earlier keys of its own chunk of `chunk` positions (counted from position 0)
   const __nv_bfloat16* gate;  // EXT: the output is multiplied by sigmoid(gate), element by element; null: no gate
   int ld_gate;
-  uint32_t inv_per, inv_h, inv_group;  // of the divisors in FwdItems (fa_reciprocal)
+  int by_length, stride;                  // how items are numbered (FwdItems)
+  uint32_t inv_stride, inv_h, inv_group;  // of the divisors in FwdItems (div_reciprocal)
   const int* cu;  // packed batch: sequence b is rows [cu[b], cu[b + 1]) of the token-major buffers; null: B sequences of S rows
   int* status;
 };
@@ -61,30 +62,25 @@ struct FlashFwdParams {
 //   * sums the exponentials on the FMA pipe: packed bf16 adds over groups of four, then fp32.
 // TMEM columns per CTA: S [0,128) fp32, O [128,128+D) fp32, P packed bf16: [192,256) for D = 64, [0,64) for D = 128.
 // ------------------------------------------------------------------------------------------------
-// TWO: two CTAs share an SM.
-template <int ND, bool TWO>
+// TWO: two CTAs share an SM. LOOP: CTAs take several items.
+template <int ND, bool TWO, bool LOOP>
 struct Fwd3Smem {
   static constexpr int TILE = ND * 16384;
-  static constexpr int QB = ND == 1 ? 2 : 1;     // Q tiles: the next item's is loaded ahead where there is room
-  static constexpr int SLOTS = TWO && ND == 2 ? 2 : 4;
+  static constexpr int QB = ND == 1 && LOOP ? 2 : 1;     // Q tiles: the next item's is loaded ahead where there is room
+  static constexpr int SLOTS = TWO && ND == 2 ? 2 : ND == 1 && !LOOP ? 5 : 4;
   static constexpr int Q_OFF = 0;
   static constexpr int KV_OFF = QB * TILE;
   static constexpr int BAR_OFF = KV_OFF + SLOTS * TILE;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
-// Walks a CTA's items: numbered head by head and query block by query block, the longest (causal) first; every other round runs backwards over the
-// CTAs, so that long and short items even out. Blocks past the end of a packed sequence are skipped.
-__host__ __device__ inline uint32_t fa_reciprocal(int d) { return d == 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d); }
-__device__ __forceinline__ int fa_divide(int n, int d, uint32_t inv) {
-  if (inv == 0) return n;
-  const int q = (int)__umulhi((uint32_t)n, inv);       // at most one too high for n < 2^31
-  return q * d > n ? q - 1 : q;
-}
+// Walks a CTA's items. By length: all heads' longest query blocks (causal) first, then the next ones; else head by head, a head's longest first.
+// Every other round runs backwards over the CTAs, so that long and short items even out. Blocks past the end of a packed sequence are
+// skipped.
 struct FwdItems {
   int round = 0, b, h, hk, q0, q_blk, row_base, S, bz, jlo, nkb;
   bool valid = false;
-  template <bool EXT>
+  template <bool EXT, bool LOOP>
   __device__ __forceinline__ void next(const FlashFwdParams& p) {
     const int per = (p.S + FA_BM - 1) / FA_BM, total = per * p.H * p.B, grid = gridDim.x, cta = blockIdx.x;
     for (;;) {
@@ -94,17 +90,19 @@ struct FwdItems {
         valid = false;
         return;
       }
-      const int r = fa_divide(idx, per, p.inv_per), x = idx - r * per;
-      b = fa_divide(r, p.H, p.inv_h);
+      const int quot = div_by(idx, p.stride, p.inv_stride), rest = idx - quot * p.stride;
+      const int r = p.by_length ? rest : quot;
+      q_blk = per - 1 - (p.by_length ? quot : rest);
+      b = div_by(r, p.H, p.inv_h);
       h = r - b * p.H;
       row_base = p.cu ? p.cu[b] : 0;             // first row of the sequence in its tensor-map slice
       S = p.cu ? p.cu[b + 1] - row_base : p.S;
-      q_blk = (S + FA_BM - 1) / FA_BM - 1 - x;
-      if (q_blk >= 0) break;
+      valid = q_blk * FA_BM < S;
+      if (valid) break;
+      if (!LOOP) return;
     }
-    valid = true;
     bz = p.cu ? 0 : b;
-    hk = fa_divide(h, p.group, p.inv_group);
+    hk = div_by(h, p.group, p.inv_group);
     q0 = q_blk * FA_BM;
     const int nkb_all = (S + FA_BN - 1) / FA_BN;
     // key blocks visited: [jlo, jlo + nkb). A sliding window skips the blocks that lie wholly before the first query's window, a
@@ -115,12 +113,12 @@ struct FwdItems {
 };
 
 // EXT: with the chunked mask and the output gate (registers the plain form does not spend).
-template <int ND, bool EXT, bool TWO>
+template <int ND, bool EXT, bool TWO, bool LOOP>
 __global__ void __launch_bounds__(FA_THREADS, TWO ? 2 : 1)
 flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                   const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ FlashFwdParams p) {
   constexpr int D = 64 * ND;
-  using L = Fwd3Smem<ND, TWO>;
+  using L = Fwd3Smem<ND, TWO, LOOP>;
   constexpr int SLOTS = L::SLOTS, QB = L::QB;
   constexpr bool ALIAS = TWO && ND == 2;      // P over the scores: the next scores wait for the values' product
   extern __shared__ uint8_t smem_raw[];
@@ -140,6 +138,11 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (p.cu) {                          // packed prompts: a block past the end of its sequence, where each CTA has one
+    FwdItems first;
+    first.next<EXT, LOOP>(p);
+    if (!first.valid) return;
+  }
   constexpr uint32_t TMEM_COLS = TWO ? 256 : 512;
   constexpr uint32_t O_COL = 128, P_COL = ALIAS ? 0 : 128 + D;
 
@@ -176,8 +179,8 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       bool ok = true;
       int load = 0;                    // K and V tiles over all items
       FwdItems w;
-      w.next<EXT>(p);
-      for (int n = 0; ok && w.valid; ++n, w.next<EXT>(p)) {
+      w.next<EXT, LOOP>(p);
+      for (int n = 0; ok && w.valid; ++n) {
         const int qb = n % QB;
         if (!mbar_wait(&q_empty[qb], ((n / QB) & 1) ^ 1, abort_flag, p.status, ERR_WAIT_EMPTY)) break;
         mbar_expect_tx(&q_full[qb], L::TILE);
@@ -193,6 +196,8 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           for (int a = 0; a < ND; ++a)
             tma_load_3d(sKV + slot * L::TILE + a * 16384, tm, &kv_full[slot], w.hk * D + a * 64, w.row_base + j * FA_BN, w.bz);
         }
+        if (!LOOP) break;
+        w.next<EXT, LOOP>(p);
       }
     }
   } else if (warp == 1) {
@@ -219,12 +224,13 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         return true;
       };
       FwdItems w;
-      w.next<EXT>(p);
+      w.next<EXT, LOOP>(p);
       bool ok = w.valid && issue_qk(0, 0, 0, 0, w.nkb);
       int g = 0, load = 0;             // load: the item's first K tile
       for (int n = 0; ok && w.valid; ++n) {
         FwdItems nx = w;
-        nx.next<EXT>(p);
+        if (LOOP) nx.next<EXT, LOOP>(p);
+        else nx.valid = false;
         for (int j = 0; j < w.nkb; ++j, ++g) {
           // the scores behind these: this item's next block or the next item's first
           auto ahead = [&]() {
@@ -262,7 +268,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     bool ok = true;
     int g = 0;                         // key blocks over all items
     FwdItems w;
-    w.next<EXT>(p);
+    w.next<EXT, LOOP>(p);
     while (ok && w.valid) {
     const int h = w.h, b = w.b, row_base = w.row_base, S = w.S, q0 = w.q0, jlo = w.jlo, nkb = w.nkb;
     const int row = q0 + r;
@@ -343,7 +349,8 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
     }
-    w.next<EXT>(p);                    // while the last product runs
+    if (LOOP) w.next<EXT, LOOP>(p);    // while the last product runs
+    else w.valid = false;
     uint4 gv[EXT ? D / 8 : 1];                    // the row's gate, requested while the last PV MMA runs
     const bool gated = EXT && p.gate != nullptr;
     if (gated && row < S) {
@@ -470,23 +477,48 @@ static int flash_fwd_launch(const void* q, const void* k, const void* v, void* o
   p.gate = (const __nv_bfloat16*)gate; p.ld_gate = ld_gate;
   const int per = (max_len + FA_BM - 1) / FA_BM;
   p.group = H / Hkv;
-  p.inv_per = fa_reciprocal(per); p.inv_h = fa_reciprocal(H); p.inv_group = fa_reciprocal(p.group);
+  p.inv_h = div_reciprocal(H); p.inv_group = div_reciprocal(p.group);
   const long items = (long)per * H * n_seq;
-  // 128-wide heads: while every item has an SM to itself, one CTA an SM with scores and P side by side (2 x 300 tokens, 16 heads on 4: 8.8 us
-  // against 12.5); beyond, two CTAs that overlap (64 x 512, 32 heads on 8: 442 -> 307 us).
-  const bool two = head_dim == 64 || items > 148;
-  const dim3 grid((unsigned)(items < (two ? 2 * 148 : 148) ? items : (two ? 2 * 148 : 148)));
+  // 128-wide heads: one CTA an SM with scores and P side by side, or two with P over the scores, which serialises a CTA's own products and
+  // exponentials but overlaps the two. Two where items are short (three key blocks or fewer on average) and fill most SMs twice; one-block items
+  // gain as soon as an SM has a second one. one / two: 6 x 128, 32 heads on 8 (192 items) 12.7 / 11.0 us; 64 x 512 321 / 308; but 3 x 500, 16 heads
+  // on 4 (192 items) 14.0 / 16.4, 1 x 1200, 32 heads 26.2 / 30.5, 2 x 2048, 16 heads 49.5 / 51.6, 8 x 1024 without a mask 82 / 94.
+  const int halves = causal ? per + 1 : 2 * per;     // twice the key blocks of an item
+  const bool two = head_dim == 64 || (halves <= 6 && items > (halves <= 3 ? 148 : 2 * 148));
+  int ctas = two ? 2 * 148 : 148;
+  // Order: by length, so that few rounds of items come out even (1 x 2600, 16 heads of 128: 78 -> 42 us, 1 x 4096, 12 heads of 64 86 -> 52; one CTA an
+  // item, 56 and 77). Many rounds of short sequences do so in any order and run head by head, whose blocks share keys and values (32 x 1024, 12 heads
+  // of 64: 136.7 -> 133 us).
+  p.by_length = causal && (head_dim == 128 || per >= 16 || items <= 8 * 2 * 148);
+  // Packed sequences of unequal length: where the items of a CTA lie is not known here, so the hardware hands them out, one a CTA; by length unless
+  // most of them are empty (3000 tokens and twenty of 60, 12 heads of 64: by length 80 us, by head 68).
+  if (cu != nullptr && (long)map_s * 10 < (long)n_seq * max_len * 9) {
+    p.by_length = (long)map_s * 4 >= (long)n_seq * max_len;
+    ctas = (int)items;
+  }
+  // A CTA that has one item only runs a form without the walk, and with a fifth tile on its way for 64-wide heads (1 x 300, 12 heads of 64: 9.2 -> 8.8 us).
+  const bool loop = items > ctas;
+  p.stride = p.by_length ? H * n_seq : per;
+  p.inv_stride = div_reciprocal(p.stride);
+  const dim3 grid((unsigned)(items < ctas ? items : ctas));
   cudaStream_t st = (cudaStream_t)stream;
   static bool configured = false;
   if (!configured) {
-#define INV_FA(ND, EXT, TWO) \
-  cudaFuncSetAttribute(flash_fwd3_kernel<ND, EXT, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd3Smem<ND, TWO>::TOTAL)
-    INV_FA(1, false, true); INV_FA(1, true, true); INV_FA(2, false, true); INV_FA(2, true, true); INV_FA(2, false, false); INV_FA(2, true, false);
+#define INV_FA(ND, EXT, TWO, LOOP) \
+  cudaFuncSetAttribute(flash_fwd3_kernel<ND, EXT, TWO, LOOP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd3Smem<ND, TWO, LOOP>::TOTAL)
+    INV_FA(1, false, true, true); INV_FA(1, true, true, true); INV_FA(2, false, true, true); INV_FA(2, true, true, true); INV_FA(2, false, false, true);
+    INV_FA(2, true, false, true);
+    INV_FA(1, false, true, false); INV_FA(1, true, true, false); INV_FA(2, false, true, false); INV_FA(2, true, true, false); INV_FA(2, false, false, false);
+    INV_FA(2, true, false, false);
 #undef INV_FA
     configured = true;
   }
   const bool ext = p.gate || p.chunk;
-#define INV_FA(ND, EXT, TWO) flash_fwd3_kernel<ND, EXT, TWO><<<grid, FA_THREADS, Fwd3Smem<ND, TWO>::TOTAL, st>>>(tq, tk, tv, p)
+#define INV_FA(ND, EXT, TWO)                                                                                                       \
+  do {                                                                                                                             \
+    if (loop) flash_fwd3_kernel<ND, EXT, TWO, true><<<grid, FA_THREADS, Fwd3Smem<ND, TWO, true>::TOTAL, st>>>(tq, tk, tv, p);        \
+    else flash_fwd3_kernel<ND, EXT, TWO, false><<<grid, FA_THREADS, Fwd3Smem<ND, TWO, false>::TOTAL, st>>>(tq, tk, tv, p);           \
+  } while (0)
   if (head_dim == 64) { if (ext) INV_FA(1, true, true); else INV_FA(1, false, true); }
   else if (two) { if (ext) INV_FA(2, true, true); else INV_FA(2, false, true); }
   else { if (ext) INV_FA(2, true, false); else INV_FA(2, false, false); }

@@ -11,6 +11,14 @@
 
 namespace inv {
 
+// n / d for 0 <= n < 2^31 and a divisor that the host knows: inv = div_reciprocal(d).
+__host__ __device__ inline uint32_t div_reciprocal(int d) { return d == 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d); }
+__device__ __forceinline__ int div_by(int n, int d, uint32_t inv) {
+  if (inv == 0) return n;
+  const uint32_t q = __umulhi((uint32_t)n, inv);       // at most one too high
+  return (int)(q * (uint32_t)d > (uint32_t)n ? q - 1 : q);
+}
+
 // ----- error/status word ---------------------------------------------------------------------
 // Kernels report a non-zero code here; the host reads it after synchronisation.
 enum : int {

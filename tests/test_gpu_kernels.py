@@ -423,6 +423,55 @@ def test_flash_attention(D, B, S, H, Hkv, causal):
     assert _rel_err(dq, rq) < 3e-2
 
 
+# Persistent CTAs: several work items each, in both orders (by length, and head by head beyond twelve rounds), both forms for 128-wide heads.
+# Items of a round: 296 forward (148 where 128-wide heads take one CTA an SM), 148 backward.
+@pytest.mark.parametrize("D,B,S,H,Hkv,causal,window", [
+    (64, 26, 333, 8, 8, True, 0), (64, 26, 333, 8, 4, True, 0), (64, 26, 333, 8, 4, False, 0), (64, 16, 640, 8, 8, True, 100), (64, 224, 200, 8, 8, True, 0),
+    (128, 26, 333, 8, 4, True, 0), (128, 26, 333, 8, 8, False, 0), (128, 10, 1000, 8, 4, True, 0), (128, 13, 700, 8, 4, False, 0), (128, 8, 1100, 8, 8, True, 200),
+    (128, 28, 900, 8, 2, True, 0), (128, 150, 130, 16, 8, True, 0)])
+def test_flash_attention_over_many_items(D, B, S, H, Hkv, causal, window):
+    """Outputs, statistics and gradients of every head of every sequence: what one item leaves behind for the next one on its CTA (barrier phases, Q, K and V
+    loaded ahead, sums and statistics) would show in single heads. Bounds: those of the single-item tests, per head."""
+    from innova_b200.ops.attention import _FlashAttnFn, attention_reference
+    torch.manual_seed(S)
+    dev = _dev()
+    qkv = (torch.randn(B, S, (H + 2 * Hkv) * D, device=dev) * 0.7).bfloat16()
+
+    class Ctx:
+        def save_for_backward(self, *a):
+            self.saved_tensors = a
+
+    ctx = Ctx()
+    out = _FlashAttnFn.forward(ctx, qkv, H, Hkv, D, causal, D ** -0.5, window)
+    lse = ctx.saved_tensors[2]
+    go = torch.randn_like(out)
+    grad = _FlashAttnFn.backward(ctx, go)[0]
+
+    def off(a, b, heads):                               # per sequence and head
+        a, b = (x.float().reshape(-1, S, heads, D) for x in (a, b))
+        return float(((a - b).norm(dim=(1, 3)) / b.norm(dim=(1, 3))).max())
+
+    for b0 in range(0, B, 8):                           # a few sequences at a time: the reference keeps all scores
+        sl = slice(b0, b0 + 8)
+        qr = qkv[sl].float().requires_grad_(True)
+        ref = attention_reference(qr, H, Hkv, D, causal=causal, scale=D ** -0.5, window=window)
+        ref.backward(go[sl].float())
+        n = ref.shape[0]
+        q, k, _ = qr.detach().split([H * D, Hkv * D, Hkv * D], dim=-1)
+        q, k = q.view(n, S, H, D).transpose(1, 2), k.view(n, S, Hkv, D).transpose(1, 2).repeat_interleave(H // Hkv, dim=1)
+        z = q @ k.transpose(-1, -2) * D ** -0.5
+        pos = torch.arange(S, device=dev)
+        if causal:
+            z = z.masked_fill(pos[None, :] > pos[:, None], float("-inf"))
+        if window:
+            z = z.masked_fill(pos[:, None] - pos[None, :] >= window, float("-inf"))
+        # the kernel adds the exponentials as packed bf16 in fours: 2^-8 of the denominator, a hundredth of a power of two
+        assert float((lse[sl] - torch.logsumexp(z, -1) * 1.4426950408889634).abs().max()) < 2e-2
+        assert off(out[sl], ref, H) < 2e-2
+        for a, r, heads in zip(grad[sl].split([H * D, Hkv * D, Hkv * D], dim=-1), qr.grad.split([H * D, Hkv * D, Hkv * D], dim=-1), (H, Hkv, Hkv)):
+            assert off(a, r, heads) < 3e-2
+
+
 # ------------------------------------------------------------------------------------------ model
 @pytest.mark.parametrize("D,B,S,H,Hkv,window", [(64, 2, 1024, 4, 4, 256), (64, 1, 640, 4, 2, 100), (128, 1, 768, 4, 2, 300), (64, 1, 512, 2, 2, 33),
                                                  (64, 1, 384, 2, 1, 128)])

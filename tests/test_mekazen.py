@@ -337,6 +337,26 @@ def test_packed_flash_attention_in_chunks(D, chunk):
         at += n
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("chunk", [63, 256, None])
+@pytest.mark.parametrize("lens", [[1, 300, 129, 128, 600, 17] * 4, [900, 40, 130] * 4])
+def test_packed_flash_attention_over_many_items(D, chunk, lens):
+    """More work items than CTAs, blocks past the end of a sequence between valid ones: every sequence and head by itself, gated and not."""
+    H, G = 8, 2
+    q, k, v = (torch.randn(sum(lens), n * D, device="cuda").bfloat16() for n in (H, G, G))
+    gate = torch.randn(sum(lens), H * D + 8, device="cuda").bfloat16()[:, : H * D]
+    b = Rows("cuda", torch.bfloat16, 1, 16, n=len(lens), max_seq=912).batch(lens, [0] * len(lens), range(len(lens)))
+    got = {name: la.packed_flash(q, k, v, H, D, D ** -0.5, None, b, kv_heads=G, chunk=chunk, gate=x).double().cpu() for name, x in (("gate", gate), ("none", None))}
+    at = 0
+    for n in lens:
+        x = [a[at:at + n].double().cpu().view(n, -1, D) for a in (q, k, v)]
+        want = oracle.softmax_attention(*x, D ** -0.5, oracle.chunk_visible(n, chunk))
+        assert torch.allclose(got["none"][at:at + n], want, atol=2e-2, rtol=2e-2)
+        assert torch.allclose(got["gate"][at:at + n], want * oracle.sigmoid(gate[at:at + n].double().cpu()), atol=2e-2, rtol=2e-2)
+        at += n
+
+
 # ------------------------------------------------------------------------------------------------ whole models
 @pytest.mark.parametrize("name", CONFIGS)
 def test_logits_and_residuals(dev, name):
