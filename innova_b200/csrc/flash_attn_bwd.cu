@@ -58,6 +58,8 @@ struct FlashBwdParams {
   float scale;
   int causal;
   int window;  // > 0 (causal only): a query sees the `window` most recent keys, its own position included
+  int by_length, stride, group;               // how items are numbered (BwdItem); query heads of a key head
+  uint32_t inv_stride, inv_hkv;               // of its divisors (div_reciprocal)
   int* status;
 };
 
@@ -79,8 +81,8 @@ struct BwdSmem {
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
-// Work item `round` of a CTA: items are numbered head by head (so that the SMs share a head's Q and dO in L2), key block by key block, and every
-// other round runs backwards over the CTAs, so that a CTA's long and short items (causal: key block j sees all later queries) even out.
+// Work item `round` of a CTA. Items are numbered by length, all heads' first key blocks (causal: those that all queries see) first, or head by head
+// (so that the SMs share a head's Q and dO in L2), and every other round runs backwards over the CTAs, so that long and short items even out.
 struct BwdItem {
   int j, hk, b, k0, i0, nq_it, n_it;
   bool valid;
@@ -88,16 +90,16 @@ struct BwdItem {
     const int nb = (p.S + 127) / 128, total = nb * p.Hkv * p.B, grid = gridDim.x, cta = blockIdx.x;
     const int idx = round * grid + ((round & 1) ? grid - 1 - cta : cta);
     valid = idx < total;
-    const int r = idx / nb;
-    j = idx - r * nb;
-    b = r / p.Hkv;
+    const int quot = div_by(idx, p.stride, p.inv_stride), rest = idx - quot * p.stride, r = p.by_length ? rest : quot;
+    j = p.by_length ? quot : rest;
+    b = div_by(r, p.Hkv, p.inv_hkv);
     hk = r - b * p.Hkv;
     k0 = j * 128;
     i0 = p.causal ? j : 0;
     // with a sliding window the last query that sees key k0 + 127 is row k0 + 126 + window
     const int i_end = (p.causal && p.window > 0) ? min(nb, (k0 + 126 + p.window) / 128 + 1) : nb;
     nq_it = i_end - i0;
-    n_it = (p.H / p.Hkv) * nq_it;
+    n_it = p.group * nq_it;
   }
 };
 
@@ -112,7 +114,7 @@ __device__ long long fb_trace_buf[64];
 #define FB_STAMP(i) do {} while (0)
 #endif
 
-template <int ND>
+template <int ND, bool LOOP>       // LOOP: CTAs take several items
 __global__ void __launch_bounds__(FB_THREADS, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                  const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
@@ -149,7 +151,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int G = p.H / p.Hkv;
+  const int G = p.group;
   if (threadIdx.x == 0) FB_STAMP(0);
 
   if (threadIdx.x == 0) {
@@ -188,6 +190,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       bool ok = true;
       int g = 0;                       // query blocks over all items
       for (int n = 0; ok; ++n) {
+        if (!LOOP && n > 0) break;
         const BwdItem w(p, n);
         if (!w.valid) break;
         for (int it = 0; it < w.n_it; ++it, ++g) {
@@ -248,6 +251,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       bool ok = true;
       int g = 0;
       for (int n = 0; ok; ++n) {
+        if (!LOOP && n > 0) break;
         const BwdItem w(p, n);
         if (!w.valid) break;
         if (!mbar_wait(kv_full, n & 1, abort_flag, p.status, ERR_WAIT_FULL)) break;
@@ -358,7 +362,9 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
     int g = 0;                         // query blocks over all items: phase of the barriers, stage of the statistics
     for (int n = 0; ok && w.valid; ++n) {
-    const BwdItem next(p, n + 1);
+    BwdItem next = w;
+    if (LOOP) next = BwdItem(p, n + 1);
+    else next.valid = false;
     const int k0 = w.k0, key = k0 + r;
     for (int it = 0; it < w.n_it; ++it, ++g) {
       const int q0 = (w.i0 + it % w.nq_it) * 128;
@@ -625,15 +631,27 @@ extern "C" int inv_flash_attn_bwd(const void* q, const void* k, const void* v, c
   p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv; p.ld_dk = ld_dk; p.ld_dv = ld_dv;
   p.B = B; p.S = S; p.H = H; p.Hkv = Hkv; p.scale = scale; p.causal = causal ? 1 : 0; p.window = window >= S ? 0 : window; p.status = status;
   const long items = (long)((S + 127) / 128) * Hkv * B;
+  // By length, so that few rounds of items come out even (1 x 6000 tokens, 16 heads of 128 on 4: 1612 -> 949 us, one CTA an item 1183; 1 x 2600, 12
+  // heads of 64: 115 -> 65, 99); many rounds of short sequences go head by head (64 x 1024, 12 heads of 64: 831 -> 735; 20 x 1000, 32 heads of 128
+  // on 8: 1228 -> 1120).
+  const int nb = (S + 127) / 128;
+  p.by_length = causal && (nb >= 32 || items <= 8 * 148);
+  p.stride = p.by_length ? Hkv * B : nb;
+  p.group = H / Hkv;
+  p.inv_stride = div_reciprocal(p.stride); p.inv_hkv = div_reciprocal(Hkv);
   const dim3 grid((unsigned)(items < 148 ? items : 148));
   static bool configured = false;
   if (!configured) {
-    cudaFuncSetAttribute(flash_bwd_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<1>::TOTAL);
-    cudaFuncSetAttribute(flash_bwd_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<2>::TOTAL);
+    cudaFuncSetAttribute(flash_bwd_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<1>::TOTAL);
+    cudaFuncSetAttribute(flash_bwd_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<2>::TOTAL);
+    cudaFuncSetAttribute(flash_bwd_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<1>::TOTAL);
+    cudaFuncSetAttribute(flash_bwd_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<2>::TOTAL);
     configured = true;
   }
-  if (head_dim == 64) flash_bwd_kernel<1><<<grid, FB_THREADS, BwdSmem<1>::TOTAL, st>>>(tq, tk, tv, tdo, tdq, p);
-  else flash_bwd_kernel<2><<<grid, FB_THREADS, BwdSmem<2>::TOTAL, st>>>(tq, tk, tv, tdo, tdq, p);
+#define INV_FB(ND, LOOP) flash_bwd_kernel<ND, LOOP><<<grid, FB_THREADS, BwdSmem<ND>::TOTAL, st>>>(tq, tk, tv, tdo, tdq, p)
+  if (head_dim == 64) { if (items > 148) INV_FB(1, true); else INV_FB(1, false); }
+  else { if (items > 148) INV_FB(2, true); else INV_FB(2, false); }
+#undef INV_FB
   {
     const long n = T * H * head_dim / 8;
     long g = (n + 255) / 256;
