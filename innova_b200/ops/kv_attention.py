@@ -80,7 +80,7 @@ def first_visible(pos: int, window: Optional[int], chunk: Optional[int]) -> int:
     return pos - pos % chunk if chunk else max(0, pos - window + 1) if window else 0
 
 
-def cluster_shape(rows: int, groups: int, span: int):
+def cluster_shape(rows: int, groups: int, span: int, dim: int = 128):
     """(CTAs, warps per CTA) that share one (row, key head): about 1024 warps in flight altogether, at least two pages each."""
     pages, units = -(-span // PAGE), rows * groups
     if 444 < units <= 888 and pages >= 128:
@@ -90,8 +90,8 @@ def cluster_shape(rows: int, groups: int, span: int):
         warps *= 2
     if warps == 32 and units <= 8 and pages >= 256:
         return 8, 8
-    if warps == 16 and units > 32:
-        return 2, 8                  # 64 units, 500 / 1500 / 4000 tokens on average: 9.6, 16.1, 30.0 us; clusters of four 10.7, 17.8, 32.2
+    if warps == 16 and units > 32 and dim > 64:
+        return 2, 8      # heads of 128, 500 / 1500 / 4000 tokens: 64 units 6.6, 10.9, 24.6 us (clusters of four 7.2, 12.1, 26.4), 48 alike; of 64: 5.9, 9.4, 17.8 (5.7, 8.6, 15.9)
     return {4: (1, 4), 8: (1, 8), 16: (4, 4), 32: (8, 4)}[warps]
 
 
@@ -111,7 +111,7 @@ def kv_attend(q: torch.Tensor, pool, page_table, heads: int, scale: float, batch
         return out if gate is None else (out.float() * torch.sigmoid(gate.float())).to(q.dtype)
     out = torch.empty(T, heads * D, dtype=q.dtype, device=q.device)
     span = min(chunk or window or page_table.shape[1] * PAGE, page_table.shape[1] * PAGE)
-    splits, warps = cluster_shape(T, G * -(-(heads // G) // 8), span)
+    splits, warps = cluster_shape(T, G * -(-(heads // G) // 8), span, D)
     rt.check(rt.lib().inv_kv_attend(q.data_ptr(), pool.data_ptr(), int(pool.dtype == torch.float32), page_table.data_ptr(), page_table.shape[1],
                                     batch.rows.data_ptr(), batch.tok_seq.data_ptr(), batch.tok_pos.data_ptr(), int(window or 0), int(chunk or 0),
                                     float(scale), rt.ptr(gate), 0 if gate is None else gate.stride(0),

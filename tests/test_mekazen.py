@@ -319,6 +319,35 @@ def test_every_cluster_shape_gives_the_same(splits, warps, chunk, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("splits,warps", [(s, w) for s in (1, 2, 4, 8) for w in (4, 8)])
+@pytest.mark.parametrize("H,G,D", [(12, 2, 64), (16, 2, 128), (9, 1, 128), (16, 2, 192), (20, 1, 256)])
+@pytest.mark.parametrize("chunk", [20, 400, None])
+def test_clusters_of_every_shape_and_size(splits, warps, H, G, D, chunk, monkeypatch):
+    """Every cluster that the kernel takes, for groups of one to eight heads and more, head sizes whose output pieces need one to several turns of a
+    CTA's threads, gated and not: against fp64 over the stored keys and values. One rounding to bf16 of the queries' scores' weights (2^-9) and
+    of the result."""
+    n = 500
+    R = Rows("cuda", torch.bfloat16, G, D, chunk=chunk)
+    R.batch([n], [0], [2])
+    R.c.kv[0].normal_()
+    pos = [0, 1, 15, 16, 19, 20, 255, 399, 400, 499]
+    q = torch.randn(len(pos), H * D, device="cuda").bfloat16()
+    gate = torch.randn(len(pos), H * D, device="cuda")
+    monkeypatch.setattr(ka, "cluster_shape", lambda *_: (splits, warps))
+    got = ka.kv_attend(q, R.c.kv[0], R.c.page_table, H, D ** -0.5, R.at(pos, 2), chunk=chunk).double().cpu()
+    gated = ka.kv_attend(q, R.c.kv[0], R.c.page_table, H, D ** -0.5, R.at(pos, 2), chunk=chunk, gate=gate).double().cpu()
+    kv = R.stored(2, n).double()
+    for i, p in enumerate(pos):
+        first = p - p % chunk if chunk else 0
+        k, v = kv[first:p + 1, :, 0], kv[first:p + 1, :, 1]
+        w = torch.softmax(torch.einsum("ghd,ngd->ghn", q[i].double().cpu().view(G, H // G, D), k) * D ** -0.5, -1)
+        want = torch.einsum("ghn,ngd->ghd", w, v).reshape(-1)
+        assert float((got[i] - want).norm() / want.norm()) < 2.0 ** -7
+        want = want * torch.sigmoid(gate[i].double().cpu())
+        assert float((gated[i] - want).norm() / want.norm()) < 2.0 ** -7
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("chunk", [1, 63, 128, 200, 256, 290, None])
 def test_packed_flash_attention_in_chunks(D, chunk):
