@@ -155,17 +155,23 @@ static int launch_skinny(const void* x, int ldx, const void* W, int ldw, int M, 
 }
 // Sixteen warps: where every tile has an SM to itself and a row has more slices than eight warps keep in flight (K > 2048): a second CTA would find
 // no tile, so eight warps left half of the SM's loads unissued and walked a chain of slices twice as long. Back to back, 2048 x 5632: one row
-// 9.4 -> 6.3 us, 16 rows 9.9 -> 6.7, 32 rows 13.7 -> 9.6; 1024 x 2816, 16 rows: 3.8 -> 2.8. Shorter rows (2048 x 2048, 3.2 us) fit in the eight
-// warps' rings. With more tiles than that, where it takes less than twice as many rounds as two CTAs an SM and every warp has two slices or more:
-// the last round is less empty (6656 x 2048, 3 rounds instead of 2 double ones: 7.5 -> 6.6 us; gated 5632 x 2048, 5 instead of 3: 10.1 -> 9.6).
+// 9.7 -> 6.5 us, 16 rows 10.1 -> 7.0, 32 rows 14.1 -> 9.9; 1024 x 2816, 16 rows: 3.9 -> 3.0. Shorter rows (2048 x 2048, 3.2 us) fit in the eight
+// warps' rings. With more tiles, where single CTAs take an odd number of rounds, which two CTAs an SM round up to an even one:
+//   three rounds of long rows: 5632 x 3072, 16 rows 11.2 -> 8.4, 32 rows 17.5 -> 15.2; of 2048 (weights in whole lines) only if the last one is filled
+//     by a quarter: 5920 x 2048 7.7 -> 6.5, 4752 x 2048 (one tile in it) 5.5 -> 6.1; in halves of lines 7104 x 1032 6.1 -> 6.6, 7104 x 2056 alike;
+//   five rounds of 2048 likewise (gated 5632 x 2048, 16 rows: 10.3 -> 9.7, 32 rows 16.4 -> 14.6), seven and more: one row 5 % slower;
+//   up to 16 rows any number of rounds of long rows: 21312 x 3072 26.8 -> 23.2, 54464 x 4096 86 -> 80; 17 to 32 rows 21312 x 3072 41.3 -> 45.8.
 // Above 32 rows the accumulators of four row tiles take the registers.
 template <int MT, int P, bool SILU>
 static int launch_skinny(const void* x, int ldx, const void* W, int ldw, int M, int N, int K, int half, void* out, int ldo, int out_f32, float cap,
                          bool early, cudaStream_t st) {
   const int tiles = SILU ? (N + 7) / 8 : (N + 15) / 16, slices = (K + 32 * P - 1) / (32 * P);
   if constexpr (MT <= 2) {
-    if (tiles <= 148 ? slices > 8 * (8 / P) : slices >= 32 && (tiles + 147) / 148 < 2 * ((tiles + 295) / 296))
-      return launch_skinny<MT, P, SILU, 16>(x, ldx, W, ldw, M, N, K, half, out, ldo, out_f32, cap, tiles, early, st);
+    const int rounds = (tiles + 147) / 148, last = tiles - 148 * (rounds - 1);
+    const bool rows_long = slices >= (P == 2 ? 48 : 96), worth = rows_long || (P == 2 && slices >= 32 && last >= 37);
+    const bool wide = rounds == 1 ? slices > 8 * (8 / P)
+                                  : rounds % 2 == 1 && worth && (rounds == 3 || (P == 2 && (rows_long ? MT == 1 : rounds == 5)));
+    if (wide) return launch_skinny<MT, P, SILU, 16>(x, ldx, W, ldw, M, N, K, half, out, ldo, out_f32, cap, tiles, early, st);
   }
   return launch_skinny<MT, P, SILU, 8>(x, ldx, W, ldw, M, N, K, half, out, ldo, out_f32, cap, tiles, early, st);
 }
