@@ -362,154 +362,154 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
     int g = 0;                         // query blocks over all items: phase of the barriers, stage of the statistics
     for (int n = 0; ok && w.valid; ++n) {
-    BwdItem next = w;
-    if (LOOP) next = BwdItem(p, n + 1);
-    else next.valid = false;
-    const int k0 = w.k0, key = k0 + r;
-    for (int it = 0; it < w.n_it; ++it, ++g) {
-      const int q0 = (w.i0 + it % w.nq_it) * 128;
-      const float* stat = wstat + (g & 1) * 64;
-      if (!mbar_wait_warp(s_full, g & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
-      tc_fence_after();
-      if (threadIdx.x == 64) FB_STAMP(8 + 3 * it);
-      __syncwarp();  // the statistics of this block are in place (written by this warp)
-      const bool windowed = p.causal && p.window > 0;
-      const bool need_mask = (p.causal && q0 < k0 + 127) || (q0 + 128 > p.S) || (k0 + 128 > p.S) || (windowed && q0 + 127 - k0 >= p.window);
-      // The thread's 32 columns of S^T and dP^T come in as two halves of 16 (the register file holds 96 registers per
-      // thread at this block size: both halves at once spill). The TMEM columns go back to the tensor core after the
-      // second load. A column i of the thread is live iff lim_lo <= i < lim_hi (causal diagonal, sequence end, window).
-      uint32_t pk[16], dk[16];  // P^T and dS^T of this thread's 32 columns as packed bf16 pairs, kept in registers until the
-                                // shared-memory tiles are free
-      float stat_next_l = 0.f, stat_next_d = 0.f;
-      const int col0 = cq * 32;
-      int lim_lo = 0, lim_hi = 32;
-      if (need_mask) {
-        if (p.causal) lim_lo = key - q0 - col0;
-        lim_hi = min(32, p.S - q0 - col0);
-        if (windowed) lim_hi = min(lim_hi, key + p.window - q0 - col0);
-        if (key >= p.S) lim_hi = 0;
-      }
-      auto softmax_block = [&](auto masked_tag) {
-      constexpr bool MASKED = decltype(masked_tag)::value;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t s_r[16], dp_r[16];
-        tmem_ld_32x16(t_lane + ST_COL + col0 + half * 16, s_r);
-        tmem_ld_32x16(t_lane + DPT_COL + col0 + half * 16, dp_r);
-        tmem_ld_wait();
-        if (half == 1) {
-          if (threadIdx.x == 64) FB_STAMP(32 + 3 * it);
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(s_empty);  // one arrival per warp: arrivals on one mbarrier are serialised
-          if (it + 1 < w.n_it) stat_load(w, it + 1, stat_next_l, stat_next_d);
-          else if (next.valid) stat_load(next, 0, stat_next_l, stat_next_d);
-        }
-        // statistics as 16-byte broadcast loads; one MUFU op and half a conversion per element
-        const float4* l4 = reinterpret_cast<const float4*>(stat + half * 16);
-        const float4* d4 = reinterpret_cast<const float4*>(stat + 32 + half * 16);
-#pragma unroll
-        for (int i4 = 0; i4 < 4; ++i4) {
-          const float4 l = l4[i4], dl = d4[i4];
-          const int i = i4 * 4;
-          float e0 = exp2f(fmaf(__uint_as_float(s_r[i]), c, -l.x)), e1 = exp2f(fmaf(__uint_as_float(s_r[i + 1]), c, -l.y));
-          float e2 = exp2f(fmaf(__uint_as_float(s_r[i + 2]), c, -l.z)), e3 = exp2f(fmaf(__uint_as_float(s_r[i + 3]), c, -l.w));
-          if (MASKED) {
-            const int ci = half * 16 + i;
-            e0 = (ci >= lim_lo && ci < lim_hi) ? e0 : 0.f;
-            e1 = (ci + 1 >= lim_lo && ci + 1 < lim_hi) ? e1 : 0.f;
-            e2 = (ci + 2 >= lim_lo && ci + 2 < lim_hi) ? e2 : 0.f;
-            e3 = (ci + 3 >= lim_lo && ci + 3 < lim_hi) ? e3 : 0.f;
-          }
-          const int o = half * 8 + i4 * 2;
-          pk[o] = cvt_bf16x2(e0, e1);
-          pk[o + 1] = cvt_bf16x2(e2, e3);
-          dk[o] = cvt_bf16x2(e0 * (__uint_as_float(dp_r[i]) - dl.x), e1 * (__uint_as_float(dp_r[i + 1]) - dl.y));
-          dk[o + 1] = cvt_bf16x2(e2 * (__uint_as_float(dp_r[i + 2]) - dl.z), e3 * (__uint_as_float(dp_r[i + 3]) - dl.w));
-        }
-      }
-      };
-      if (need_mask) softmax_block(std::true_type{});   // two copies of the loop: interior blocks carry no selects
-      else softmax_block(std::false_type{});
-      // the warp's other statistics stage was last read in the block before
-      wstat[((g + 1) & 1) * 64 + lane] = stat_next_l;
-      wstat[((g + 1) & 1) * 64 + 32 + lane] = stat_next_d;
-      // Software pipeline (when dQ has its own TMEM columns): the arithmetic above ran while the MMAs of the previous
-      // block were still reading its P^T / dS^T tiles; only now wait for them, publish this block's tiles, and read the
-      // previous block's dQ out of TMEM while this block's MMAs run.
-      if (threadIdx.x == 64) FB_STAMP(33 + 3 * it);
-      if (OVERLAP && it > 0) {
-        if (!mbar_wait_warp(mma2_done, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+      BwdItem next = w;
+      if (LOOP) next = BwdItem(p, n + 1);
+      else next.valid = false;
+      const int k0 = w.k0, key = k0 + r;
+      for (int it = 0; it < w.n_it; ++it, ++g) {
+        const int q0 = (w.i0 + it % w.nq_it) * 128;
+        const float* stat = wstat + (g & 1) * 64;
+        if (!mbar_wait_warp(s_full, g & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
         tc_fence_after();
-      }
-      if (!OVERLAP && g > 0) {         // every warp's dQ boxes of the block before, which lie in the tiles, have been read
-        if (lane == 0) {
-          bulk_wait_read();
-          mbar_arrive(dqs_free);
+        if (threadIdx.x == 64) FB_STAMP(8 + 3 * it);
+        __syncwarp();  // the statistics of this block are in place (written by this warp)
+        const bool windowed = p.causal && p.window > 0;
+        const bool need_mask = (p.causal && q0 < k0 + 127) || (q0 + 128 > p.S) || (k0 + 128 > p.S) || (windowed && q0 + 127 - k0 >= p.window);
+        // The thread's 32 columns of S^T and dP^T come in as two halves of 16 (the register file holds 96 registers per
+        // thread at this block size: both halves at once spill). The TMEM columns go back to the tensor core after the
+        // second load. A column i of the thread is live iff lim_lo <= i < lim_hi (causal diagonal, sequence end, window).
+        uint32_t pk[16], dk[16];  // P^T and dS^T of this thread's 32 columns as packed bf16 pairs, kept in registers until the
+                                  // shared-memory tiles are free
+        float stat_next_l = 0.f, stat_next_d = 0.f;
+        const int col0 = cq * 32;
+        int lim_lo = 0, lim_hi = 32;
+        if (need_mask) {
+          if (p.causal) lim_lo = key - q0 - col0;
+          lim_hi = min(32, p.S - q0 - col0);
+          if (windowed) lim_hi = min(lim_hi, key + p.window - q0 - col0);
+          if (key >= p.S) lim_hi = 0;
         }
-        if (!mbar_wait_warp(dqs_free, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_MISC)) { ok = false; break; }
-      }
-      if (threadIdx.x == 64) FB_STAMP(34 + 3 * it);
+        auto softmax_block = [&](auto masked_tag) {
+        constexpr bool MASKED = decltype(masked_tag)::value;
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        const int chunk = ((cq & 1) * 4 + g) ^ (r & 7);
-        *reinterpret_cast<uint4*>(pt_row + chunk * 16) = make_uint4(pk[g * 4], pk[g * 4 + 1], pk[g * 4 + 2], pk[g * 4 + 3]);
-        *reinterpret_cast<uint4*>(dst_row + chunk * 16) = make_uint4(dk[g * 4], dk[g * 4 + 1], dk[g * 4 + 2], dk[g * 4 + 3]);
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(pds_full);
-      if (threadIdx.x == 64) FB_STAMP(9 + 3 * it);
-      if (OVERLAP) {
-        if (it > 0) dq_readout(w, it - 1);
-        if (threadIdx.x == 64) FB_STAMP(10 + 3 * it);
-      } else {
-        if (!mbar_wait_warp(mma2_done, g & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
-        tc_fence_after();
-        dq_readout(w, it);
-      }
-    }
-    if (OVERLAP && ok) {
-      if (mbar_wait_warp(mma2_done, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) {
-        tc_fence_after();
-        dq_readout(w, w.n_it - 1);
-      } else {
-        ok = false;
-      }
-    }
-    // dK, dV: the last mma2_done covers every accumulation. TMEM lanes are key rows.
-    if (ok) {
-      tc_fence_after();
-#pragma unroll
-      for (int which = 0; which < 2; ++which) {
-        const uint32_t colbase = which == 0 ? DV_COL : DK_COL;
-        __nv_bfloat16* outp = which == 0 ? p.dv : p.dk;
-        const int ld = which == 0 ? p.ld_dv : p.ld_dk;
-        const float sc = which == 0 ? 1.f : p.scale;
-        {
-          const int col0 = cq * DC;
-          uint32_t rr[DC];
-          if (DC == 16) tmem_ld_32x16(t_lane + colbase + col0, rr);
-          else tmem_ld_32x32(t_lane + colbase + col0, rr);
+        for (int half = 0; half < 2; ++half) {
+          uint32_t s_r[16], dp_r[16];
+          tmem_ld_32x16(t_lane + ST_COL + col0 + half * 16, s_r);
+          tmem_ld_32x16(t_lane + DPT_COL + col0 + half * 16, dp_r);
           tmem_ld_wait();
-          if (key < p.S) {
-            __nv_bfloat16* dst = outp + ((size_t)w.b * p.S + key) * ld + w.hk * D + col0;
+          if (half == 1) {
+            if (threadIdx.x == 64) FB_STAMP(32 + 3 * it);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(s_empty);  // one arrival per warp: arrivals on one mbarrier are serialised
+            if (it + 1 < w.n_it) stat_load(w, it + 1, stat_next_l, stat_next_d);
+            else if (next.valid) stat_load(next, 0, stat_next_l, stat_next_d);
+          }
+          // statistics as 16-byte broadcast loads; one MUFU op and half a conversion per element
+          const float4* l4 = reinterpret_cast<const float4*>(stat + half * 16);
+          const float4* d4 = reinterpret_cast<const float4*>(stat + 32 + half * 16);
 #pragma unroll
-            for (int g = 0; g < DC / 8; ++g) {
-              uint4 o;
-              o.x = pack_bf16x2(__uint_as_float(rr[g * 8 + 0]) * sc, __uint_as_float(rr[g * 8 + 1]) * sc);
-              o.y = pack_bf16x2(__uint_as_float(rr[g * 8 + 2]) * sc, __uint_as_float(rr[g * 8 + 3]) * sc);
-              o.z = pack_bf16x2(__uint_as_float(rr[g * 8 + 4]) * sc, __uint_as_float(rr[g * 8 + 5]) * sc);
-              o.w = pack_bf16x2(__uint_as_float(rr[g * 8 + 6]) * sc, __uint_as_float(rr[g * 8 + 7]) * sc);
-              *reinterpret_cast<uint4*>(dst + g * 8) = o;
+          for (int i4 = 0; i4 < 4; ++i4) {
+            const float4 l = l4[i4], dl = d4[i4];
+            const int i = i4 * 4;
+            float e0 = exp2f(fmaf(__uint_as_float(s_r[i]), c, -l.x)), e1 = exp2f(fmaf(__uint_as_float(s_r[i + 1]), c, -l.y));
+            float e2 = exp2f(fmaf(__uint_as_float(s_r[i + 2]), c, -l.z)), e3 = exp2f(fmaf(__uint_as_float(s_r[i + 3]), c, -l.w));
+            if (MASKED) {
+              const int ci = half * 16 + i;
+              e0 = (ci >= lim_lo && ci < lim_hi) ? e0 : 0.f;
+              e1 = (ci + 1 >= lim_lo && ci + 1 < lim_hi) ? e1 : 0.f;
+              e2 = (ci + 2 >= lim_lo && ci + 2 < lim_hi) ? e2 : 0.f;
+              e3 = (ci + 3 >= lim_lo && ci + 3 < lim_hi) ? e3 : 0.f;
+            }
+            const int o = half * 8 + i4 * 2;
+            pk[o] = cvt_bf16x2(e0, e1);
+            pk[o + 1] = cvt_bf16x2(e2, e3);
+            dk[o] = cvt_bf16x2(e0 * (__uint_as_float(dp_r[i]) - dl.x), e1 * (__uint_as_float(dp_r[i + 1]) - dl.y));
+            dk[o + 1] = cvt_bf16x2(e2 * (__uint_as_float(dp_r[i + 2]) - dl.z), e3 * (__uint_as_float(dp_r[i + 3]) - dl.w));
+          }
+        }
+        };
+        if (need_mask) softmax_block(std::true_type{});   // two copies of the loop: interior blocks carry no selects
+        else softmax_block(std::false_type{});
+        // the warp's other statistics stage was last read in the block before
+        wstat[((g + 1) & 1) * 64 + lane] = stat_next_l;
+        wstat[((g + 1) & 1) * 64 + 32 + lane] = stat_next_d;
+        // Software pipeline (when dQ has its own TMEM columns): the arithmetic above ran while the MMAs of the previous
+        // block were still reading its P^T / dS^T tiles; only now wait for them, publish this block's tiles, and read the
+        // previous block's dQ out of TMEM while this block's MMAs run.
+        if (threadIdx.x == 64) FB_STAMP(33 + 3 * it);
+        if (OVERLAP && it > 0) {
+          if (!mbar_wait_warp(mma2_done, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+          tc_fence_after();
+        }
+        if (!OVERLAP && g > 0) {         // every warp's dQ boxes of the block before, which lie in the tiles, have been read
+          if (lane == 0) {
+            bulk_wait_read();
+            mbar_arrive(dqs_free);
+          }
+          if (!mbar_wait_warp(dqs_free, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_MISC)) { ok = false; break; }
+        }
+        if (threadIdx.x == 64) FB_STAMP(34 + 3 * it);
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          const int chunk = ((cq & 1) * 4 + g) ^ (r & 7);
+          *reinterpret_cast<uint4*>(pt_row + chunk * 16) = make_uint4(pk[g * 4], pk[g * 4 + 1], pk[g * 4 + 2], pk[g * 4 + 3]);
+          *reinterpret_cast<uint4*>(dst_row + chunk * 16) = make_uint4(dk[g * 4], dk[g * 4 + 1], dk[g * 4 + 2], dk[g * 4 + 3]);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(pds_full);
+        if (threadIdx.x == 64) FB_STAMP(9 + 3 * it);
+        if (OVERLAP) {
+          if (it > 0) dq_readout(w, it - 1);
+          if (threadIdx.x == 64) FB_STAMP(10 + 3 * it);
+        } else {
+          if (!mbar_wait_warp(mma2_done, g & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+          tc_fence_after();
+          dq_readout(w, it);
+        }
+      }
+      if (OVERLAP && ok) {
+        if (mbar_wait_warp(mma2_done, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) {
+          tc_fence_after();
+          dq_readout(w, w.n_it - 1);
+        } else {
+          ok = false;
+        }
+      }
+      // dK, dV: the last mma2_done covers every accumulation. TMEM lanes are key rows.
+      if (ok) {
+        tc_fence_after();
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {
+          const uint32_t colbase = which == 0 ? DV_COL : DK_COL;
+          __nv_bfloat16* outp = which == 0 ? p.dv : p.dk;
+          const int ld = which == 0 ? p.ld_dv : p.ld_dk;
+          const float sc = which == 0 ? 1.f : p.scale;
+          {
+            const int col0 = cq * DC;
+            uint32_t rr[DC];
+            if (DC == 16) tmem_ld_32x16(t_lane + colbase + col0, rr);
+            else tmem_ld_32x32(t_lane + colbase + col0, rr);
+            tmem_ld_wait();
+            if (key < p.S) {
+              __nv_bfloat16* dst = outp + ((size_t)w.b * p.S + key) * ld + w.hk * D + col0;
+#pragma unroll
+              for (int g = 0; g < DC / 8; ++g) {
+                uint4 o;
+                o.x = pack_bf16x2(__uint_as_float(rr[g * 8 + 0]) * sc, __uint_as_float(rr[g * 8 + 1]) * sc);
+                o.y = pack_bf16x2(__uint_as_float(rr[g * 8 + 2]) * sc, __uint_as_float(rr[g * 8 + 3]) * sc);
+                o.z = pack_bf16x2(__uint_as_float(rr[g * 8 + 4]) * sc, __uint_as_float(rr[g * 8 + 5]) * sc);
+                o.w = pack_bf16x2(__uint_as_float(rr[g * 8 + 6]) * sc, __uint_as_float(rr[g * 8 + 7]) * sc);
+                *reinterpret_cast<uint4*>(dst + g * 8) = o;
+              }
             }
           }
         }
+        tc_fence_before();
+        if (threadIdx.x == 64) FB_STAMP(4);
       }
-      tc_fence_before();
-      if (threadIdx.x == 64) FB_STAMP(4);
-    }
-    w = next;
+      w = next;
     }
     if (lane == 0) bulk_wait_all();  // this warp's reduce copies must have landed before the grid ends
   }

@@ -270,132 +270,132 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     FwdItems w;
     w.next<EXT, LOOP>(p);
     while (ok && w.valid) {
-    const int h = w.h, b = w.b, row_base = w.row_base, S = w.S, q0 = w.q0, jlo = w.jlo, nkb = w.nkb;
-    const int row = q0 + r;
-    float m_used = -INFINITY, l = 0.f;
-    for (int j = 0; j < nkb; ++j, ++g) {
-      if (!mbar_wait_warp(s_full, g & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
-      tc_fence_after();
-      const int k0 = (jlo + j) * FA_BN;
-      const bool windowed = p.causal && p.window > 0, chunked = EXT && p.causal && p.chunk > 0;
-      const int last = q0 + FA_BM - 1;           // the block's last row has the highest first visible key
-      const bool need_mask = (p.causal && k0 + FA_BN - 1 > q0) || (k0 + FA_BN > S) || (windowed && k0 <= last - p.window) ||
-                             (chunked && k0 < last - last % p.chunk);
-      const int kmax = p.causal ? min(row, S - 1) : S - 1;
-      const int kmin = windowed ? row - p.window + 1 : chunked ? row - row % p.chunk : 0;
-      uint32_t sr[128];
-      tmem_ld_32x32(t_lane, sr);
-      tmem_ld_32x32(t_lane + 32, sr + 32);
-      tmem_ld_32x32(t_lane + 64, sr + 64);
-      tmem_ld_32x32(t_lane + 96, sr + 96);
-      tmem_ld_wait();
-      tc_fence_before();
-      if (!ALIAS) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(s_empty);  // the scores live in registers now: the next QK^T may start (one arrival per warp)
-      }
-      if (need_mask) {
-#pragma unroll
-        for (int i = 0; i < 128; ++i)
-          if (k0 + i > kmax || k0 + i < kmin) sr[i] = 0xff800000u;  // -inf
-      }
-      float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-#pragma unroll
-      for (int i = 0; i < 128; i += 8) {
-        mx0 = fmax3(mx0, __uint_as_float(sr[i + 0]), __uint_as_float(sr[i + 1]));
-        mx1 = fmax3(mx1, __uint_as_float(sr[i + 2]), __uint_as_float(sr[i + 3]));
-        mx2 = fmax3(mx2, __uint_as_float(sr[i + 4]), __uint_as_float(sr[i + 5]));
-        mx3 = fmax3(mx3, __uint_as_float(sr[i + 6]), __uint_as_float(sr[i + 7]));
-      }
-      const float m_blk = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-      const bool raise = j == 0 || (m_blk - m_used) * c > 8.0f;  // lazy: tolerate exponents up to 2^8
-      const float m_new = raise ? fmaxf(m_used, m_blk) : m_used;
-      const float alpha = (j == 0 || !raise) ? 1.0f : exp2f((m_used - m_new) * c);
-      m_used = m_new;
-      const bool any_rescale = __any_sync(0xffffffffu, j > 0 && raise);
-      const float mc = m_used == -INFINITY ? 0.f : m_used * c;  // a row that has seen no key yet (window edge): every exponential is 0
-      // exponentials into registers (packed bf16 pairs overwrite the scores) and their sum: one MUFU op per element and
-      // one hardware conversion per pair
-      float rs0 = 0.f, rs1 = 0.f;
-#pragma unroll
-      for (int i = 0; i < 128; i += 2) {
-        const float e0 = exp2f(fmaf(__uint_as_float(sr[i]), c, -mc));
-        const float e1 = exp2f(fmaf(__uint_as_float(sr[i + 1]), c, -mc));
-        rs0 += e0;
-        rs1 += e1;
-        sr[i >> 1] = cvt_bf16x2(e0, e1);  // slot i/2 <= i: never read again as a score
-      }
-      l = l * alpha + (rs0 + rs1);
-      if (j > 0) {
-        // PV of the previous block is complete: P may be overwritten, O is stable
-        if (!mbar_wait_warp(o_full, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+      const int h = w.h, b = w.b, row_base = w.row_base, S = w.S, q0 = w.q0, jlo = w.jlo, nkb = w.nkb;
+      const int row = q0 + r;
+      float m_used = -INFINITY, l = 0.f;
+      for (int j = 0; j < nkb; ++j, ++g) {
+        if (!mbar_wait_warp(s_full, g & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
         tc_fence_after();
-        if (any_rescale) {
-#pragma unroll 1
-          for (int cc = 0; cc < D / 32; ++cc) {
-            uint32_t rr[32];
-            tmem_ld_32x32(t_lane + O_COL + cc * 32, rr);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) rr[i] = __float_as_uint(__uint_as_float(rr[i]) * alpha);
-            tmem_st_32x32(t_lane + O_COL + cc * 32, rr);
-          }
-        }
-      }
-      tmem_st_32x32(t_lane + P_COL, sr);
-      tmem_st_32x32(t_lane + P_COL + 32, sr + 32);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
-    }
-    if (LOOP) w.next<EXT, LOOP>(p);    // while the last product runs
-    else w.valid = false;
-    uint4 gv[EXT ? D / 8 : 1];                    // the row's gate, requested while the last PV MMA runs
-    const bool gated = EXT && p.gate != nullptr;
-    if (gated && row < S) {
-      const __nv_bfloat16* gate = p.gate + ((p.cu ? (size_t)row_base : (size_t)b * S) + row) * p.ld_gate + h * D;
-#pragma unroll
-      for (int i = 0; i < (EXT ? D / 8 : 1); ++i) gv[i] = *reinterpret_cast<const uint4*>(gate + i * 8);
-    }
-    if (ok) ok = mbar_wait_warp(o_full, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
-    if (ok) {
-      tc_fence_after();
-      const float inv_l = l > 0.f ? 1.f / l : 0.f;
-      __nv_bfloat16* dst = p.out + ((p.cu ? (size_t)row_base : (size_t)b * S) + row) * p.ld_o + h * D;
-#pragma unroll (EXT ? D / 32 : 1)
-      for (int cc = 0; cc < D / 32; ++cc) {
-        uint32_t rr[32];
-        tmem_ld_32x32(t_lane + O_COL + cc * 32, rr);
+        const int k0 = (jlo + j) * FA_BN;
+        const bool windowed = p.causal && p.window > 0, chunked = EXT && p.causal && p.chunk > 0;
+        const int last = q0 + FA_BM - 1;           // the block's last row has the highest first visible key
+        const bool need_mask = (p.causal && k0 + FA_BN - 1 > q0) || (k0 + FA_BN > S) || (windowed && k0 <= last - p.window) ||
+                               (chunked && k0 < last - last % p.chunk);
+        const int kmax = p.causal ? min(row, S - 1) : S - 1;
+        const int kmin = windowed ? row - p.window + 1 : chunked ? row - row % p.chunk : 0;
+        uint32_t sr[128];
+        tmem_ld_32x32(t_lane, sr);
+        tmem_ld_32x32(t_lane + 32, sr + 32);
+        tmem_ld_32x32(t_lane + 64, sr + 64);
+        tmem_ld_32x32(t_lane + 96, sr + 96);
         tmem_ld_wait();
-        if (row < S) {
-          if (gated) {
+        tc_fence_before();
+        if (!ALIAS) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(s_empty);  // the scores live in registers now: the next QK^T may start (one arrival per warp)
+        }
+        if (need_mask) {
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              const uint4 g4 = gv[EXT ? cc * 4 + g : 0];
-              const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w};
+          for (int i = 0; i < 128; ++i)
+            if (k0 + i > kmax || k0 + i < kmin) sr[i] = 0xff800000u;  // -inf
+        }
+        float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const float g0 = __uint_as_float(gw[i] << 16), g1 = __uint_as_float(gw[i] & 0xffff0000u);
-                rr[g * 8 + 2 * i] = __float_as_uint(__uint_as_float(rr[g * 8 + 2 * i]) / (1.0f + __expf(-g0)));
-                rr[g * 8 + 2 * i + 1] = __float_as_uint(__uint_as_float(rr[g * 8 + 2 * i + 1]) / (1.0f + __expf(-g1)));
-              }
+        for (int i = 0; i < 128; i += 8) {
+          mx0 = fmax3(mx0, __uint_as_float(sr[i + 0]), __uint_as_float(sr[i + 1]));
+          mx1 = fmax3(mx1, __uint_as_float(sr[i + 2]), __uint_as_float(sr[i + 3]));
+          mx2 = fmax3(mx2, __uint_as_float(sr[i + 4]), __uint_as_float(sr[i + 5]));
+          mx3 = fmax3(mx3, __uint_as_float(sr[i + 6]), __uint_as_float(sr[i + 7]));
+        }
+        const float m_blk = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+        const bool raise = j == 0 || (m_blk - m_used) * c > 8.0f;  // lazy: tolerate exponents up to 2^8
+        const float m_new = raise ? fmaxf(m_used, m_blk) : m_used;
+        const float alpha = (j == 0 || !raise) ? 1.0f : exp2f((m_used - m_new) * c);
+        m_used = m_new;
+        const bool any_rescale = __any_sync(0xffffffffu, j > 0 && raise);
+        const float mc = m_used == -INFINITY ? 0.f : m_used * c;  // a row that has seen no key yet (window edge): every exponential is 0
+        // exponentials into registers (packed bf16 pairs overwrite the scores) and their sum: one MUFU op per element and
+        // one hardware conversion per pair
+        float rs0 = 0.f, rs1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 128; i += 2) {
+          const float e0 = exp2f(fmaf(__uint_as_float(sr[i]), c, -mc));
+          const float e1 = exp2f(fmaf(__uint_as_float(sr[i + 1]), c, -mc));
+          rs0 += e0;
+          rs1 += e1;
+          sr[i >> 1] = cvt_bf16x2(e0, e1);  // slot i/2 <= i: never read again as a score
+        }
+        l = l * alpha + (rs0 + rs1);
+        if (j > 0) {
+          // PV of the previous block is complete: P may be overwritten, O is stable
+          if (!mbar_wait_warp(o_full, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+          tc_fence_after();
+          if (any_rescale) {
+#pragma unroll 1
+            for (int cc = 0; cc < D / 32; ++cc) {
+              uint32_t rr[32];
+              tmem_ld_32x32(t_lane + O_COL + cc * 32, rr);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) rr[i] = __float_as_uint(__uint_as_float(rr[i]) * alpha);
+              tmem_st_32x32(t_lane + O_COL + cc * 32, rr);
             }
           }
+        }
+        tmem_st_32x32(t_lane + P_COL, sr);
+        tmem_st_32x32(t_lane + P_COL + 32, sr + 32);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+      }
+      if (LOOP) w.next<EXT, LOOP>(p);    // while the last product runs
+      else w.valid = false;
+      uint4 gv[EXT ? D / 8 : 1];                    // the row's gate, requested while the last PV MMA runs
+      const bool gated = EXT && p.gate != nullptr;
+      if (gated && row < S) {
+        const __nv_bfloat16* gate = p.gate + ((p.cu ? (size_t)row_base : (size_t)b * S) + row) * p.ld_gate + h * D;
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint4 o;
-            o.x = pack_bf16x2(__uint_as_float(rr[g * 8 + 0]) * inv_l, __uint_as_float(rr[g * 8 + 1]) * inv_l);
-            o.y = pack_bf16x2(__uint_as_float(rr[g * 8 + 2]) * inv_l, __uint_as_float(rr[g * 8 + 3]) * inv_l);
-            o.z = pack_bf16x2(__uint_as_float(rr[g * 8 + 4]) * inv_l, __uint_as_float(rr[g * 8 + 5]) * inv_l);
-            o.w = pack_bf16x2(__uint_as_float(rr[g * 8 + 6]) * inv_l, __uint_as_float(rr[g * 8 + 7]) * inv_l);
-            *reinterpret_cast<uint4*>(dst + cc * 32 + g * 8) = o;
+        for (int i = 0; i < (EXT ? D / 8 : 1); ++i) gv[i] = *reinterpret_cast<const uint4*>(gate + i * 8);
+      }
+      if (ok) ok = mbar_wait_warp(o_full, (g - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
+      if (ok) {
+        tc_fence_after();
+        const float inv_l = l > 0.f ? 1.f / l : 0.f;
+        __nv_bfloat16* dst = p.out + ((p.cu ? (size_t)row_base : (size_t)b * S) + row) * p.ld_o + h * D;
+#pragma unroll (EXT ? D / 32 : 1)
+        for (int cc = 0; cc < D / 32; ++cc) {
+          uint32_t rr[32];
+          tmem_ld_32x32(t_lane + O_COL + cc * 32, rr);
+          tmem_ld_wait();
+          if (row < S) {
+            if (gated) {
+#pragma unroll
+              for (int g = 0; g < 4; ++g) {
+                const uint4 g4 = gv[EXT ? cc * 4 + g : 0];
+                const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const float g0 = __uint_as_float(gw[i] << 16), g1 = __uint_as_float(gw[i] & 0xffff0000u);
+                  rr[g * 8 + 2 * i] = __float_as_uint(__uint_as_float(rr[g * 8 + 2 * i]) / (1.0f + __expf(-g0)));
+                  rr[g * 8 + 2 * i + 1] = __float_as_uint(__uint_as_float(rr[g * 8 + 2 * i + 1]) / (1.0f + __expf(-g1)));
+                }
+              }
+            }
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+              uint4 o;
+              o.x = pack_bf16x2(__uint_as_float(rr[g * 8 + 0]) * inv_l, __uint_as_float(rr[g * 8 + 1]) * inv_l);
+              o.y = pack_bf16x2(__uint_as_float(rr[g * 8 + 2]) * inv_l, __uint_as_float(rr[g * 8 + 3]) * inv_l);
+              o.z = pack_bf16x2(__uint_as_float(rr[g * 8 + 4]) * inv_l, __uint_as_float(rr[g * 8 + 5]) * inv_l);
+              o.w = pack_bf16x2(__uint_as_float(rr[g * 8 + 6]) * inv_l, __uint_as_float(rr[g * 8 + 7]) * inv_l);
+              *reinterpret_cast<uint4*>(dst + cc * 32 + g * 8) = o;
+            }
           }
         }
+        if (p.lse && row < S) p.lse[((size_t)b * p.H + h) * S + row] = m_used * c + log2f(l);
+        tc_fence_before();
       }
-      if (p.lse && row < S) p.lse[((size_t)b * p.H + h) * S + row] = m_used * c + log2f(l);
-      tc_fence_before();
-    }
     }
   }
 

@@ -293,16 +293,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
       } else {
 #pragma unroll 1
-      for (int c = half * 4; c < half * 4 + 4; c += 2) {
-        const int col0 = u.n0 + c * 32;
-        if (col0 >= p.N) break;  // uniform across the warp
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32(t_row + c * 32, r0);
-        tmem_ld_32x32(t_row + c * 32 + 32, r1);
-        tmem_ld_wait();
-        gemm_epilogue_chunk(p, C, bias, row, row_ok, col0, r0);
-        if (col0 + 32 < p.N) gemm_epilogue_chunk(p, C, bias, row, row_ok, col0 + 32, r1);
-      }
+        for (int c = half * 4; c < half * 4 + 4; c += 2) {
+          const int col0 = u.n0 + c * 32;
+          if (col0 >= p.N) break;  // uniform across the warp
+          uint32_t r0[32], r1[32];
+          tmem_ld_32x32(t_row + c * 32, r0);
+          tmem_ld_32x32(t_row + c * 32 + 32, r1);
+          tmem_ld_wait();
+          gemm_epilogue_chunk(p, C, bias, row, row_ok, col0, r0);
+          if (col0 + 32 < p.N) gemm_epilogue_chunk(p, C, bias, row, row_ok, col0 + 32, r1);
+        }
       }
       tc_fence_before();
       __syncwarp();

@@ -390,106 +390,106 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       }
       if (lane == 0) tma_store_wait_all();       // shared memory must outlive the stores that read it
     } else {
-    const bool staged = !p.c_f32;
-    const bool staged_aux = staged && INV_EPI_WRITES_AUX(p.epilogue) && p.aux_out != nullptr;
-    // Second operand of the epilogue (residual to add, pre-activation of the GELU backward) through TMA: the warp's two
-    // 4 KB boxes alternate; box i is loaded while box i-1 is computed, the result overwrites the operand in place and
-    // leaves through a TMA store. Per-thread global loads of a row-strided operand serialise on memory latency
-    // (sixteen dependent round trips per tile) and made these epilogues three times as long as the main loop.
-    const bool aux_tma = staged && INV_EPI_READS_AUX(p.epilogue);
-    uint8_t* my_stage = sStage + (warp - 2) * 8192;
-    uint64_t* my_aux_bar = aux_bar + (warp - 2) * 2;
-    const int row_in_tile = (int)cta * 128 + q * 32;
-    // (w, j): j-th 64-column box of this warp in work unit w; false when the unit or the box does not exist
-    auto box_of = [&](int w, int j, int& col0, int& row0) -> bool {
-      if (w >= total_work) return false;
-      const WorkUnit2 u = decode_work2<TN>(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
-      col0 = u.n0 + (half * 4 + 2 * j) * 32;
-      row0 = u.m0 + row_in_tile;
-      return col0 < p.N;
-    };
-    uint32_t boxes_done = 0;       // boxes this warp has computed: box i uses buffer i & 1, phase (i >> 1) & 1 of its barrier
-    int nw = pair, nj = 0;          // next box to prefetch
-    auto prefetch_next = [&](uint32_t box_index) {   // lane 0 only
-      int col0, row0;
-      while (nw < total_work && !box_of(nw, nj, col0, row0)) { nw += npairs; nj = 0; }   // a missing box 0 or 1 ends the unit for this warp
-      if (nw >= total_work) return;
-      const uint32_t b = box_index & 1;
-      mbar_expect_tx(&my_aux_bar[b], 4096);
-      tma_load_2d(my_stage + b * 4096, &tmap_aux, &my_aux_bar[b], col0, row0);
-      if (nj == 0) nj = 1; else { nj = 0; nw += npairs; }
-    };
-    if (aux_tma && lane == 0) prefetch_next(0);
-    int tile_i = 0;
-    bool ok = true;
-    for (int w = pair; ok && w < total_work; w += npairs, ++tile_i) {
-      const WorkUnit2 u = decode_work2<TN>(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
-      const int acc = tile_i & 1;
-      const uint32_t acc_ph = (tile_i >> 1) & 1;
-      if (!mbar_wait_warp(&tmem_full[acc], acc_ph, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) break;
-      tc_fence_after();
-      const int row = u.m0 + row_in_tile + lane;
-      const bool row_ok = row < p.M;
-      const CUtensorMap* c_map = &tmap_c;
-      int row_shift = 0;
-      if (p.rs_world > 1) {  // this tile's rows belong to one owner: the staged tile is TMA-stored into its buffer (peer memory) at the shard-relative row
-        const int owner = u.m0 / p.rs_shard_rows;
-        c_map = &rs_maps.m[owner];
-        row_shift = owner * p.rs_shard_rows;
-      }
-      const uint32_t t_row = tmem_base + acc * BN + (uint32_t(q * 32) << 16);
-      const int row0_abs = u.m0 + row_in_tile;
-#pragma unroll 1
-      for (int c = half * 4; c < half * 4 + 4; c += 2) {
-        const int col0 = u.n0 + c * 32;
-        if (col0 >= p.N) break;
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32(t_row + c * 32, r0);
-        tmem_ld_32x32(t_row + c * 32 + 32, r1);
-        tmem_ld_wait();
-        if (aux_tma) {
-          const uint32_t b = boxes_done & 1;
-          if (lane == 0) {
-            tma_store_wait_read();          // the other buffer's store (box i-1) has left shared memory
-            prefetch_next(boxes_done + 1);  // ... so box i+1 may land there while box i is computed
-          }
-          if (!mbar_wait_warp(&my_aux_bar[b], (boxes_done >> 1) & 1, abort_flag, p.status, ERR_WAIT_MISC)) { ok = false; break; }
-          uint8_t* sc = my_stage + b * 4096 + lane * 128;
-          gemm_epilogue_chunk(p, p.C, p.bias, row, row_ok, col0, r0, sc, nullptr, 0, lane, sc);
-          if (col0 + 32 < p.N) gemm_epilogue_chunk(p, p.C, p.bias, row, row_ok, col0 + 32, r1, sc, nullptr, 1, lane, sc);
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            tma_store_2d(c_map, my_stage + b * 4096, col0, row0_abs - row_shift);
-            tma_store_commit();
-          }
-          ++boxes_done;
-        } else if (staged) {
-          // bf16 output: registers -> swizzled 32x64 box in shared memory -> one TMA store per box
-          if (lane == 0) tma_store_wait_read();  // the previous box of this warp has left shared memory
-          __syncwarp();
-          uint8_t* sc = my_stage + lane * 128;
-          uint8_t* sa = staged_aux ? sc + 4096 : nullptr;
-          gemm_epilogue_chunk(p, p.C, p.bias, row, row_ok, col0, r0, sc, sa, 0, lane);
-          if (col0 + 32 < p.N) gemm_epilogue_chunk(p, p.C, p.bias, row, row_ok, col0 + 32, r1, sc, sa, 1, lane);
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            tma_store_2d(c_map, my_stage, col0, row0_abs - row_shift);
-            if (staged_aux) tma_store_2d(&tmap_aux, my_stage + 4096, col0, row0_abs);
-            tma_store_commit();
-          }
-        } else {
-          gemm_epilogue_chunk(p, p.C, p.bias, row, row_ok, col0, r0);
-          if (col0 + 32 < p.N) gemm_epilogue_chunk(p, p.C, p.bias, row, row_ok, col0 + 32, r1);
+      const bool staged = !p.c_f32;
+      const bool staged_aux = staged && INV_EPI_WRITES_AUX(p.epilogue) && p.aux_out != nullptr;
+      // Second operand of the epilogue (residual to add, pre-activation of the GELU backward) through TMA: the warp's two
+      // 4 KB boxes alternate; box i is loaded while box i-1 is computed, the result overwrites the operand in place and
+      // leaves through a TMA store. Per-thread global loads of a row-strided operand serialise on memory latency
+      // (sixteen dependent round trips per tile) and made these epilogues three times as long as the main loop.
+      const bool aux_tma = staged && INV_EPI_READS_AUX(p.epilogue);
+      uint8_t* my_stage = sStage + (warp - 2) * 8192;
+      uint64_t* my_aux_bar = aux_bar + (warp - 2) * 2;
+      const int row_in_tile = (int)cta * 128 + q * 32;
+      // (w, j): j-th 64-column box of this warp in work unit w; false when the unit or the box does not exist
+      auto box_of = [&](int w, int j, int& col0, int& row0) -> bool {
+        if (w >= total_work) return false;
+        const WorkUnit2 u = decode_work2<TN>(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
+        col0 = u.n0 + (half * 4 + 2 * j) * 32;
+        row0 = u.m0 + row_in_tile;
+        return col0 < p.N;
+      };
+      uint32_t boxes_done = 0;       // boxes this warp has computed: box i uses buffer i & 1, phase (i >> 1) & 1 of its barrier
+      int nw = pair, nj = 0;          // next box to prefetch
+      auto prefetch_next = [&](uint32_t box_index) {   // lane 0 only
+        int col0, row0;
+        while (nw < total_work && !box_of(nw, nj, col0, row0)) { nw += npairs; nj = 0; }   // a missing box 0 or 1 ends the unit for this warp
+        if (nw >= total_work) return;
+        const uint32_t b = box_index & 1;
+        mbar_expect_tx(&my_aux_bar[b], 4096);
+        tma_load_2d(my_stage + b * 4096, &tmap_aux, &my_aux_bar[b], col0, row0);
+        if (nj == 0) nj = 1; else { nj = 0; nw += npairs; }
+      };
+      if (aux_tma && lane == 0) prefetch_next(0);
+      int tile_i = 0;
+      bool ok = true;
+      for (int w = pair; ok && w < total_work; w += npairs, ++tile_i) {
+        const WorkUnit2 u = decode_work2<TN>(w, p, m_tiles, n_tiles, kb_total, kb_per_split);
+        const int acc = tile_i & 1;
+        const uint32_t acc_ph = (tile_i >> 1) & 1;
+        if (!mbar_wait_warp(&tmem_full[acc], acc_ph, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) break;
+        tc_fence_after();
+        const int row = u.m0 + row_in_tile + lane;
+        const bool row_ok = row < p.M;
+        const CUtensorMap* c_map = &tmap_c;
+        int row_shift = 0;
+        if (p.rs_world > 1) {  // this tile's rows belong to one owner: the staged tile is TMA-stored into its buffer (peer memory) at the shard-relative row
+          const int owner = u.m0 / p.rs_shard_rows;
+          c_map = &rs_maps.m[owner];
+          row_shift = owner * p.rs_shard_rows;
         }
+        const uint32_t t_row = tmem_base + acc * BN + (uint32_t(q * 32) << 16);
+        const int row0_abs = u.m0 + row_in_tile;
+#pragma unroll 1
+        for (int c = half * 4; c < half * 4 + 4; c += 2) {
+          const int col0 = u.n0 + c * 32;
+          if (col0 >= p.N) break;
+          uint32_t r0[32], r1[32];
+          tmem_ld_32x32(t_row + c * 32, r0);
+          tmem_ld_32x32(t_row + c * 32 + 32, r1);
+          tmem_ld_wait();
+          if (aux_tma) {
+            const uint32_t b = boxes_done & 1;
+            if (lane == 0) {
+              tma_store_wait_read();          // the other buffer's store (box i-1) has left shared memory
+              prefetch_next(boxes_done + 1);  // ... so box i+1 may land there while box i is computed
+            }
+            if (!mbar_wait_warp(&my_aux_bar[b], (boxes_done >> 1) & 1, abort_flag, p.status, ERR_WAIT_MISC)) { ok = false; break; }
+            uint8_t* sc = my_stage + b * 4096 + lane * 128;
+            gemm_epilogue_chunk(p, p.C, p.bias, row, row_ok, col0, r0, sc, nullptr, 0, lane, sc);
+            if (col0 + 32 < p.N) gemm_epilogue_chunk(p, p.C, p.bias, row, row_ok, col0 + 32, r1, sc, nullptr, 1, lane, sc);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(c_map, my_stage + b * 4096, col0, row0_abs - row_shift);
+              tma_store_commit();
+            }
+            ++boxes_done;
+          } else if (staged) {
+            // bf16 output: registers -> swizzled 32x64 box in shared memory -> one TMA store per box
+            if (lane == 0) tma_store_wait_read();  // the previous box of this warp has left shared memory
+            __syncwarp();
+            uint8_t* sc = my_stage + lane * 128;
+            uint8_t* sa = staged_aux ? sc + 4096 : nullptr;
+            gemm_epilogue_chunk(p, p.C, p.bias, row, row_ok, col0, r0, sc, sa, 0, lane);
+            if (col0 + 32 < p.N) gemm_epilogue_chunk(p, p.C, p.bias, row, row_ok, col0 + 32, r1, sc, sa, 1, lane);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(c_map, my_stage, col0, row0_abs - row_shift);
+              if (staged_aux) tma_store_2d(&tmap_aux, my_stage + 4096, col0, row0_abs);
+              tma_store_commit();
+            }
+          } else {
+            gemm_epilogue_chunk(p, p.C, p.bias, row, row_ok, col0, r0);
+            if (col0 + 32 < p.N) gemm_epilogue_chunk(p, p.C, p.bias, row, row_ok, col0 + 32, r1);
+          }
+        }
+        if (!ok) break;
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&tmem_empty[acc]), 0));
       }
-      if (!ok) break;
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&tmem_empty[acc]), 0));
-    }
-    if (lane == 0) tma_store_wait_all();  // shared memory must outlive the stores that read it
+      if (lane == 0) tma_store_wait_all();  // shared memory must outlive the stores that read it
     }
   }
 
