@@ -243,6 +243,9 @@ extern "C" int inv_block_bytes(int which, long B, long S, long E, long H, long H
   return 0;
 }
 
+// The cut that the products of the backward pass take (ops/gemm.py states the same rule).
+extern "C" int inv_block_split_k(long M, long N, long K) { return split_k_for(M, N, K); }
+
 // Pre-norm block: y = x2 + MLP(norm2(x2)), x2 = x + attention(norm1(x)); causal. Returns the number of launches, or a negative code.
 extern "C" int inv_block_fwd(const BlockDesc* d) {
   BlockRun r(*d);

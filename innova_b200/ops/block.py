@@ -21,7 +21,8 @@ from .quant import BLOCK, MODES, default_codebook
 
 _gemm = importlib.import_module(".gemm", __package__)      # the module: the package exports the function under this name
 
-_native.register_cuda_sigs({"inv_block_fwd": [_native.vp], "inv_block_bwd": [_native.vp], "inv_block_bytes": [_native.i32] + [_native.i64] * 9 + [_native.vp]})
+_native.register_cuda_sigs({"inv_block_fwd": [_native.vp], "inv_block_bwd": [_native.vp], "inv_block_bytes": [_native.i32] + [_native.i64] * 9 + [_native.vp],
+                              "inv_block_split_k": [_native.i64] * 3})
 
 # BlockDesc: 12 parameters, tables, positions, codebook, x, y, saved, status, stream | dy, dx, two column sums, 12 gradients, scratch | 14 sizes |
 # eps1, eps2, scale

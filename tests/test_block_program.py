@@ -184,6 +184,15 @@ def test_block_buffers_are_sized_by_their_layout():
         block._bytes(block.SAVED, 0, 1, 64, 1, 1, 64, 8, 0, 0)
 
 
+def test_block_cuts_its_weight_gradients_as_the_layers_do():
+    from innova_b200.ops import block, runtime as rt  # noqa: F401
+    from innova_b200.ops.gemm import _split_k_for
+    for M in (8, 128, 129, 256, 257, 768, 2048, 11264):
+        for N in (8, 128, 136, 264, 2048, 5632):
+            for K in (1, 64, 65, 1024, 3003, 65536):
+                assert rt.lib().inv_block_split_k(M, N, K) == _split_k_for(M, N, K), (M, N, K)
+
+
 def test_train_step_puts_parts_in_eval_mode_back():
     from innova_b200.training.trainer import Trainer
     m = DenseModel(PRESETS["tiny"](num_layers=1, vocab_size=64, max_seq_len=16, hidden_size=32, num_heads=1, head_dim=32, ffn_hidden_size=32), dtype=torch.float32)
