@@ -97,9 +97,11 @@ __device__ __forceinline__ float code_threshold(float c0, float c1) {
 
 // Whole blocks of 32 values, 16-byte aligned. One read of a table entry gives a value's code: x falls into one of BUCKETS buckets of
 // [-1, 1] (the bits of x * BUCKETS / 2 + 2^23 + BUCKETS / 2), which knows the thresholds below it and the one inside it. Codebooks with
-// several thresholds in a bucket walk on from there; the next block's values are requested before this one is coded. Bound by issue
-// and, from fp32, by memory: 11008 x 4096 fp32 to packed nibbles and bf16 scales in 55 us, 3.8 TB/s (one warp per block with a binary
-// search per value, then a packing and a rounding launch: 270 us); 20 M values bf16 to bf16 through 256 entries in 33 us (107 us).
+// several thresholds in a bucket walk on from there; the next block's values are requested before this one is coded. Bound by the table:
+// each lane reads an entry of eight bytes at a place of its own, which takes a warp 5.8 passes for Gaussian blocks where 2 would do (simulated on
+// the bucket rule), 30 us of shared memory for 11008 x 4096; then by issue and, from fp32, by memory: 11008 x 4096 fp32 to packed nibbles and
+// bf16 scales in 55 us, 3.8 TB/s (one warp per block with a binary search per value, then a packing and a rounding launch: 270 us); 20 M
+// values bf16 to bf16 through 256 entries in 33 us (107 us).
 template <typename TIn, int MODE>
 __global__ void __launch_bounds__(256) block_quant8_kernel(const TIn* __restrict__ in, QuantOut out, const float* __restrict__ codebook,
                                                            long nblocks) {
