@@ -249,16 +249,14 @@ static int launch_oil_skinny(const OilSkinnyParams& p, bool early, int smem, cud
   return e == cudaSuccess ? 0 : -(int)e;
 }
 // Sixteen warps where a tile has an SM to itself and more slices than eight warps: all of its weights are then in flight at once and the
-// expansion, which is bound by instruction issue, has four warps a scheduler (2048 x 5632: eight tokens 6.6 -> 5.8 us, three 6.3 -> 5.0). One token
-// expands little: with 4- and 8-bit codes only where half of the SMs have no tile (1024 x 4096 3.4 alike and 4.3 -> 4.0; 2048 x 5632 4.5 -> 4.65 and 5.8
-// -> 5.95; 2-bit codes there 8.4 -> 6.3).
+// expansion, which is bound by instruction issue, has four warps a scheduler (2048 x 5632: eight tokens 6.5 -> 5.5 us, one token alike, 4.3).
 // With several tiles an SM two CTAs of eight warps do the same and overlap their reductions.
 template <int BITS, int MT>
 static int launch_oil_skinny(const OilSkinnyParams& p, bool early, cudaStream_t st) {
   using namespace os;
   const int slices = (p.K + SLICE - 1) / SLICE;
   const int x = slices * 128 * (4 * p.M + 1), sums = ROWS * (MT * 8 + 1) * 4;
-  if (p.n_tiles <= (p.M > 1 || BITS == 2 ? 148 : 74) && slices > 8 && x + 16 * sums <= 190 * 1024) return launch_oil_skinny<BITS, MT, 16>(p, early, x + 16 * sums, st);
+  if (p.n_tiles <= 148 && slices > 8 && x + 16 * sums <= 190 * 1024) return launch_oil_skinny<BITS, MT, 16>(p, early, x + 16 * sums, st);
   return launch_oil_skinny<BITS, MT, 8>(p, early, x + 8 * sums, st);
 }
 
