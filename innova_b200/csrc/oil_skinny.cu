@@ -249,7 +249,9 @@ static int launch_oil_skinny(const OilSkinnyParams& p, bool early, int smem, cud
   return e == cudaSuccess ? 0 : -(int)e;
 }
 // Sixteen warps where a tile has an SM to itself and more slices than eight warps: all of its weights are then in flight at once and the
-// expansion, which is bound by instruction issue, has four warps a scheduler (2048 x 5632: eight tokens 6.5 -> 5.5 us, one token alike, 4.3).
+// expansion, which is bound by instruction issue, has four warps a scheduler (2048 x 5632: eight tokens 6.6 -> 5.8 us, three 6.3 -> 5.0; one token back
+// to back 4.5 with eight and 4.65 with sixteen, but behind the attention and gate/up products of a decode step, whose end its loads overlap,
+// sixteen take 1 us a layer less: generate of one sequence, 8 layers, 64 steps: 18.05 -> 17.5 ms).
 // With several tiles an SM two CTAs of eight warps do the same and overlap their reductions.
 template <int BITS, int MT>
 static int launch_oil_skinny(const OilSkinnyParams& p, bool early, cudaStream_t st) {
