@@ -97,11 +97,8 @@ class FFN(nn.Module):
         return ops.linear(act, _ste(self.down_proj.weight, cfg), self.down_proj.bias, residual=residual, mode="add")
 
 
-def _steps(cls):
-    return cls.forward, getattr(cls, "with_residual", None)
-
-
-_AS_WRITTEN = {cls: _steps(cls) for cls in (Attention, FFN, Norm)}     # a class whose steps were replaced since (by a profiler, say) is called itself
+# The steps as written: a class in which one was replaced since (by a profiler, say) is called itself.
+_ATTENTION, _FFN, _NORM = Attention.forward, FFN.forward, (Norm.forward, Norm.with_residual)
 
 
 class TransformerBlock(nn.Module):
@@ -115,11 +112,12 @@ class TransformerBlock(nn.Module):
 
     def _whole(self):
         """Whether nothing inside the block was hooked, replaced or configured on its own, so that its launches may be issued together."""
-        if self.attention.cfg is not self.cfg or self.ffn.cfg is not self.cfg:
+        if (self.attention.cfg is not self.cfg or self.ffn.cfg is not self.cfg or Attention.forward is not _ATTENTION or FFN.forward is not _FFN
+                or Norm.forward is not _NORM[0] or Norm.with_residual is not _NORM[1]):
             return False
         for m, cls in ((self.attention, Attention), (self.ffn, FFN), (self.attention_norm, Norm), (self.ffn_norm, Norm)):
             if (type(m) is not cls or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__
-                    or "with_residual" in m.__dict__ or _steps(cls) != _AS_WRITTEN[cls]):
+                    or "with_residual" in m.__dict__):
                 return False
         return True
 
