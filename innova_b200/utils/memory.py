@@ -11,7 +11,7 @@ from __future__ import annotations
 
 import ctypes as C
 import threading
-from typing import Dict, Optional, Sequence
+from typing import List, Optional, Sequence, Tuple
 
 import torch
 
@@ -152,24 +152,24 @@ class ThreadLocalPoolRegistry:
     def __init__(self, capacity_per_thread: int, device="cpu", pin: bool = False):
         self.capacity, self.device, self.pin = capacity_per_thread, device, pin
         self._local = threading.local()
-        self._all: Dict[int, MemoryPool] = {}
+        self._all: List[Tuple[threading.Thread, MemoryPool]] = []
         self._lock = threading.Lock()
 
     def get(self) -> MemoryPool:
         p = getattr(self._local, "pool", None)
         if p is None:
             p = self._local.pool = MemoryPool(self.capacity, self.device, self.pin)
-            with self._lock:
-                self._all[threading.get_ident()] = p
+            with self._lock:        # by the thread itself: numbers are given again; an ended thread's pool stays while it holds something
+                self._all = [(t, q) for t, q in self._all if t.is_alive() or q.bytes_used] + [(threading.current_thread(), p)]
         return p
 
     def total_used(self) -> int:
         with self._lock:
-            return sum(p.bytes_used for p in self._all.values())
+            return sum(p.bytes_used for _, p in self._all)
 
     def reset_all(self):
         with self._lock:
-            for p in self._all.values():
+            for _, p in self._all:
                 p.reset()
 
 

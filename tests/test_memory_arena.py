@@ -69,6 +69,23 @@ def test_thread_local_registry_and_buffer():
     assert buf.data_ptr() % 512 == 0 and buf.nbytes == 1000 and buf.view(torch.float32, (5, 5), 64).shape == (5, 5)
 
 
+def test_threads_one_after_the_other_keep_their_pools():
+    """They get the same number: nothing that an ended one holds drops out of the registry; what holds nothing does."""
+    reg = ThreadLocalPoolRegistry(1 << 12)
+
+    def one_after_the_other():
+        for _ in range(8):
+            t = threading.Thread(target=lambda: reg.get().allocate((16,), torch.float32))
+            t.start()
+            t.join()
+
+    one_after_the_other()
+    assert reg.total_used() == 8 * 64
+    reg.reset_all()
+    one_after_the_other()
+    assert reg.total_used() == 8 * 64 and len(reg._all) == 8
+
+
 def test_tensor_view():
     base = torch.arange(24.0)
     v = TensorView(base, (2, 3, 4))
