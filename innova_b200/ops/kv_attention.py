@@ -91,7 +91,9 @@ def cluster_shape(rows: int, groups: int, span: int, dim: int = 128):
     if warps == 32 and units <= 8 and pages >= 256:
         return 8, 8
     if warps == 16 and units > 32 and dim > 64:
-        return 2, 8      # heads of 128, 500 / 1500 / 4000 tokens: 64 units 6.6, 10.9, 24.6 us (clusters of four 7.2, 12.1, 26.4), 48 alike; of 64: 5.9, 9.4, 17.8 (5.7, 8.6, 15.9)
+        # heads of 128, 500 / 1500 / 4000 tokens: 64 units 6.6, 10.9, 24.6 us (clusters of four 7.2, 12.1, 26.4), 48 alike;
+        # heads of 64, 64 units: 5.9, 9.4, 17.8 (5.7, 8.6, 15.9)
+        return 2, 8
     return {4: (1, 4), 8: (1, 8), 16: (4, 4), 32: (8, 4)}[warps]
 
 
