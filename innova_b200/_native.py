@@ -39,6 +39,7 @@ _CUDA_SIGS = {
     "inv_scale_bf16": [vp, vp, vp, i64, vp],
     "inv_cross_entropy": [vp, vp, vp, vp, i32, i32, i32, f32, f32, i32, vp],
     "inv_sumsq": [vp, i64, vp, vp],
+    "inv_event_wait": [vp],
     "inv_adamw": [vp, vp, vp, vp, vp, i64, vp, vp, i32, vp],
 }
 

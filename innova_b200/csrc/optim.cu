@@ -109,3 +109,12 @@ extern "C" int inv_adamw(float* p, float* m, float* v, float* g, void* p16, long
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
+
+// Waits on the host for an event, also while another thread captures a graph (a plain wait would end that capture).
+extern "C" int inv_event_wait(void* event) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const cudaError_t e = cudaEventSynchronize((cudaEvent_t)event);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return e == cudaSuccess ? 0 : -(int)e;
+}

@@ -30,26 +30,39 @@ class HyperRows:
 
     def __init__(self, rows: int, device, event=None):
         self.rows = torch.zeros(rows, 16, dtype=torch.float32)
-        if device.type == "cuda":
+        self._cuda = device.type == "cuda"
+        if self._cuda:
             self.rows = self.rows.pin_memory()
         self._values = self.rows.numpy()        # the same memory: a row is written in one assignment
-        self._event = event or (torch.cuda.Event if device.type == "cuda" else None)
+        self._event = event or (torch.cuda.Event if self._cuda else None)
         self._read = [None] * rows              # the event behind the last copy of each row ...
         self._sent = [False] * rows             # ... where there was one since the row was written
         self._slot = 0
+
+    def _wait(self, event):
+        if not self._cuda:
+            return event.synchronize()
+        from ..ops import runtime as rt
+        rc = rt.lib().inv_event_wait(event.cuda_event)
+        if rc != 0:
+            raise RuntimeError(f"inv_event_wait failed with code {rc}")
+
+    def _capturing(self) -> bool:
+        return self._cuda and torch.cuda.is_current_stream_capturing()
 
     def fill(self, *values) -> torch.Tensor:
         """The next row, holding ``values`` (numbers, or tensors of one)."""
         self._slot = slot = (self._slot + 1) % len(self._read)
         if self._sent[slot]:
-            self._read[slot].synchronize()
+            if not self._capturing():           # (a captured copy reads the row when it is replayed)
+                self._wait(self._read[slot])
             self._sent[slot] = False
         self._values[slot, :len(values)] = [float(v) for v in values]
         return self.rows[slot]
 
     def send(self, dst: torch.Tensor, row: torch.Tensor):
         dst.copy_(row, non_blocking=True)
-        if self._event is None or (dst.is_cuda and torch.cuda.is_current_stream_capturing()):
+        if self._event is None or self._capturing():
             return
         slot = row.storage_offset() // 16
         if self._read[slot] is None:

@@ -400,6 +400,66 @@ def test_adamw_matches_torch():
     assert float(eng.flat_grad.abs().max()) == 0.0
 
 
+def test_an_optimizer_step_is_captured_after_many():
+    """The step's row of hyperparameters has been sent before by then; a capture permits no wait for that."""
+    from innova_b200.training.flat_engine import FlatParamEngine
+    dev = _dev()
+    out = []
+    for graph in (False, True):
+        torch.manual_seed(4)
+        lin = torch.nn.Linear(64, 64).to(dev).bfloat16()
+        eng = FlatParamEngine(lin, lr=1e-2)
+        grads = torch.randn(41, eng.total, device=dev)
+        for g in grads[:40]:
+            eng.flat_grad.copy_(g)
+            eng.step()
+        eng.flat_grad.copy_(grads[40])
+        if graph:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                eng.step()
+            g.replay()
+        else:
+            eng.step()
+        torch.cuda.synchronize()
+        out.append(eng.master.clone())
+    # the squares of the gradient norm are added in any order: 2^-23 of 41 steps of 1e-2, and as many roundings of values below one half
+    assert torch.allclose(*out, rtol=0, atol=1e-6)
+
+
+def test_optimizer_steps_beside_a_capture_on_another_thread():
+    """More steps than rows of hyperparameters, on a stream of their own, while this thread captures: neither disturbs the other."""
+    import threading
+    from innova_b200.training.flat_engine import FlatParamEngine
+    dev = _dev()
+    torch.manual_seed(4)
+    lin = torch.nn.Linear(64, 64).to(dev).bfloat16()
+    eng = FlatParamEngine(lin, lr=1e-2)
+    eng.step()
+    x, y = torch.ones(64, device=dev), torch.empty(64, device=dev)
+    errors, side = [], torch.cuda.Stream()
+
+    def steps():
+        try:
+            with torch.cuda.stream(side):
+                for _ in range(40):
+                    eng.step()
+        except Exception as e:
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        torch.mul(x, 2.0, out=y)
+        t = threading.Thread(target=steps)
+        t.start()
+        t.join()
+        torch.add(y, 1.0, out=y)
+    g.replay()
+    torch.cuda.synchronize()
+    assert not errors and eng.step_count == 41 and torch.equal(y, torch.full_like(y, 3.0))
+
+
 # ------------------------------------------------------------------------------------------ attention
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,S,H,Hkv,causal", [(2, 256, 4, 4, True), (1, 384, 4, 2, True), (2, 200, 2, 2, True), (1, 256, 2, 1, False),
